@@ -33,6 +33,7 @@ namespace {
 thread_local std::string g_last_error;
 
 constexpr int MAX_SWEEPS = 40;
+constexpr int MESH_LANES = 2;   // streams a mesh's groups of updates are spread over
 
 struct DevBuf {
   void* p = nullptr;
@@ -107,15 +108,14 @@ struct bsmpo_ctx {
   int tc_mask = 1;
   // side streams (0-3, BSMPO_TD_FORK) for the tridiagonalisation's size-class launches:
   // the largest class present runs on the update's stream, the others on the side
-  // streams, forked and joined with events.  With concurrent updates the streams of all
-  // workers share the device's hardware queues (CUDA_DEVICE_MAX_CONNECTIONS, at most
-  // 32); streams beyond that count are serialised with others
-  int td_fork = 1;
+  // streams, forked and joined with events.  Two lanes of one stream and three side
+  // streams each are the device's 8 hardware queues (CUDA_DEVICE_MAX_CONNECTIONS' default)
+  int td_fork = 3;
   int n_aux = 0;   // side streams created
   HostStage stage, stage2, hres;
   // last update diagnostics (host)
   std::vector<int> last_cc, last_shape, last_kept, last_k;
-  std::vector<int64_t> last_soff;
+  int64_t last_sig_off = 0;   // first singular value of that update in `sig`
   double last_trunc = 0.0, last_gemm = 0.0, last_svd = 0.0, last_bytes = 0.0;
   int last_sweeps = 0;
   // opt-in stage timing (BSMPO_PROFILE=1): synchronises after every stage
@@ -241,26 +241,37 @@ void block_offsets(const int* cnt, int d, int* off) {
   for (int q = 0; q < d * d; ++q) off[q + 1] = off[q] + cnt[q];
 }
 
+// One update of a group: where it acts, its gate tensor, and (mesh) its index.
+struct Job {
+  int mode = 0;
+  const cplx* u3 = nullptr;
+  int index = 0;
+};
+
+// The launches of a group of updates that touch disjoint sites: every table is the
+// concatenation of the updates' tables, every workspace offset runs through the group.
 struct Plan {
-  UpdateTables tab;
-  std::vector<int> tidx;
+  std::vector<UpdateTables> tab;  // one per update
+  std::vector<int> tidx;          // d^4 per update
   std::vector<ThetaDesc> td;
   std::vector<SectorDesc> sd;
   std::vector<MixPair> pairs;
   std::vector<GemmGroup> gg;
   std::vector<GemmGroup> ggram;   // Gram G_s = X^H X of every sector (Gram route)
+  std::vector<GemmGroup> gv, gw;  // V = T Y diag(1/sigma) (Gram route, X = T) and W = V^H C
   std::vector<int> tdlist;        // sectors by tridiagonalisation size class (Gram route)
   std::vector<TcGroup> tcg;       // Theta groups on the tensor cores (TF32X3)
-  std::vector<unsigned char> tcmaps;   // their two tensor maps (Gamma_L, Gamma_R)
+  std::vector<unsigned char> tcmaps;   // two tensor maps per update (Gamma_L, Gamma_R)
   int tc_tiles = 0;
-  int td_count[4] = {0, 0, 0, 0}, td_kmax[4] = {0, 0, 0, 0};
+  int td_count[TD_CLASSES] = {}, td_kmax[TD_CLASSES] = {};
   std::vector<JacobiWork> jw;
-  int mix_tiles = 0, gemm_tiles = 0, max_rounds = 0, max_k = 0, max_left_m2 = 0;
+  int mix_tiles = 0, gemm_tiles = 0, max_rounds = 0, max_k = 0, max_left_m2 = 0, max_v = 0;
+  int gram_tiles = 0, v_tiles = 0, w_tiles = 0;
   int gram_ctas = 0, apply_ctas = 0, jac_slots = 0;   // every sector in one round
   int64_t theta_elems = 0, c_elems = 0, a_elems = 0, s_elems = 0, w_elems = 0, v_elems = 0;
   int64_t g_elems = 0, y_elems = 0;
-  int gram_tiles = 0;
-  double flops_theta = 0.0;
+  std::vector<double> flops_theta;   // per update
+  bool gram = false;                 // the group's route (one for all of its updates)
 };
 
 // Orders a round's work entries (most rounds per sweep first: those sectors set the
@@ -284,17 +295,56 @@ void jacobi_launch_list(std::vector<JacobiWork>& w, int* gram_ctas, int* apply_c
   *slots = sl;
 }
 
-int make_plan(bsmpo_ctx* h, int mode, Plan& P) {
+// The candidates of an update, sum over its sectors of min(|L_s|, |R_s|).
+int64_t candidates(bsmpo_ctx* h, int mode) {
+  const int d = h->d, dd = d * d;
+  const int* cL = &mirror(h)[(size_t)mode * dd];
+  const int* cR = &mirror(h)[(size_t)(mode + 2) * dd];
+  int64_t sum = 0;
+  for (int cc0 = 0; cc0 < d; ++cc0)
+    for (int cc1 = 0; cc1 < d; ++cc1) {
+      int m = 0, n = 0;
+      for (int x0 = 0; x0 < d; ++x0)
+        for (int x1 = 0; x1 < d; ++x1) {
+          if (x0 >= cc0 && x1 >= cc1) m += cL[x0 * d + x1];
+          if (x0 <= cc0 && x1 <= cc1) n += cR[x0 * d + x1];
+        }
+      sum += std::min(m, n);
+    }
+  return sum;
+}
+
+// Whether an update takes the Gram route.  That route drops singular values below ~2e-6
+// of a sector's largest.  Where the update does not truncate to chi that is pure loss
+// (W = V^H C carries them through 1 / Lambda_R), so such updates take the exact Jacobi
+// SVD: where the candidates cannot exceed chi, or (gram_policy 2) where the centre bond
+// holds fewer than chi vectors (it was not truncated by the last update on it and is
+// unlikely to be by this one).
+bool gram_route(bsmpo_ctx* h, int mode) {
+  if (h->precision == BSMPO_PRECISION_FP64 || candidates(h, mode) <= h->chi) return false;
+  if (h->gram_policy < 2) return true;
+  const int dd = h->d * h->d;
+  int64_t centre = 0;
+  for (int q = 0; q < dd; ++q) centre += mirror(h)[(size_t)(mode + 1) * dd + q];
+  return centre >= h->chi;
+}
+
+// Adds the update at `mode` to the plan.
+int add_update(bsmpo_ctx* h, int mode, int64_t gate_off, Plan& P) {
   const int d = h->d, dd = d * d;
   const std::vector<int>& cnt = mirror(h);
   const int* cL = &cnt[(size_t)mode * dd];
   const int* cC = &cnt[(size_t)(mode + 1) * dd];
   const int* cR = &cnt[(size_t)(mode + 2) * dd];
-  UpdateTables& T = P.tab;
+  const int upd = (int)P.tab.size(), sec0 = (int)P.sd.size();
+  P.tab.emplace_back();
+  UpdateTables& T = P.tab.back();
   std::memset(&T, 0, sizeof(T));
   T.d = d;
   T.chi = h->chi;
   T.mode = mode;
+  T.sec0 = sec0;
+  T.gate_off = gate_off;
   block_offsets(cL, d, T.offL);
   block_offsets(cC, d, T.offC);
   block_offsets(cR, d, T.offR);
@@ -308,8 +358,6 @@ int make_plan(bsmpo_ctx* h, int mode, Plan& P) {
     }
   auto rows_of = [&](int a0, int from1) { return T.offL[(a0 + 1) * d] - T.offL[a0 * d + from1]; };
   auto cols_of = [&](int b0, int to1) { return T.offR[b0 * d + to1 + 1] - T.offR[b0 * d]; };
-  P.sd.clear();
-  int64_t c_off = 0, a_off = 0, s_off = 0, w_off = 0, v_off = 0, g_off = 0, y_off = 0;
   for (int cc0 = lo0; cc0 <= hi0; ++cc0)
     for (int cc1 = lo1; cc1 <= hi1; ++cc1) {
       SectorDesc S;
@@ -326,34 +374,40 @@ int make_plan(bsmpo_ctx* h, int mode, Plan& P) {
       S.k = S.left ? m : n;
       S.rows_g = S.left ? n : m;
       S.rows_tot = S.left ? n + m : m;
-      S.c_off = c_off; c_off += (int64_t)m * n;
-      S.a_off = a_off; a_off += (int64_t)S.rows_tot * S.k;
-      S.s_off = s_off; s_off += S.k;
-      S.w_off = w_off; w_off += (int64_t)S.k * n;
-      S.v_off = v_off; v_off += (int64_t)m * S.k;
-      S.g_off = g_off; g_off += (int64_t)S.k * S.k;
-      S.y_off = y_off; y_off += (int64_t)S.k * S.k;
+      S.c_off = P.c_elems; P.c_elems += (int64_t)m * n;
+      S.a_off = P.a_elems; P.a_elems += (int64_t)S.rows_tot * S.k;
+      S.s_off = P.s_elems; P.s_elems += S.k;
+      S.w_off = P.w_elems; P.w_elems += (int64_t)S.k * n;
+      S.v_off = P.v_elems; P.v_elems += (int64_t)m * S.k;
+      S.g_off = P.g_elems; P.g_elems += (int64_t)S.k * S.k;
+      S.y_off = P.y_elems; P.y_elems += (int64_t)S.k * S.k;
       T.sidx[cc0 * d + cc1] = (int)P.sd.size();
       P.sd.push_back(S);
     }
-  const int ns = (int)P.sd.size();
+  const int ns = (int)P.sd.size() - sec0;
   if (ns > BSMPO_MAX_Q) return fail(h, BSMPO_EINVAL, "too many sectors");
-  for (int s = 0; s < ns; ++s) {
-    const int p = T.sidx[P.sd[s].cc1 * d + P.sd[s].cc0];
-    T.pair_of[s] = p;
-  }
+  if (ns == 0) return fail(h, BSMPO_EINVAL, "update with an empty left or right bond");
+  for (int s = 0; s < ns; ++s) T.pair_of[s] = T.sidx[P.sd[sec0 + s].cc1 * d + P.sd[sec0 + s].cc0];
   T.n_sectors = ns;
-  P.c_elems = c_off; P.a_elems = a_off; P.s_elems = s_off; P.w_elems = w_off; P.v_elems = v_off;
-  P.g_elems = g_off; P.y_elems = y_off;
   // Theta groups (q, a0, b0)
-  P.tidx.assign((size_t)dd * d * d, -1);
-  P.td.clear();
-  P.gg.clear();
-  int64_t t_off = 0;
-  int tiles = 0;
+  const size_t tidx0 = P.tidx.size();
+  P.tidx.resize(tidx0 + (size_t)dd * dd, -1);
   const int TMt = zgemm_tile_m(), TNt = zgemm_tile_n();
   const int64_t chi2 = (int64_t)h->chi * h->chi;
-  P.flops_theta = 0.0;
+  const bool tc_theta = h->precision == BSMPO_PRECISION_TF32X3 && (h->tc_mask & 1);
+  const int tm = tc_tile_m(), tn = tc_tile_n();
+  const size_t mb = tc_map_bytes();
+  if (tc_theta) {
+    // Theta on the tensor cores: one tensor map per site tensor, groups address blocks
+    P.tcmaps.resize(P.tcmaps.size() + 2 * mb, 0);
+    unsigned char* maps = P.tcmaps.data() + (size_t)2 * upd * mb;
+    const cplx* gl = h->gamma + (size_t)mode * chi2;
+    const cplx* gr = h->gamma + (size_t)(mode + 1) * chi2;
+    if (tc_encode_map(maps, gl, h->chi, h->chi, h->chi, 0) != cudaSuccess ||
+        tc_encode_map(maps + mb, gr, h->chi, h->chi, h->chi, 2) != cudaSuccess)
+      return fail(h, BSMPO_ECUDA, "tensor map encoding failed");
+  }
+  double flops_theta = 0.0;
   for (int q0 = 0; q0 < d; ++q0)
     for (int q1 = 0; q1 < d; ++q1) {
       const int nk = cC[q0 * d + q1];
@@ -369,90 +423,44 @@ int make_plan(bsmpo_ctx* h, int mode, Plan& P) {
           D.row0 = T.offL[a0 * d + q1]; D.nrow = nrow;
           D.col0 = T.offR[b0 * d]; D.ncol = ncol;
           D.k0 = T.offC[q0 * d + q1]; D.nk = nk;
-          D.off = t_off;
-          t_off += (int64_t)nrow * ncol;
-          P.tidx[((q0 * d + q1) * d + a0) * d + b0] = (int)P.td.size();
+          D.off = P.theta_elems;
+          P.theta_elems += (int64_t)nrow * ncol;
+          P.tidx[tidx0 + ((q0 * d + q1) * d + a0) * d + b0] = (int)P.td.size();
           P.td.push_back(D);
+          flops_theta += 8.0 * nrow * (double)nk * ncol;
+          if (tc_theta) {
+            TcGroup g;
+            std::memset(&g, 0, sizeof(g));
+            g.M = nrow; g.N = ncol; g.K = nk;
+            g.opA = 0; g.mapA = 2 * upd; g.mapB = 2 * upd + 1;
+            g.a_r0 = D.row0; g.a_c0 = D.k0; g.b_r0 = D.k0; g.b_c0 = D.col0;
+            g.ldc = ncol;
+            g.tiles_n = ceil_div(ncol, tn);
+            g.tile_start = P.tc_tiles;
+            P.tc_tiles += ceil_div(nrow, tm) * g.tiles_n;
+            g.c_off = D.off;
+            g.cs_off = -1;
+            P.tcg.push_back(g);
+            continue;
+          }
           GemmGroup g;
           std::memset(&g, 0, sizeof(g));
           g.M = nrow; g.N = ncol; g.K = nk;
           g.lda = h->chi; g.ldb = h->chi; g.ldc = ncol;
-          g.opA = 0; g.opB = 0; g.beta = 0;
+          g.opA = 0; g.opB = 0; g.beta = 0; g.sec = -1;
           g.tiles_n = ceil_div(ncol, TNt);
-          g.tile_start = tiles;
-          tiles += ceil_div(nrow, TMt) * g.tiles_n;
+          g.tile_start = P.gemm_tiles;
+          P.gemm_tiles += ceil_div(nrow, TMt) * g.tiles_n;
           g.a_off = (int64_t)mode * chi2 + (int64_t)D.row0 * h->chi + D.k0;
           g.b_off = (int64_t)(mode + 1) * chi2 + (int64_t)D.k0 * h->chi + D.col0;
           g.c_off = D.off;
           g.ks_off = g.rs_off = g.cs_off = -1;
           P.gg.push_back(g);
-          P.flops_theta += 8.0 * nrow * (double)nk * ncol;
         }
       }
     }
-  P.theta_elems = t_off;
-  P.gemm_tiles = tiles;
-  // Theta on the tensor cores: one tensor map per site tensor, groups address blocks
-  P.tcg.clear();
-  P.tcmaps.clear();
-  P.tc_tiles = 0;
-  if (h->precision == BSMPO_PRECISION_TF32X3 && (h->tc_mask & 1)) {
-    const size_t mb = tc_map_bytes();
-    P.tcmaps.assign(2 * mb, 0);
-    const cplx* gl = h->gamma + (size_t)mode * chi2;
-    const cplx* gr = h->gamma + (size_t)(mode + 1) * chi2;
-    if (tc_encode_map(P.tcmaps.data(), gl, h->chi, h->chi, h->chi, 0) != cudaSuccess ||
-        tc_encode_map(P.tcmaps.data() + mb, gr, h->chi, h->chi, h->chi, 2) != cudaSuccess)
-      return fail(h, BSMPO_ECUDA, "tensor map encoding failed");
-    const int tm = tc_tile_m(), tn = tc_tile_n();
-    for (const ThetaDesc& D : P.td) {
-      TcGroup g;
-      std::memset(&g, 0, sizeof(g));
-      g.M = D.nrow; g.N = D.ncol; g.K = D.nk;
-      g.opA = 0; g.mapA = 0; g.mapB = 1;
-      g.a_r0 = D.row0; g.a_c0 = D.k0; g.b_r0 = D.k0; g.b_c0 = D.col0;
-      g.ldc = D.ncol;
-      g.tiles_n = ceil_div(D.ncol, tn);
-      g.tile_start = P.tc_tiles;
-      P.tc_tiles += ceil_div(D.nrow, tm) * g.tiles_n;
-      g.c_off = D.off;
-      g.cs_off = -1;
-      P.tcg.push_back(g);
-    }
-  }
-  // Gram groups: G_s = X^H X, X = the first rows_g rows of the sector's Jacobi matrix
-  // ([rows_g][k] row-major: T, or T^H when |L| < |R|)
-  P.ggram.clear();
-  int gtiles = 0;
-  for (const SectorDesc& S : P.sd) {
-    GemmGroup g;
-    std::memset(&g, 0, sizeof(g));
-    g.M = S.k; g.N = S.k; g.K = S.rows_g;
-    g.lda = S.k; g.ldb = S.k; g.ldc = S.k;
-    g.opA = 1; g.opB = 0; g.beta = 0;
-    g.tiles_n = ceil_div(S.k, TNt);
-    g.tile_start = gtiles;
-    gtiles += ceil_div(S.k, TMt) * g.tiles_n;
-    g.a_off = S.a_off; g.b_off = S.a_off; g.c_off = S.g_off;
-    g.ks_off = g.rs_off = g.cs_off = -1;
-    P.ggram.push_back(g);
-  }
-  P.gram_tiles = gtiles;
-  P.tdlist.clear();
-  for (int c = 0; c < 4; ++c) {
-    P.td_count[c] = 0;
-    P.td_kmax[c] = 0;
-    for (int s = 0; s < (int)P.sd.size(); ++s)
-      if (tridiag_class(P.sd[s].k) == c) {
-        P.tdlist.push_back(s);
-        P.td_count[c]++;
-        P.td_kmax[c] = std::max(P.td_kmax[c], P.sd[s].k);
-      }
-  }
-  T.n_theta = (int)P.td.size();
+  P.flops_theta.push_back(flops_theta);
   // mix pairs (a >= b)
-  P.pairs.clear();
-  int mt = 0;
   for (int a0 = 0; a0 < d; ++a0)
     for (int a1 = 0; a1 < d; ++a1) {
       const int na = cL[a0 * d + a1];
@@ -465,24 +473,82 @@ int make_plan(bsmpo_ctx* h, int mode, Plan& P) {
           M.a0 = a0; M.a1 = a1; M.b0 = b0; M.b1 = b1;
           M.row0 = T.offL[a0 * d + a1]; M.nrow = na;
           M.col0 = T.offR[b0 * d + b1]; M.ncol = nb;
-          M.tile_start = mt;
-          M.pad_ = 0;
-          mt += ceil_div(na * nb, 256);
+          M.tile_start = P.mix_tiles;
+          M.upd = upd;
+          P.mix_tiles += ceil_div(na * nb, 256);
           P.pairs.push_back(M);
         }
     }
-  P.mix_tiles = mt;
-  T.n_pairs = (int)P.pairs.size();
-  // Jacobi work
-  P.jw.clear();
-  P.max_rounds = 0;
-  P.max_k = 0;
-  P.max_left_m2 = 0;
+  for (int s = sec0; s < sec0 + ns; ++s) {
+    const SectorDesc& S = P.sd[s];
+    P.max_k = std::max(P.max_k, S.k);
+    P.max_v = std::max(P.max_v, S.m * S.k);
+    // W = V^H C; the kept count (M, and V's row length) is read on the device
+    GemmGroup g;
+    std::memset(&g, 0, sizeof(g));
+    g.M = S.k; g.N = S.n; g.K = S.m;
+    g.lda = S.k; g.ldb = S.n; g.ldc = S.n;
+    g.opA = 1; g.sec = s; g.kdim = 1;
+    g.tiles_n = ceil_div(S.n, TNt);
+    g.tile_start = P.w_tiles;
+    P.w_tiles += ceil_div(S.k, TMt) * g.tiles_n;
+    g.a_off = S.v_off; g.b_off = S.c_off; g.c_off = S.w_off;
+    g.ks_off = g.rs_off = g.cs_off = -1;
+    P.gw.push_back(g);
+    if (P.gram) {
+      // Gram G_s = X^H X, X = the first rows_g rows of the sector's Jacobi matrix
+      // ([rows_g][k] row-major: T, or T^H when |L| < |R|)
+      GemmGroup r;
+      std::memset(&r, 0, sizeof(r));
+      r.M = S.k; r.N = S.k; r.K = S.rows_g;
+      r.lda = S.k; r.ldb = S.k; r.ldc = S.k;
+      r.opA = 1; r.sec = -1;
+      r.tiles_n = ceil_div(S.k, TNt);
+      r.tile_start = P.gram_tiles;
+      P.gram_tiles += ceil_div(S.k, TMt) * r.tiles_n;
+      r.a_off = S.a_off; r.b_off = S.a_off; r.c_off = S.g_off;
+      r.ks_off = r.rs_off = r.cs_off = -1;
+      P.ggram.push_back(r);
+      if (!S.left) {
+        // V [m][kept] = T [m][k] Y [k][kept] diag(1 / sigma)
+        GemmGroup v;
+        std::memset(&v, 0, sizeof(v));
+        v.M = S.m; v.N = S.k; v.K = S.k;
+        v.lda = S.k; v.ldb = S.k; v.ldc = S.k;
+        v.sec = s; v.kdim = 2;
+        v.tiles_n = ceil_div(S.k, TNt);
+        v.tile_start = P.v_tiles;
+        P.v_tiles += ceil_div(S.m, TMt) * v.tiles_n;
+        v.a_off = S.a_off; v.b_off = S.y_off; v.c_off = S.v_off;
+        v.ks_off = v.rs_off = -1;
+        v.cs_off = S.s_off;
+        P.gv.push_back(v);
+      }
+    }
+  }
+  return BSMPO_OK;
+}
+
+// The sector-wise work lists, once every update of the group is in the plan.
+void finish_plan(bsmpo_ctx* h, Plan& P) {
+  const int ns = (int)P.sd.size();
+  if (P.gram) {
+    for (int c = 0; c < TD_CLASSES; ++c) {
+      const size_t first = P.tdlist.size();
+      for (int s = 0; s < ns; ++s)
+        if (tridiag_class(P.sd[s].k) == c) P.tdlist.push_back(s);
+      // largest first: the last CTAs to start are the shortest
+      std::stable_sort(P.tdlist.begin() + first, P.tdlist.end(),
+                       [&](int x, int y) { return P.sd[x].k > P.sd[y].k; });
+      P.td_count[c] = (int)(P.tdlist.size() - first);
+      P.td_kmax[c] = P.td_count[c] ? P.sd[P.tdlist[first]].k : 0;
+    }
+    return;
+  }
   const int JBc = jacobi_block_cols();
   const int rmax = std::min(h->jac_rows, jacobi_rows_per_part());
   for (int s = 0; s < ns; ++s) {
     const SectorDesc& S = P.sd[s];
-    P.max_k = std::max(P.max_k, S.k);
     if (S.left) P.max_left_m2 = std::max(P.max_left_m2, S.m * S.m);
     JacobiWork w;
     std::memset(&w, 0, sizeof(w));
@@ -502,30 +568,52 @@ int make_plan(bsmpo_ctx* h, int mode, Plan& P) {
   }
   std::vector<JacobiWork> all(P.jw);
   jacobi_launch_list(all, &P.gram_ctas, &P.apply_ctas, &P.jac_slots);
-  return BSMPO_OK;
 }
 
 // packs plan tables into the pinned stage and copies them to the device table buffer
 struct TabLayout {
-  size_t tab, tidx, td, sd, pairs, gg, ggram, tdlist, tcmaps, tcg, jw, total;
+  size_t tab, tidx, td, sd, pairs, gg, ggram, gv, gw, tdlist, tcmaps, tcg, jw, total;
 };
 
 TabLayout layout_of(const Plan& P) {
   TabLayout L;
   size_t o = 0;
-  L.tab = o; o = align_up(o + sizeof(UpdateTables), 256);
-  L.tidx = o; o = align_up(o + P.tidx.size() * sizeof(int), 256);
-  L.td = o; o = align_up(o + P.td.size() * sizeof(ThetaDesc) + 1, 256);
-  L.sd = o; o = align_up(o + P.sd.size() * sizeof(SectorDesc) + 1, 256);
-  L.pairs = o; o = align_up(o + P.pairs.size() * sizeof(MixPair) + 1, 256);
-  L.gg = o; o = align_up(o + P.gg.size() * sizeof(GemmGroup) + 1, 256);
-  L.ggram = o; o = align_up(o + P.ggram.size() * sizeof(GemmGroup) + 1, 256);
-  L.tdlist = o; o = align_up(o + P.tdlist.size() * sizeof(int) + 1, 256);
-  L.tcmaps = o; o = align_up(o + P.tcmaps.size() + 1, 256);
-  L.tcg = o; o = align_up(o + P.tcg.size() * sizeof(TcGroup) + 1, 256);
-  L.jw = o; o = align_up(o + P.jw.size() * sizeof(JacobiWork) + 1, 256);
+  auto place = [&](size_t bytes) {
+    const size_t at = o;
+    o = align_up(o + bytes + 1, 256);
+    return at;
+  };
+  L.tab = place(P.tab.size() * sizeof(UpdateTables));
+  L.tidx = place(P.tidx.size() * sizeof(int));
+  L.td = place(P.td.size() * sizeof(ThetaDesc));
+  L.sd = place(P.sd.size() * sizeof(SectorDesc));
+  L.pairs = place(P.pairs.size() * sizeof(MixPair));
+  L.gg = place(P.gg.size() * sizeof(GemmGroup));
+  L.ggram = place(P.ggram.size() * sizeof(GemmGroup));
+  L.gv = place(P.gv.size() * sizeof(GemmGroup));
+  L.gw = place(P.gw.size() * sizeof(GemmGroup));
+  L.tdlist = place(P.tdlist.size() * sizeof(int));
+  L.tcmaps = place(P.tcmaps.size());
+  L.tcg = place(P.tcg.size() * sizeof(TcGroup));
+  L.jw = place(P.jw.size() * sizeof(JacobiWork));
   L.total = o;
   return L;
+}
+
+// The pinned words that come back from the device during a group's update.
+struct ResLayout {
+  size_t kept, trunc, err, work, rot, total;
+};
+
+ResLayout result_layout(int ns, int nj) {
+  ResLayout R;
+  R.kept = 0;                                                    // int[ns] kept, int[nj] totals
+  R.trunc = align_up((size_t)(ns + nj) * sizeof(int), 256);      // double[nj]
+  R.err = align_up(R.trunc + nj * sizeof(double), 256);          // int
+  R.work = R.err + 256;                                          // unsigned long long[2]
+  R.rot = R.work + 256;                                          // 2 x int[3 ns]
+  R.total = align_up(R.rot + (size_t)6 * ns * sizeof(int), 256);
+  return R;
 }
 
 template <typename T>
@@ -555,18 +643,299 @@ struct StageClock {
   }
 };
 
-int bs_update_impl(bsmpo_ctx* h, int mode, const cplx* u3_dev) {
-  int rc = check_mode(h, mode);
-  if (rc) return rc;
+// 3a. The Gram route's eigenvalues: Gram matrices, tridiagonalisation, bisection.
+int gram_eigenvalues(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, const GemmGroup* ggram_d,
+                     const int* tdlist_d, int* err_d) {
+  const int ns = (int)P.sd.size();
+  cudaStream_t st = h->stream;
+  int rc;
+  if (P.max_k > eigen_max_k())
+    return fail(h, BSMPO_ECAPACITY, "a sector of dimension " + std::to_string(P.max_k) +
+                                        " exceeds the Gram route's limit " + std::to_string(eigen_max_k()));
+  if ((rc = grow(h, h->gbuf, std::max<int64_t>(P.g_elems, 1) * sizeof(cplx)))) return rc;
+  if ((rc = grow(h, h->eigd, std::max<int64_t>(3 * P.s_elems, 1) * sizeof(double)))) return rc;
+  if ((rc = grow(h, h->taub, std::max<int64_t>(P.s_elems, 1) * sizeof(cplx)))) return rc;
+  if ((rc = grow(h, h->invsig, std::max<int64_t>(P.s_elems, 1) * sizeof(double)))) return rc;
+  double* dbuf_d = reinterpret_cast<double*>(h->eigd.p);
+  double* ebuf_d = dbuf_d + P.s_elems;
+  double* lam_d = ebuf_d + P.s_elems;
+  if (h->timing) CK(h, cudaEventRecord(h->ev0, st));
+  CKL(h, launch_zgemm_grouped(h->abuf.p, h->abuf.p, h->gbuf.p, nullptr, ggram_d, (int)P.ggram.size(), P.gram_tiles,
+                              nullptr, st));
+  // the largest class present on the update's stream, the others dealt out to the side
+  // streams (none: all one after another)
+  if (h->td_fork > 0 && (rc = make_fork_streams(h))) return rc;
+  const int naux = std::min(h->td_fork, h->n_aux);
+  cudaStream_t ts[TD_CLASSES];
+  bool used[3] = {false, false, false};
+  for (int c = TD_CLASSES - 1, slot = -1; c >= 0; --c) {
+    ts[c] = st;
+    if (P.td_count[c] == 0) continue;
+    if (slot >= 0 && naux > 0) {
+      ts[c] = h->aux[slot % naux];
+      used[slot % naux] = true;
+    }
+    ++slot;
+  }
+  const bool fork = used[0] || used[1] || used[2];
+  if (h->timing) {
+    if (!h->td_ev0) {
+      CK(h, cudaEventCreate(&h->td_ev0));
+      CK(h, cudaEventCreate(&h->td_ev1));
+    }
+    CK(h, cudaEventRecord(h->td_ev0, st));
+  }
+  if (fork) {
+    CK(h, cudaEventRecord(h->fork_ev, st));
+    for (int i = 0; i < 3; ++i)
+      if (used[i]) CK(h, cudaStreamWaitEvent(h->aux[i], h->fork_ev, 0));
+  }
+  CK(h, launch_tridiag(sd_d, tdlist_d, P.td_count, P.td_kmax, h->gbuf.p, dbuf_d, ebuf_d, h->taub.p, err_d, ts));
+  for (int i = 0; i < 3; ++i)
+    if (used[i]) {
+      CK(h, cudaEventRecord(h->join_ev[i], h->aux[i]));
+      CK(h, cudaStreamWaitEvent(st, h->join_ev[i], 0));
+    }
+  // the last class takes two kernels
+  for (int c = 0; c < TD_CLASSES; ++c) h->launches += P.td_count[c] > 0 ? 1 + (c == TD_CLASSES - 1) : 0;
+  if (h->timing) CK(h, cudaEventRecord(h->td_ev1, st));
+  CK(h, launch_bisect(sd_d, ns, P.max_k, dbuf_d, ebuf_d, lam_d, reinterpret_cast<double*>(h->sig.p),
+                      reinterpret_cast<double*>(h->invsig.p), st));
+  h->launches += 2;
+  if (h->timing) CK(h, cudaEventRecord(h->ev1, st));
+  h->last_sweeps = 0;
+  return BSMPO_OK;
+}
+
+// The Gram route's timing (timing mode): its events have completed when the kept counts
+// have arrived.
+int gram_timing(bsmpo_ctx* h, const Plan& P) {
+  // eigen phase of the Gram route (Gram GEMM, tridiagonalisation, bisection)
+  float ms = 0.f;
+  CK(h, cudaEventElapsedTime(&ms, h->ev0, h->ev1));
+  h->jac_ms += ms;
+  h->jac_launches += 4;
+  // algorithmic flops: the Gram (8 k^2 rows, complex MACs) and the Householder
+  // reduction of a k x k Hermitian matrix (16/3 k^3, LAPACK's zhetrd count)
+  for (const SectorDesc& S : P.sd)
+    h->jac_flops += 8.0 * (double)S.k * S.k * S.rows_g + 16.0 / 3.0 * (double)S.k * S.k * S.k;
+  float tms = 0.f;
+  CK(h, cudaEventElapsedTime(&tms, h->td_ev0, h->td_ev1));
+  h->td_ms += tms;
+  h->td_phases++;
+  for (const SectorDesc& S : P.sd) {
+    // step j reads and writes the (k - j - 1)^2 trailing matrix once: 32 B per entry
+    const double k = S.k;
+    h->td_bytes += 32.0 * (k - 1.0) * k * (2.0 * k - 1.0) / 6.0;
+    h->td_flops += 16.0 / 3.0 * k * k * k;
+  }
+  return BSMPO_OK;
+}
+
+// 3b. Blocked one-sided Jacobi of every sector of the group.
+int jacobi_svd(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, char* jw_d, const ResLayout& R) {
+  const int ns = (int)P.sd.size();
+  cudaStream_t st = h->stream;
+  int rc;
+  char* hres = static_cast<char*>(h->hres.p);
+  const size_t pair_elems = (size_t)4 * jacobi_block_cols() * jacobi_block_cols();
+  if ((rc = grow(h, h->perm, std::max<int64_t>(P.s_elems, 1) * sizeof(int)))) return rc;
+  if ((rc = grow(h, h->rot, (size_t)3 * ns * sizeof(int)))) return rc;
+  if ((rc = grow(h, h->nf2, (size_t)ns * sizeof(double)))) return rc;
+  if ((rc = grow(h, h->qbuf, std::max(P.jac_slots, 1) * pair_elems * sizeof(cplx)))) return rc;
+  if ((rc = grow(h, h->qflag, std::max(P.jac_slots, 1) * sizeof(int)))) return rc;
+  if ((rc = grow(h, h->pcnt, std::max(P.jac_slots, 1) * sizeof(int)))) return rc;
+  if ((rc = grow(h, h->pbuf, std::max(P.gram_ctas, 1) * pair_elems * sizeof(cplx)))) return rc;
+  if ((rc = grow(h, h->jwork, 2 * sizeof(unsigned long long)))) return rc;
+  double* nf2 = reinterpret_cast<double*>(h->nf2.p);
+  CKL(h, launch_sector_norms(sd_d, ns, h->abuf.p, nf2, st));
+  CK(h, cudaMemsetAsync(h->rot.p, 0, (size_t)3 * ns * sizeof(int), st));
+  CK(h, cudaMemsetAsync(h->pcnt.p, 0, std::max(P.jac_slots, 1) * sizeof(int), st));
+  CK(h, cudaMemsetAsync(h->jwork.p, 0, 2 * sizeof(unsigned long long), st));
+  std::vector<JacobiWork> active(P.jw);
+  int gram_ctas = 0, apply_ctas = 0, slots = 0;
+  jacobi_launch_list(active, &gram_ctas, &apply_ctas, &slots);
+  // Convergence polls run one chunk behind: after launching chunk c + 1 the host reads
+  // the counters copied after chunk c, so the stream always has a chunk queued while the
+  // host checks (a converged sector's rounds in the extra chunk exit at once).  Counters
+  // and compacted launch tables alternate between two pinned slots.
+  int* hrot_slot[2] = {reinterpret_cast<int*>(hres + R.rot), nullptr};
+  hrot_slot[1] = hrot_slot[0] + 3 * ns;
+  const size_t jw_bytes = align_up(std::max<size_t>(P.jw.size(), 1) * sizeof(JacobiWork), 256);
+  if ((rc = grow_host(h, h->stage2, 2 * jw_bytes))) return rc;
+  char* jw_stage[2] = {static_cast<char*>(h->stage2.p), static_cast<char*>(h->stage2.p) + jw_bytes};
+  for (cudaEvent_t& e : h->poll_ev)
+    if (!e) CK(h, cudaEventCreateWithFlags(&e, cudaEventBlockingSync | cudaEventDisableTiming));
+  int t = 0;
+  const int t_max = MAX_SWEEPS * std::max(1, P.max_rounds);
+  bool converged = false;
+  int checks = 0;
+  std::vector<int> conv_at(ns, -1);
+  if (h->timing) CK(h, cudaEventRecord(h->ev0, st));
+  const int chunk = std::max(1, P.max_rounds);   // one sweep of the largest sector
+  int t_after[2] = {0, 0};
+  auto launch_chunk = [&](int slot) -> int {
+    for (int i = 0; i < chunk && t < t_max; ++i, ++t) {
+      // tol <= 0: per-sector default 4 eps sqrt(rows of the Gram), at least 8 eps
+      CK(h, launch_jacobi_round(sd_d, reinterpret_cast<const JacobiWork*>(jw_d), (int)active.size(), gram_ctas,
+                                apply_ctas, t, h->abuf.p, reinterpret_cast<int*>(h->rot.p), nf2, 0.0, MAX_SWEEPS,
+                                h->pbuf.p, reinterpret_cast<int*>(h->pcnt.p), h->qbuf.p,
+                                reinterpret_cast<int*>(h->qflag.p),
+                                reinterpret_cast<unsigned long long*>(h->jwork.p), st));
+      h->launches += 2;
+    }
+    CK(h, cudaMemcpyAsync(hrot_slot[slot], h->rot.p, (size_t)3 * ns * sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(h, cudaEventRecord(h->poll_ev[slot], st));
+    t_after[slot] = t;
+    return BSMPO_OK;
+  };
+  if ((rc = launch_chunk(0))) return rc;
+  int cur = 0, compactions = 0;
+  for (;;) {
+    const bool more = t < t_max;
+    if (more && (rc = launch_chunk(cur ^ 1))) return rc;
+    CK(h, cudaEventSynchronize(h->poll_ev[cur]));
+    ++checks;
+    const int* hrot = hrot_slot[cur];
+    bool all = true;
+    for (int s = 0; s < ns; ++s) {
+      // a converged sector leaves the launches, and its counters are stale from then on
+      if (conv_at[s] >= 0) continue;
+      const int Rn = P.jw[s].rounds;
+      const int done = t_after[cur] / Rn;
+      if (done < 1 || hrot[3 * s + (done - 1) % 3] != 0) { all = false; continue; }
+      conv_at[s] = done;
+    }
+    if (all) { converged = true; break; }
+    if (!more) break;
+    // drop converged sectors (and those out of sweeps) from the launches after the queued
+    // chunk: the table copy is stream-ordered after it
+    std::vector<JacobiWork> next;
+    for (const auto& w : P.jw)
+      if (conv_at[w.sector] < 0 && t / w.rounds < MAX_SWEEPS) next.push_back(w);
+    if (next.size() < active.size() && !next.empty()) {
+      active.swap(next);
+      jacobi_launch_list(active, &gram_ctas, &apply_ctas, &slots);
+      char* stg = jw_stage[compactions++ & 1];
+      put(stg, 0, active);
+      CK(h, cudaMemcpyAsync(jw_d, stg, active.size() * sizeof(JacobiWork), cudaMemcpyHostToDevice, st));
+    }
+    cur ^= 1;
+  }
+  if (h->timing) {
+    CK(h, cudaMemcpyAsync(hres + R.work, h->jwork.p, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+    CK(h, cudaEventRecord(h->ev1, st));
+  }
+  // sweeps the slowest sector needed (its last one without rotations included); t also
+  // counts the chunk queued after convergence, whose rounds exit at once
+  {
+    int sw = 0;
+    for (int s = 0; s < ns; ++s) sw = std::max(sw, conv_at[s] >= 0 ? conv_at[s] : t / P.jw[s].rounds);
+    h->last_sweeps = sw;
+  }
+  h->jacobi_rounds += t;   // launched rounds, including the drained chunk
+  if (h->timing) {
+    float ms = 0.f;
+    CK(h, cudaEventSynchronize(h->ev1));
+    CK(h, cudaEventElapsedTime(&ms, h->ev0, h->ev1));
+    h->jac_ms += ms;
+    h->jac_launches += t;
+    // flops of the executed work, counted on the device: every row that formed a
+    // partial pair Gram contributes its 10 upper 8 x 8 tiles (640 complex MACs), every
+    // rotated row 32 x 32 complex MACs; 8 flops per complex MAC.  Pairs that did not
+    // rotate and sectors that had converged do no apply work and are not counted.
+    const unsigned long long* hw = reinterpret_cast<const unsigned long long*>(hres + R.work);
+    h->jac_flops += 8.0 * 640.0 * (double)hw[0] + 8.0 * 1024.0 * (double)hw[1];
+  }
+  if (!converged) {
+    std::string msg = "Jacobi SVD did not converge";
+    for (const UpdateTables& T : P.tab)
+      for (int i = 0; i < T.n_sectors; ++i) {
+        const int s = T.sec0 + i;
+        if (conv_at[s] >= 0) continue;
+        const int Rn = P.jw[s].rounds, done = t_after[cur] / Rn;
+        const SectorDesc& S = P.sd[s];
+        msg += " (mode " + std::to_string(T.mode) + "); sector (" + std::to_string(S.cc0) + "," +
+               std::to_string(S.cc1) + ") m=" + std::to_string(S.m) + " n=" + std::to_string(S.n) +
+               " sweeps=" + std::to_string(done) + " rotations=" +
+               std::to_string(hrot_slot[cur][3 * s + (done - 1 + 3) % 3]);
+        return fail(h, BSMPO_ECONVERGE, msg);
+      }
+    return fail(h, BSMPO_ECONVERGE, msg);
+  }
+  CKL(h, launch_jacobi_finish(sd_d, ns, P.max_k, h->abuf.p, nf2, reinterpret_cast<double*>(h->sig.p),
+                              reinterpret_cast<int*>(h->perm.p), st));
+  return BSMPO_OK;
+}
+
+// W = V^H C on the tensor cores (TF32X3 with bit 1 of tc_mask): two tensor maps per
+// sector, built from the kept counts on the host.
+int tc_w_gemm(bsmpo_ctx* h, const Plan& P, const int* hk, int* err_d) {
+  const size_t mb = tc_map_bytes();
+  cudaStream_t st = h->stream;
+  std::vector<unsigned char> maps;
+  std::vector<TcGroup> tw;
+  int tw_tiles = 0, rc;
+  const int tm = tc_tile_m(), tn = tc_tile_n();
+  bool enc_ok = true;
+  auto add_map = [&](const void* base, int rows, int cols, int ld, int kind) -> int {
+    const int idx = (int)(maps.size() / mb);
+    maps.resize(maps.size() + mb);
+    if (tc_encode_map(maps.data() + (size_t)idx * mb, base, rows, cols, ld, kind) != cudaSuccess) enc_ok = false;
+    return idx;
+  };
+  const cplx* V0 = reinterpret_cast<const cplx*>(h->vbuf.p);
+  const cplx* C0 = reinterpret_cast<const cplx*>(h->cbuf.p);
+  for (int s = 0; s < (int)P.sd.size(); ++s) {
+    const SectorDesc& S = P.sd[s];
+    const int kp = hk[s];
+    if (kp == 0) continue;
+    TcGroup g;
+    std::memset(&g, 0, sizeof(g));
+    g.M = kp; g.N = S.n; g.K = S.m; g.opA = 1;
+    g.mapA = add_map(V0 + S.v_off, S.m, kp, kp, 1);
+    g.mapB = add_map(C0 + S.c_off, S.m, S.n, S.n, 2);
+    g.ldc = S.n;
+    g.tiles_n = ceil_div(S.n, tn);
+    g.tile_start = tw_tiles;
+    tw_tiles += ceil_div(kp, tm) * g.tiles_n;
+    g.c_off = S.w_off;
+    g.cs_off = -1;
+    tw.push_back(g);
+  }
+  if (!enc_ok) return fail(h, BSMPO_ECUDA, "tensor map encoding failed");
+  const size_t o_tw = align_up(maps.size(), 256);
+  const size_t total = align_up(o_tw + tw.size() * sizeof(TcGroup) + 1, 256);
+  if ((rc = grow(h, h->tab3, total))) return rc;
+  if ((rc = grow_host(h, h->stage3, total))) return rc;
+  if (!maps.empty()) std::memcpy(h->stage3.p, maps.data(), maps.size());
+  put(h->stage3.p, o_tw, tw);
+  CK(h, cudaMemcpyAsync(h->tab3.p, h->stage3.p, total, cudaMemcpyHostToDevice, st));
+  const char* t3 = static_cast<const char*>(h->tab3.p);
+  CKL(h, launch_tc_zgemm(reinterpret_cast<const TcGroup*>(t3 + o_tw), (int)tw.size(), tw_tiles, t3, h->wbuf.p,
+                         nullptr, err_d, st));
+  return BSMPO_OK;
+}
+
+// Updates at the modes of `jobs` (disjoint sites, one route), all in the same launches.
+// Every sector computes exactly what it computes in a group of its own; trunc[j], if
+// given, receives job j's truncation weight.  Returns with the kept counts on the host
+// (the plan of a following update needs them) and the group's last kernels in flight.
+int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
+  int rc = BSMPO_OK;
+  for (int j = 0; j < nj; ++j)
+    if ((rc = check_mode(h, jobs[j].mode))) return rc;
   StageClock clk(h);
-  h->updates++;
+  h->updates += nj;
   const int d = h->d, chi = h->chi, dd = d * d;
   cudaStream_t st = h->stream;
   Plan P;
-  if ((rc = make_plan(h, mode, P))) return rc;
+  P.gram = gram_route(h, jobs[0].mode);
+  const cplx* u3_base = jobs[0].u3;
+  for (int j = 0; j < nj; ++j)
+    if ((rc = add_update(h, jobs[j].mode, jobs[j].u3 - u3_base, P))) return rc;
+  finish_plan(h, P);
   const int ns = (int)P.sd.size();
-  h->last_ns = ns;
-  if (ns == 0) return fail(h, BSMPO_EINVAL, "update with an empty left or right bond");
   // workspaces
   if ((rc = grow(h, h->theta, std::max<int64_t>(P.theta_elems, 1) * sizeof(cplx)))) return rc;
   if ((rc = grow(h, h->cbuf, std::max<int64_t>(P.c_elems, 1) * sizeof(cplx)))) return rc;
@@ -575,34 +944,32 @@ int bs_update_impl(bsmpo_ctx* h, int mode, const cplx* u3_dev) {
   if ((rc = grow(h, h->vbuf, std::max<int64_t>(P.v_elems, 1) * sizeof(cplx)))) return rc;
   if ((rc = grow(h, h->sig, std::max<int64_t>(P.s_elems, 1) * sizeof(double)))) return rc;
   if ((rc = grow(h, h->keys, std::max<int64_t>(P.s_elems, 1) * sizeof(double)))) return rc;
-  if ((rc = grow(h, h->perm, std::max<int64_t>(P.s_elems, 1) * sizeof(int)))) return rc;
-  if ((rc = grow(h, h->rot, (size_t)3 * ns * sizeof(int)))) return rc;
-  if ((rc = grow(h, h->nf2, (size_t)ns * sizeof(double)))) return rc;
-  const size_t pair_elems = (size_t)4 * jacobi_block_cols() * jacobi_block_cols();
-  if ((rc = grow(h, h->qbuf, std::max(P.jac_slots, 1) * pair_elems * sizeof(cplx)))) return rc;
-  if ((rc = grow(h, h->qflag, std::max(P.jac_slots, 1) * sizeof(int)))) return rc;
-  if ((rc = grow(h, h->pcnt, std::max(P.jac_slots, 1) * sizeof(int)))) return rc;
-  if ((rc = grow(h, h->pbuf, std::max(P.gram_ctas, 1) * pair_elems * sizeof(cplx)))) return rc;
-  if ((rc = grow(h, h->kept, (size_t)(ns + 1) * sizeof(int) + 64))) return rc;
+  const size_t kept_bytes = align_up((size_t)(ns + nj) * sizeof(int), 256);
+  if ((rc = grow(h, h->kept, kept_bytes + nj * sizeof(double)))) return rc;
   const TabLayout L = layout_of(P);
+  const ResLayout R = result_layout(ns, nj);
   if ((rc = grow(h, h->tab, L.total))) return rc;
   if ((rc = grow_host(h, h->stage, L.total))) return rc;
-  if ((rc = grow_host(h, h->hres, 4096 + (size_t)(ns + 2) * sizeof(int) + 6 * ns * sizeof(int)))) return rc;
+  if ((rc = grow_host(h, h->hres, R.total))) return rc;
   char* hs = static_cast<char*>(h->stage.p);
-  std::memcpy(hs + L.tab, &P.tab, sizeof(UpdateTables));
+  put(hs, L.tab, P.tab);
   put(hs, L.tidx, P.tidx);
   put(hs, L.td, P.td);
   put(hs, L.sd, P.sd);
   put(hs, L.pairs, P.pairs);
   put(hs, L.gg, P.gg);
   put(hs, L.ggram, P.ggram);
+  put(hs, L.gv, P.gv);
+  put(hs, L.gw, P.gw);
   put(hs, L.tdlist, P.tdlist);
   put(hs, L.tcmaps, P.tcmaps);
   put(hs, L.tcg, P.tcg);
-  std::vector<JacobiWork> active(P.jw);
-  int gram_ctas = 0, apply_ctas = 0, slots = 0;
-  jacobi_launch_list(active, &gram_ctas, &apply_ctas, &slots);
-  put(hs, L.jw, active);
+  {
+    std::vector<JacobiWork> active(P.jw);
+    int a, b, c;
+    jacobi_launch_list(active, &a, &b, &c);
+    put(hs, L.jw, active);
+  }
   char* dt = static_cast<char*>(h->tab.p);
   CK(h, cudaMemcpyAsync(dt, hs, L.total, cudaMemcpyHostToDevice, st));
   const UpdateTables* tab_d = reinterpret_cast<const UpdateTables*>(dt + L.tab);
@@ -610,9 +977,7 @@ int bs_update_impl(bsmpo_ctx* h, int mode, const cplx* u3_dev) {
   const ThetaDesc* td_d = reinterpret_cast<const ThetaDesc*>(dt + L.td);
   SectorDesc* sd_d = reinterpret_cast<SectorDesc*>(dt + L.sd);
   const MixPair* pairs_d = reinterpret_cast<const MixPair*>(dt + L.pairs);
-  const GemmGroup* gg_d = reinterpret_cast<const GemmGroup*>(dt + L.gg);
-  const GemmGroup* ggram_d = reinterpret_cast<const GemmGroup*>(dt + L.ggram);
-  const int* tdlist_d = reinterpret_cast<const int*>(dt + L.tdlist);
+  auto groups_at = [&](size_t off) { return reinterpret_cast<const GemmGroup*>(dt + off); };
   const bool tc = h->precision == BSMPO_PRECISION_TF32X3;
   const bool tc_theta = tc && (h->tc_mask & 1), tc_w = tc && (h->tc_mask & 2);
   // error word of the asynchronous pipelines (tensor-core GEMM, streamed
@@ -622,23 +987,6 @@ int bs_update_impl(bsmpo_ctx* h, int mode, const cplx* u3_dev) {
     CK(h, cudaMemsetAsync(h->tcerr.p, 0, sizeof(int), st));
   }
   int* tcerr_d = reinterpret_cast<int*>(h->tcerr.p);
-  // The Gram route drops singular values below ~2e-6 of a sector's largest.  Where the
-  // update does not truncate to chi that is pure loss (W = V^H C carries them through
-  // 1 / Lambda_R), so such updates take the exact Jacobi SVD: up front when the
-  // candidates cannot exceed chi or the centre bond holds fewer than chi vectors, and
-  // after the selection when fewer than chi survive.
-  bool gram = h->precision != BSMPO_PRECISION_FP64;
-  {
-    // the centre bond's current dimension predicts the outcome: a bond below chi was not
-    // truncated by the last update on it and is unlikely to be by this one
-    int64_t sum_k = 0, centre = 0;
-    for (const SectorDesc& S : P.sd) sum_k += S.k;
-    const std::vector<int>& cm = mirror(h);
-    for (int q = 0; q < dd; ++q) centre += cm[(size_t)(mode + 1) * dd + q];
-    if (sum_k <= chi || (h->gram_policy >= 2 && centre < chi)) gram = false;
-  }
-  const JacobiWork* jw_d = reinterpret_cast<const JacobiWork*>(dt + L.jw);
-  const int64_t chi2 = (int64_t)chi * chi;
 
   if ((rc = clk.mark(0))) return rc;
   // 1. Theta_q = Glc[a, q] Gcr[q, b] for every valid triple
@@ -646,413 +994,155 @@ int bs_update_impl(bsmpo_ctx* h, int mode, const cplx* u3_dev) {
     CKL(h, launch_tc_zgemm(reinterpret_cast<const TcGroup*>(dt + L.tcg), (int)P.tcg.size(), P.tc_tiles,
                            dt + L.tcmaps, h->theta.p, nullptr, tcerr_d, st));
   else
-    CKL(h, launch_zgemm_grouped(h->gamma, h->gamma, h->theta.p, nullptr, gg_d, (int)P.gg.size(),
-                                P.gemm_tiles, st));
+    CKL(h, launch_zgemm_grouped(h->gamma, h->gamma, h->theta.p, nullptr, groups_at(L.gg), (int)P.gg.size(),
+                                P.gemm_tiles, nullptr, st));
   if ((rc = clk.mark(1))) return rc;
   // 2. identity rows of [T^H; I] and the gate mix
-  if (!gram) CKL(h, launch_identity_rows(sd_d, ns, P.max_left_m2, h->abuf.p, st));
-  CKL(h, launch_mix_d(d, tab_d, tidx_d, td_d, sd_d, pairs_d, (int)P.pairs.size(), P.mix_tiles,
-                      u3_dev, h->theta.p, h->lam + (size_t)(mode + 2) * chi, h->cbuf.p, h->abuf.p,
-                      st));
+  if (!P.gram) CKL(h, launch_identity_rows(sd_d, ns, P.max_left_m2, h->abuf.p, st));
+  CKL(h, launch_mix_d(d, tab_d, tidx_d, td_d, sd_d, pairs_d, (int)P.pairs.size(), P.mix_tiles, u3_base, h->theta.p,
+                      h->lam, h->cbuf.p, h->abuf.p, st));
   if ((rc = clk.mark(2))) return rc;
-  // 3. the sector SVD: Gram + Hermitian eigenproblem, or blocked one-sided Jacobi
-  double* lam_d = nullptr;
-  double* dbuf_d = nullptr;
-  double* ebuf_d = nullptr;
-  int* hk = reinterpret_cast<int*>(h->hres.p);
-  double* htw = reinterpret_cast<double*>(static_cast<char*>(h->hres.p) + 512);
-  int total_kept = 0;
-  for (;;) {
-  if (gram) {
-    if (P.max_k > eigen_max_k())
-      return fail(h, BSMPO_ECAPACITY, "a sector of dimension " + std::to_string(P.max_k) +
-                                          " exceeds the Gram route's limit " + std::to_string(eigen_max_k()));
-    if ((rc = grow(h, h->gbuf, std::max<int64_t>(P.g_elems, 1) * sizeof(cplx)))) return rc;
-    if ((rc = grow(h, h->eigd, std::max<int64_t>(3 * P.s_elems, 1) * sizeof(double)))) return rc;
-    if ((rc = grow(h, h->taub, std::max<int64_t>(P.s_elems, 1) * sizeof(cplx)))) return rc;
-    if ((rc = grow(h, h->invsig, std::max<int64_t>(P.s_elems, 1) * sizeof(double)))) return rc;
-    dbuf_d = reinterpret_cast<double*>(h->eigd.p);
-    ebuf_d = dbuf_d + P.s_elems;
-    lam_d = ebuf_d + P.s_elems;
-    if (h->timing) CK(h, cudaEventRecord(h->ev0, st));
-    CKL(h, launch_zgemm_grouped(h->abuf.p, h->abuf.p, h->gbuf.p, nullptr, ggram_d, (int)P.ggram.size(),
-                                P.gram_tiles, st));
-    {
-      // the largest class present on the update's stream, the others spread over the
-      // side streams (none: all one after another)
-      if (h->td_fork > 0 && (rc = make_fork_streams(h))) return rc;
-      const int naux = std::min(h->td_fork, h->n_aux);
-      cudaStream_t ts[4] = {st, st, st, st};
-      bool used[3] = {false, false, false};
-      for (int c = 3, slot = -1; c >= 0; --c) {
-        if (P.td_count[c] == 0) continue;
-        if (slot >= 0 && naux > 0) {
-          ts[3 - c] = h->aux[slot % naux];
-          used[slot % naux] = true;
-        }
-        ++slot;
-      }
-      const bool fork = used[0] || used[1] || used[2];
-      if (h->timing) {
-        if (!h->td_ev0) {
-          CK(h, cudaEventCreate(&h->td_ev0));
-          CK(h, cudaEventCreate(&h->td_ev1));
-        }
-        CK(h, cudaEventRecord(h->td_ev0, st));
-      }
-      if (fork) {
-        CK(h, cudaEventRecord(h->fork_ev, st));
-        for (int i = 0; i < 3; ++i)
-          if (used[i]) CK(h, cudaStreamWaitEvent(h->aux[i], h->fork_ev, 0));
-      }
-      CK(h, launch_tridiag(sd_d, tdlist_d, P.td_count, P.td_kmax, h->gbuf.p, dbuf_d, ebuf_d, h->taub.p,
-                           tcerr_d, ts));
-      for (int i = 0; i < 3; ++i)
-        if (used[i]) {
-          CK(h, cudaEventRecord(h->join_ev[i], h->aux[i]));
-          CK(h, cudaStreamWaitEvent(st, h->join_ev[i], 0));
-        }
-      for (int c = 0; c < 4; ++c) h->launches += P.td_count[c] > 0;
-      if (h->timing) CK(h, cudaEventRecord(h->td_ev1, st));
-    }
-    CK(h, launch_bisect(sd_d, ns, P.max_k, dbuf_d, ebuf_d, lam_d, reinterpret_cast<double*>(h->sig.p),
-                        reinterpret_cast<double*>(h->invsig.p), st));
-    h->launches += 2;
-    if (h->timing) CK(h, cudaEventRecord(h->ev1, st));
-    h->last_sweeps = 0;
-    if ((rc = clk.mark(3))) return rc;
-  } else {
-    // 3. blocked one-sided Jacobi
-    double* nf2 = reinterpret_cast<double*>(h->nf2.p);
-    CKL(h, launch_sector_norms(sd_d, ns, h->abuf.p, nf2, st));
-    CK(h, cudaMemsetAsync(h->rot.p, 0, (size_t)3 * ns * sizeof(int), st));
-    CK(h, cudaMemsetAsync(h->pcnt.p, 0, std::max(P.jac_slots, 1) * sizeof(int), st));
-    if ((rc = grow(h, h->jwork, 2 * sizeof(unsigned long long)))) return rc;
-    CK(h, cudaMemsetAsync(h->jwork.p, 0, 2 * sizeof(unsigned long long), st));
-    // Convergence polls run one chunk behind: after launching chunk c + 1 the host reads
-    // the counters copied after chunk c, so the stream always has a chunk queued while the
-    // host checks (a converged sector's rounds in the extra chunk exit at once).  Counters
-    // and compacted launch tables alternate between two pinned slots.
-    int* hrot_slot[2] = {reinterpret_cast<int*>(static_cast<char*>(h->hres.p) + 1024), nullptr};
-    hrot_slot[1] = hrot_slot[0] + 3 * ns;
-    const size_t jw_bytes = align_up(std::max<size_t>(P.jw.size(), 1) * sizeof(JacobiWork), 256);
-    if ((rc = grow_host(h, h->stage2, 2 * jw_bytes))) return rc;
-    char* jw_stage[2] = {static_cast<char*>(h->stage2.p), static_cast<char*>(h->stage2.p) + jw_bytes};
-    for (cudaEvent_t& e : h->poll_ev)
-      if (!e) CK(h, cudaEventCreateWithFlags(&e, cudaEventBlockingSync | cudaEventDisableTiming));
-    int t = 0;
-    const int t_max = MAX_SWEEPS * std::max(1, P.max_rounds);
-    bool converged = false;
-    int checks = 0;
-    std::vector<int> conv_at(ns, -1);
-    if (h->timing) CK(h, cudaEventRecord(h->ev0, st));
-    const int chunk = std::max(1, P.max_rounds);   // one sweep of the largest sector
-    int t_after[2] = {0, 0};
-    auto launch_chunk = [&](int slot) -> int {
-      for (int i = 0; i < chunk && t < t_max; ++i, ++t) {
-        // tol <= 0: per-sector default 4 eps sqrt(rows of the Gram), at least 8 eps
-        CK(h, launch_jacobi_round(sd_d, jw_d, (int)active.size(), gram_ctas, apply_ctas, t,
-                                  h->abuf.p, reinterpret_cast<int*>(h->rot.p), nf2, 0.0, MAX_SWEEPS,
-                                  h->pbuf.p, reinterpret_cast<int*>(h->pcnt.p), h->qbuf.p,
-                                  reinterpret_cast<int*>(h->qflag.p),
-                                  reinterpret_cast<unsigned long long*>(h->jwork.p), st));
-        h->launches += 2;
-      }
-      CK(h, cudaMemcpyAsync(hrot_slot[slot], h->rot.p, (size_t)3 * ns * sizeof(int),
-                            cudaMemcpyDeviceToHost, st));
-      CK(h, cudaEventRecord(h->poll_ev[slot], st));
-      t_after[slot] = t;
-      return BSMPO_OK;
-    };
-    if ((rc = launch_chunk(0))) return rc;
-    int cur = 0, compactions = 0;
-    for (;;) {
-      const bool more = t < t_max;
-      if (more && (rc = launch_chunk(cur ^ 1))) return rc;
-      CK(h, cudaEventSynchronize(h->poll_ev[cur]));
-      ++checks;
-      const int* hrot = hrot_slot[cur];
-      bool all = true;
-      for (int s = 0; s < ns; ++s) {
-        // a converged sector leaves the launches, and its counters are stale from then on
-        if (conv_at[s] >= 0) continue;
-        const int R = P.jw[s].rounds;
-        const int done = t_after[cur] / R;
-        if (done < 1 || hrot[3 * s + (done - 1) % 3] != 0) { all = false; continue; }
-        conv_at[s] = done;
-      }
-      if (all) { converged = true; break; }
-      if (!more) break;
-      // drop converged sectors (and those out of sweeps) from the launches after the queued
-      // chunk: the table copy is stream-ordered after it
-      std::vector<JacobiWork> next;
-      for (const auto& w : P.jw)
-        if (conv_at[w.sector] < 0 && t / w.rounds < MAX_SWEEPS) next.push_back(w);
-      if (next.size() < active.size() && !next.empty()) {
-        active.swap(next);
-        jacobi_launch_list(active, &gram_ctas, &apply_ctas, &slots);
-        char* stg = jw_stage[compactions++ & 1];
-        put(stg, 0, active);
-        CK(h, cudaMemcpyAsync(dt + L.jw, stg, active.size() * sizeof(JacobiWork),
-                              cudaMemcpyHostToDevice, st));
-      }
-      cur ^= 1;
-    }
-    if (h->timing) {
-      CK(h, cudaMemcpyAsync(static_cast<char*>(h->hres.p) + 2048, h->jwork.p, 2 * sizeof(unsigned long long),
-                            cudaMemcpyDeviceToHost, st));
-      CK(h, cudaEventRecord(h->ev1, st));
-    }
-    // sweeps the slowest sector needed (its last one without rotations included); t also
-    // counts the chunk queued after convergence, whose rounds exit at once
-    {
-      int sw = 0;
-      for (int s = 0; s < ns; ++s) sw = std::max(sw, conv_at[s] >= 0 ? conv_at[s] : t / P.jw[s].rounds);
-      h->last_sweeps = sw;
-    }
-    h->jacobi_rounds += t;   // launched rounds, including the drained chunk
-    if (h->timing) {
-      float ms = 0.f;
-      CK(h, cudaEventSynchronize(h->ev1));
-      CK(h, cudaEventElapsedTime(&ms, h->ev0, h->ev1));
-      h->jac_ms += ms;
-      h->jac_launches += t;
-      // flops of the executed work, counted on the device: every row that formed a
-      // partial pair Gram contributes its 10 upper 8 x 8 tiles (640 complex MACs), every
-      // rotated row 32 x 32 complex MACs; 8 flops per complex MAC.  Pairs that did not
-      // rotate and sectors that had converged do no apply work and are not counted.
-      const unsigned long long* hw =
-          reinterpret_cast<const unsigned long long*>(static_cast<char*>(h->hres.p) + 2048);
-      h->jac_flops += 8.0 * 640.0 * (double)hw[0] + 8.0 * 1024.0 * (double)hw[1];
-    }
-    if ((rc = clk.mark(3))) return rc;
-    if (!converged) {
-      std::string msg = "Jacobi SVD did not converge (mode " + std::to_string(mode) + ")";
-      for (int s = 0; s < ns; ++s) {
-        const int R = P.jw[s].rounds, done = t_after[cur] / R;
-        if (conv_at[s] >= 0) continue;
-        const SectorDesc& S = P.sd[s];
-        msg += "; sector (" + std::to_string(S.cc0) + "," + std::to_string(S.cc1) + ") m=" +
-               std::to_string(S.m) + " n=" + std::to_string(S.n) + " sweeps=" + std::to_string(done) +
-               " rotations=" + std::to_string(hrot_slot[cur][3 * s + (done - 1 + 3) % 3]);
-        break;
-      }
-      return fail(h, BSMPO_ECONVERGE, msg);
-    }
-    CKL(h, launch_jacobi_finish(sd_d, ns, P.max_k, h->abuf.p, nf2,
-                                reinterpret_cast<double*>(h->sig.p),
-                                reinterpret_cast<int*>(h->perm.p), st));
-  }
-  // 4. selection -> kept counts (the one host sync of the update)
+  // 3. the sector SVD: Gram + Hermitian eigenproblem, or blocked one-sided Jacobi;
+  // 4. selection -> kept counts
+  char* hres = static_cast<char*>(h->hres.p);
+  const int* hk = reinterpret_cast<const int*>(hres + R.kept);
+  const double* htw = reinterpret_cast<const double*>(hres + R.trunc);
+  const int* htc = reinterpret_cast<const int*>(hres + R.err);
   int* kept_d = reinterpret_cast<int*>(h->kept.p);
-  double* trunc_d = reinterpret_cast<double*>(static_cast<char*>(h->kept.p) +
-                                              align_up((size_t)(ns + 1) * sizeof(int), 16));
-  CKL(h, launch_select(tab_d, sd_d, ns, reinterpret_cast<double*>(h->sig.p),
-                       reinterpret_cast<double*>(h->keys.p), h->cutoff, chi, kept_d, trunc_d, st));
-  CK(h, cudaMemcpyAsync(hk, kept_d, (size_t)(ns + 1) * sizeof(int), cudaMemcpyDeviceToHost, st));
-  CK(h, cudaMemcpyAsync(htw, trunc_d, sizeof(double), cudaMemcpyDeviceToHost, st));
-  int* htc = reinterpret_cast<int*>(static_cast<char*>(h->hres.p) + 1000);
-  CK(h, cudaMemcpyAsync(htc, tcerr_d, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CK(h, host_wait(h));
-  if (*htc != 0)
-    return fail(h, BSMPO_ECUDA, "tensor-core GEMM or tridiagonalisation: a pipeline wait expired (error word set)");
-  total_kept = hk[ns];
-  if (gram && total_kept < chi && h->cutoff == 0.0 && h->gram_policy >= 1) {
-    // not truncated to chi: redo the SVD exactly (the Gram matrix and the eigen buffers
-    // are not needed any more; the Jacobi matrix is intact)
-    gram = false;
-    CKL(h, launch_identity_rows(sd_d, ns, P.max_left_m2, h->abuf.p, st));
-    continue;
-  }
-  break;
-  }
-  h->route_count[gram ? 1 : 0]++;
-  if (gram && h->timing) {
-    // eigen phase of the Gram route (Gram GEMM, tridiagonalisation, bisection): both
-    // events completed before the kept counts arrived
-    float ms = 0.f;
-    CK(h, cudaEventElapsedTime(&ms, h->ev0, h->ev1));
-    h->jac_ms += ms;
-    h->jac_launches += 4;
-    // algorithmic flops: the Gram (8 k^2 rows, complex MACs) and the Householder
-    // reduction of a k x k Hermitian matrix (16/3 k^3, LAPACK's zhetrd count)
-    for (const SectorDesc& S : P.sd)
-      h->jac_flops += 8.0 * (double)S.k * S.k * S.rows_g + 16.0 / 3.0 * (double)S.k * S.k * S.k;
-    float tms = 0.f;
-    CK(h, cudaEventElapsedTime(&tms, h->td_ev0, h->td_ev1));
-    h->td_ms += tms;
-    h->td_phases++;
-    for (const SectorDesc& S : P.sd) {
-      // step j reads and writes the (k - j - 1)^2 trailing matrix once: 32 B per entry
-      const double k = S.k;
-      h->td_bytes += 32.0 * (k - 1.0) * k * (2.0 * k - 1.0) / 6.0;
-      h->td_flops += 16.0 / 3.0 * k * k * k;
+  double* trunc_d = reinterpret_cast<double*>(static_cast<char*>(h->kept.p) + kept_bytes);
+  if (!h->wait_ev) CK(h, cudaEventCreateWithFlags(&h->wait_ev, cudaEventBlockingSync | cudaEventDisableTiming));
+  rc = P.gram ? gram_eigenvalues(h, P, sd_d, groups_at(L.ggram), reinterpret_cast<const int*>(dt + L.tdlist), tcerr_d)
+              : jacobi_svd(h, P, sd_d, dt + L.jw, R);
+  if (rc || (rc = clk.mark(3))) return rc;
+  auto select = [&]() -> int {
+    CKL(h, launch_select(tab_d, sd_d, nj, ns, reinterpret_cast<double*>(h->sig.p),
+                         reinterpret_cast<double*>(h->keys.p), h->cutoff, chi, kept_d, trunc_d, st));
+    CK(h, cudaMemcpyAsync(hres + R.kept, kept_d, (size_t)(ns + nj) * sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(h, cudaMemcpyAsync(hres + R.trunc, trunc_d, nj * sizeof(double), cudaMemcpyDeviceToHost, st));
+    CK(h, cudaMemcpyAsync(hres + R.err, tcerr_d, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(h, cudaEventRecord(h->wait_ev, st));
+    return BSMPO_OK;
+  };
+  if ((rc = select())) return rc;
+  if (P.gram && h->gram_policy >= 1) {
+    CK(h, cudaEventSynchronize(h->wait_ev));
+    if (*htc == 0 && hk[ns] < chi && h->cutoff == 0.0) {
+      // not truncated to chi (groups of one update under this policy): redo the SVD
+      // exactly; the Jacobi matrix is intact
+      Plan J;
+      if ((rc = add_update(h, jobs[0].mode, 0, J))) return rc;
+      finish_plan(h, J);
+      std::vector<JacobiWork> active(J.jw);
+      int a, b, c;
+      jacobi_launch_list(active, &a, &b, &c);
+      const size_t bytes = std::max<size_t>(active.size(), 1) * sizeof(JacobiWork);
+      if ((rc = grow(h, h->tab2, bytes))) return rc;
+      if ((rc = grow_host(h, h->stage3, bytes))) return rc;
+      put(h->stage3.p, 0, active);
+      CK(h, cudaMemcpyAsync(h->tab2.p, h->stage3.p, bytes, cudaMemcpyHostToDevice, st));
+      CKL(h, launch_identity_rows(sd_d, ns, J.max_left_m2, h->abuf.p, st));
+      if ((rc = jacobi_svd(h, J, sd_d, static_cast<char*>(h->tab2.p), R))) return rc;
+      P.gram = false;
+      if ((rc = select())) return rc;
     }
   }
   if ((rc = clk.mark(4))) return rc;
   // 5. V (Jacobi: extracted from the converged columns; Gram route: eigenvectors, and
-  // V = T Y diag(1/sigma) where X = T) and W = V^H C
-  std::vector<GemmGroup> wg, vg;
-  int wtiles = 0, vtiles = 0, max_vm = 0, kept_max = 0;
-  double flops_w = 0.0;
-  const int TMt = zgemm_tile_m(), TNt = zgemm_tile_n();
-  for (int s = 0; s < ns; ++s) {
-    const SectorDesc& S = P.sd[s];
-    const int kp = hk[s];
-    max_vm = std::max(max_vm, kp * S.m);
-    kept_max = std::max(kept_max, kp);
-    if (kp == 0) continue;
-    GemmGroup g;
-    std::memset(&g, 0, sizeof(g));
-    g.M = kp; g.N = S.n; g.K = S.m;
-    g.lda = kp; g.ldb = S.n; g.ldc = S.n;
-    g.opA = 1; g.opB = 0; g.beta = 0;
-    g.tiles_n = ceil_div(S.n, TNt);
-    g.tile_start = wtiles;
-    wtiles += ceil_div(kp, TMt) * g.tiles_n;
-    g.a_off = S.v_off; g.b_off = S.c_off; g.c_off = S.w_off;
-    g.ks_off = g.rs_off = g.cs_off = -1;
-    wg.push_back(g);
-    flops_w += 8.0 * kp * (double)S.m * S.n;
-    if (gram && !S.left) {
-      // V [m][kp] = T [m][k] Y [k][kp] diag(1 / sigma)
-      GemmGroup v;
-      std::memset(&v, 0, sizeof(v));
-      v.M = S.m; v.N = kp; v.K = S.k;
-      v.lda = S.k; v.ldb = kp; v.ldc = kp;
-      v.opA = 0; v.opB = 0; v.beta = 0;
-      v.tiles_n = ceil_div(kp, TNt);
-      v.tile_start = vtiles;
-      vtiles += ceil_div(S.m, TMt) * v.tiles_n;
-      v.a_off = S.a_off; v.b_off = S.y_off; v.c_off = S.v_off;
-      v.ks_off = v.rs_off = -1;
-      v.cs_off = S.s_off;
-      vg.push_back(v);
-      flops_w += 8.0 * kp * (double)S.m * S.k;
-    }
-  }
-  const size_t wbytes = align_up(wg.size() * sizeof(GemmGroup) + 1, 256);
-  const size_t vbytes = align_up(vg.size() * sizeof(GemmGroup) + 1, 256);
-  if ((rc = grow(h, h->tab2, wbytes + vbytes))) return rc;
-  if ((rc = grow_host(h, h->stage2, wbytes + vbytes))) return rc;
-  put(h->stage2.p, 0, wg);
-  put(h->stage2.p, wbytes, vg);
-  CK(h, cudaMemcpyAsync(h->tab2.p, h->stage2.p, wbytes + vbytes, cudaMemcpyHostToDevice, st));
-  const GemmGroup* wg_d = reinterpret_cast<const GemmGroup*>(h->tab2.p);
-  const GemmGroup* vg_d = reinterpret_cast<const GemmGroup*>(static_cast<char*>(h->tab2.p) + wbytes);
-  if (gram) {
+  // V = T Y diag(1/sigma) where X = T) and W = V^H C; the kernels read the kept counts on
+  // the device, so the host does not wait for them before these launches
+  if (P.gram) {
     const size_t ye = (size_t)std::max<int64_t>(P.y_elems, 1);
     if ((rc = grow(h, h->escr, 4 * ye * sizeof(double)))) return rc;
     if ((rc = grow(h, h->swp, ye))) return rc;
     if ((rc = grow(h, h->zbuf, ye * sizeof(double)))) return rc;
     if ((rc = grow(h, h->ybuf, ye * sizeof(cplx)))) return rc;
-    CK(h, launch_eigvec(sd_d, ns, P.max_k, kept_max, dbuf_d, ebuf_d, lam_d,
-                        reinterpret_cast<double*>(h->escr.p), reinterpret_cast<unsigned char*>(h->swp.p),
-                        reinterpret_cast<double*>(h->zbuf.p), h->gbuf.p, h->taub.p, h->vbuf.p, h->ybuf.p,
-                        st));
+    double* dbuf_d = reinterpret_cast<double*>(h->eigd.p);
+    double* ebuf_d = dbuf_d + P.s_elems;
+    double* lam_d = ebuf_d + P.s_elems;
+    CK(h, launch_eigvec(sd_d, ns, P.max_k, P.max_k, dbuf_d, ebuf_d, lam_d, reinterpret_cast<double*>(h->escr.p),
+                        reinterpret_cast<unsigned char*>(h->swp.p), reinterpret_cast<double*>(h->zbuf.p), h->gbuf.p,
+                        h->taub.p, h->vbuf.p, h->ybuf.p, st));
     h->launches += 2;
     // V = T Y diag(1/sigma) stays FP64: it divides by sigma (down to ~3e-3 of the largest
     // at the cut), which would magnify a TF32 error into V's orthogonality, and a
     // non-orthonormal V leaks into W = V^H C at the scale of C
-    if (!vg.empty())
+    if (!P.gv.empty())
       CKL(h, launch_zgemm_grouped(h->abuf.p, h->ybuf.p, h->vbuf.p, reinterpret_cast<double*>(h->invsig.p),
-                                  vg_d, (int)vg.size(), vtiles, st));
+                                  groups_at(L.gv), (int)P.gv.size(), P.v_tiles, sd_d, st));
   } else {
-    CKL(h, launch_extract_v(sd_d, ns, max_vm, h->abuf.p, reinterpret_cast<double*>(h->sig.p),
+    CKL(h, launch_extract_v(sd_d, ns, P.max_v, h->abuf.p, reinterpret_cast<double*>(h->sig.p),
                             reinterpret_cast<int*>(h->perm.p), h->vbuf.p, st));
   }
   if (tc_w) {
-    // W = V^H C on the tensor cores: two tensor maps per group
-    const size_t mb = tc_map_bytes();
-    std::vector<unsigned char> maps;
-    std::vector<TcGroup> tw;
-    int tw_tiles = 0;
-    const int tm = tc_tile_m(), tn = tc_tile_n();
-    bool enc_ok = true;
-    auto add_map = [&](const void* base, int rows, int cols, int ld, int kind) -> int {
-      const int idx = (int)(maps.size() / mb);
-      maps.resize(maps.size() + mb);
-      if (tc_encode_map(maps.data() + (size_t)idx * mb, base, rows, cols, ld, kind) != cudaSuccess) enc_ok = false;
-      return idx;
-    };
-    const cplx* V0 = reinterpret_cast<const cplx*>(h->vbuf.p);
-    const cplx* C0 = reinterpret_cast<const cplx*>(h->cbuf.p);
-    for (int s = 0; s < ns; ++s) {
-      const SectorDesc& S = P.sd[s];
-      const int kp = hk[s];
-      if (kp == 0) continue;
-      TcGroup g;
-      std::memset(&g, 0, sizeof(g));
-      g.M = kp; g.N = S.n; g.K = S.m; g.opA = 1;
-      g.mapA = add_map(V0 + S.v_off, S.m, kp, kp, 1);
-      g.mapB = add_map(C0 + S.c_off, S.m, S.n, S.n, 2);
-      g.ldc = S.n;
-      g.tiles_n = ceil_div(S.n, tn);
-      g.tile_start = tw_tiles;
-      tw_tiles += ceil_div(kp, tm) * g.tiles_n;
-      g.c_off = S.w_off;
-      g.cs_off = -1;
-      tw.push_back(g);
-    }
-    if (!enc_ok) return fail(h, BSMPO_ECUDA, "tensor map encoding failed");
-    const size_t o_tw = align_up(maps.size(), 256);
-    const size_t total = align_up(o_tw + tw.size() * sizeof(TcGroup) + 1, 256);
-    if ((rc = grow(h, h->tab3, total))) return rc;
-    if ((rc = grow_host(h, h->stage3, total))) return rc;
-    std::memcpy(h->stage3.p, maps.data(), maps.size());
-    put(h->stage3.p, o_tw, tw);
-    CK(h, cudaMemcpyAsync(h->tab3.p, h->stage3.p, total, cudaMemcpyHostToDevice, st));
-    const char* t3 = static_cast<const char*>(h->tab3.p);
-    CKL(h, launch_tc_zgemm(reinterpret_cast<const TcGroup*>(t3 + o_tw), (int)tw.size(), tw_tiles, t3,
-                           h->wbuf.p, nullptr, tcerr_d, st));
+    CK(h, cudaEventSynchronize(h->wait_ev));
+    if ((rc = tc_w_gemm(h, P, hk, tcerr_d))) return rc;
   } else {
-    CKL(h, launch_zgemm_grouped(h->vbuf.p, h->cbuf.p, h->wbuf.p, nullptr, wg_d, (int)wg.size(), wtiles, st));
+    CKL(h, launch_zgemm_grouped(h->vbuf.p, h->cbuf.p, h->wbuf.p, nullptr, groups_at(L.gw), (int)P.gw.size(),
+                                P.w_tiles, sd_d, st));
   }
   if ((rc = clk.mark(5))) return rc;
   // 6. scatter into Gamma[mode], Gamma[mode+1], Lambda / charge of bond mode+1
-  CKL(h, launch_scatter(tab_d, sd_d, ns, total_kept, chi, h->charge + (size_t)mode * chi * 2,
-                        h->charge + (size_t)(mode + 2) * chi * 2, h->vbuf.p, h->wbuf.p,
-                        reinterpret_cast<double*>(h->sig.p), h->gamma + (size_t)mode * chi2,
-                        h->gamma + (size_t)(mode + 1) * chi2, h->lam + (size_t)(mode + 1) * chi,
-                        h->charge + (size_t)(mode + 1) * chi * 2, st));
+  CKL(h, launch_scatter(tab_d, sd_d, nj, kept_d + ns, chi, h->vbuf.p, h->wbuf.p,
+                        reinterpret_cast<double*>(h->sig.p), h->gamma, h->lam, h->charge, st));
   if ((rc = clk.mark(6))) return rc;
-  // algorithmic minimum bytes: read Glc, Gcr, write Gamma_L, Gamma_R (complex128)
-  {
-    double nl = 0, nc = 0, nr = 0;
-    const std::vector<int>& cnt = mirror(h);
-    for (int q = 0; q < dd; ++q) {
-      nl += cnt[(size_t)mode * dd + q];
-      nc += cnt[(size_t)(mode + 1) * dd + q];
-      nr += cnt[(size_t)(mode + 2) * dd + q];
+  CK(h, cudaEventSynchronize(h->wait_ev));
+  if (*htc != 0)
+    return fail(h, BSMPO_ECUDA, "tensor-core GEMM or tridiagonalisation: a pipeline wait expired (error word set)");
+  h->route_count[P.gram ? 1 : 0] += nj;
+  if (P.gram && h->timing && (rc = gram_timing(h, P))) return rc;
+  // host mirror, truncation weights, and the diagnostics of the group's last update
+  for (int j = 0; j < nj; ++j) {
+    const UpdateTables& T = P.tab[j];
+    std::vector<int>& cnt = mirror(h);
+    if (trunc) trunc[j] = htw[j];
+    if (j == nj - 1) {
+      double nl = 0, nc = 0, nr = 0, flops_w = 0.0, svd_flops = 0.0;
+      for (int q = 0; q < dd; ++q) {
+        nl += cnt[(size_t)T.mode * dd + q];
+        nc += cnt[(size_t)(T.mode + 1) * dd + q];
+        nr += cnt[(size_t)(T.mode + 2) * dd + q];
+      }
+      // algorithmic minimum bytes: read Glc, Gcr, write Gamma_L, Gamma_R (complex128)
+      h->last_bytes = 16.0 * (nl * nc + nc * nr + (nl + nr) * hk[ns + j]);
+      h->last_ns = T.n_sectors;
+      h->last_sig_off = P.sd[T.sec0].s_off;
+      h->last_cc.assign(2 * T.n_sectors, 0);
+      h->last_shape.assign(2 * T.n_sectors, 0);
+      h->last_kept.assign(T.n_sectors, 0);
+      h->last_k.assign(T.n_sectors, 0);
+      for (int i = 0; i < T.n_sectors; ++i) {
+        const SectorDesc& S = P.sd[T.sec0 + i];
+        const int kp = hk[T.sec0 + i];
+        h->last_cc[2 * i] = S.cc0;
+        h->last_cc[2 * i + 1] = S.cc1;
+        h->last_shape[2 * i] = S.m;
+        h->last_shape[2 * i + 1] = S.n;
+        h->last_kept[i] = kp;
+        h->last_k[i] = S.k;
+        flops_w += 8.0 * kp * (double)S.m * S.n;
+        if (P.gram && !S.left) flops_w += 8.0 * kp * (double)S.m * S.k;
+        // one sweep: every column pair's Gram (rows_g) and rotation (rows_tot), 8 flops / complex MAC
+        svd_flops += 4.0 * (double)S.k * S.k * (S.rows_g + S.rows_tot);
+      }
+      h->last_trunc = htw[j];
+      h->last_gemm = P.flops_theta[j] + flops_w;
+      h->last_svd = svd_flops * h->last_sweeps;
     }
-    h->last_bytes = 16.0 * (nl * nc + nc * nr + ((double)nl + nr) * total_kept);
+    int* cM = &cnt[(size_t)(T.mode + 1) * dd];
+    std::fill(cM, cM + dd, 0);
+    for (int i = 0; i < T.n_sectors; ++i) {
+      const SectorDesc& S = P.sd[T.sec0 + i];
+      cM[S.cc0 * d + S.cc1] = hk[T.sec0 + i];
+    }
   }
-  // host mirror and diagnostics
-  int* cM = &mirror(h)[(size_t)(mode + 1) * dd];
-  std::fill(cM, cM + dd, 0);
-  h->last_cc.assign(2 * ns, 0);
-  h->last_shape.assign(2 * ns, 0);
-  h->last_kept.assign(ns, 0);
-  h->last_k.assign(ns, 0);
-  h->last_soff.assign(ns, 0);
-  double svd_flops = 0.0;
-  for (int s = 0; s < ns; ++s) {
-    const SectorDesc& S = P.sd[s];
-    cM[S.cc0 * d + S.cc1] = hk[s];
-    h->last_cc[2 * s] = S.cc0;
-    h->last_cc[2 * s + 1] = S.cc1;
-    h->last_shape[2 * s] = S.m;
-    h->last_shape[2 * s + 1] = S.n;
-    h->last_kept[s] = hk[s];
-    h->last_k[s] = S.k;
-    h->last_soff[s] = S.s_off;
-    // one sweep: every column pair's Gram (rows_g) and rotation (rows_tot), 8 flops / complex MAC
-    svd_flops += 4.0 * (double)S.k * S.k * (S.rows_g + S.rows_tot);
-  }
-  h->last_trunc = *htw;
-  h->last_gemm = P.flops_theta + flops_w;
-  h->last_svd = svd_flops * h->last_sweeps;
   return BSMPO_OK;
+}
+
+int bs_update_impl(bsmpo_ctx* h, int mode, const cplx* u3_dev) {
+  Job job;
+  job.mode = mode;
+  job.u3 = u3_dev;
+  return update_group(h, &job, 1, nullptr);
 }
 
 M8 transpose_to_m8(const double* S) {
@@ -1126,14 +1216,20 @@ void destroy_worker(bsmpo_ctx* w) {
   delete w;   // the state belongs to the owner
 }
 
-// Runs the updates of a mesh on the owner's workers.  Two beam splitters conflict when
-// their modes differ by 0 or 1 (shared site); update k depends on the latest earlier
-// update at modes m_k - 1, m_k and m_k + 1 -- nothing else it touches is written by
-// another update (modes 2 apart share only a bond both read).  Workers take the
-// lowest-numbered update whose dependencies have finished (host side: after their
-// host mirror entries are written; device side: the worker's stream waits for the
-// events recorded at their ends), so consecutive brick-wall layers overlap.  Every
-// update computes exactly what it computes alone.
+// Runs the updates of a mesh on the owner's workers, in groups.  Two beam splitters
+// conflict when their modes differ by 0 or 1 (shared site); update k depends on the latest
+// earlier update at modes m_k - 1, m_k and m_k + 1 -- nothing else it touches is written
+// by another update (modes 2 apart share only a bond both read).  At most `nw` updates run
+// at once, on MESH_LANES streams (fewer where nw is smaller): a lane takes the
+// lowest-numbered updates whose dependencies have finished (host side: after their host
+// mirror entries are written; device side: the lane's stream waits for the events recorded
+// at their ends) as one group, so an update's launches are shared by its layer's other
+// updates and consecutive brick-wall layers overlap.  Every update computes exactly what
+// it computes alone.
+// Why groups on few streams: an update's ~25 sectors fill a fraction of the GPU, and one
+// stream per update ran into the device's hardware queues (8 by default): two layers at
+// N = 64, chi = 1024 with 16 updates at once took 142 ms, in groups on two lanes 92 (with
+// the eigen kernels of that time).
 // The host side of a mesh over a host-resident state: the first update touching site s,
 // first[s], copies the site in on its own stream before it starts, and the last, last[s],
 // copies it out after it ends.  Every later update touching the site depends on the
@@ -1152,12 +1248,15 @@ int run_mesh_concurrent(bsmpo_ctx* h, int n_bs, const int* modes, const cplx* u3
                         HostStream* hs = nullptr) {
   const int d3 = h->d * h->d * h->d;
   int rc;
-  while ((int)h->workers.size() < nw) {
+  const int lanes = std::min(nw, MESH_LANES);
+  // updates per group; a policy that may redo an update's SVD takes them one by one
+  const int cap = h->gram_policy >= 1 && h->precision != BSMPO_PRECISION_FP64 ? 1 : ceil_div(nw, lanes);
+  while ((int)h->workers.size() < lanes) {
     bsmpo_ctx* w = nullptr;
     if ((rc = make_worker(h, &w))) return rc;
     h->workers.push_back(w);
   }
-  for (int k = 0; k < nw; ++k) {
+  for (int k = 0; k < lanes; ++k) {
     bsmpo_ctx* w = h->workers[k];
     w->cutoff = h->cutoff;
     w->precision = h->precision;
@@ -1190,72 +1289,109 @@ int run_mesh_concurrent(bsmpo_ctx* h, int n_bs, const int* modes, const cplx* u3
       last[m] = k;
     }
   }
-  std::vector<cudaEvent_t> done_ev(n_bs, nullptr);
-  for (int k = 0; k < n_bs; ++k)
-    if (cudaEventCreateWithFlags(&done_ev[k], cudaEventDisableTiming) != cudaSuccess) {
-      cudaGetLastError();
-      for (cudaEvent_t e : done_ev) if (e) cudaEventDestroy(e);
-      return fail(h, BSMPO_ECUDA, "event creation failed");
-    }
+  std::vector<int> group_of(n_bs, -1);      // update -> its group
+  std::vector<cudaEvent_t> done_ev;         // group -> event recorded behind its last kernel
+  std::vector<int> lane_of;                 // group -> lane
+  done_ev.reserve(n_bs);
+  lane_of.reserve(n_bs);
   std::mutex mu;
   std::condition_variable cv;
-  std::priority_queue<int, std::vector<int>, std::greater<int>> ready;
+  std::vector<int> ready;                   // ascending
   for (int k = 0; k < n_bs; ++k)
-    if (remaining[k] == 0) ready.push(k);
-  int finished = 0;
+    if (remaining[k] == 0) ready.push_back(k);
+  int finished = 0, idle = lanes;
   int err_code = BSMPO_OK;
   std::string err_msg;
   std::vector<std::thread> pool;
-  for (int wk = 0; wk < nw; ++wk)
+  for (int wk = 0; wk < lanes; ++wk)
     pool.emplace_back([&, wk]() {
       bsmpo_ctx* w = h->workers[wk];
       cudaSetDevice(h->device);
+      std::vector<Job> jobs;
+      std::vector<cudaEvent_t> waits;
+      std::vector<double> tw;
       for (;;) {
-        int k;
+        cudaEvent_t mine = nullptr;
         {
           std::unique_lock<std::mutex> lock(mu);
           cv.wait(lock, [&] { return err_code || finished == n_bs || !ready.empty(); });
           if (err_code || ready.empty()) break;
-          k = ready.top();
-          ready.pop();
+          if (cudaEventCreateWithFlags(&mine, cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            err_code = BSMPO_ECUDA;
+            err_msg = "event creation failed";
+            cv.notify_all();
+            break;
+          }
+          // an even share of the ready updates for each lane without work, of one SVD route
+          const int share = std::min(cap, ceil_div((int)ready.size(), idle));
+          --idle;
+          const int gid = (int)done_ev.size();
+          done_ev.push_back(mine);
+          lane_of.push_back(wk);
+          jobs.clear();
+          const bool route = gram_route(w, modes[ready[0]]);
+          for (size_t i = 0; i < ready.size() && (int)jobs.size() < share;) {
+            const int k = ready[i];
+            if (gram_route(w, modes[k]) != route) { ++i; continue; }
+            ready.erase(ready.begin() + i);
+            Job j;
+            j.mode = modes[k];
+            j.u3 = u3 + (size_t)k * d3;
+            j.index = k;
+            jobs.push_back(j);
+            group_of[k] = gid;
+          }
+          waits.clear();
+          for (const Job& j : jobs)
+            for (int c = 0; c < 3; ++c) {
+              const int p = pred[(size_t)3 * j.index + c];
+              if (p < 0 || lane_of[group_of[p]] == wk) continue;   // stream order covers its own lane
+              const cudaEvent_t e = done_ev[group_of[p]];
+              if (std::find(waits.begin(), waits.end(), e) == waits.end()) waits.push_back(e);
+            }
         }
         int r = BSMPO_OK;
-        for (int c = 0; c < 3 && !r; ++c) {
-          const int j = pred[(size_t)3 * k + c];
-          if (j >= 0 && cudaStreamWaitEvent(w->stream, done_ev[j], 0) != cudaSuccess)
+        for (cudaEvent_t e : waits)
+          if (!r && cudaStreamWaitEvent(w->stream, e, 0) != cudaSuccess)
             r = fail(w, BSMPO_ECUDA, "cudaStreamWaitEvent failed");
-        }
-        for (int site = modes[k]; hs && site <= modes[k] + 1 && !r; ++site)
-          if (hs->first[site] == k &&
-              cudaMemcpyAsync(reinterpret_cast<char*>(h->gamma) + (size_t)site * hs->site_bytes,
-                              hs->gamma_in + (size_t)site * hs->site_bytes, hs->site_bytes,
-                              cudaMemcpyHostToDevice, w->stream) != cudaSuccess)
-            r = fail(w, BSMPO_ECUDA, "site copy-in failed");
-        if (!r) r = bs_update_impl(w, modes[k], u3 + (size_t)k * d3);
-        if (!r) h->mesh_tw[k] = w->last_trunc;   // each k is written by one worker only
-        if (!r && cudaEventRecord(done_ev[k], w->stream) != cudaSuccess)
+        for (const Job& j : jobs)
+          for (int site = j.mode; hs && site <= j.mode + 1 && !r; ++site)
+            if (hs->first[site] == j.index &&
+                cudaMemcpyAsync(reinterpret_cast<char*>(h->gamma) + (size_t)site * hs->site_bytes,
+                                hs->gamma_in + (size_t)site * hs->site_bytes, hs->site_bytes,
+                                cudaMemcpyHostToDevice, w->stream) != cudaSuccess)
+              r = fail(w, BSMPO_ECUDA, "site copy-in failed");
+        tw.assign(jobs.size(), 0.0);
+        if (!r) r = update_group(w, jobs.data(), (int)jobs.size(), tw.data());
+        // each update's weight is written by the one lane that ran it
+        for (size_t i = 0; i < jobs.size() && !r; ++i) h->mesh_tw[jobs[i].index] = tw[i];
+        if (!r && cudaEventRecord(mine, w->stream) != cudaSuccess)
           r = fail(w, BSMPO_ECUDA, "cudaEventRecord failed");
-        for (int site = modes[k]; hs && site <= modes[k] + 1 && !r; ++site)
-          // the site's final value of this mesh: copied out behind the update
-          if (hs->last[site] == k &&
-              cudaMemcpyAsync(hs->gamma_out + (size_t)site * hs->site_bytes,
-                              reinterpret_cast<const char*>(h->gamma) + (size_t)site * hs->site_bytes,
-                              hs->site_bytes, cudaMemcpyDeviceToHost, w->stream) != cudaSuccess)
-            r = fail(w, BSMPO_ECUDA, "site copy-out failed");
+        for (const Job& j : jobs)
+          for (int site = j.mode; hs && site <= j.mode + 1 && !r; ++site)
+            // the site's final value of this mesh: copied out behind the update
+            if (hs->last[site] == j.index &&
+                cudaMemcpyAsync(hs->gamma_out + (size_t)site * hs->site_bytes,
+                                reinterpret_cast<const char*>(h->gamma) + (size_t)site * hs->site_bytes,
+                                hs->site_bytes, cudaMemcpyDeviceToHost, w->stream) != cudaSuccess)
+              r = fail(w, BSMPO_ECUDA, "site copy-out failed");
         std::lock_guard<std::mutex> lock(mu);
+        ++idle;
         if (r) {
           if (!err_code) { err_code = r; err_msg = w->err; }
         } else {
-          w->last_index = std::max(w->last_index, k);
-          ++finished;
-          for (int s2 : succ[k])
-            if (--remaining[s2] == 0) ready.push(s2);
+          w->last_index = jobs.back().index;
+          finished += (int)jobs.size();
+          for (const Job& j : jobs)
+            for (int s2 : succ[j.index])
+              if (--remaining[s2] == 0) ready.insert(std::upper_bound(ready.begin(), ready.end(), s2), s2);
         }
         cv.notify_all();
       }
     });
   for (auto& t : pool) t.join();
-  for (int wk = 0; wk < nw; ++wk) {
+  for (int wk = 0; wk < lanes; ++wk) {
     const cudaError_t e = host_wait(h->workers[wk]);
     if (e != cudaSuccess && !err_code) { err_code = BSMPO_ECUDA; err_msg = cudaGetErrorString(e); }
   }
@@ -1263,7 +1399,7 @@ int run_mesh_concurrent(bsmpo_ctx* h, int n_bs, const int* modes, const cplx* u3
   if (err_code) return fail(h, err_code, err_msg);
   // counters and the last update's diagnostics
   int best = -1;
-  for (int k = 0; k < nw; ++k) {
+  for (int k = 0; k < lanes; ++k) {
     bsmpo_ctx* w = h->workers[k];
     h->launches += w->launches;
     h->updates += w->updates;
@@ -1939,7 +2075,8 @@ int bsmpo_last_update_info(const bsmpo_ctx* hc, int* n_sectors, int* sector_cc, 
     int64_t tot = 0;
     for (int k : h->last_k) tot += k;
     if (tot > sigma_cap) return fail(const_cast<bsmpo_ctx*>(hc), BSMPO_ECAPACITY, "sigma buffer too small");
-    CK(h, cudaMemcpyAsync(sigma, h->sig.p, tot * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    CK(h, cudaMemcpyAsync(sigma, reinterpret_cast<const double*>(h->sig.p) + h->last_sig_off, tot * sizeof(double),
+                          cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
   }
   return BSMPO_OK;

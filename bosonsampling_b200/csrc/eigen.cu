@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -35,27 +36,14 @@ namespace cg = cooperative_groups;
 namespace {
 
 constexpr double EPS = 2.220446049250313e-16;
-// Threads per CTA of the tridiagonalisation: two instantiations, 128 threads (6 CTAs per
-// SM by registers) for the small size classes and 256 threads (2 per SM) for the classes
-// from BSMPO_TD_WIDE on (0-4, default 4: none).  Measured at chi = 1024 with 16
-// concurrent updates: 256 threads for every class 656-672 BS-updates/s against 733-744
-// for none; for the classes with k > 320 only (BSMPO_TD_WIDE=2) 760-776 against 790-793
-// in the same run -- the wider CTAs shorten the largest sector's chain but cost resident
-// CTA slots the concurrent updates share.
-constexpr int TD_NT = 128;
-constexpr int TD_NT_WIDE = 256;
-constexpr int TD_CLASSES = 4;   // cluster sizes 1, 2, 4, 8 CTAs per sector, by sector size
-constexpr int TD_NW_MAX = TD_NT_WIDE / 32;
-// bulk-copy ring of each warp: about BSMPO_TD_RING_KB per CTA, 1, 2 or TD_MAXSLOT row
-// slots (pairs of rows share one pass over the vectors)
-#ifndef BSMPO_TD_RING_KB
-#define BSMPO_TD_RING_KB 64
-#endif
+// Streamed tridiagonalisation (sectors too large for tridiag_resident_kernel): one cluster of
+// TD_CL CTAs per sector
+constexpr int TD_NT = 256, TD_NW = TD_NT / 32;
+constexpr int TD_CL = 16;
+// bulk-copy ring of each warp: about TD_RING_KB per CTA, 1, 2 or TD_MAXSLOT row slots (pairs
+// of rows share one pass over the vectors)
+constexpr int TD_RING_KB = 64;
 constexpr int TD_MAXSLOT = 4;
-#ifndef BSMPO_TD_PAIRS
-#define BSMPO_TD_PAIRS 1   // rows two at a time (0: one at a time)
-#endif
-static_assert(TD_NW_MAX <= 8, "the per-warp scalars of the tridiagonalisation hold 8 warps");
 
 // shared memory of the tridiagonalisation with `slots` ring slots per warp (kmax = the
 // launch's largest k, cl = CTAs per sector): the row rings, v and w of two steps, the
@@ -67,12 +55,12 @@ __host__ __device__ inline size_t td_smem_for(int kmax, int cl, int slots, int n
          64 * sizeof(double) + nw * TD_MAXSLOT * sizeof(uint64_t);
 }
 
-// ring slots per warp: a power of two, 2 to TD_MAXSLOT within about BSMPO_TD_RING_KB per
-// CTA, fewer where a one-CTA sector of size kmax would not fit in 227 KB
+// ring slots per warp: a power of two, 2 to TD_MAXSLOT within about TD_RING_KB per
+// CTA, fewer where a sector of size kmax would not fit in 227 KB
 __host__ __device__ inline int td_slots(int kmax, int nw) {
-  const long long fit = (long long)BSMPO_TD_RING_KB * 1024 / ((long long)nw * kmax * (long long)sizeof(cplx));
+  const long long fit = (long long)TD_RING_KB * 1024 / ((long long)nw * kmax * (long long)sizeof(cplx));
   int s = fit >= TD_MAXSLOT ? TD_MAXSLOT : 2;
-  while (s > 1 && td_smem_for(kmax, 1, s, nw) > 227 * 1024) s >>= 1;
+  while (s > 1 && td_smem_for(kmax, TD_CL, s, nw) > 227 * 1024) s >>= 1;
   return s;
 }
 
@@ -90,10 +78,19 @@ __device__ __forceinline__ cplx warp_sum(cplx v) {
   return v;
 }
 
+// The warp's sum in every lane: as the right operand of an FP64 m8n8k4 product with ones,
+// lane 4 n + c's value is entry (c, n), so the product holds the sums over c; of those,
+// lane x holds two, and a second product adds the four pairs.  Two matrix instructions and
+// an addition (60 cycles) where five shuffles and additions take 210.
 __device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+  double a = 0.0, b = 0.0, t = 0.0, u = 0.0;
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(a), "+d"(b)
+               : "d"(1.0), "d"(v));
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(t), "+d"(u)
+               : "d"(1.0), "d"(a + b));
+  return t;
 }
 
 // a - (x conj(y) + u conj(z)), eight fused multiply-adds (the rank-2 update of one entry)
@@ -116,7 +113,355 @@ __device__ __forceinline__ cplx cdiv(cplx a, cplx b) {
 }
 
 // ---------------------------------------------------------------------------------
-// 1. Tridiagonalisation.  Cluster c handles sector list[c]; its cl CTAs (1, 2, 4 or 8,
+// 1a. Tridiagonalisation with the matrix resident in shared memory: cluster c handles
+//     sector list[c]; CTA `rank` of its cl CTAs holds the rows i = rank (mod cl), stored by
+//     columns so that a lane works on a row of its own and a row's dot product needs no
+//     exchange between lanes.  Step j (trailing size t = k - j - 1), all in shared memory:
+//     1   alpha = -|tau|^2 v^H A v / 2 of step j - 1 from the partials (zhetd2's
+//         -tau p^H v / 2, which is real because A is Hermitian); v = sc y and
+//         w = p + alpha v of step j - 1 (in y's and p's place); row j minus the pending
+//         rank-2 update gives d_j and, conjugated, y, the vector the reflector is formed
+//         from; its norm.  Done redundantly in every CTA on bit-identical inputs and in the
+//         same order, so every CTA holds the same y without exchanging it;
+//     2   own rows i > j, up to four to a lane, the columns dealt out to the warps and spare
+//         lanes in runs: A[i][l] -= v'_i conj(w'_l) + w'_i conj(v'_l)
+//         (v', w' of step j - 1) and the dot products with y.  A warp of its own computes
+//         the reflector beside them (zlarfg: beta real, tau_j, v_j = sc y but 1 at j + 1);
+//         it enters in 3, so its square root and division are off the step's chain;
+//     3   p_i = tau (A[i][j + 1] + sc sum_l A[i][l] y_l); p_i, A[i][j + 1] (row j + 1 of the
+//         next step, by symmetry) and the rows' part of alpha go into every CTA of the
+//         cluster.
+//     Two barriers within a CTA and one of the cluster per step; p, the row and the partials
+//     of alpha are double-buffered by step parity, so a CTA that runs ahead writes what nobody
+//     reads before the next barrier.
+//     What bounds it: shared-memory instructions -- a 128-bit access of a warp takes four
+//     cycles of the SM even where all lanes read one address, so an entry's load and store
+//     and three vector loads would take longer than its 12 fused multiply-adds; four rows to
+//     a lane share the vector loads (44 cycles for 128 entries) -- and the latency of the
+//     step's chain (three warp sums, three barriers).
+//     Measured, one sector alone, us (k = 27, 50, 100, 209, 310, 430): 41, 84, 213, 594,
+//     1,062, 1,565, where the streamed form with 1 to 4 CTAs of 128 threads took 120, 312, 756,
+//     2,847, 7,205, 8,553.  31 sectors of k = 430 at once take 7.8 ms against 9.0 (seven
+//     clusters of 16 fit the GPU).
+constexpr int TD_RES_CLASSES = 7;
+// largest k, CTAs per sector and threads per CTA of a class.  The bounds of the classes
+// from 2 on are what 227 KB of shared memory per CTA hold; below, several sectors share an
+// SM, with about four warps to every 32 rows.
+constexpr int TD_RES_K[TD_RES_CLASSES] = {28, 56, 113, 158, 224, 310, 430};
+constexpr int TD_RES_MAX = TD_RES_K[TD_RES_CLASSES - 1];
+constexpr int TD_RES_CL[TD_RES_CLASSES] = {1, 1, 1, 2, 4, 8, 16};
+constexpr int TD_RES_NT[TD_RES_CLASSES] = {128, 256, 256, 256, 256, 256, 256};
+
+// v, p and the next row, two of each; the partials of the dot products and (two sets, real)
+// of alpha; 64 scalars; the rows
+__host__ __device__ constexpr int td_res_rows(int k, int cl) { return (k + cl - 1) / cl; }
+// 32-row slots of a CTA's rows, a power of two
+__host__ __device__ constexpr int td_res_slots(int k, int cl) {
+  const int rows = td_res_rows(k, cl);
+  return rows > 64 ? 4 : rows > 32 ? 2 : 1;
+}
+__host__ __device__ constexpr size_t td_res_smem(int k, int cl, int nt) {
+  return sizeof(cplx) * (6 * (size_t)k + (size_t)nt * td_res_slots(k, cl) + (size_t)cl * td_res_slots(k, cl) +
+                         (size_t)td_res_rows(k, cl) * k) +
+         64 * sizeof(double);
+}
+constexpr bool td_res_fits() {
+  for (int c = 0; c < TD_RES_CLASSES; ++c)
+    if (td_res_smem(TD_RES_K[c], TD_RES_CL[c], TD_RES_NT[c]) > 227 * 1024 ||
+        td_res_rows(TD_RES_K[c], TD_RES_CL[c]) > 128 || td_res_slots(TD_RES_K[c], TD_RES_CL[c]) > TD_RES_NT[c] / 32)
+      return false;
+  return true;
+}
+static_assert(td_res_fits(), "a class exceeds a CTA's shared memory, or its warps do not cover its rows");
+
+// Phase 2 of one group of lanes: rows r, r + RL, .. (RPL of them, the first n stored), columns
+// l .. end - 1.  UPD: with the rank-2 update (not in step 0).
+template <int RPL, bool UPD>
+__device__ __forceinline__ void td_res_columns(cplx* ap, const int (&ro)[4], int ld, int n, const cplx* vprev,
+                                               const cplx* wprev, const cplx* ycur, const int (&ri)[4], int l, int end,
+                                               cplx (&acc)[4]) {
+  constexpr int UN = RPL > 2 ? 2 : 4;  // columns in flight
+  cplx vi[RPL], wi[RPL];
+  if (UPD) {
+#pragma unroll
+    for (int q = 0; q < RPL; ++q) {
+      vi[q] = ldc(vprev + ri[q]);
+      wi[q] = ldc(wprev + ri[q]);
+    }
+  }
+  auto columns = [&](auto un) {
+    constexpr int U = decltype(un)::value;
+    cplx y[U], vp[U], wp[U], a[U][RPL];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+#pragma unroll
+      for (int q = 0; q < RPL; ++q) a[u][q] = ldc(ap + u * ld + ro[q]);
+      if (UPD) {
+        wp[u] = ldc(wprev + l + u);
+        vp[u] = ldc(vprev + l + u);
+      }
+      y[u] = ldc(ycur + l + u);
+    }
+    if (UPD) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int q = 0; q < RPL; ++q) a[u][q] = crank2(a[u][q], vi[q], wp[u], wi[q], vp[u]);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int q = 0; q < RPL; ++q)
+          if (q < n) stc(ap + u * ld + ro[q], a[u][q]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int q = 0; q < RPL; ++q) cfma(acc[q], a[u][q], y[u]);
+    l += U;
+    ap += U * ld;
+  };
+#pragma unroll 1
+  while (l + UN <= end) columns(std::integral_constant<int, UN>());
+#pragma unroll 1
+  while (l < end) columns(std::integral_constant<int, 1>());
+}
+
+// NT worker threads and one warp more, which forms the reflectors
+template <int NT>
+__global__ void __launch_bounds__(NT + 32)
+    tridiag_resident_kernel(const SectorDesc* __restrict__ sd, const int* __restrict__ list,
+                            cplx* __restrict__ gbuf, double* __restrict__ dbuf,
+                            double* __restrict__ ebuf, cplx* __restrict__ taubuf) {
+  constexpr int NW = NT / 32;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank();
+  const int cl = (int)cluster.num_blocks(), cls = __ffs(cl) - 1;   // a power of two
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const SectorDesc& S = sd[list[blockIdx.x >> cls]];
+  // what is left of the sector where the streamed kernel has reduced its first `off` rows
+  const int ldg = S.k, off = max(S.k - TD_RES_MAX, 0);
+  const int k = S.k - off;             // the same for every CTA of the cluster
+  const int slots = td_res_slots(k, cl), nc = cl * slots;   // partials of alpha, at most 32
+  const int sls = slots >> 1;          // log2 of 1, 2, 4
+  const int ld = td_res_rows(k, cl);
+  cplx* vb = reinterpret_cast<cplx*>(smem_raw);   // y, then v, of step j: vb + (j & 1) k
+  cplx* pb = vb + 2 * k;               // p, then w, of step j: pb + (j & 1) k
+  cplx* xb = pb + 2 * k;               // row j + 1 as step j left it: xb + (j & 1) k
+  cplx* part = xb + 2 * k;             // partials of the dot products: part + warp 32 slots
+  double* cb = reinterpret_cast<double*>(part + NT * slots);   // partials of alpha of step j: cb + (j & 1) nc
+  double* scal = cb + 2 * nc;          // [0, NW) norm, [46, 48) diagonal, [48, 50) first of y, [50, 54) tau, sc
+  cplx* As = reinterpret_cast<cplx*>(scal + 64);   // row i = rank + r cl: As[l ld + r] = A[i][l]
+  cplx* A = gbuf + S.g_off + (int64_t)off * ldg + off;
+  double* dd = dbuf + S.s_off + off;
+  double* ee = ebuf + S.s_off + off;
+  cplx* tt = taubuf + S.s_off + off;
+  if (k <= 1) {
+    if (k == 1 && rank == 0 && tid == 0) dd[0] = A[0].x;
+    return;                            // uniform over the cluster
+  }
+  const int own = (k - rank + cl - 1) >> cls;
+  if (off > 0) {
+    // the streamed kernel's last rank-2 update is pending: v in the row above, w in column
+    // 0 of the whole matrix
+    for (int l = tid; l < k; l += NT + 32) {
+      stc(vb + l, ldc(A - ldg + l));
+      stc(pb + l, ldc(A + (int64_t)l * ldg - off));
+    }
+    __syncthreads();
+  }
+  auto entry = [&](int i, int l) {
+    const cplx a = ldc(A + (int64_t)i * ldg + l);
+    return off > 0 ? crank2(a, ldc(vb + i), ldc(pb + l), ldc(pb + i), ldc(vb + l)) : a;
+  };
+  // A[i][l] = conj(A[l][i]): a warp reads along a row of the matrix
+  for (int l = warp; l < k; l += NW + 1)
+    for (int r = lane; r < own; r += 32) stc(As + l * ld + r, cconj(entry(l, rank + (r << cls))));
+  // row 0 to every CTA (step -1 of the row buffers)
+  for (int l = tid; l < k; l += NT + 32) stc(xb + k + l, entry(0, l));
+  cluster.sync();                      // row 0 of the global matrix is overwritten from here on
+  // alpha of step j from the partials
+  auto alpha_of = [&](int j) { return warp_sum(lane < nc ? cb[(j & 1) * nc + lane] : 0.0); };
+  for (int j = 0; j < k - 1; ++j) {
+    const int par = j & 1;
+    cplx* ycur = vb + par * k;
+    cplx* vprev = vb + (par ^ 1) * k;  // y of step j - 1 until phase 1 has scaled it
+    cplx* wprev = pb + (par ^ 1) * k;  // p of step j - 1 likewise
+    // ---- 1 (v'_j = 1; entry j of v' and w' is not read again, so it is not written)
+    const int na = min(NW, (k - j + 31) >> 5);   // warps with an entry
+    if (warp < na) {
+      const cplx* x = xb + (par ^ 1) * k;
+      double al = 0.0;
+      cplx w1 = cmake(0.0, 0.0), sc = w1;
+      if (j > 0) {
+        al = alpha_of(j - 1);
+        w1 = ldc(wprev + j);
+        w1.x += al;
+        sc = cmake(scal[52], scal[53]);
+      }
+      const bool keeper = j > 0 && rank == ((j - 1) & (cl - 1));   // stores v_{j-1} for the back-transformation
+      double part2 = 0.0;
+      for (int l = j + tid; l < k; l += NT) {
+        cplx a = ldc(x + l);
+        if (j > 0) {
+          cplx v = cmul(sc, ldc(vprev + l)), w = ldc(wprev + l);
+          w = cmake(fma(al, v.x, w.x), fma(al, v.y, w.y));
+          if (l > j) {
+            stc(vprev + l, v);
+            stc(wprev + l, w);
+          } else {
+            v = cmake(1.0, 0.0);
+            w = w1;
+          }
+          if (keeper) stc(A + (int64_t)(j - 1) * ldg + l, v);
+          // row j: a - (conj(w_l) + w_j conj(v_l))
+          a = csub(a, cadd(cconj(w), cmulc(w1, v)));
+        }
+        // d_j, then the first of y: its part of the dot products is added in phase 3
+        const bool head = l <= j + 1;
+        if (head) {
+          scal[46 + 2 * (l - j)] = a.x;
+          scal[47 + 2 * (l - j)] = -a.y;
+          a = cmake(0.0, 0.0);
+        }
+        stc(ycur + l, cconj(a));
+        part2 += cabs2(a);
+      }
+      part2 = warp_sum(part2);
+      if (lane == 0) scal[warp] = part2;
+    }
+    __syncthreads();
+    // ---- 2: own rows r = r0 .. own - 1 (i = rank + r cl > j); 8, 16 or 32 lanes across them
+    const int r0 = j >= rank ? ((j - rank) >> cls) + 1 : 0;
+    const int rows = own - r0;
+    if (warp == NW) {
+      // the reflector
+      double xn2 = scal[0];
+      for (int q = 1; q < na; ++q) xn2 += scal[q];
+      const cplx alpha = cmake(scal[48], scal[49]);
+      double beta = alpha.x;
+      cplx tau = cmake(0.0, 0.0), sc = tau;
+      if (xn2 != 0.0 || alpha.y != 0.0) {
+        beta = -copysign(sqrt(fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, xn2))), alpha.x);
+        const double rb = 1.0 / beta;
+        tau = cmake((beta - alpha.x) * rb, -alpha.y * rb);
+        sc = cdiv(cmake(1.0, 0.0), cmake(alpha.x - beta, alpha.y));
+      }
+      if (lane == 0) {
+        scal[50] = tau.x; scal[51] = tau.y;
+        scal[52] = sc.x; scal[53] = sc.y;
+        if (rank == (j & (cl - 1))) { dd[j] = scal[46]; ee[j] = beta; tt[j] = tau; }
+      }
+    } else if (rows > 0) {
+      const int rls = rows > 64 ? 5 : rows > 32 ? 4 : 3;   // log2 of the lanes across rows
+      const int idx = lane & ((1 << rls) - 1);
+      // rows past the end repeat the last one; they are not stored
+      int ro[4], ri[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        ro[q] = min(r0 + idx + (q << rls), own - 1);
+        ri[q] = rank + (ro[q] << cls);
+      }
+      const int n = (rows - idx + (1 << rls) - 1) >> rls;   // rows of this lane
+      // the columns j + 1 .. k - 1 in equal runs, one to each group of lanes
+      constexpr int NWS = NW == 4 ? 2 : 3;
+      const int gs = NWS + 5 - rls;        // log2 of the groups
+      const int run = (k - j - 2 + (1 << gs)) >> gs;
+      const int l = j + 1 + ((warp << (5 - rls)) + (lane >> rls)) * run, end = min(l + run, k);
+      cplx acc[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[q] = cmake(0.0, 0.0);
+      cplx* ap = As + l * ld;
+      const int rpl = (rows + (1 << rls) - 1) >> rls;       // 1 .. 4, warp-uniform
+      if (j == 0) td_res_columns<4, false>(ap, ro, ld, n, vprev, wprev, ycur, ri, l, end, acc);
+      else if (rpl > 3) td_res_columns<4, true>(ap, ro, ld, n, vprev, wprev, ycur, ri, l, end, acc);
+      else if (rpl > 2) td_res_columns<3, true>(ap, ro, ld, n, vprev, wprev, ycur, ri, l, end, acc);
+      else if (rpl > 1) td_res_columns<2, true>(ap, ro, ld, n, vprev, wprev, ycur, ri, l, end, acc);
+      else td_res_columns<1, true>(ap, ro, ld, n, vprev, wprev, ycur, ri, l, end, acc);
+      __syncwarp();
+      // sums over the groups within the warp, each exchange halving the rows a lane keeps:
+      // with 8 lanes across the rows lane x ends with row x, with 16 with rows
+      // (x mod 16) + 32 (x / 16) and 16 more
+      const bool h16 = (lane & 16) != 0, h8 = (lane & 8) != 0;
+      cplx* pp = part + (warp * slots << 5);
+      if (rls == 5) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (q < n) stc(pp + idx + 32 * q, acc[q]);
+      } else {
+        const cplx s0 = h16 ? acc[0] : acc[2], s1 = h16 ? acc[1] : acc[3];
+        cplx k0 = h16 ? acc[2] : acc[0], k1 = h16 ? acc[3] : acc[1];
+        k0.x += __shfl_xor_sync(0xffffffffu, s0.x, 16);
+        k0.y += __shfl_xor_sync(0xffffffffu, s0.y, 16);
+        k1.x += __shfl_xor_sync(0xffffffffu, s1.x, 16);
+        k1.y += __shfl_xor_sync(0xffffffffu, s1.y, 16);
+        if (rls == 4) {
+          const int x = idx + (h16 ? 32 : 0);
+          if (x < rows) stc(pp + x, k0);
+          if (x + 16 < rows) stc(pp + x + 16, k1);
+        } else {
+          const cplx s = h8 ? k0 : k1;
+          cplx p = h8 ? k1 : k0;
+          p.x += __shfl_xor_sync(0xffffffffu, s.x, 8);
+          p.y += __shfl_xor_sync(0xffffffffu, s.y, 8);
+          if (lane < rows) stc(pp + lane, p);
+        }
+      }
+    }
+    __syncthreads();
+    // ---- 3: a warp to a slot of 32 rows and every (NW >> sls)-th receiving CTA
+    if (warp < NW && (warp >> sls) < cl) {
+      const int slot = warp & (slots - 1), idx = (slot << 5) + lane;
+      cplx p = cmake(0.0, 0.0), xi = p;
+      double ai = 0.0;
+      const int i = rank + ((r0 + idx) << cls);
+      if (idx < rows) {
+        const cplx tau = cmake(scal[50], scal[51]), sc = cmake(scal[52], scal[53]);
+        cplx acc = ldc(part + idx);
+#pragma unroll
+        for (int c = 1; c < NW; ++c) acc = cadd(acc, ldc(part + (c * slots << 5) + idx));
+        const cplx aj = ldc(As + (j + 1) * ld + r0 + idx);
+        xi = cconj(aj);
+        const cplx av = cadd(aj, cmul(sc, acc));   // (A v)_i
+        p = cmul(tau, av);
+        const cplx v = i == j + 1 ? cmake(1.0, 0.0) : cmul(sc, ldc(ycur + i));
+        ai = -0.5 * cabs2(tau) * fma(v.x, av.x, v.y * av.y);
+      }
+      cplx* pd = pb + par * k + i;
+      cplx* xd = xb + par * k + i;
+      double* ad = cb + par * nc + rank * slots + slot;
+      if (cl == 1) {
+        if (idx < rows) { stc(pd, p); stc(xd, xi); }
+        ai = warp_sum(ai);
+        if (lane == 0) *ad = ai;
+      } else {
+        for (int q = warp >> sls; q < cl; q += NW >> sls)
+          if (idx < rows) {
+            stc(cluster.map_shared_rank(pd, q), p);
+            stc(cluster.map_shared_rank(xd, q), xi);
+          }
+        ai = warp_sum(ai);
+        for (int q = warp >> sls; q < cl; q += NW >> sls)
+          if (lane == 0) *cluster.map_shared_rank(ad, q) = ai;
+      }
+    }
+    if (cl > 1) cluster.sync(); else __syncthreads();
+  }
+  // last diagonal entry: row k - 1 minus the update of step k - 2 (v = 1 there)
+  if (rank == 0 && warp == 0) {
+    const int j = k - 1, par = (k - 2) & 1;
+    const double w = pb[par * k + j].x + alpha_of(k - 2);
+    if (lane == 0) {
+      dd[j] = xb[par * k + j].x - 2.0 * w;
+      stc(A + (int64_t)(k - 2) * ldg + j, cmake(1.0, 0.0));
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------
+// 1b. The first k - TD_RES_MAX steps of the larger sectors, rows streamed from L2; the
+//    resident kernel takes over there (a step costs about 10 us here at k = 445, 30 at 1,024,
+//    and 3.6 in the resident kernel).  Cluster c handles sector list[c]; its cl CTAs (1, 2, 4 or 8,
 //    by sector size: a small sector would spend its steps waiting at barriers of a big
 //    cluster) own the rows i = rank (mod cl).  Every CTA holds the reflector vectors
 //    and a copy of the row being reduced, so one cluster barrier per step suffices.
@@ -136,7 +481,7 @@ __device__ __forceinline__ cplx cdiv(cplx a, cplx b) {
 //    again only cl steps later: every next write follows the next barrier, which no CTA
 //    passes before every CTA has finished its G.
 //    Rows stream through shared memory.  Warp w of a CTA handles its own rows number
-//    r = w (mod 4) in every step (row i = rank + r cl), through a private ring of row
+//    r = w (mod 8) in every step (row i = rank + r cl), through a private ring of row
 //    slots: its lane 0 issues a bulk copy (cp.async.bulk, completion counted on the
 //    slot's mbarrier) of the row's trailing segment as soon as the slot is free and the
 //    warp has written that row back in the previous step, so the copies run ahead of
@@ -144,18 +489,15 @@ __device__ __forceinline__ cplx cdiv(cplx a, cplx b) {
 //    -- instead of one L2 round trip per load.  A row is read and written by one warp
 //    only; its write-back is ordered before the next bulk read of it by a proxy fence
 //    of the writing lanes and the warp's synchronisation.
-template <int TD_NT_, int MINB>
-__global__ void __launch_bounds__(TD_NT_, MINB)
+__global__ void __launch_bounds__(TD_NT, 2)
     tridiag_kernel(const SectorDesc* __restrict__ sd, const int* __restrict__ list, int kmax,
                    cplx* __restrict__ gbuf, double* __restrict__ dbuf, double* __restrict__ ebuf,
                    cplx* __restrict__ taubuf, int* __restrict__ err) {
-  constexpr int TD_NT = TD_NT_;        // threads of this instantiation
-  constexpr int TD_NW = TD_NT_ / 32;   // its warps, each streaming its own rows
   extern __shared__ __align__(128) unsigned char smem_raw[];
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
-  const int TD_CL = (int)cluster.num_blocks();   // 1, 2, 4 or 8
-  const int cls = __ffs(TD_CL) - 1;                // log2 of it
+  constexpr int cls = 4;               // log2 of TD_CL
+  static_assert(TD_CL == 1 << cls, "rows are dealt out by shifts");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int own_cap = kmax / TD_CL + 1;
   const int nslot = td_slots(kmax, TD_NW);         // 1, 2 or 4
@@ -172,14 +514,11 @@ __global__ void __launch_bounds__(TD_NT_, MINB)
   cplx* wring = ring + (size_t)warp * nslot * kmax;
   const SectorDesc& S = sd[list[blockIdx.x / TD_CL]];
   const int k = S.k;                   // the same for every CTA of the cluster
+  const int steps = k - TD_RES_MAX;    // >= 1; the rest is the resident kernel's
   cplx* A = gbuf + S.g_off;
   double* dd = dbuf + S.s_off;
   double* ee = ebuf + S.s_off;
   cplx* tt = taubuf + S.s_off;
-  if (k <= 1) {
-    if (k == 1 && rank == 0 && tid == 0) dd[0] = A[0].x;
-    return;                            // uniform over the cluster
-  }
   if (lane < TD_MAXSLOT) {
     mbar_init(bars + lane, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -187,7 +526,7 @@ __global__ void __launch_bounds__(TD_NT_, MINB)
   __syncthreads();
 
   // ---- this warp's row sequence: (step s, own row r) with rows i = rank + r cl > s,
-  // r = warp (mod 4), in step order, then row order; copies are issued in the same order
+  // r = warp (mod 8), in step order, then row order; copies are issued in the same order
   // as the pass consumes them, element q into slot q mod nslot
   auto first_row = [&](int s) {
     const int r0 = s >= rank ? ((s - rank) >> cls) + 1 : 0;
@@ -199,7 +538,7 @@ __global__ void __launch_bounds__(TD_NT_, MINB)
   auto issue = [&]() {
     // a free slot, and the row's write-back of the previous step done (consumption is in
     // sequence order, so the last consumed element tells)
-    while (is < k - 1 && rank + (ir << cls) < k && issued < done + nslot &&
+    while (is < steps && rank + (ir << cls) < k && issued < done + nslot &&
            (is == 0 || ls > is - 1 || (ls == is - 1 && lr >= ir))) {
       if (lane == 0) {
         const int slot = issued & (nslot - 1);
@@ -216,7 +555,7 @@ __global__ void __launch_bounds__(TD_NT_, MINB)
   issue();
 
   double beta = 0.0;                   // this step's e_j (warp 0)
-  for (int j = 0; j < k - 1; ++j) {
+  for (int j = 0; j < steps; ++j) {
     const int par = j & 1;
     const bool owner = rank == (j & (TD_CL - 1));
     cplx* vcur = vb + par * kmax;
@@ -271,7 +610,7 @@ __global__ void __launch_bounds__(TD_NT_, MINB)
       for (int r = first_row(j); rank + (r << cls) < k;) {
         const int r2 = r + TD_NW;
         const int i = rank + (r << cls), i2 = rank + (r2 << cls);
-        const bool two = BSMPO_TD_PAIRS && nslot >= 2 && i2 < k;   // warp-uniform
+        const bool two = nslot >= 2 && i2 < k;   // warp-uniform
         const int slot = done & (nslot - 1), slot2 = (done + 1) & (nslot - 1);
         // on expiry the error word is set and the pass goes on with what the slot holds
         mbar_wait_fast(bars + slot, (uint32_t)(done >> nss) & 1u, err);
@@ -401,12 +740,10 @@ __global__ void __launch_bounds__(TD_NT_, MINB)
       __syncthreads();
     }
   }
-  // last diagonal entry: row k - 1 (copied in the last G) minus the update of step k - 2
-  if (rank == ((k - 1) & (TD_CL - 1)) && tid == 0) {
-    const int j = k - 1;
-    const cplx v = vb[((k - 2) & 1) * kmax + j], w = wb[((k - 2) & 1) * kmax + j];
-    const cplx a = crank2(nrow[j], v, w, w, v);
-    dd[j] = a.x;
+  // w of the last step, whose update of the rows i >= steps is pending, into column 0
+  for (int r = tid; rank + (r << cls) < k; r += TD_NT) {
+    const int i = rank + (r << cls);
+    if (i >= steps) stc(A + (int64_t)i * k, wb[((steps - 1) & 1) * kmax + i]);
   }
   cluster.sync();   // no CTA leaves while another may still read its shared memory
 }
@@ -538,13 +875,21 @@ __global__ __launch_bounds__(FI_NT) void eig_finish_kernel(const SectorDesc* __r
 
 // ---------------------------------------------------------------------------------
 // 3a. Eigenvectors of the tridiagonal by inverse iteration, one thread per kept
-//     eigenvalue.  T - lambda I = P L U with partial pivoting (U has two
-//     superdiagonals), stored column-interleaved in the scratch (entry l of vector t
+//     eigenvalue, one CTA per sector.  T - lambda I = P L U with partial pivoting (U has
+//     two superdiagonals), stored column-interleaved in the scratch (entry l of vector t
 //     at l * kept + t, so a warp's accesses coalesce).  Start vector: a fixed
 //     pseudo-random one; three solves, normalised.  Eigenvalues closer than `gaptol`
-//     form a group handled by its first member, each vector orthogonalised against
-//     the group's earlier ones after every solve.
+//     form a group; after the second and the third solve the whole CTA orthogonalises each
+//     group's vectors in order (classical Gram-Schmidt, twice).
+//     What bounds it: each thread's recurrences (k dependent steps, seven passes).  The
+//     passes move IV_B steps of a column between registers and scratch at a time, one
+//     batch ahead, and the factorisation keeps the pivots' reciprocals, so a step costs its
+//     two or three dependent operations and not a division and an L2 round trip.
+//     Measured: 3.1 ms of kernel time in two layers at N = 64, chi = 1024 (62 updates)
+//     against 33.5 with one thread per group and a division and scratch access per step.
 constexpr int IV_NT = 128;
+constexpr int IV_B = 8;        // steps of a batch
+constexpr int IV_GT = 32;      // group members one pass of the orthogonalisation takes
 
 __device__ __forceinline__ double start_entry(int l, int t) {
   unsigned h = (unsigned)l * 2654435761u ^ ((unsigned)t * 40503u + 0x9e3779b9u);
@@ -562,101 +907,180 @@ __global__ __launch_bounds__(IV_NT) void invit_kernel(const SectorDesc* __restri
                                                       unsigned char* __restrict__ swp,
                                                       double* __restrict__ zbuf) {
   extern __shared__ double ism[];
-  const SectorDesc& S = sd[blockIdx.y];
+  __shared__ double dots[IV_NT / 32][IV_GT], coef[IV_GT], nrm2[IV_NT / 32];
+  const SectorDesc& S = sd[blockIdx.x];
   const int k = S.k, kept = S.kept;
-  const int t0 = blockIdx.x * IV_NT;
-  if (t0 >= kept) return;
+  if (kept == 0) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double* d = ism;
   double* e = ism + k;
-  for (int i = threadIdx.x; i < k; i += IV_NT) {
+  for (int i = tid; i < k; i += IV_NT) {
     d[i] = dbuf[S.s_off + i];
     e[i] = i < k - 1 ? ebuf[S.s_off + i] : 0.0;
   }
-  __syncthreads();
-  const int t = t0 + threadIdx.x;
-  if (t >= kept) return;
   const double* lv = lam + S.s_off;
   const double norm = fmax(fabs(lv[0]), fabs(lv[k - 1]));
   const double gaptol = 1e-9 * norm;
-  // group membership: not a leader if the previous kept eigenvalue is within gaptol
-  if (t > 0 && lv[t - 1] - lv[t] <= gaptol) return;
-  int g_end = t + 1;
-  while (g_end < kept && lv[g_end - 1] - lv[g_end] <= gaptol) ++g_end;
   const double tiny = EPS * norm + 1e-300;
-  // scratch layout of this sector: 4 arrays [k][kept] (u0, u1, u2, mult)
-  double* U0 = scratch + 4 * S.y_off;   // 4 arrays of k x kept in the sector's 4 k^2 slots
-  double* U1 = U0 + (int64_t)k * kept;
+  // scratch of this sector: 1 / pivot, the superdiagonals, the multipliers (k x kept
+  // each), and the row exchanges, IV_B of them to a byte
+  double* RP = scratch + 4 * S.y_off;
+  double* U1 = RP + (int64_t)k * kept;
   double* U2 = U1 + (int64_t)k * kept;
   double* MU = U2 + (int64_t)k * kept;
   unsigned char* SW = swp + S.y_off;
   double* Z = zbuf + S.y_off;
-  for (int m = t; m < g_end; ++m) {
-    const double lambda = lv[m];
+  __syncthreads();
+  bool grouped = false;
+  for (int m = tid; m < kept; m += IV_NT) grouped |= m > 0 && lv[m - 1] - lv[m] <= gaptol;
+  grouped = __syncthreads_or(grouped);
+  for (int m = tid; m < kept; m += IV_NT) {
     // factor T - lambda I
+    const double lambda = lv[m];
     double p = d[0] - lambda, q = k > 1 ? e[0] : 0.0;
-#pragma unroll 4
-    for (int i = 0; i < k - 1; ++i) {
-      const double ei = e[i], an = d[i + 1] - lambda, en = i + 1 < k - 1 ? e[i + 1] : 0.0;
-      const int64_t o = (int64_t)i * kept + m;
-      if (fabs(ei) > fabs(p)) {
-        const double mu = p / ei;
-        U0[o] = ei; U1[o] = an; U2[o] = en; MU[o] = mu; SW[o] = 1;
-        const double np = q - mu * an, nq = -mu * en;
-        p = np;
-        q = nq;
-      } else {
-        if (p == 0.0) p = tiny;
-        const double mu = ei / p;
-        U0[o] = p; U1[o] = q; U2[o] = 0.0; MU[o] = mu; SW[o] = 0;
-        p = an - mu * q;
-        q = en;
+    for (int i0 = 0; i0 < k; i0 += IV_B) {
+      unsigned sw = 0;
+#pragma unroll
+      for (int b = 0; b < IV_B; ++b) {
+        const int i = i0 + b;
+        if (i >= k) break;
+        const int64_t o = (int64_t)i * kept + m;
+        const double ei = i < k - 1 ? e[i] : 0.0, en = i + 1 < k - 1 ? e[i + 1] : 0.0;
+        const double an = i < k - 1 ? d[i + 1] - lambda : 0.0;
+        const bool x = fabs(ei) > fabs(p);
+        if (!x && p == 0.0) p = tiny;
+        const double r = 1.0 / (x ? ei : p), mu = (x ? p : ei) * r;
+        RP[o] = r;
+        U1[o] = x ? an : q;
+        U2[o] = x ? en : 0.0;
+        MU[o] = mu;
+        sw |= x ? 1u << b : 0u;
+        p = x ? q - mu * an : an - mu * q;
+        q = x ? -mu * en : en;
       }
+      SW[(int64_t)(i0 / IV_B) * kept + m] = (unsigned char)sw;
     }
-    if (p == 0.0) p = tiny;
-    {
-      const int64_t o = (int64_t)(k - 1) * kept + m;
-      U0[o] = p; U1[o] = 0.0; U2[o] = 0.0; MU[o] = 0.0; SW[o] = 0;
-    }
-    for (int it = 0; it < 3; ++it) {
-      // right-hand side: start vector, or L^{-1} P z
+  }
+  for (int it = 0; it < 3; ++it) {
+    for (int m = tid; m < kept; m += IV_NT) {
+      // right-hand side: the start vector, or L^{-1} P z; the solution's scale is applied
+      // where it is read next (a solve's scale is dropped before the next one's matters)
       if (it == 0) {
         for (int i = 0; i < k; ++i) Z[(int64_t)i * kept + m] = start_entry(i, m);
       } else {
-#pragma unroll 4
-        for (int i = 0; i < k - 1; ++i) {
-          const int64_t o = (int64_t)i * kept + m, o1 = o + kept;
-          double bi = Z[o], bn = Z[o1];
-          if (SW[o]) { const double x = bi; bi = bn; bn = x; }
-          Z[o] = bi;
-          Z[o1] = bn - MU[o] * bi;
+        double zc = Z[m];
+        double zn[IV_B], mu[IV_B];
+        unsigned sw = 0;
+        auto load = [&](int i0) {
+#pragma unroll
+          for (int b = 0; b < IV_B; ++b) {
+            const int i = i0 + b;
+            zn[b] = i + 1 < k ? Z[(int64_t)(i + 1) * kept + m] : 0.0;
+            mu[b] = i < k ? MU[(int64_t)i * kept + m] : 0.0;
+          }
+          sw = i0 < k ? SW[(int64_t)(i0 / IV_B) * kept + m] : 0;
+        };
+        load(0);
+        for (int i0 = 0; i0 < k - 1; i0 += IV_B) {
+          double cz[IV_B], cm[IV_B];
+          const unsigned cs = sw;
+#pragma unroll
+          for (int b = 0; b < IV_B; ++b) { cz[b] = zn[b]; cm[b] = mu[b]; }
+          load(i0 + IV_B);
+#pragma unroll
+          for (int b = 0; b < IV_B; ++b) {
+            if (i0 + b >= k - 1) break;
+            const bool x = (cs >> b) & 1u;
+            const double bi = x ? cz[b] : zc, bn = x ? zc : cz[b];
+            Z[(int64_t)(i0 + b) * kept + m] = bi;
+            zc = fma(-cm[b], bi, bn);
+          }
         }
+        Z[(int64_t)(k - 1) * kept + m] = zc;
       }
-      // back substitution U z = b, then normalise
+      // back substitution U z = b, batches from the last row up
       double z1 = 0.0, z2 = 0.0, nrm = 0.0;
-#pragma unroll 4
-      for (int i = k - 1; i >= 0; --i) {
-        const int64_t o = (int64_t)i * kept + m;
-        double u0 = U0[o];
-        if (u0 == 0.0) u0 = tiny;
-        const double z = (Z[o] - U1[o] * z1 - U2[o] * z2) / u0;
-        Z[o] = z;
-        z2 = z1;
-        z1 = z;
-        nrm += z * z;
-      }
-      // orthogonalise against the group's earlier vectors
-      for (int g = t; g < m; ++g) {
-        double dot = 0.0;
-        for (int i = 0; i < k; ++i) dot += Z[(int64_t)i * kept + g] * Z[(int64_t)i * kept + m];
-        nrm = 0.0;
-        for (int i = 0; i < k; ++i) {
-          const double z = Z[(int64_t)i * kept + m] - dot * Z[(int64_t)i * kept + g];
-          Z[(int64_t)i * kept + m] = z;
-          nrm += z * z;
+      double zb[IV_B], rp[IV_B], u1[IV_B], u2[IV_B];
+      auto load = [&](int i1) {   // rows i1, i1 - 1, ...
+#pragma unroll
+        for (int b = 0; b < IV_B; ++b) {
+          const int i = i1 - b;
+          const int64_t o = (int64_t)i * kept + m;
+          zb[b] = i >= 0 ? Z[o] : 0.0;
+          rp[b] = i >= 0 ? RP[o] : 0.0;
+          u1[b] = i >= 0 ? U1[o] : 0.0;
+          u2[b] = i >= 0 ? U2[o] : 0.0;
+        }
+      };
+      load(k - 1);
+      for (int i1 = k - 1; i1 >= 0; i1 -= IV_B) {
+        double cb[IV_B], cr[IV_B], c1[IV_B], c2[IV_B];
+#pragma unroll
+        for (int b = 0; b < IV_B; ++b) { cb[b] = zb[b]; cr[b] = rp[b]; c1[b] = u1[b]; c2[b] = u2[b]; }
+        load(i1 - IV_B);
+#pragma unroll
+        for (int b = 0; b < IV_B; ++b) {
+          if (i1 - b < 0) break;
+          const double z = fma(-c1[b], z1, fma(-c2[b], z2, cb[b])) * cr[b];
+          Z[(int64_t)(i1 - b) * kept + m] = z;
+          z2 = z1;
+          z1 = z;
+          nrm = fma(z, z, nrm);
         }
       }
       const double inv = nrm > 0.0 ? 1.0 / sqrt(nrm) : 0.0;
-      for (int i = 0; i < k; ++i) Z[(int64_t)i * kept + m] *= inv;
+      for (int i0 = 0; i0 < k; i0 += IV_B) {
+        double zs[IV_B];
+#pragma unroll
+        for (int b = 0; b < IV_B; ++b) zs[b] = i0 + b < k ? Z[(int64_t)(i0 + b) * kept + m] : 0.0;
+#pragma unroll
+        for (int b = 0; b < IV_B; ++b)
+          if (i0 + b < k) Z[(int64_t)(i0 + b) * kept + m] = zs[b] * inv;
+      }
+    }
+    if (!grouped || it == 0) continue;   // uniform over the CTA
+    __syncthreads();
+    int first = 0;
+    for (int m = 1; m < kept; ++m) {
+      if (lv[m - 1] - lv[m] > gaptol) { first = m; continue; }
+      // z_m against the group's earlier vectors first .. m - 1, twice
+      for (int pass = 0; pass < 2; ++pass) {
+        for (int g0 = first; g0 < m; g0 += IV_GT) {
+          const int g = g0 + lane, ng = min(IV_GT, m - g0);
+          double dot = 0.0;
+          if (g < m)
+            for (int i = warp; i < k; i += IV_NT / 32)
+              dot = fma(Z[(int64_t)i * kept + g], Z[(int64_t)i * kept + m], dot);
+          dots[warp][lane] = dot;
+          __syncthreads();
+          if (tid < IV_GT) {
+            double s = 0.0;
+            for (int w = 0; w < IV_NT / 32; ++w) s += dots[w][tid];
+            coef[tid] = s;
+          }
+          __syncthreads();
+          // a thread per entry of z_m
+          for (int i = tid; i < k; i += IV_NT) {
+            double z = Z[(int64_t)i * kept + m];
+            for (int c = 0; c < ng; ++c) z = fma(-coef[c], Z[(int64_t)i * kept + g0 + c], z);
+            Z[(int64_t)i * kept + m] = z;
+          }
+          __syncthreads();
+        }
+      }
+      double s = 0.0;
+      for (int i = tid; i < k; i += IV_NT) {
+        const double z = Z[(int64_t)i * kept + m];
+        s = fma(z, z, s);
+      }
+      s = warp_sum(s);
+      if (lane == 0) nrm2[warp] = s;
+      __syncthreads();
+      s = 0.0;
+      for (int w = 0; w < IV_NT / 32; ++w) s += nrm2[w];
+      const double inv = s > 0.0 ? 1.0 / sqrt(s) : 0.0;
+      for (int i = tid; i < k; i += IV_NT) Z[(int64_t)i * kept + m] *= inv;
+      __syncthreads();
     }
   }
 }
@@ -718,7 +1142,7 @@ int eigen_max_k() {
   static const int kmax = [] {
     int best = 0;
     for (int k = 1; k <= 32 * 32; ++k) {   // the back-transformation keeps 32 entries per lane
-      if (td_smem_bytes(k, 1, TD_NT / 32) > 227 * 1024) break;
+      if (td_smem_bytes(k, TD_CL, TD_NW) > 227 * 1024) break;
       best = k;
     }
     return best;
@@ -726,69 +1150,75 @@ int eigen_max_k() {
   return kmax;
 }
 
-// Size-class bounds (largest k of classes 0, 1, 2); BSMPO_TD_CLASSES="a,b,c" in the
-// environment replaces them (read once).
+// Size class of a sector: the resident kernel's classes, then the streamed kernel's.
 int tridiag_class(int k) {
-  static const int* bounds = [] {
-    static int b[3] = {64, 320, 1024};   // the 8-CTA class stays unused up to k = 1024
-    const char* e = std::getenv("BSMPO_TD_CLASSES");
-    int x, y, z;
-    if (e && std::sscanf(e, "%d,%d,%d", &x, &y, &z) == 3 && 0 < x && x < y && y < z) {
-      b[0] = x; b[1] = y; b[2] = z;
-    }
-    return b;
-  }();
-  return k <= bounds[0] ? 0 : k <= bounds[1] ? 1 : k <= bounds[2] ? 2 : 3;
+  for (int c = 0; c < TD_RES_CLASSES; ++c)
+    if (k <= TD_RES_K[c]) return c;
+  return TD_RES_CLASSES;
 }
+
+namespace {
+
+template <typename F, typename... Args>
+cudaError_t launch_cluster(F* kernel, int grid, int cl, int nt, size_t smem, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(nt);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cl;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+}  // namespace
 
 cudaError_t launch_tridiag(const SectorDesc* sd_dev, const int* list_dev, const int* class_count,
                            const int* class_kmax, void* gbuf, double* dbuf, double* ebuf,
                            void* taubuf, int* err, const cudaStream_t* streams) {
-  // once per process: the largest dynamic shared memory any launch may ask for
+  static_assert(TD_CLASSES == TD_RES_CLASSES + 1, "one class more than the resident kernel's");
+  // once per process: the largest dynamic shared memory any launch may ask for, and
+  // clusters of 16 CTAs
   static const cudaError_t attr = [] {
-    size_t most = 0, most_w = 0;
-    for (int k = 1; k <= eigen_max_k(); ++k) {
-      most = std::max(most, td_smem_bytes(k, 1, TD_NT / 32));
-      const size_t w = td_smem_bytes(k, 1, TD_NT_WIDE / 32);
-      if (w <= 227 * 1024) most_w = std::max(most_w, w);
-    }
-    cudaError_t e = cudaFuncSetAttribute(tridiag_kernel<TD_NT, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    size_t most = 0;
+    for (int k = 1; k <= eigen_max_k(); ++k) most = std::max(most, td_smem_bytes(k, TD_CL, TD_NW));
+    const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(tridiag_kernel, dyn, (int)most);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(tridiag_resident_kernel<128>, dyn, 227 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(tridiag_resident_kernel<256>, dyn, 227 * 1024);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(tridiag_kernel<TD_NT_WIDE, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most_w);
+      e = cudaFuncSetAttribute(tridiag_resident_kernel<256>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(tridiag_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
   }();
   if (attr != cudaSuccess) return attr;
-  // the first size class on 256-thread CTAs (BSMPO_TD_WIDE, 0-4; 4: none), read once
-  static const int wide = [] {
-    const char* e = std::getenv("BSMPO_TD_WIDE");
-    return (e && e[0] >= '0' && e[0] <= '4') ? e[0] - '0' : TD_CLASSES;
-  }();
+  cplx* G = reinterpret_cast<cplx*>(gbuf);
+  cplx* tau = reinterpret_cast<cplx*>(taubuf);
   int first = 0;
   for (int c = 0; c < TD_CLASSES; ++c) {
     const int count = class_count[c];
     if (count == 0) continue;
-    const int cl = 1 << c;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(count * cl);
-    // 256 threads where asked and where their larger rings fit the launch's shared memory
-    const bool w = c >= wide && td_smem_bytes(class_kmax[c], 1, TD_NT_WIDE / 32) <= 227 * 1024;
-    const int nt = w ? TD_NT_WIDE : TD_NT;
-    cfg.blockDim = dim3(nt);
-    cfg.dynamicSmemBytes = td_smem_bytes(class_kmax[c], cl, nt / 32);
-    cfg.stream = streams[TD_CLASSES - 1 - c];   // the largest class on the caller's stream
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cl;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaError_t e = w ? cudaLaunchKernelEx(&cfg, tridiag_kernel<TD_NT_WIDE, 2>, sd_dev, list_dev + first,
-                                           class_kmax[c], reinterpret_cast<cplx*>(gbuf), dbuf, ebuf,
-                                           reinterpret_cast<cplx*>(taubuf), err)
-                      : cudaLaunchKernelEx(&cfg, tridiag_kernel<TD_NT, 6>, sd_dev, list_dev + first,
-                                           class_kmax[c], reinterpret_cast<cplx*>(gbuf), dbuf, ebuf,
-                                           reinterpret_cast<cplx*>(taubuf), err);
+    const int* list = list_dev + first;
+    cudaStream_t s = streams[c];
+    cudaError_t e;
+    if (c == TD_RES_CLASSES) {
+      e = launch_cluster(tridiag_kernel, count * TD_CL, TD_CL, TD_NT, td_smem_bytes(class_kmax[c], TD_CL, TD_NW), s,
+                         sd_dev, list, class_kmax[c], G, dbuf, ebuf, tau, err);
+      if (e != cudaSuccess) return e;
+    }
+    {
+      const int rc = std::min(c, TD_RES_CLASSES - 1);
+      const int cl = TD_RES_CL[rc], nt = TD_RES_NT[rc];
+      const auto kernel = nt == 128 ? tridiag_resident_kernel<128> : tridiag_resident_kernel<256>;
+      e = launch_cluster(kernel, count * cl, cl, nt + 32, td_res_smem(std::min(class_kmax[c], TD_RES_MAX), cl, nt), s,
+                         sd_dev, list, G, dbuf, ebuf, tau);
+    }
     if (e != cudaSuccess) return e;
     first += count;
   }
@@ -822,8 +1252,7 @@ cudaError_t launch_eigvec(const SectorDesc* sd_dev, int n_sectors, int kmax, int
     cudaError_t e = cudaFuncSetAttribute(invit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  invit_kernel<<<dim3(ceil_div(kept_max, IV_NT), n_sectors), IV_NT, smem, s>>>(sd_dev, dbuf, ebuf, lam,
-                                                                               scratch, swp, zbuf);
+  invit_kernel<<<n_sectors, IV_NT, smem, s>>>(sd_dev, dbuf, ebuf, lam, scratch, swp, zbuf);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   dim3 grid(ceil_div(kept_max, BT_NT / 32), n_sectors);

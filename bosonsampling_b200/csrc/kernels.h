@@ -31,7 +31,8 @@ cudaError_t launch_fock_tensor_single(int d, M8 m, void* u_re_or_cplx, double* u
 // One group of a grouped complex128 GEMM:  C = rs[m] cs[n] sum_k op(A)(m,k) ks[k] op(B)(k,n)
 // op 0: as stored (row-major A[m][k], B[k][n]); op 1: conjugate transpose (A stored
 // [k][m], B stored [n][k]).  Offsets are in complex elements (scales in doubles) from
-// the launch's base pointers; a negative scale offset means "none".
+// the launch's base pointers; a negative scale offset means "none".  sd is read only for
+// groups with sec >= 0.
 struct GemmGroup {
   int M, N, K;
   int lda, ldb, ldc;
@@ -39,6 +40,8 @@ struct GemmGroup {
   int beta;          // 0: C = result, 1: C += result
   int tiles_n;       // ceil(N / tile N)
   int tile_start;    // first flat tile index of this group
+  int sec;           // >= 0: a dimension is sector sec's kept count, read on the device
+  int kdim;          // (1: M and lda; 2: N, ldb and ldc); the host's value is its bound
   int pad_;
   int64_t a_off, b_off, c_off;
   int64_t ks_off, rs_off, cs_off;
@@ -46,7 +49,7 @@ struct GemmGroup {
 
 cudaError_t launch_zgemm_grouped(const void* a, const void* b, void* c, const double* scale,
                                  const GemmGroup* groups_dev, int n_groups, int total_tiles,
-                                 cudaStream_t s);
+                                 const struct SectorDesc* sd_dev, cudaStream_t s);
 int zgemm_tile_m();
 int zgemm_tile_n();
 
@@ -86,16 +89,18 @@ struct MixPair {
   int row0, nrow;      // left-bond rows of block a
   int col0, ncol;      // right-bond columns of block b
   int tile_start;      // first flat CTA index of this pair
-  int pad_;
+  int upd;             // its update in the group
 };
 
-// Per-update tables shared by several kernels (device copy, one per update).
+// Tables of one update of a group, shared by several kernels (device copy).  Sector indices
+// are the group's; the update's own sectors are sec0 .. sec0 + n_sectors - 1.
 struct UpdateTables {
   int d, chi, mode;
-  int n_sectors, n_theta, n_pairs;
+  int n_sectors, sec0, pad_;
+  int64_t gate_off;                               // its gate tensor, from the launch's base
   int offL[BSMPO_MAX_Q + 1], offC[BSMPO_MAX_Q + 1], offR[BSMPO_MAX_Q + 1];
   int sidx[BSMPO_MAX_Q];                          // sector index of centre charge, or -1
-  int pair_of[BSMPO_MAX_Q];                       // sector index of the (cc1, cc0) sector, or -1
+  int pair_of[BSMPO_MAX_Q];                       // per own sector: the (cc1, cc0) sector, or -1
 };
 
 // ---------------------------------------------------------------- sector.cu
@@ -103,25 +108,26 @@ struct UpdateTables {
 cudaError_t launch_mix_d(int d, const UpdateTables* tab_dev, const int* tidx_dev,
                          const ThetaDesc* td_dev, const SectorDesc* sd_dev,
                          const MixPair* pairs_dev, int n_pairs, int total_tiles, const void* u3,
-                         const void* theta, const double* lam_r, void* cbuf, void* abuf,
+                         const void* theta, const double* lam, void* cbuf, void* abuf,
                          cudaStream_t s);
 // Identity rows of [T^H; I_m] for the `left` sectors.
 cudaError_t launch_identity_rows(const SectorDesc* sd_dev, int n_sectors, int max_elems,
                                  void* abuf, cudaStream_t s);
-// Deterministic top-chi with ket/bra pair symmetrisation; writes kept counts into
-// sd_dev[s].kept and kept_out[s], slot starts, and the truncation weight.
-cudaError_t launch_select(const UpdateTables* tab_dev, SectorDesc* sd_dev, int n_sectors,
-                          const double* sig, double* keys, double cutoff, int chi,
+// Deterministic top-chi with ket/bra pair symmetrisation, one CTA per update; writes kept
+// counts into sd_dev[s].kept and kept_out[s], slot starts, every update's total into
+// kept_out[n_sectors + u] and its truncation weight into trunc_out[u].
+cudaError_t launch_select(const UpdateTables* tab_dev, SectorDesc* sd_dev, int n_updates,
+                          int n_sectors, const double* sig, double* keys, double cutoff, int chi,
                           int* kept_out, double* trunc_out, cudaStream_t s);
 // conj(V) rows for the kept vectors of every sector.
 cudaError_t launch_extract_v(const SectorDesc* sd_dev, int n_sectors, int max_elems,
                              const void* abuf, const double* sig, const int* perm, void* vbuf,
                              cudaStream_t s);
-// New Gamma_L (= Gamma[mode]), Gamma_R (= Gamma[mode+1]), Lambda and charges of bond mode+1.
-cudaError_t launch_scatter(const UpdateTables* tab_dev, const SectorDesc* sd_dev, int n_sectors,
-                           int total_kept, int chi, const int* charge_l, const int* charge_r,
-                           const void* vbuf, const void* wbuf, const double* sig,
-                           void* gamma_l, void* gamma_r, double* lam_c, int* charge_c,
+// New Gamma_L (= Gamma[mode]), Gamma_R (= Gamma[mode+1]), Lambda and charges of bond mode+1
+// of every update; gamma, lam, charge: the whole state's; totals: kept vectors per update.
+cudaError_t launch_scatter(const UpdateTables* tab_dev, const SectorDesc* sd_dev, int n_updates,
+                           const int* totals, int chi, const void* vbuf, const void* wbuf,
+                           const double* sig, void* gamma, double* lam, int* charge,
                            cudaStream_t s);
 // exp(i phi (n_ket - n_bra)) on every element of one site tensor.
 cudaError_t launch_phase(int d, int chi, double phi, const int* charge_l, const int* charge_r,
@@ -169,11 +175,12 @@ cudaError_t launch_jacobi_finish(const SectorDesc* sd_dev, int n_sectors, int ma
 // Gram / Hermitian-eigen route of the sector SVD (see eigen.cu).  gbuf holds every
 // sector's Gram G = X^H X (k x k at g_off), overwritten by the Householder vectors.
 int eigen_max_k();
-// Sectors go in four launches by size class (tridiag_class: 1, 2, 4 or 8 CTAs per
-// sector): list_dev holds the sector indices grouped by class, class_count / class_kmax
-// (host, 4 entries) the number of sectors and their largest k per class.  Class c goes
-// on streams[3 - c] (the caller forks and joins them; streams[0] is its own).  err: a
-// device word set to 1 when a bulk-copy wait expired (zeroed by the caller).
+// Sectors go in one launch per size class (tridiag_class): list_dev holds the sector
+// indices grouped by class, class_count / class_kmax (host, TD_CLASSES entries) the number
+// of sectors and their largest k per class.  Class c goes on streams[c] (the caller forks
+// and joins them).  err: a device word set to 1 when a bulk-copy wait expired (zeroed by
+// the caller).
+constexpr int TD_CLASSES = 8;
 int tridiag_class(int k);
 cudaError_t launch_tridiag(const SectorDesc* sd_dev, const int* list_dev, const int* class_count,
                            const int* class_kmax, void* gbuf, double* dbuf, double* ebuf,

@@ -19,14 +19,14 @@ namespace {
 constexpr int MIX_NT = 256;
 
 template <int MD>
-__global__ __launch_bounds__(MIX_NT) void mix_kernel(const UpdateTables* __restrict__ tab,
-                                                     const int* __restrict__ tidx,
+__global__ __launch_bounds__(MIX_NT) void mix_kernel(const UpdateTables* __restrict__ tabs,
+                                                     const int* __restrict__ tidxs,
                                                      const ThetaDesc* __restrict__ td,
                                                      const SectorDesc* __restrict__ sd,
                                                      const MixPair* __restrict__ pairs, int n_pairs,
-                                                     const cplx* __restrict__ u3,
+                                                     const cplx* __restrict__ u3s,
                                                      const cplx* __restrict__ theta,
-                                                     const double* __restrict__ lam_r,
+                                                     const double* __restrict__ lam_all,
                                                      cplx* __restrict__ cbuf,
                                                      cplx* __restrict__ abuf) {
   __shared__ MixPair P;
@@ -36,7 +36,6 @@ __global__ __launch_bounds__(MIX_NT) void mix_kernel(const UpdateTables* __restr
   __shared__ int64_t cb[MD][MD], ab[MD][MD];
   __shared__ int cn[MD][MD], ck[MD][MD], cleft[MD][MD], crow[MD][MD], ccol[MD][MD], crt[MD][MD];
   const int tid = threadIdx.x;
-  const int d = tab->d;
   if (tid == 0) {
     int lo = 0, hi = n_pairs - 1;
     const int t = blockIdx.x;
@@ -47,6 +46,11 @@ __global__ __launch_bounds__(MIX_NT) void mix_kernel(const UpdateTables* __restr
     P = pairs[lo];
   }
   __syncthreads();
+  const UpdateTables* tab = tabs + P.upd;
+  const int d = tab->d;
+  const int* tidx = tidxs + (int64_t)P.upd * d * d * d * d;
+  const cplx* u3 = u3s + tab->gate_off;
+  const double* lam_r = lam_all + (int64_t)(tab->mode + 2) * tab->chi;
   const int D0 = P.a0 - P.b0 + 1, D1 = P.a1 - P.b1 + 1;
   // per-box tables: index i0 <-> charge b0 + i0, i1 <-> b1 + i1
   if (tid < MD * MD) {
@@ -188,12 +192,16 @@ __device__ T block_sum(T v, T* red) {
   return r;
 }
 
-__global__ __launch_bounds__(SEL_NT) void select_kernel(const UpdateTables* __restrict__ tab,
-                                                        SectorDesc* __restrict__ sd, int ns,
+__global__ __launch_bounds__(SEL_NT) void select_kernel(const UpdateTables* __restrict__ tabs,
+                                                        SectorDesc* __restrict__ sds, int n_sectors,
                                                         const double* __restrict__ sig,
                                                         double* __restrict__ keys, double cutoff,
-                                                        int chi, int* __restrict__ kept_out,
-                                                        double* __restrict__ trunc_out) {
+                                                        int chi, int* __restrict__ kept_all,
+                                                        double* __restrict__ trunc_all) {
+  const UpdateTables* tab = tabs + blockIdx.x;
+  const int sec0 = tab->sec0, ns = tab->n_sectors;
+  SectorDesc* sd = sds + sec0;
+  int* kept_out = kept_all + sec0;
   __shared__ double redd[SEL_NT];
   __shared__ long long redi[SEL_NT];
   __shared__ int kept_s[BSMPO_MAX_Q];
@@ -205,7 +213,7 @@ __global__ __launch_bounds__(SEL_NT) void select_kernel(const UpdateTables* __re
   if (own) { k = sd[s].k; off = sd[s].s_off; }
   // keys: singular values made equal within ket/bra-swapped sector pairs
   if (own) {
-    const int p = tab->pair_of[s];
+    const int p = tab->pair_of[s] - sec0;
     int kp = 0;
     int64_t poff = 0;
     if (p >= 0 && p != s) { kp = sd[p].k; poff = sd[p].s_off; }
@@ -266,7 +274,7 @@ __global__ __launch_bounds__(SEL_NT) void select_kernel(const UpdateTables* __re
   __syncthreads();
   // a cut inside a degenerate swapped pair keeps neither member
   if (own) {
-    const int p = tab->pair_of[s];
+    const int p = tab->pair_of[s] - sec0;
     if (p >= 0 && p != s) kept = min(kept, kept_s[p]);
   }
   __syncthreads();
@@ -285,8 +293,8 @@ __global__ __launch_bounds__(SEL_NT) void select_kernel(const UpdateTables* __re
       kept_out[i] = kept_s[i];
       slot += kept_s[i];
     }
-    kept_out[ns] = slot;
-    trunc_out[0] = tw;
+    kept_all[n_sectors + blockIdx.x] = slot;
+    trunc_all[blockIdx.x] = tw;
   }
 }
 
@@ -312,18 +320,25 @@ __global__ void extract_v_kernel(const SectorDesc* __restrict__ sd, const cplx* 
 
 constexpr int SC_NT = 256;
 
-__global__ __launch_bounds__(SC_NT) void scatter_kernel(const UpdateTables* __restrict__ tab,
-                                                        const SectorDesc* __restrict__ sd, int ns,
-                                                        int total_kept,
-                                                        const int2* __restrict__ charge_l,
-                                                        const int2* __restrict__ charge_r,
+__global__ __launch_bounds__(SC_NT) void scatter_kernel(const UpdateTables* __restrict__ tabs,
+                                                        const SectorDesc* __restrict__ sds,
+                                                        const int* __restrict__ totals,
                                                         const cplx* __restrict__ vbuf,
                                                         const cplx* __restrict__ wbuf,
                                                         const double* __restrict__ sig,
-                                                        cplx* __restrict__ gamma_l,
-                                                        cplx* __restrict__ gamma_r,
-                                                        double* __restrict__ lam_c,
-                                                        int2* __restrict__ charge_c) {
+                                                        cplx* __restrict__ gamma,
+                                                        double* __restrict__ lam,
+                                                        int2* __restrict__ charge) {
+  const UpdateTables* tab = tabs + blockIdx.y;
+  const SectorDesc* sd = sds + tab->sec0;
+  const int ns = tab->n_sectors, total_kept = totals[blockIdx.y];
+  const int64_t site = (int64_t)tab->chi * tab->chi;
+  cplx* gamma_l = gamma + tab->mode * site;
+  cplx* gamma_r = gamma_l + site;
+  const int2* charge_l = charge + (int64_t)tab->mode * tab->chi;
+  int2* charge_c = charge + (int64_t)(tab->mode + 1) * tab->chi;
+  const int2* charge_r = charge + (int64_t)(tab->mode + 2) * tab->chi;
+  double* lam_c = lam + (int64_t)(tab->mode + 1) * tab->chi;
   __shared__ int slot0[BSMPO_MAX_Q + 1];
   __shared__ SectorDesc S[BSMPO_MAX_Q];
   const int tid = threadIdx.x;
@@ -409,7 +424,7 @@ __global__ void phase_kernel(int d, int chi, double phi, const int2* __restrict_
 cudaError_t launch_mix_d(int d, const UpdateTables* tab_dev, const int* tidx_dev,
                          const ThetaDesc* td_dev, const SectorDesc* sd_dev,
                          const MixPair* pairs_dev, int n_pairs, int total_tiles, const void* u3,
-                         const void* theta, const double* lam_r, void* cbuf, void* abuf,
+                         const void* theta, const double* lam, void* cbuf, void* abuf,
                          cudaStream_t s) {
   if (total_tiles <= 0) return cudaSuccess;
   const cplx* U = reinterpret_cast<const cplx*>(u3);
@@ -418,7 +433,7 @@ cudaError_t launch_mix_d(int d, const UpdateTables* tab_dev, const int* tidx_dev
   cplx* A = reinterpret_cast<cplx*>(abuf);
 #define BSMPO_MIX(MD)                                                                        \
   mix_kernel<MD><<<total_tiles, MIX_NT, 0, s>>>(tab_dev, tidx_dev, td_dev, sd_dev, pairs_dev, \
-                                                n_pairs, U, T, lam_r, C, A)
+                                                n_pairs, U, T, lam, C, A)
   switch (d) {
     case 1: case 2: BSMPO_MIX(2); break;
     case 3: BSMPO_MIX(3); break;
@@ -439,11 +454,12 @@ cudaError_t launch_identity_rows(const SectorDesc* sd_dev, int n_sectors, int ma
   return cudaGetLastError();
 }
 
-cudaError_t launch_select(const UpdateTables* tab_dev, SectorDesc* sd_dev, int n_sectors,
+cudaError_t launch_select(const UpdateTables* tab_dev, SectorDesc* sd_dev, int n_updates, int n_sectors,
                           const double* sig, double* keys, double cutoff, int chi, int* kept_out,
                           double* trunc_out, cudaStream_t s) {
-  select_kernel<<<1, SEL_NT, 0, s>>>(tab_dev, sd_dev, n_sectors, sig, keys, cutoff, chi,
-                                     kept_out, trunc_out);
+  if (n_updates <= 0) return cudaSuccess;
+  select_kernel<<<n_updates, SEL_NT, 0, s>>>(tab_dev, sd_dev, n_sectors, sig, keys, cutoff, chi, kept_out,
+                                             trunc_out);
   return cudaGetLastError();
 }
 
@@ -457,17 +473,15 @@ cudaError_t launch_extract_v(const SectorDesc* sd_dev, int n_sectors, int max_el
   return cudaGetLastError();
 }
 
-cudaError_t launch_scatter(const UpdateTables* tab_dev, const SectorDesc* sd_dev, int n_sectors,
-                           int total_kept, int chi, const int* charge_l, const int* charge_r,
-                           const void* vbuf, const void* wbuf, const double* sig, void* gamma_l,
-                           void* gamma_r, double* lam_c, int* charge_c, cudaStream_t s) {
+cudaError_t launch_scatter(const UpdateTables* tab_dev, const SectorDesc* sd_dev, int n_updates,
+                           const int* totals, int chi, const void* vbuf, const void* wbuf,
+                           const double* sig, void* gamma, double* lam, int* charge, cudaStream_t s) {
+  if (n_updates <= 0) return cudaSuccess;
   const int64_t total = 2 * (int64_t)chi * chi + chi;
   const int blocks = (int)std::min<int64_t>((total + SC_NT - 1) / SC_NT, 148 * 16);
-  scatter_kernel<<<blocks, SC_NT, 0, s>>>(
-      tab_dev, sd_dev, n_sectors, total_kept, reinterpret_cast<const int2*>(charge_l),
-      reinterpret_cast<const int2*>(charge_r), reinterpret_cast<const cplx*>(vbuf),
-      reinterpret_cast<const cplx*>(wbuf), sig, reinterpret_cast<cplx*>(gamma_l),
-      reinterpret_cast<cplx*>(gamma_r), lam_c, reinterpret_cast<int2*>(charge_c));
+  scatter_kernel<<<dim3(blocks, n_updates), SC_NT, 0, s>>>(
+      tab_dev, sd_dev, totals, reinterpret_cast<const cplx*>(vbuf), reinterpret_cast<const cplx*>(wbuf), sig,
+      reinterpret_cast<cplx*>(gamma), lam, reinterpret_cast<int2*>(charge));
   return cudaGetLastError();
 }
 

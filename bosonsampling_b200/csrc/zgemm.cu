@@ -23,7 +23,8 @@ __global__ __launch_bounds__(NT) void zgemm_grouped_kernel(const cplx* __restric
                                                            cplx* __restrict__ C,
                                                            const double* __restrict__ scale,
                                                            const GemmGroup* __restrict__ groups,
-                                                           int n_groups) {
+                                                           int n_groups,
+                                                           const SectorDesc* __restrict__ sd) {
   __shared__ double2 As[TK][TM + 1];
   __shared__ double2 Bs[TK][TN + 1];
   __shared__ GemmGroup g;
@@ -36,12 +37,18 @@ __global__ __launch_bounds__(NT) void zgemm_grouped_kernel(const cplx* __restric
       if (groups[mid].tile_start <= t) lo = mid; else hi = mid - 1;
     }
     g = groups[lo];
+    if (g.sec >= 0) {
+      const int kept = sd[g.sec].kept;
+      if (g.kdim == 1) { g.M = kept; g.lda = kept; }
+      else { g.N = kept; g.ldb = kept; g.ldc = kept; }
+    }
   }
   __syncthreads();
   const int tile = blockIdx.x - g.tile_start;
   const int m0 = (tile / g.tiles_n) * TM;
   const int n0 = (tile % g.tiles_n) * TN;
   const int M = g.M, N = g.N, K = g.K;
+  if (m0 >= M || n0 >= N) return;   // tiles are laid out for the host's bound
   const cplx* a = A + g.a_off;
   const cplx* b = B + g.b_off;
   const double* ks = g.ks_off >= 0 ? scale + g.ks_off : nullptr;
@@ -150,10 +157,10 @@ int zgemm_tile_n() { return TN; }
 
 cudaError_t launch_zgemm_grouped(const void* a, const void* b, void* c, const double* scale,
                                  const GemmGroup* groups_dev, int n_groups, int total_tiles,
-                                 cudaStream_t s) {
+                                 const SectorDesc* sd_dev, cudaStream_t s) {
   if (total_tiles <= 0 || n_groups <= 0) return cudaSuccess;
   zgemm_grouped_kernel<<<total_tiles, NT, 0, s>>>(
       reinterpret_cast<const cplx*>(a), reinterpret_cast<const cplx*>(b),
-      reinterpret_cast<cplx*>(c), scale, groups_dev, n_groups);
+      reinterpret_cast<cplx*>(c), scale, groups_dev, n_groups, sd_dev);
   return cudaGetLastError();
 }
