@@ -75,14 +75,13 @@ struct bsmpo_ctx {
   // host mirror of block sizes: cnt[b * d*d + c0*d + c1]
   std::vector<int> cnt;
   // workspaces
-  DevBuf theta, cbuf, abuf, wbuf, vbuf, sig, keys, perm, tab, tab2, rot, kept, u3, m4, env_l,
+  DevBuf theta, cbuf, abuf, wbuf, vbuf, sig, keys, perm, tab, tab2, rot, u3, m4, env_l,
       env_r, part, outv, dims, nf2, qbuf, qflag, pbuf, pcnt;
   // Gram / eigen route of the sector SVD (precision != BSMPO_PRECISION_FP64)
   DevBuf gbuf, eigd, taub, invsig, escr, swp, zbuf, ybuf;
   // tensor-core contractions (BSMPO_PRECISION_TF32X3): groups and tensor maps of the
-  // V / W GEMMs, and the pipeline's error word
-  DevBuf tab3, tcerr;
-  DevBuf jwork;   // executed Jacobi rows: pair-Gram rows, rotated rows (unsigned long long[2])
+  // V / W GEMMs
+  DevBuf tab3;
   HostStage stage3;
   int precision = BSMPO_PRECISION_FP64;
   // the tridiagonalisation's size classes run side by side: three more streams, forked
@@ -259,7 +258,10 @@ struct Plan {
   std::vector<GemmGroup> gg;
   std::vector<GemmGroup> ggram;   // Gram G_s = X^H X of every sector (Gram route)
   std::vector<GemmGroup> gv, gw;  // V = T Y diag(1/sigma) (Gram route, X = T) and W = V^H C
-  std::vector<int> tdlist;        // sectors by tridiagonalisation size class (Gram route)
+  // sectors by tridiagonalisation size class (Gram route); the small sectors, then the
+  // others (Jacobi)
+  std::vector<int> tdlist;
+  int n_small = 0, small_elems = 0, small_k = 0, big_k = 0;
   std::vector<TcGroup> tcg;       // Theta groups on the tensor cores (TF32X3)
   std::vector<unsigned char> tcmaps;   // two tensor maps per update (Gamma_L, Gamma_R)
   int tc_tiles = 0;
@@ -447,14 +449,14 @@ int add_update(bsmpo_ctx* h, int mode, int64_t gate_off, Plan& P) {
           std::memset(&g, 0, sizeof(g));
           g.M = nrow; g.N = ncol; g.K = nk;
           g.lda = h->chi; g.ldb = h->chi; g.ldc = ncol;
-          g.opA = 0; g.opB = 0; g.beta = 0; g.sec = -1;
+          g.opA = 0; g.sec = -1;
           g.tiles_n = ceil_div(ncol, TNt);
           g.tile_start = P.gemm_tiles;
           P.gemm_tiles += ceil_div(nrow, TMt) * g.tiles_n;
           g.a_off = (int64_t)mode * chi2 + (int64_t)D.row0 * h->chi + D.k0;
           g.b_off = (int64_t)(mode + 1) * chi2 + (int64_t)D.k0 * h->chi + D.col0;
           g.c_off = D.off;
-          g.ks_off = g.rs_off = g.cs_off = -1;
+          g.cs_off = -1;
           P.gg.push_back(g);
         }
       }
@@ -493,7 +495,7 @@ int add_update(bsmpo_ctx* h, int mode, int64_t gate_off, Plan& P) {
     g.tile_start = P.w_tiles;
     P.w_tiles += ceil_div(S.k, TMt) * g.tiles_n;
     g.a_off = S.v_off; g.b_off = S.c_off; g.c_off = S.w_off;
-    g.ks_off = g.rs_off = g.cs_off = -1;
+    g.cs_off = -1;
     P.gw.push_back(g);
     if (P.gram) {
       // Gram G_s = X^H X, X = the first rows_g rows of the sector's Jacobi matrix
@@ -502,12 +504,12 @@ int add_update(bsmpo_ctx* h, int mode, int64_t gate_off, Plan& P) {
       std::memset(&r, 0, sizeof(r));
       r.M = S.k; r.N = S.k; r.K = S.rows_g;
       r.lda = S.k; r.ldb = S.k; r.ldc = S.k;
-      r.opA = 1; r.sec = -1;
+      r.opA = 1; r.herm = 1; r.sec = -1;
       r.tiles_n = ceil_div(S.k, TNt);
       r.tile_start = P.gram_tiles;
       P.gram_tiles += ceil_div(S.k, TMt) * r.tiles_n;
       r.a_off = S.a_off; r.b_off = S.a_off; r.c_off = S.g_off;
-      r.ks_off = r.rs_off = r.cs_off = -1;
+      r.cs_off = -1;
       P.ggram.push_back(r);
       if (!S.left) {
         // V [m][kept] = T [m][k] Y [k][kept] diag(1 / sigma)
@@ -520,7 +522,6 @@ int add_update(bsmpo_ctx* h, int mode, int64_t gate_off, Plan& P) {
         v.tile_start = P.v_tiles;
         P.v_tiles += ceil_div(S.m, TMt) * v.tiles_n;
         v.a_off = S.a_off; v.b_off = S.y_off; v.c_off = S.v_off;
-        v.ks_off = v.rs_off = -1;
         v.cs_off = S.s_off;
         P.gv.push_back(v);
       }
@@ -547,9 +548,18 @@ void finish_plan(bsmpo_ctx* h, Plan& P) {
   }
   const int JBc = jacobi_block_cols();
   const int rmax = std::min(h->jac_rows, jacobi_rows_per_part());
+  std::vector<int> big;
   for (int s = 0; s < ns; ++s) {
     const SectorDesc& S = P.sd[s];
     if (S.left) P.max_left_m2 = std::max(P.max_left_m2, S.m * S.m);
+    if (jacobi_is_small(S.rows_tot, S.k)) {
+      P.tdlist.push_back(s);
+      P.small_elems = std::max(P.small_elems, jacobi_small_elems(S.rows_tot, S.k));
+      P.small_k = std::max(P.small_k, S.k);
+      continue;
+    }
+    big.push_back(s);
+    P.big_k = std::max(P.big_k, S.k);
     JacobiWork w;
     std::memset(&w, 0, sizeof(w));
     w.sector = s;
@@ -566,16 +576,41 @@ void finish_plan(bsmpo_ctx* h, Plan& P) {
     P.max_rounds = std::max(P.max_rounds, w.rounds);
     P.jw.push_back(w);
   }
+  // the most work first
+  std::stable_sort(P.tdlist.begin(), P.tdlist.end(), [&](int x, int y) {
+    return (int64_t)P.sd[x].k * P.sd[x].k * P.sd[x].rows_tot > (int64_t)P.sd[y].k * P.sd[y].k * P.sd[y].rows_tot;
+  });
+  P.n_small = (int)P.tdlist.size();
+  P.tdlist.insert(P.tdlist.end(), big.begin(), big.end());
   std::vector<JacobiWork> all(P.jw);
   jacobi_launch_list(all, &P.gram_ctas, &P.apply_ctas, &P.jac_slots);
 }
 
 // packs plan tables into the pinned stage and copies them to the device table buffer
 struct TabLayout {
-  size_t tab, tidx, td, sd, pairs, gg, ggram, gv, gw, tdlist, tcmaps, tcg, jw, total;
+  size_t tab, tidx, td, sd, pairs, gg, ggram, gv, gw, tdlist, tcmaps, tcg, jw, res, total;
 };
 
-TabLayout layout_of(const Plan& P) {
+// The words that come back from the device at the end of a group's update, at L.res of the
+// table buffer (zeroed with the upload of the tables).
+struct ResLayout {
+  size_t kept, trunc, err, work, total;
+  size_t rot;   // host only: the Jacobi polls' counters
+};
+
+ResLayout result_layout(int ns, int nj) {
+  ResLayout R;
+  R.kept = 0;                                                  // int[ns] kept, int[nj] totals
+  R.trunc = align_up((size_t)(ns + nj) * sizeof(int), 16);     // double[nj]
+  R.err = R.trunc + nj * sizeof(double);                       // int: a pipeline wait expired; int: no convergence
+  // unsigned long long[4]: pair-Gram rows, rotated rows; small sectors: complex MACs, sweeps
+  R.work = align_up(R.err + 2 * sizeof(int), 16);
+  R.total = R.work + 4 * sizeof(unsigned long long);
+  R.rot = align_up(R.total, 256);                              // 2 x int[3 ns]
+  return R;
+}
+
+TabLayout layout_of(const Plan& P, const ResLayout& R) {
   TabLayout L;
   size_t o = 0;
   auto place = [&](size_t bytes) {
@@ -596,24 +631,9 @@ TabLayout layout_of(const Plan& P) {
   L.tcmaps = place(P.tcmaps.size());
   L.tcg = place(P.tcg.size() * sizeof(TcGroup));
   L.jw = place(P.jw.size() * sizeof(JacobiWork));
+  L.res = place(R.total);
   L.total = o;
   return L;
-}
-
-// The pinned words that come back from the device during a group's update.
-struct ResLayout {
-  size_t kept, trunc, err, work, rot, total;
-};
-
-ResLayout result_layout(int ns, int nj) {
-  ResLayout R;
-  R.kept = 0;                                                    // int[ns] kept, int[nj] totals
-  R.trunc = align_up((size_t)(ns + nj) * sizeof(int), 256);      // double[nj]
-  R.err = align_up(R.trunc + nj * sizeof(double), 256);          // int
-  R.work = R.err + 256;                                          // unsigned long long[2]
-  R.rot = R.work + 256;                                          // 2 x int[3 ns]
-  R.total = align_up(R.rot + (size_t)6 * ns * sizeof(int), 256);
-  return R;
 }
 
 template <typename T>
@@ -732,26 +752,49 @@ int gram_timing(bsmpo_ctx* h, const Plan& P) {
   return BSMPO_OK;
 }
 
-// 3b. Blocked one-sided Jacobi of every sector of the group.
-int jacobi_svd(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, char* jw_d, const ResLayout& R) {
-  const int ns = (int)P.sd.size();
+// 3b. One-sided Jacobi of every sector of the group: the small sectors in one launch, the
+// others in blocked rounds.
+int jacobi_svd(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, char* jw_d, const int* list_d, char* res_d,
+               const ResLayout& R) {
+  const int ns = (int)P.sd.size(), n_big = (int)P.jw.size();
   cudaStream_t st = h->stream;
   int rc;
   char* hres = static_cast<char*>(h->hres.p);
-  const size_t pair_elems = (size_t)4 * jacobi_block_cols() * jacobi_block_cols();
+  unsigned long long* work_d = reinterpret_cast<unsigned long long*>(res_d + R.work);
   if ((rc = grow(h, h->perm, std::max<int64_t>(P.s_elems, 1) * sizeof(int)))) return rc;
+  double* sig = reinterpret_cast<double*>(h->sig.p);
+  int* perm = reinterpret_cast<int*>(h->perm.p);
+  if (h->timing) CK(h, cudaEventRecord(h->ev0, st));
+  // beside the blocked rounds, where there are any, on the first side stream
+  cudaStream_t small_st = st;
+  if (P.n_small && n_big && h->td_fork > 0) {
+    if ((rc = make_fork_streams(h))) return rc;
+    if (h->n_aux > 0) {
+      small_st = h->aux[0];
+      CK(h, cudaEventRecord(h->fork_ev, st));
+      CK(h, cudaStreamWaitEvent(small_st, h->fork_ev, 0));
+    }
+  }
+  if (P.n_small)
+    CKL(h, launch_jacobi_small(sd_d, list_d, P.n_small, P.small_elems, P.small_k, h->abuf.p, MAX_SWEEPS, sig, perm,
+                               reinterpret_cast<int*>(res_d + R.err) + 1, work_d + 2, small_st));
+  if (small_st != st) CK(h, cudaEventRecord(h->join_ev[0], small_st));
+  h->last_sweeps = 0;
+  if (!n_big) {
+    if (h->timing) CK(h, cudaEventRecord(h->ev1, st));
+    return BSMPO_OK;
+  }
+  const size_t pair_elems = (size_t)4 * jacobi_block_cols() * jacobi_block_cols();
   if ((rc = grow(h, h->rot, (size_t)3 * ns * sizeof(int)))) return rc;
   if ((rc = grow(h, h->nf2, (size_t)ns * sizeof(double)))) return rc;
   if ((rc = grow(h, h->qbuf, std::max(P.jac_slots, 1) * pair_elems * sizeof(cplx)))) return rc;
   if ((rc = grow(h, h->qflag, std::max(P.jac_slots, 1) * sizeof(int)))) return rc;
   if ((rc = grow(h, h->pcnt, std::max(P.jac_slots, 1) * sizeof(int)))) return rc;
   if ((rc = grow(h, h->pbuf, std::max(P.gram_ctas, 1) * pair_elems * sizeof(cplx)))) return rc;
-  if ((rc = grow(h, h->jwork, 2 * sizeof(unsigned long long)))) return rc;
   double* nf2 = reinterpret_cast<double*>(h->nf2.p);
-  CKL(h, launch_sector_norms(sd_d, ns, h->abuf.p, nf2, st));
+  CKL(h, launch_sector_norms(sd_d, list_d + P.n_small, n_big, h->abuf.p, nf2, st));
   CK(h, cudaMemsetAsync(h->rot.p, 0, (size_t)3 * ns * sizeof(int), st));
   CK(h, cudaMemsetAsync(h->pcnt.p, 0, std::max(P.jac_slots, 1) * sizeof(int), st));
-  CK(h, cudaMemsetAsync(h->jwork.p, 0, 2 * sizeof(unsigned long long), st));
   std::vector<JacobiWork> active(P.jw);
   int gram_ctas = 0, apply_ctas = 0, slots = 0;
   jacobi_launch_list(active, &gram_ctas, &apply_ctas, &slots);
@@ -770,8 +813,7 @@ int jacobi_svd(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, char* jw_d, 
   const int t_max = MAX_SWEEPS * std::max(1, P.max_rounds);
   bool converged = false;
   int checks = 0;
-  std::vector<int> conv_at(ns, -1);
-  if (h->timing) CK(h, cudaEventRecord(h->ev0, st));
+  std::vector<int> conv_at(n_big, -1);   // by entry of P.jw
   const int chunk = std::max(1, P.max_rounds);   // one sweep of the largest sector
   int t_after[2] = {0, 0};
   auto launch_chunk = [&](int slot) -> int {
@@ -781,7 +823,7 @@ int jacobi_svd(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, char* jw_d, 
                                 apply_ctas, t, h->abuf.p, reinterpret_cast<int*>(h->rot.p), nf2, 0.0, MAX_SWEEPS,
                                 h->pbuf.p, reinterpret_cast<int*>(h->pcnt.p), h->qbuf.p,
                                 reinterpret_cast<int*>(h->qflag.p),
-                                reinterpret_cast<unsigned long long*>(h->jwork.p), st));
+                                work_d, st));
       h->launches += 2;
     }
     CK(h, cudaMemcpyAsync(hrot_slot[slot], h->rot.p, (size_t)3 * ns * sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -798,21 +840,20 @@ int jacobi_svd(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, char* jw_d, 
     ++checks;
     const int* hrot = hrot_slot[cur];
     bool all = true;
-    for (int s = 0; s < ns; ++s) {
+    for (int w = 0; w < n_big; ++w) {
       // a converged sector leaves the launches, and its counters are stale from then on
-      if (conv_at[s] >= 0) continue;
-      const int Rn = P.jw[s].rounds;
-      const int done = t_after[cur] / Rn;
-      if (done < 1 || hrot[3 * s + (done - 1) % 3] != 0) { all = false; continue; }
-      conv_at[s] = done;
+      if (conv_at[w] >= 0) continue;
+      const int done = t_after[cur] / P.jw[w].rounds;
+      if (done < 1 || hrot[3 * P.jw[w].sector + (done - 1) % 3] != 0) { all = false; continue; }
+      conv_at[w] = done;
     }
     if (all) { converged = true; break; }
     if (!more) break;
     // drop converged sectors (and those out of sweeps) from the launches after the queued
     // chunk: the table copy is stream-ordered after it
     std::vector<JacobiWork> next;
-    for (const auto& w : P.jw)
-      if (conv_at[w.sector] < 0 && t / w.rounds < MAX_SWEEPS) next.push_back(w);
+    for (int w = 0; w < n_big; ++w)
+      if (conv_at[w] < 0 && t / P.jw[w].rounds < MAX_SWEEPS) next.push_back(P.jw[w]);
     if (next.size() < active.size() && !next.empty()) {
       active.swap(next);
       jacobi_launch_list(active, &gram_ctas, &apply_ctas, &slots);
@@ -822,49 +863,43 @@ int jacobi_svd(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, char* jw_d, 
     }
     cur ^= 1;
   }
-  if (h->timing) {
-    CK(h, cudaMemcpyAsync(hres + R.work, h->jwork.p, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    CK(h, cudaEventRecord(h->ev1, st));
-  }
+  if (small_st != st) CK(h, cudaStreamWaitEvent(st, h->join_ev[0], 0));
+  if (h->timing) CK(h, cudaEventRecord(h->ev1, st));
   // sweeps the slowest sector needed (its last one without rotations included); t also
   // counts the chunk queued after convergence, whose rounds exit at once
-  {
-    int sw = 0;
-    for (int s = 0; s < ns; ++s) sw = std::max(sw, conv_at[s] >= 0 ? conv_at[s] : t / P.jw[s].rounds);
-    h->last_sweeps = sw;
-  }
+  for (int w = 0; w < n_big; ++w)
+    h->last_sweeps = std::max(h->last_sweeps, conv_at[w] >= 0 ? conv_at[w] : t / P.jw[w].rounds);
   h->jacobi_rounds += t;   // launched rounds, including the drained chunk
-  if (h->timing) {
-    float ms = 0.f;
-    CK(h, cudaEventSynchronize(h->ev1));
-    CK(h, cudaEventElapsedTime(&ms, h->ev0, h->ev1));
-    h->jac_ms += ms;
-    h->jac_launches += t;
-    // flops of the executed work, counted on the device: every row that formed a
-    // partial pair Gram contributes its 10 upper 8 x 8 tiles (640 complex MACs), every
-    // rotated row 32 x 32 complex MACs; 8 flops per complex MAC.  Pairs that did not
-    // rotate and sectors that had converged do no apply work and are not counted.
-    const unsigned long long* hw = reinterpret_cast<const unsigned long long*>(hres + R.work);
-    h->jac_flops += 8.0 * 640.0 * (double)hw[0] + 8.0 * 1024.0 * (double)hw[1];
-  }
+  if (h->timing) h->jac_launches += t;
   if (!converged) {
     std::string msg = "Jacobi SVD did not converge";
-    for (const UpdateTables& T : P.tab)
-      for (int i = 0; i < T.n_sectors; ++i) {
-        const int s = T.sec0 + i;
-        if (conv_at[s] >= 0) continue;
-        const int Rn = P.jw[s].rounds, done = t_after[cur] / Rn;
-        const SectorDesc& S = P.sd[s];
-        msg += " (mode " + std::to_string(T.mode) + "); sector (" + std::to_string(S.cc0) + "," +
-               std::to_string(S.cc1) + ") m=" + std::to_string(S.m) + " n=" + std::to_string(S.n) +
-               " sweeps=" + std::to_string(done) + " rotations=" +
-               std::to_string(hrot_slot[cur][3 * s + (done - 1 + 3) % 3]);
-        return fail(h, BSMPO_ECONVERGE, msg);
-      }
+    for (int w = 0; w < n_big; ++w) {
+      if (conv_at[w] >= 0) continue;
+      const int sec = P.jw[w].sector, done = t_after[cur] / P.jw[w].rounds;
+      const SectorDesc& S = P.sd[sec];
+      int mode = 0;
+      for (const UpdateTables& T : P.tab)
+        if (sec >= T.sec0) mode = T.mode;
+      msg += " (mode " + std::to_string(mode) + "); sector (" + std::to_string(S.cc0) + "," + std::to_string(S.cc1) +
+             ") m=" + std::to_string(S.m) + " n=" + std::to_string(S.n) + " sweeps=" + std::to_string(done) +
+             " rotations=" + std::to_string(hrot_slot[cur][3 * sec + (done - 1 + 3) % 3]);
+      break;
+    }
     return fail(h, BSMPO_ECONVERGE, msg);
   }
-  CKL(h, launch_jacobi_finish(sd_d, ns, P.max_k, h->abuf.p, nf2, reinterpret_cast<double*>(h->sig.p),
-                              reinterpret_cast<int*>(h->perm.p), st));
+  CKL(h, launch_jacobi_finish(sd_d, list_d + P.n_small, n_big, P.big_k, h->abuf.p, nf2, sig, perm, st));
+  return BSMPO_OK;
+}
+
+// The Jacobi route's timing likewise, from the work counted on the device: every row that
+// formed a partial pair Gram contributes its 10 upper 8 x 8 tiles (640 complex MACs), every
+// rotated row 32 x 32, the small sectors' kernel counts MACs; 8 flops per complex MAC.  Pairs
+// that did not rotate and sectors that had converged do no apply work and are not counted.
+int jacobi_timing(bsmpo_ctx* h, const unsigned long long* w) {
+  float ms = 0.f;
+  CK(h, cudaEventElapsedTime(&ms, h->ev0, h->ev1));
+  h->jac_ms += ms;
+  h->jac_flops += 8.0 * (640.0 * (double)w[0] + 1024.0 * (double)w[1] + (double)w[2]);
   return BSMPO_OK;
 }
 
@@ -944,13 +979,11 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
   if ((rc = grow(h, h->vbuf, std::max<int64_t>(P.v_elems, 1) * sizeof(cplx)))) return rc;
   if ((rc = grow(h, h->sig, std::max<int64_t>(P.s_elems, 1) * sizeof(double)))) return rc;
   if ((rc = grow(h, h->keys, std::max<int64_t>(P.s_elems, 1) * sizeof(double)))) return rc;
-  const size_t kept_bytes = align_up((size_t)(ns + nj) * sizeof(int), 256);
-  if ((rc = grow(h, h->kept, kept_bytes + nj * sizeof(double)))) return rc;
-  const TabLayout L = layout_of(P);
   const ResLayout R = result_layout(ns, nj);
+  const TabLayout L = layout_of(P, R);
   if ((rc = grow(h, h->tab, L.total))) return rc;
   if ((rc = grow_host(h, h->stage, L.total))) return rc;
-  if ((rc = grow_host(h, h->hres, R.total))) return rc;
+  if ((rc = grow_host(h, h->hres, R.rot + (size_t)6 * ns * sizeof(int)))) return rc;
   char* hs = static_cast<char*>(h->stage.p);
   put(hs, L.tab, P.tab);
   put(hs, L.tidx, P.tidx);
@@ -970,6 +1003,7 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
     jacobi_launch_list(active, &a, &b, &c);
     put(hs, L.jw, active);
   }
+  std::memset(hs + L.res, 0, R.total);
   char* dt = static_cast<char*>(h->tab.p);
   CK(h, cudaMemcpyAsync(dt, hs, L.total, cudaMemcpyHostToDevice, st));
   const UpdateTables* tab_d = reinterpret_cast<const UpdateTables*>(dt + L.tab);
@@ -980,13 +1014,11 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
   auto groups_at = [&](size_t off) { return reinterpret_cast<const GemmGroup*>(dt + off); };
   const bool tc = h->precision == BSMPO_PRECISION_TF32X3;
   const bool tc_theta = tc && (h->tc_mask & 1), tc_w = tc && (h->tc_mask & 2);
-  // error word of the asynchronous pipelines (tensor-core GEMM, streamed
-  // tridiagonalisation): set on the device when a bounded wait expires
-  if (!h->tcerr.p) {
-    if ((rc = grow(h, h->tcerr, sizeof(int)))) return rc;
-    CK(h, cudaMemsetAsync(h->tcerr.p, 0, sizeof(int), st));
-  }
-  int* tcerr_d = reinterpret_cast<int*>(h->tcerr.p);
+  // results of the group; the error word of the asynchronous pipelines (tensor-core GEMM,
+  // streamed tridiagonalisation) is set on the device when a bounded wait expires
+  char* res_d = dt + L.res;
+  int* tcerr_d = reinterpret_cast<int*>(res_d + R.err);
+  const int* list_d = reinterpret_cast<const int*>(dt + L.tdlist);
 
   if ((rc = clk.mark(0))) return rc;
   // 1. Theta_q = Glc[a, q] Gcr[q, b] for every valid triple
@@ -1008,18 +1040,17 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
   const int* hk = reinterpret_cast<const int*>(hres + R.kept);
   const double* htw = reinterpret_cast<const double*>(hres + R.trunc);
   const int* htc = reinterpret_cast<const int*>(hres + R.err);
-  int* kept_d = reinterpret_cast<int*>(h->kept.p);
-  double* trunc_d = reinterpret_cast<double*>(static_cast<char*>(h->kept.p) + kept_bytes);
+  const unsigned long long* hwork = reinterpret_cast<const unsigned long long*>(hres + R.work);
+  int* kept_d = reinterpret_cast<int*>(res_d + R.kept);
+  double* trunc_d = reinterpret_cast<double*>(res_d + R.trunc);
   if (!h->wait_ev) CK(h, cudaEventCreateWithFlags(&h->wait_ev, cudaEventBlockingSync | cudaEventDisableTiming));
-  rc = P.gram ? gram_eigenvalues(h, P, sd_d, groups_at(L.ggram), reinterpret_cast<const int*>(dt + L.tdlist), tcerr_d)
-              : jacobi_svd(h, P, sd_d, dt + L.jw, R);
+  rc = P.gram ? gram_eigenvalues(h, P, sd_d, groups_at(L.ggram), list_d, tcerr_d)
+              : jacobi_svd(h, P, sd_d, dt + L.jw, list_d, res_d, R);
   if (rc || (rc = clk.mark(3))) return rc;
   auto select = [&]() -> int {
     CKL(h, launch_select(tab_d, sd_d, nj, ns, reinterpret_cast<double*>(h->sig.p),
                          reinterpret_cast<double*>(h->keys.p), h->cutoff, chi, kept_d, trunc_d, st));
-    CK(h, cudaMemcpyAsync(hres + R.kept, kept_d, (size_t)(ns + nj) * sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(h, cudaMemcpyAsync(hres + R.trunc, trunc_d, nj * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CK(h, cudaMemcpyAsync(hres + R.err, tcerr_d, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(h, cudaMemcpyAsync(hres, res_d, R.total, cudaMemcpyDeviceToHost, st));
     CK(h, cudaEventRecord(h->wait_ev, st));
     return BSMPO_OK;
   };
@@ -1035,13 +1066,16 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
       std::vector<JacobiWork> active(J.jw);
       int a, b, c;
       jacobi_launch_list(active, &a, &b, &c);
-      const size_t bytes = std::max<size_t>(active.size(), 1) * sizeof(JacobiWork);
+      const size_t jbytes = align_up(active.size() * sizeof(JacobiWork) + 1, 256);
+      const size_t bytes = jbytes + J.tdlist.size() * sizeof(int);
       if ((rc = grow(h, h->tab2, bytes))) return rc;
       if ((rc = grow_host(h, h->stage3, bytes))) return rc;
       put(h->stage3.p, 0, active);
-      CK(h, cudaMemcpyAsync(h->tab2.p, h->stage3.p, bytes, cudaMemcpyHostToDevice, st));
+      put(h->stage3.p, jbytes, J.tdlist);
+      char* t2 = static_cast<char*>(h->tab2.p);
+      CK(h, cudaMemcpyAsync(t2, h->stage3.p, bytes, cudaMemcpyHostToDevice, st));
       CKL(h, launch_identity_rows(sd_d, ns, J.max_left_m2, h->abuf.p, st));
-      if ((rc = jacobi_svd(h, J, sd_d, static_cast<char*>(h->tab2.p), R))) return rc;
+      if ((rc = jacobi_svd(h, J, sd_d, t2, reinterpret_cast<const int*>(t2 + jbytes), res_d, R))) return rc;
       P.gram = false;
       if ((rc = select())) return rc;
     }
@@ -1088,8 +1122,10 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
   CK(h, cudaEventSynchronize(h->wait_ev));
   if (*htc != 0)
     return fail(h, BSMPO_ECUDA, "tensor-core GEMM or tridiagonalisation: a pipeline wait expired (error word set)");
+  if (htc[1] != 0) return fail(h, BSMPO_ECONVERGE, "Jacobi SVD did not converge (a small sector)");
   h->route_count[P.gram ? 1 : 0] += nj;
-  if (P.gram && h->timing && (rc = gram_timing(h, P))) return rc;
+  if (!P.gram) h->last_sweeps = std::max(h->last_sweeps, (int)hwork[3]);
+  if (h->timing && (rc = P.gram ? gram_timing(h, P) : jacobi_timing(h, hwork))) return rc;
   // host mirror, truncation weights, and the diagnostics of the group's last update
   for (int j = 0; j < nj; ++j) {
     const UpdateTables& T = P.tab[j];
@@ -1157,10 +1193,10 @@ M8 transpose_to_m8(const double* S) {
 
 void free_workspaces(bsmpo_ctx* h) {
   DevBuf* bufs[] = {&h->theta, &h->cbuf, &h->abuf, &h->wbuf, &h->vbuf, &h->sig, &h->keys,
-                    &h->perm, &h->tab, &h->tab2, &h->rot, &h->kept, &h->u3, &h->m4,
+                    &h->perm, &h->tab, &h->tab2, &h->rot, &h->u3, &h->m4,
                     &h->env_l, &h->env_r, &h->part, &h->outv, &h->dims, &h->nf2, &h->qbuf,
                     &h->qflag, &h->pbuf, &h->pcnt, &h->gbuf, &h->eigd, &h->taub, &h->invsig,
-                    &h->escr, &h->swp, &h->zbuf, &h->ybuf, &h->tab3, &h->tcerr, &h->jwork};
+                    &h->escr, &h->swp, &h->zbuf, &h->ybuf, &h->tab3};
   for (DevBuf* b : bufs)
     if (b->p) cudaFreeAsync(b->p, h->stream);
   cudaStreamSynchronize(h->stream);
@@ -1419,40 +1455,6 @@ int run_mesh_concurrent(bsmpo_ctx* h, int n_bs, const int* modes, const cplx* u3
     for (int q = 0; q < 8; ++q) w->stage_ms[q] = 0.0;
     if (w->last_index > best) { best = w->last_index; h->diag = w; }
   }
-  return BSMPO_OK;
-}
-
-int env_all(bsmpo_ctx* h) {
-  const int n = h->n, d = h->d, chi = h->chi, dd = d * d;
-  cudaStream_t st = h->stream;
-  int rc;
-  if ((rc = grow(h, h->env_l, (size_t)(n + 1) * chi * sizeof(cplx)))) return rc;
-  if ((rc = grow(h, h->env_r, (size_t)(n + 1) * chi * sizeof(cplx)))) return rc;
-  std::vector<int> dims(n + 1);
-  for (int b = 0; b <= n; ++b) {
-    int s = 0;
-    for (int q = 0; q < dd; ++q) s += h->cnt[(size_t)b * dd + q];
-    dims[b] = s;
-  }
-  if ((rc = grow(h, h->dims, (size_t)(n + 1) * sizeof(int)))) return rc;
-  if ((rc = grow_host(h, h->stage2, std::max<size_t>(h->stage2.bytes, (n + 1) * sizeof(int))))) return rc;
-  std::memcpy(h->stage2.p, dims.data(), (n + 1) * sizeof(int));
-  CK(h, cudaMemcpyAsync(h->dims.p, h->stage2.p, (n + 1) * sizeof(int), cudaMemcpyHostToDevice, st));
-  cplx* R = reinterpret_cast<cplx*>(h->env_r.p);
-  cplx* Lv = reinterpret_cast<cplx*>(h->env_l.p);
-  const int64_t chi2 = (int64_t)chi * chi;
-  CKL(h, launch_env_init(d, chi, h->charge + (size_t)n * chi * 2, h->lam + (size_t)n * chi,
-                         R + (size_t)n * chi, st));
-  for (int b = n - 1; b >= 0; --b)
-    CKL(h, launch_env_right_step(d, chi, h->gamma + (size_t)b * chi2, h->charge + (size_t)b * chi * 2,
-                                 h->lam + (size_t)b * chi, R + (size_t)(b + 1) * chi,
-                                 R + (size_t)b * chi, dims[b], dims[b + 1], st));
-  CKL(h, launch_env_init(d, chi, h->charge, h->lam, Lv, st));
-  for (int b = 0; b < n; ++b)
-    CKL(h, launch_env_left_step(d, chi, h->gamma + (size_t)b * chi2,
-                                h->charge + (size_t)(b + 1) * chi * 2, h->lam + (size_t)(b + 1) * chi,
-                                Lv + (size_t)b * chi, Lv + (size_t)(b + 1) * chi, dims[b], dims[b + 1],
-                                st));
   return BSMPO_OK;
 }
 
@@ -2034,19 +2036,33 @@ int bsmpo_apply_phases(bsmpo_ctx* h, const double* phases) {
 int bsmpo_observables(bsmpo_ctx* h, double* trace, double* marginals) {
   if (!h || !trace) return fail(h, BSMPO_EINVAL, "bad argument");
   if (!h->loaded) return fail(h, BSMPO_EINVAL, "no state loaded");
-  const int n = h->n, d = h->d, chi = h->chi;
+  const int n = h->n, d = h->d, chi = h->chi, dd = d * d;
+  cudaStream_t st = h->stream;
   int rc;
-  if ((rc = env_all(h))) return rc;
-  const int chunk_rows = 32;
-  const int nchunk = ceil_div(chi, chunk_rows);
-  if ((rc = grow(h, h->part, (size_t)n * nchunk * d * sizeof(cplx)))) return rc;
+  if ((rc = grow(h, h->env_l, (size_t)(n + 1) * chi * sizeof(cplx)))) return rc;
+  if ((rc = grow(h, h->env_r, (size_t)(n + 1) * chi * sizeof(cplx)))) return rc;
+  if ((rc = grow(h, h->dims, ((size_t)(n + 1) * chi + n + 1) * sizeof(int)))) return rc;
   if ((rc = grow(h, h->outv, ((size_t)n * d + 1) * sizeof(cplx)))) return rc;
+  // kept entries of every bond, from the host mirror (the kernels use their own counts: an
+  // entry also needs Lambda > 0)
+  std::vector<int> kept(n + 1, 0);
+  int most = 0;
+  for (int b = 0; b <= n; ++b) {
+    for (int c = 0; c < d; ++c) kept[b] += h->cnt[(size_t)b * dd + c * d + c];
+    most = std::max(most, kept[b]);
+  }
+  const int chunk_rows = 32;
+  const int nchunk = marginals ? std::max(ceil_div(most, chunk_rows), 1) : 0;
+  if ((rc = grow(h, h->part, std::max((size_t)n * nchunk * d, (size_t)1) * sizeof(cplx)))) return rc;
+  int* list = reinterpret_cast<int*>(h->dims.p);
+  int* count = list + (size_t)(n + 1) * chi;
+  CKL(h, launch_diag_lists(n, d, chi, h->charge, h->lam, list, count, h->env_r.p, h->env_l.p, st));
+  for (int t = 0; t < n; ++t)
+    CKL(h, launch_env_step(n, chi, t, std::max(kept[n - 1 - t], marginals ? kept[t + 1] : 0),
+                           marginals != nullptr, h->gamma, list, count, h->env_r.p, h->env_l.p, st));
   cplx* out = reinterpret_cast<cplx*>(h->outv.p);
-  CKL(h, launch_sum_vector(h->env_r.p, chi, out + (size_t)n * d, h->stream));
-  if (marginals)
-    CKL(h, launch_marginals(n, d, chi, h->gamma, h->charge, h->env_l.p, h->env_r.p,
-                            reinterpret_cast<const int*>(h->dims.p), h->part.p, chunk_rows, out,
-                            h->stream));
+  CKL(h, launch_marginals(n, d, chi, h->gamma, h->charge, list, count, h->env_l.p, h->env_r.p, h->part.p, chunk_rows,
+                          nchunk, out, st));
   if ((rc = grow_host(h, h->hres, std::max(h->hres.bytes, ((size_t)n * d + 1) * sizeof(cplx) + 8192)))) return rc;
   cplx* ho = reinterpret_cast<cplx*>(static_cast<char*>(h->hres.p) + 4096);
   CK(h, cudaMemcpyAsync(ho, out, ((size_t)n * d + 1) * sizeof(cplx), cudaMemcpyDeviceToHost, h->stream));
@@ -2113,10 +2129,10 @@ int bsmpo_workspace_stats(const bsmpo_ctx* h, int64_t* out) {
   int64_t dev = 0, host = 0;
   auto add = [&](const bsmpo_ctx* c) {
     const DevBuf* bufs[] = {&c->theta, &c->cbuf, &c->abuf, &c->wbuf, &c->vbuf, &c->sig, &c->keys,
-                            &c->perm, &c->tab, &c->tab2, &c->rot, &c->kept, &c->u3, &c->m4,
+                            &c->perm, &c->tab, &c->tab2, &c->rot, &c->u3, &c->m4,
                             &c->env_l, &c->env_r, &c->part, &c->outv, &c->dims, &c->nf2, &c->qbuf,
                             &c->qflag, &c->pbuf, &c->pcnt, &c->gbuf, &c->eigd, &c->taub, &c->invsig,
-                            &c->escr, &c->swp, &c->zbuf, &c->ybuf, &c->tab3, &c->tcerr, &c->jwork};
+                            &c->escr, &c->swp, &c->zbuf, &c->ybuf, &c->tab3};
     for (const DevBuf* b : bufs) dev += (int64_t)b->bytes;
     const HostStage* hs[] = {&c->stage, &c->stage2, &c->stage3, &c->hres};
     for (const HostStage* b : hs) host += (int64_t)b->bytes;

@@ -5,55 +5,207 @@
 //
 // with each charge taken per row / column / centre entry (so no x8 alignment
 // padding or centre-charge change list is needed) and the term zero unless every U
-// index lies in [0, d).  FP64, 16 x 16 output tile per CTA, centre index staged
-// through shared memory 16 at a time.  The whole-BS path (bsmpo_bs_update) does not
-// use these kernels; it contracts charge blocks as GEMMs instead.
-#include "common.cuh"
+// index lies in [0, d).  The whole-BS path (bsmpo_bs_update) does not use these kernels; it
+// contracts charge blocks as GEMMs instead.
+//
+// The weight depends on the centre entry through its charge only.  So the centre entries are
+// taken in runs of equal charge (any order of the entries is allowed; an order by charge has
+// the fewest runs): a run's plain products are accumulated on the FP64 tensor path (m8n8k4),
+// and at its end each output adds its weight times the run's sum.  A run that no row and
+// column of the tile can use is not read.  What bounds it: the FP64 tensor rate, at a small
+// grid (32 x 32 tiles, 4 warps, so that a sector of 443 x 389 is 182 CTAs).  Measured there with
+// 1,024 centre entries, d = 5: 93 us; 16 x 16 tiles with the weight applied per entry took 270.
+#include "dmma.cuh"
 #include "kernels.h"
 
 namespace {
 
-constexpr int CT = 16;
+static_assert(BSMPO_MAX_D <= 1 << 10, "charges are far below the sentinel");
+constexpr int CT = 32, CK = 8, CNT = 128, CSTAGES = 3;
+constexpr int CWIN = 1024;                 // centre entries whose runs are listed at once
+constexpr int CLDA = CK + 4, CLDB = CT + 2;
+constexpr int CSTAGE = CT * CLDA + CK * CLDB;
 
-__global__ void contract_sector_kernel(int d, int cc0, int cc1, const cplx* __restrict__ u,
-                                       const cplx* __restrict__ glc, const cplx* __restrict__ gcr,
-                                       const int2* __restrict__ cl, const int2* __restrict__ cc,
-                                       const int2* __restrict__ cr, int len_l, int len_c,
-                                       int len_r, cplx* __restrict__ out) {
-  __shared__ cplx us[BSMPO_MAX_D * BSMPO_MAX_D * BSMPO_MAX_D];
-  __shared__ cplx ga[CT][CT + 1], gb[CT][CT + 1];
-  __shared__ int2 qc[CT];
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * CT + tx;
-  const int d3 = d * d * d;
-  for (int i = tid; i < d3; i += CT * CT) us[i] = u[i];
-  const int l = blockIdx.y * CT + ty, r = blockIdx.x * CT + tx;
-  const int2 a = l < len_l ? cl[l] : make_int2(d, d);
-  const int2 b = r < len_r ? cr[r] : make_int2(d, d);
-  const bool row_ok = a.x < d && a.y < d && a.x >= cc0 && a.y >= cc1;
-  const bool col_ok = b.x < d && b.y < d && b.x <= cc0 && b.y <= cc1;
-  cplx acc = cmake(0.0, 0.0);
-  for (int c0 = 0; c0 < len_c; c0 += CT) {
+// (a, b) >= (x, y) in both components
+__device__ __forceinline__ bool ge2(int2 a, int2 b) { return a.x >= b.x && a.y >= b.y; }
+
+// The product of one tile over the centre entries, run by run: fold(q) is called with the
+// run's first centre index once re / im hold its sum.  use is called by whole warps.
+template <typename Same, typename Use, typename Fold>
+__device__ __forceinline__ void run_products(const cplx* __restrict__ glc, const cplx* __restrict__ gcr, int len_l,
+                                             int len_c, int len_r, double2* smem, int* runs, double2 (&re)[2][2],
+                                             double2 (&im)[2][2], Same same, Use use, Fold fold) {
+  __shared__ int wsum[CNT / 32], n_runs;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int m0 = blockIdx.y * CT, n0 = blockIdx.x * CT;
+  const int wm = (warp >> 1) * 16, wn = (warp & 1) * 16, li = lane >> 2, lk = lane & 3;
+  for (int w0 = 0; w0 < len_c; w0 += CWIN) {
+    const int w1 = min(w0 + CWIN, len_c);
+    // starts of the window's runs, in order
+    if (tid == 0) n_runs = 0;
     __syncthreads();
-    {
-      const int lr = blockIdx.y * CT + ty, cc_ = c0 + tx;
-      ga[ty][tx] = (lr < len_l && cc_ < len_c) ? ldc(glc + (int64_t)lr * len_c + cc_) : cmake(0.0, 0.0);
-      const int cr_ = c0 + ty, rc = blockIdx.x * CT + tx;
-      gb[ty][tx] = (cr_ < len_c && rc < len_r) ? ldc(gcr + (int64_t)cr_ * len_r + rc) : cmake(0.0, 0.0);
-      if (ty == 0) qc[tx] = (c0 + tx < len_c) ? cc[c0 + tx] : make_int2(d, d);
+    for (int i0 = w0; i0 < w1; i0 += CNT) {
+      const int i = i0 + tid;
+      const bool start = i < w1 && (i == w0 || !same(i - 1, i));
+      const unsigned m = __ballot_sync(0xffffffffu, start);
+      if (lane == 0) wsum[warp] = __popc(m);
+      __syncthreads();
+      int at = n_runs + __popc(m & ((1u << lane) - 1));
+      for (int w = 0; w < warp; ++w) at += wsum[w];
+      if (start) runs[at] = i;
+      __syncthreads();
+      if (tid == 0)
+        for (int w = 0; w < CNT / 32; ++w) n_runs += wsum[w];
+      __syncthreads();
     }
-    __syncthreads();
-    if (!(row_ok && col_ok)) continue;
-    for (int j = 0; j < CT; ++j) {
-      const int2 q = qc[j];
-      if (q.x >= d || q.y >= d) continue;
-      if (!(a.x >= q.x && q.x >= b.x && a.y >= q.y && q.y >= b.y)) continue;
-      const cplx u0 = us[((a.x - cc0) * d + (cc0 - b.x)) * d + (a.x - q.x)];
-      const cplx u1 = us[((a.y - cc1) * d + (cc1 - b.y)) * d + (a.y - q.y)];
-      const cplx w = cmulc(u0, u1);
-      cfma(acc, w, cmul(ga[ty][j], gb[j][tx]));
+    const int nr = n_runs;
+    // slabs of CK entries within a run, over the window's used runs; (run, k) walk in
+    // step for the fills and the products
+    auto end_of = [&](int r) { return r + 1 < nr ? runs[r + 1] : w1; };
+    auto next_used = [&](int r) {
+      while (r < nr && !use(runs[r])) ++r;
+      return r;
+    };
+    int fr = next_used(0), fk = fr < nr ? runs[fr] : 0;   // next slab to fill
+    auto fill = [&](int s) {
+      if (fr >= nr) return;
+      const int end = end_of(fr);
+      double2 *as = smem + s * CSTAGE, *bs = as + CT * CLDA;
+#pragma unroll
+      for (int i = 0; i < CT * CK / CNT; ++i) {
+        const int e = tid + i * CNT, m = e / CK, k = e % CK;
+        const bool ok = m0 + m < len_l && fk + k < end;
+        cp_async16(as + m * CLDA + k, ok ? glc + (int64_t)(m0 + m) * len_c + fk + k : glc, ok);
+      }
+#pragma unroll
+      for (int i = 0; i < CT * CK / CNT; ++i) {
+        const int e = tid + i * CNT, k = e / CT, n = e % CT;
+        const bool ok = n0 + n < len_r && fk + k < end;
+        cp_async16(bs + k * CLDB + n, ok ? gcr + (int64_t)(fk + k) * len_r + n0 + n : gcr, ok);
+      }
+      fk += CK;
+      if (fk >= end) {
+        fr = next_used(fr + 1);
+        if (fr < nr) fk = runs[fr];
+      }
+    };
+    int cr = fr, ck = fk;                                 // next slab to multiply
+#pragma unroll
+    for (int s = 0; s < CSTAGES - 1; ++s) {
+      fill(s);
+      cp_async_commit();
     }
+    for (int t = 0; cr < nr; ++t) {
+      cp_async_wait<CSTAGES - 2>();
+      __syncthreads();
+      fill((t + CSTAGES - 1) % CSTAGES);
+      cp_async_commit();
+      const double2 *as = smem + (t % CSTAGES) * CSTAGE, *bs = as + CT * CLDA;
+      cmma_tile<2, 2, CK / 4, false>(
+          re, im, [&](int i, int k) { return as[(wm + 8 * i + li) * CLDA + k + lk]; },
+          [&](int j, int k) { return bs[(k + lk) * CLDB + wn + 8 * j + li]; });
+      ck += CK;
+      if (ck >= end_of(cr)) {
+        fold(runs[cr]);
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) re[i][j] = im[i][j] = make_double2(0.0, 0.0);
+        cr = next_used(cr + 1);
+        if (cr < nr) ck = runs[cr];
+      }
+    }
+    __syncthreads();   // the stages and the run list are free for the next window
   }
-  if (l < len_l && r < len_r) out[(int64_t)l * len_r + r] = acc;
+}
+
+// this lane's outputs of the tile: row of (i), column of (j, x)
+struct TileLane {
+  int row0, col0;
+  __device__ TileLane() {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    row0 = blockIdx.y * CT + (warp >> 1) * 16 + (lane >> 2);
+    col0 = blockIdx.x * CT + (warp & 1) * 16 + 2 * (lane & 3);
+  }
+  __device__ int row(int i) const { return row0 + 8 * i; }
+  __device__ int col(int j, int x) const { return col0 + 8 * j + x; }
+};
+
+__global__ __launch_bounds__(CNT) void contract_sector_kernel(int d, int cc0, int cc1, const cplx* __restrict__ u,
+                                                              const cplx* __restrict__ glc, const cplx* __restrict__ gcr,
+                                                              const int2* __restrict__ cl, const int2* __restrict__ cc,
+                                                              const int2* __restrict__ cr, int len_l, int len_c, int len_r,
+                                                              cplx* __restrict__ out) {
+  __shared__ __align__(16) double2 smem[CSTAGES * CSTAGE];
+  __shared__ cplx us[BSMPO_MAX_D * BSMPO_MAX_D * BSMPO_MAX_D];
+  __shared__ int2 rows[CT], cols[CT];
+  __shared__ int runs[CWIN];
+  const int tid = threadIdx.x, d3 = d * d * d;
+  for (int i = tid; i < d3; i += CNT) us[i] = u[i];
+  // charges of the tile's rows and columns; (-1, -1) / (BIG, BIG): contributes nothing
+  constexpr int BIG = 1 << 20;
+  if (tid < CT) {
+    const int l = blockIdx.y * CT + tid;
+    const int2 a = l < len_l ? cl[l] : make_int2(d, d);
+    rows[tid] = a.x < d && a.y < d && a.x >= cc0 && a.y >= cc1 ? a : make_int2(-1, -1);
+  } else if (tid < 2 * CT) {
+    const int r = blockIdx.x * CT + tid - CT;
+    const int2 b = r < len_r ? cr[r] : make_int2(d, d);
+    cols[tid - CT] = b.x < d && b.y < d && b.x <= cc0 && b.y <= cc1 ? b : make_int2(BIG, BIG);
+  }
+  __syncthreads();
+  const TileLane T;
+  int2 a[2], b[2][2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    a[i] = rows[T.row(i) - blockIdx.y * CT];
+    b[i][0] = cols[T.col(i, 0) - blockIdx.x * CT];
+    b[i][1] = cols[T.col(i, 1) - blockIdx.x * CT];
+  }
+  double2 re[2][2], im[2][2];
+  cplx acc[2][2][2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      re[i][j] = im[i][j] = make_double2(0.0, 0.0);
+      acc[i][j][0] = acc[i][j][1] = cmake(0.0, 0.0);
+    }
+  run_products(
+      glc, gcr, len_l, len_c, len_r, smem, runs, re, im,
+      [&](int i, int j) { return cc[i].x == cc[j].x && cc[i].y == cc[j].y; },
+      [&](int i) {
+        const int2 q = cc[i];
+        if (q.x >= d || q.y >= d) return false;
+        const int t = threadIdx.x & 31;   // a lane to a row and a column of the tile
+        const bool r = __any_sync(0xffffffffu, ge2(rows[t], q)), c = __any_sync(0xffffffffu, ge2(q, cols[t]));
+        return r && c;
+      },
+      [&](int i0) {
+        const int2 q = cc[i0];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          if (!ge2(a[i], q)) continue;
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+              const int2 c = b[j][x];
+              if (!ge2(q, c)) continue;
+              const cplx u0 = us[((a[i].x - cc0) * d + (cc0 - c.x)) * d + (a[i].x - q.x)];
+              const cplx u1 = us[((a[i].y - cc1) * d + (cc1 - c.y)) * d + (a[i].y - q.y)];
+              cfma(acc[i][j][x], cmulc(u0, u1),
+                   x ? cmake(re[i][j].y, im[i][j].y) : cmake(re[i][j].x, im[i][j].x));
+            }
+        }
+      });
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+        if (T.row(i) < len_l && T.col(j, x) < len_r) stc(out + (int64_t)T.row(i) * len_r + T.col(j, x), acc[i][j][x]);
 }
 
 // The pure-state (MPS) variant: the drop-in for cuda_kernels.update_MPS
@@ -63,6 +215,7 @@ __global__ void contract_sector_kernel(int d, int cc0, int cc1, const cplx* __re
 // the term zero unless cl >= q(c) >= cr and every U index lies in [0, d).  The reference
 // reloads LC in tiles of 256 centre indices and, on its last partial tile, from offset 0
 // (src/update_kernel.cu:632-638) -- a quirk for k > 256; here LC[c] is read per index.
+constexpr int MT = 16;
 __global__ void contract_mps_kernel(int d, int tau, const cplx* __restrict__ u,
                                     const cplx* __restrict__ glc, const cplx* __restrict__ gcr,
                                     const double* __restrict__ ll, const double* __restrict__ lc,
@@ -70,23 +223,23 @@ __global__ void contract_mps_kernel(int d, int tau, const cplx* __restrict__ u,
                                     const int* __restrict__ cc, const int* __restrict__ cr, int len_l,
                                     int len_c, int len_r, cplx* __restrict__ out) {
   __shared__ cplx us[BSMPO_MAX_D * BSMPO_MAX_D * BSMPO_MAX_D];
-  __shared__ cplx ga[CT][CT + 1], gb[CT][CT + 1];
-  __shared__ int qc[CT];
-  __shared__ double lcs[CT];
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * CT + tx;
+  __shared__ cplx ga[MT][MT + 1], gb[MT][MT + 1];
+  __shared__ int qc[MT];
+  __shared__ double lcs[MT];
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * MT + tx;
   const int d3 = d * d * d;
-  for (int i = tid; i < d3; i += CT * CT) us[i] = u[i];
-  const int l = blockIdx.y * CT + ty, r = blockIdx.x * CT + tx;
+  for (int i = tid; i < d3; i += MT * MT) us[i] = u[i];
+  const int l = blockIdx.y * MT + ty, r = blockIdx.x * MT + tx;
   const int a = l < len_l ? cl[l] : -1;
   const int b = r < len_r ? cr[r] : -1;
   const bool ok = a >= 0 && b >= 0 && a - tau >= 0 && a - tau < d && tau - b >= 0 && tau - b < d;
   cplx acc = cmake(0.0, 0.0);
-  for (int c0 = 0; c0 < len_c; c0 += CT) {
+  for (int c0 = 0; c0 < len_c; c0 += MT) {
     __syncthreads();
     {
-      const int lrow = blockIdx.y * CT + ty, ccol = c0 + tx;
+      const int lrow = blockIdx.y * MT + ty, ccol = c0 + tx;
       ga[ty][tx] = (lrow < len_l && ccol < len_c) ? ldc(glc + (int64_t)lrow * len_c + ccol) : cmake(0.0, 0.0);
-      const int crow = c0 + ty, rc = blockIdx.x * CT + tx;
+      const int crow = c0 + ty, rc = blockIdx.x * MT + tx;
       gb[ty][tx] = (crow < len_c && rc < len_r) ? ldc(gcr + (int64_t)crow * len_r + rc) : cmake(0.0, 0.0);
       if (ty == 0) {
         qc[tx] = (c0 + tx < len_c) ? cc[c0 + tx] : -1;
@@ -95,7 +248,7 @@ __global__ void contract_mps_kernel(int d, int tau, const cplx* __restrict__ u,
     }
     __syncthreads();
     if (!ok) continue;
-    for (int j = 0; j < CT; ++j) {
+    for (int j = 0; j < MT; ++j) {
       const int q = qc[j];
       if (q < 0 || !(a >= q && q >= b) || a - q >= d) continue;
       const cplx w = cscale(us[((a - tau) * d + (tau - b)) * d + (a - q)], lcs[j]);
@@ -112,8 +265,8 @@ cudaError_t launch_contract_mps(int d, int tau, const void* u, const void* glc, 
                                 const int* cc, const int* cr, int len_l, int len_c, int len_r, void* t,
                                 cudaStream_t s) {
   if (len_l <= 0 || len_r <= 0) return cudaSuccess;
-  dim3 grid(ceil_div(len_r, CT), ceil_div(len_l, CT));
-  dim3 block(CT, CT);
+  dim3 grid(ceil_div(len_r, MT), ceil_div(len_l, MT));
+  dim3 block(MT, MT);
   contract_mps_kernel<<<grid, block, 0, s>>>(d, tau, reinterpret_cast<const cplx*>(u),
                                              reinterpret_cast<const cplx*>(glc), reinterpret_cast<const cplx*>(gcr),
                                              ll, lc, lr, cl, cc, cr, len_l, len_c, len_r, reinterpret_cast<cplx*>(t));
@@ -125,8 +278,7 @@ cudaError_t launch_contract_sector(int d, int cc0, int cc1, const void* u, const
                                    int len_l, int len_c, int len_r, void* c, cudaStream_t s) {
   if (len_l <= 0 || len_r <= 0) return cudaSuccess;
   dim3 grid(ceil_div(len_r, CT), ceil_div(len_l, CT));
-  dim3 block(CT, CT);
-  contract_sector_kernel<<<grid, block, 0, s>>>(
+  contract_sector_kernel<<<grid, CNT, 0, s>>>(
       d, cc0, cc1, reinterpret_cast<const cplx*>(u), reinterpret_cast<const cplx*>(glc),
       reinterpret_cast<const cplx*>(gcr), reinterpret_cast<const int2*>(cl),
       reinterpret_cast<const int2*>(cc), reinterpret_cast<const int2*>(cr), len_l, len_c, len_r,

@@ -485,12 +485,13 @@ __global__ __launch_bounds__(JNT) void jacobi_apply_kernel(const SectorDesc* __r
 constexpr int FNT = 512;
 
 __global__ __launch_bounds__(FNT) void jacobi_finish_kernel(const SectorDesc* __restrict__ sd,
+                                                            const int* __restrict__ list,
                                                             const cplx* __restrict__ abuf,
                                                             const double* __restrict__ nf2,
                                                             double* __restrict__ sig,
                                                             int* __restrict__ perm) {
   extern __shared__ unsigned char smem_raw[];
-  const SectorDesc& S = sd[blockIdx.x];
+  const SectorDesc& S = sd[list[blockIdx.x]];
   const int k = S.k;
   if (k == 0) return;
   int np2 = 1;
@@ -499,7 +500,7 @@ __global__ __launch_bounds__(FNT) void jacobi_finish_kernel(const SectorDesc* __
   int* si = reinterpret_cast<int*>(sv + np2);
   const cplx* A = abuf + S.a_off;
   const double zf = 16.0 * 2.220446049250313e-16 * sqrt((double)S.rows_g);
-  const double z2 = zf * zf * nf2[blockIdx.x];
+  const double z2 = zf * zf * nf2[list[blockIdx.x]];
   for (int j = threadIdx.x; j < np2; j += FNT) {
     double s2 = -1.0;
     if (j < k) {
@@ -540,10 +541,11 @@ __global__ __launch_bounds__(FNT) void jacobi_finish_kernel(const SectorDesc* __
 // ||T_s||_F^2 over the Gram rows, one CTA per sector, fixed-order reduction
 constexpr int NNT = 256;
 __global__ __launch_bounds__(NNT) void sector_norm_kernel(const SectorDesc* __restrict__ sd,
+                                                          const int* __restrict__ list,
                                                           const cplx* __restrict__ abuf,
                                                           double* __restrict__ nf2) {
   __shared__ double red[NNT];
-  const SectorDesc& S = sd[blockIdx.x];
+  const SectorDesc& S = sd[list[blockIdx.x]];
   const int64_t total = (int64_t)S.rows_g * S.k;
   const cplx* A = abuf + S.a_off;
   double acc = 0.0;
@@ -554,17 +556,244 @@ __global__ __launch_bounds__(NNT) void sector_norm_kernel(const SectorDesc* __re
     if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
     __syncthreads();
   }
-  if (threadIdx.x == 0) nf2[blockIdx.x] = red[0];
+  if (threadIdx.x == 0) nf2[list[blockIdx.x]] = red[0];
+}
+
+// ---------------------------------------------------------------------------------
+// Small sectors: the whole SVD of a sector in one CTA.  The Jacobi matrix lives in shared
+// memory by columns; a sweep is the circle method over single columns, a warp to a column
+// pair: dot products over the Gram rows, the rotation, its application to all rows, with
+// the tests and the floor of the blocked form above.  All sweeps, the column norms and the
+// sort run here, so such a sector needs no rounds of launches and no convergence polls.
+// What bounds it: the latency of a step (loads, 130 cycles of reduction, 200 of reciprocal
+// square roots, a barrier), k - 1 steps a sweep.  The blocked form pays two launches of
+// ~45 us a round and the host's polls: a 9-mode chi = 50 circuit took 16 ms with it and takes
+// 5.9, one update at chi = 32 1.58 ms and 0.47.
+constexpr int JS_KMAX = 48;
+
+// leading dimension of a column: odd in units of 16 B, so lanes across columns fall on
+// different banks
+__host__ __device__ inline int js_ld(int rows) { return rows | 1; }
+inline size_t js_smem(int rows, int k) { return (size_t)js_ld(rows) * k * sizeof(double2) + JS_KMAX * sizeof(double); }
+
+// (a, b, gx, gy) summed over the warp, in every lane.  Each value's product with ones leaves
+// a lane its four-lane sums of columns 2 (lane & 3) and 2 (lane & 3) + 1; a last product
+// whose right operand is value n in column n adds the four pairs of all values at once.
+__device__ __forceinline__ void sum4(double& a, double& b, double& gx, double& gy) {
+  const int lane = threadIdx.x & 31, n = (lane >> 2) & 3;
+  double2 s0 = make_double2(0, 0), s1 = s0, s2 = s0, s3 = s0, t = s0;
+  dmma(s0, 1.0, a);
+  dmma(s1, 1.0, b);
+  dmma(s2, 1.0, gx);
+  dmma(s3, 1.0, gy);
+  const double e0 = s0.x + s0.y, e1 = s1.x + s1.y, e2 = s2.x + s2.y, e3 = s3.x + s3.y;
+  dmma(t, 1.0, n == 0 ? e0 : n == 1 ? e1 : n == 2 ? e2 : e3);
+  // lanes with an even lane & 3 hold (a, b), the others (gx, gy)
+  const double ox = __shfl_xor_sync(0xffffffffu, t.x, 1), oy = __shfl_xor_sync(0xffffffffu, t.y, 1);
+  const bool ab = (lane & 1) == 0;
+  a = ab ? t.x : ox;
+  b = ab ? t.y : oy;
+  gx = ab ? ox : t.x;
+  gy = ab ? oy : t.y;
+}
+
+// One column pair: RC chunks of 32 rows held in registers between the dot products and the
+// rotation (0: read again).  Returns whether it rotated.
+template <int RC>
+__device__ __forceinline__ bool js_pair(double2* x, double2* y, int rows_g, int rows, double z2, double t2) {
+  const int lane = threadIdx.x & 31;
+  constexpr int R = RC > 0 ? RC : 1;
+  double2 u[R], v[R];
+  double a = 0.0, b = 0.0, gx = 0.0, gy = 0.0;
+  auto dot = [&](double2 p, double2 q) {
+    a = fma(p.x, p.x, fma(p.y, p.y, a));
+    b = fma(q.x, q.x, fma(q.y, q.y, b));
+    gx = fma(p.x, q.x, fma(p.y, q.y, gx));
+    gy = fma(p.x, q.y, fma(-p.y, q.x, gy));
+  };
+  if (RC > 0) {
+#pragma unroll
+    for (int c = 0; c < R; ++c) {
+      const int r = lane + 32 * c;
+      u[c] = v[c] = make_double2(0.0, 0.0);
+      if (r < rows) { u[c] = x[r]; v[c] = y[r]; }
+    }
+#pragma unroll
+    for (int c = 0; c < R; ++c)
+      if (lane + 32 * c < rows_g) dot(u[c], v[c]);
+  } else {
+#pragma unroll 4
+    for (int r = lane; r < rows_g; r += 32) dot(x[r], y[r]);
+  }
+  sum4(a, b, gx, gy);
+  const double g2 = gx * gx + gy * gy;
+  if (!(a > z2 && b > z2 && a > t2 * b && b > t2 * a && g2 > t2 * a * b)) return false;   // warp-uniform
+  // the rotation of the blocked form: c, s e^{i alpha} of the small angle
+  const double dd = b - a, ir = rsqrt(fma(dd, dd, 4.0 * g2)), c2 = fma(0.5 * fabs(dd), ir, 0.5), ic = rsqrt(c2);
+  const double c = c2 * ic, f = copysign(ir * ic, dd), sx = f * gx, sy = f * gy;
+  auto turn = [&](double2& p, double2& q) {
+    // p' = c p - conj(s) q, q' = s p + c q
+    const double2 n = make_double2(c * p.x - (sx * q.x + sy * q.y), c * p.y - (sx * q.y - sy * q.x));
+    q = make_double2(fma(c, q.x, sx * p.x - sy * p.y), fma(c, q.y, sx * p.y + sy * p.x));
+    p = n;
+  };
+  if (RC > 0) {
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      const int r = lane + 32 * k;
+      if (r < rows) {
+        turn(u[k], v[k]);
+        x[r] = u[k];
+        y[r] = v[k];
+      }
+    }
+  } else {
+#pragma unroll 4
+    for (int r = lane; r < rows; r += 32) {
+      double2 p = x[r], q = y[r];
+      turn(p, q);
+      x[r] = p;
+      y[r] = q;
+    }
+  }
+  return true;
+}
+
+template <int NT>
+__global__ __launch_bounds__(NT) void jacobi_small_kernel(const SectorDesc* __restrict__ sd,
+                                                          const int* __restrict__ list, cplx* __restrict__ abuf,
+                                                          int max_sweeps, double* __restrict__ sig,
+                                                          int* __restrict__ perm, int* __restrict__ fail,
+                                                          unsigned long long* __restrict__ executed) {
+  constexpr int NW = NT / 32;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double red[NW];
+  __shared__ int rot[2];
+  const SectorDesc& S = sd[list[blockIdx.x]];
+  const int k = S.k, rows = S.rows_tot, rows_g = S.rows_g, ld = js_ld(rows);
+  double2* X = reinterpret_cast<double2*>(smem_raw);   // column c: X + c ld
+  double* nrm = reinterpret_cast<double*>(X + (size_t)k * ld);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  cplx* A = abuf + S.a_off;
+  double f2 = 0.0;
+  for (int e = tid; e < rows * k; e += NT) {
+    const int r = e / k, c = e - r * k;
+    const cplx v = ldc(A + e);
+    X[c * ld + r] = make_double2(v.x, v.y);
+    if (r < rows_g) f2 += cabs2(v);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) f2 += __shfl_xor_sync(0xffffffffu, f2, o);
+  if (lane == 0) red[warp] = f2;
+  if (tid < 2) rot[tid] = 0;
+  __syncthreads();
+  f2 = 0.0;
+  for (int w = 0; w < NW; ++w) f2 += red[w];
+  const double zf = 16.0 * 2.220446049250313e-16 * sqrt((double)rows_g), z2 = zf * zf * f2;
+  const double tol = fmax(8.0 * 2.220446049250313e-16, 4.0 * 2.220446049250313e-16 * sqrt((double)rows_g));
+  const double t2 = tol * tol;
+  const int n = k + (k & 1), chunks = (rows + 31) / 32;
+  int sweep = 0;
+  unsigned long long turned = 0;
+  if (k > 1)
+    for (;; ++sweep) {
+      if (sweep == max_sweeps) {
+        if (tid == 0) *fail = 1;
+        break;
+      }
+      int mine = 0;
+      for (int step = 0; step < n - 1; ++step) {
+        for (int P = warp; P < n / 2; P += NW) {
+          int p = circle_at(P, step, n), q = circle_at(n - 1 - P, step, n);
+          if (p > q) { const int x = p; p = q; q = x; }
+          if (q >= k) continue;          // the padding column
+          double2 *x = X + p * ld, *y = X + q * ld;
+          bool r;
+          if (chunks <= 1) r = js_pair<1>(x, y, rows_g, rows, z2, t2);
+          else if (chunks == 2) r = js_pair<2>(x, y, rows_g, rows, z2, t2);
+          else if (chunks <= 4) r = js_pair<4>(x, y, rows_g, rows, z2, t2);
+          else r = js_pair<0>(x, y, rows_g, rows, z2, t2);
+          mine += r;
+        }
+        __syncthreads();
+      }
+      turned += mine;
+      if (lane == 0 && mine) rot[sweep & 1] = 1;
+      __syncthreads();
+      const bool again = rot[sweep & 1] != 0;
+      if (tid == 0) rot[(sweep + 1) & 1] = 0;   // the next sweep's flag, which nobody sets before its barriers
+      if (!again) break;
+    }
+  if (lane == 0 && turned) atomicAdd(executed, turned * 4ull * rows);
+  if (tid == 0) {
+    atomicAdd(executed, (unsigned long long)(sweep + 1) * (unsigned)(k * (k - 1) / 2) * 2ull * rows_g);
+    atomicMax(executed + 1, (unsigned long long)(sweep + 1));
+  }
+  __syncthreads();
+  // column norms (0 below the numerical-rank floor), the descending order (ties by column)
+  for (int c = warp; c < k; c += NW) {
+    double s2 = 0.0;
+    for (int r = lane; r < rows_g; r += 32) {
+      const double2 v = X[c * ld + r];
+      s2 = fma(v.x, v.x, fma(v.y, v.y, s2));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+    if (lane == 0) nrm[c] = s2 <= z2 ? 0.0 : sqrt(s2);
+  }
+  __syncthreads();
+  if (tid < k) {
+    const double s = nrm[tid];
+    int at = 0;
+    for (int c = 0; c < k; ++c) at += nrm[c] > s || (nrm[c] == s && c < tid);
+    sig[S.s_off + at] = s;
+    perm[S.s_off + at] = tid;
+  }
+  for (int e = tid; e < rows * k; e += NT) {
+    const int r = e / k, c = e - r * k;
+    const double2 v = X[c * ld + r];
+    stc(A + e, cmake(v.x, v.y));
+  }
 }
 
 }  // namespace
 
 int jacobi_block_cols() { return JB; }
 
-cudaError_t launch_sector_norms(const SectorDesc* sd_dev, int n_sectors, const void* abuf,
+// The whole SVD in one CTA, by the shape of the Jacobi matrix.  Measured against the blocked
+// form's rounds (two launches of 45 us a round and sweep): k = 9, 958 rows 121 us (270);
+// k = 17, 128 rows 101 (270); k = 28, 128 rows 236 (315), 256 rows 336 (315); k = 48, 128 rows
+// 768 (1,080), 256 rows 1,000 (945); k = 64, 128 rows 1,195 (1,080).
+bool jacobi_is_small(int rows, int k) {
+  return (k <= 16 || (k <= 32 && rows <= 256) || (k <= JS_KMAX && rows <= 192)) && js_smem(rows, k) <= 220 * 1024;
+}
+
+cudaError_t launch_jacobi_small(const SectorDesc* sd_dev, const int* list_dev, int count, int max_rows_k, int max_k,
+                                void* abuf, int max_sweeps, double* sig, int* perm, int* fail,
+                                unsigned long long* executed, cudaStream_t s) {
+  if (count <= 0) return cudaSuccess;
+  static const cudaError_t attr = [] {
+    cudaError_t e = cudaFuncSetAttribute(jacobi_small_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, 221 * 1024);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(jacobi_small_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, 221 * 1024);
+    return e;
+  }();
+  if (attr != cudaSuccess) return attr;
+  const size_t smem = (size_t)max_rows_k * sizeof(double2) + JS_KMAX * sizeof(double);
+  cplx* A = reinterpret_cast<cplx*>(abuf);
+  // a warp to a column pair: 8 warps cover a step of up to 16 columns
+  if (max_k <= 16)
+    jacobi_small_kernel<256><<<count, 256, smem, s>>>(sd_dev, list_dev, A, max_sweeps, sig, perm, fail, executed);
+  else
+    jacobi_small_kernel<512><<<count, 512, smem, s>>>(sd_dev, list_dev, A, max_sweeps, sig, perm, fail, executed);
+  return cudaGetLastError();
+}
+int jacobi_small_elems(int rows, int k) { return js_ld(rows) * k; }
+
+cudaError_t launch_sector_norms(const SectorDesc* sd_dev, const int* list_dev, int count, const void* abuf,
                                 double* nf2, cudaStream_t s) {
-  if (n_sectors <= 0) return cudaSuccess;
-  sector_norm_kernel<<<n_sectors, NNT, 0, s>>>(sd_dev, reinterpret_cast<const cplx*>(abuf), nf2);
+  if (count <= 0) return cudaSuccess;
+  sector_norm_kernel<<<count, NNT, 0, s>>>(sd_dev, list_dev, reinterpret_cast<const cplx*>(abuf), nf2);
   return cudaGetLastError();
 }
 
@@ -592,10 +821,10 @@ cudaError_t launch_jacobi_round(const SectorDesc* sd_dev, const JacobiWork* work
 
 int jacobi_rows_per_part() { return RMAX; }
 
-cudaError_t launch_jacobi_finish(const SectorDesc* sd_dev, int n_sectors, int max_k,
+cudaError_t launch_jacobi_finish(const SectorDesc* sd_dev, const int* list_dev, int count, int max_k,
                                  const void* abuf, const double* nf2, double* sig, int* perm,
                                  cudaStream_t s) {
-  if (n_sectors <= 0) return cudaSuccess;
+  if (count <= 0) return cudaSuccess;
   int np2 = 1;
   while (np2 < max_k) np2 <<= 1;
   const size_t smem = (size_t)np2 * (sizeof(double) + sizeof(int));
@@ -604,7 +833,6 @@ cudaError_t launch_jacobi_finish(const SectorDesc* sd_dev, int n_sectors, int ma
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  jacobi_finish_kernel<<<n_sectors, FNT, smem, s>>>(sd_dev, reinterpret_cast<const cplx*>(abuf),
-                                                    nf2, sig, perm);
+  jacobi_finish_kernel<<<count, FNT, smem, s>>>(sd_dev, list_dev, reinterpret_cast<const cplx*>(abuf), nf2, sig, perm);
   return cudaGetLastError();
 }

@@ -28,23 +28,21 @@ cudaError_t launch_fock_tensor_single(int d, M8 m, void* u_re_or_cplx, double* u
                                       cudaStream_t s);
 
 // ---------------------------------------------------------------- zgemm.cu
-// One group of a grouped complex128 GEMM:  C = rs[m] cs[n] sum_k op(A)(m,k) ks[k] op(B)(k,n)
-// op 0: as stored (row-major A[m][k], B[k][n]); op 1: conjugate transpose (A stored
-// [k][m], B stored [n][k]).  Offsets are in complex elements (scales in doubles) from
-// the launch's base pointers; a negative scale offset means "none".  sd is read only for
-// groups with sec >= 0.
+// One group of a grouped complex128 GEMM:  C = cs[n] sum_k op(A)(m,k) B(k,n), row-major
+// A[m][k] (opA 0) or its conjugate transpose, A stored [k][m] (opA 1); B[k][n].  Offsets are
+// in complex elements (the scale's in doubles) from the launch's base pointers; a negative
+// scale offset means "none".  sd is read only for groups with sec >= 0.
 struct GemmGroup {
   int M, N, K;
   int lda, ldb, ldc;
-  int opA, opB;
-  int beta;          // 0: C = result, 1: C += result
+  int opA;
+  int herm;          // 1: C is Hermitian (M = N), its lower tiles are written as adjoints
   int tiles_n;       // ceil(N / tile N)
   int tile_start;    // first flat tile index of this group
   int sec;           // >= 0: a dimension is sector sec's kept count, read on the device
   int kdim;          // (1: M and lda; 2: N, ldb and ldc); the host's value is its bound
-  int pad_;
   int64_t a_off, b_off, c_off;
-  int64_t ks_off, rs_off, cs_off;
+  int64_t cs_off;
 };
 
 cudaError_t launch_zgemm_grouped(const void* a, const void* b, void* c, const double* scale,
@@ -161,13 +159,21 @@ cudaError_t launch_jacobi_round(const SectorDesc* sd_dev, const JacobiWork* work
                                 const double* nf2, double tol, int max_sweeps, void* pbuf,
                                 int* pcnt, void* qbuf, int* qflag, unsigned long long* executed,
                                 cudaStream_t s);
-// Largest number of Jacobi-matrix rows (|L| + |R| or |L|) a sector may have.
-// ||T_s||_F^2 of each sector's Jacobi matrix (Gram rows), fixed-order reduction.
-cudaError_t launch_sector_norms(const SectorDesc* sd_dev, int n_sectors, const void* abuf,
+// Small sectors: the whole SVD (all sweeps, column norms, sort) in one CTA per listed
+// sector.  jacobi_is_small: whether a rows x k Jacobi matrix goes there; max_elems: the
+// largest jacobi_small_elems of the list.  fail is set to 1 where max_sweeps do not
+// converge; executed[0] += complex MACs done, executed[1] = the most sweeps.
+bool jacobi_is_small(int rows, int k);
+int jacobi_small_elems(int rows, int k);
+cudaError_t launch_jacobi_small(const SectorDesc* sd_dev, const int* list_dev, int count, int max_elems, int max_k,
+                                void* abuf, int max_sweeps, double* sig, int* perm, int* fail,
+                                unsigned long long* executed, cudaStream_t s);
+// ||T_s||_F^2 of the listed sectors' Jacobi matrices (Gram rows), fixed-order reduction.
+cudaError_t launch_sector_norms(const SectorDesc* sd_dev, const int* list_dev, int count, const void* abuf,
                                 double* nf2, cudaStream_t s);
 // Column norms (0 below the numerical-rank floor), descending sort (ties by column
-// index): sig[s_off..], perm[s_off..].
-cudaError_t launch_jacobi_finish(const SectorDesc* sd_dev, int n_sectors, int max_k,
+// index) of the listed sectors: sig[s_off..], perm[s_off..].
+cudaError_t launch_jacobi_finish(const SectorDesc* sd_dev, const int* list_dev, int count, int max_k,
                                  const void* abuf, const double* nf2, double* sig, int* perm,
                                  cudaStream_t s);
 
@@ -242,17 +248,16 @@ cudaError_t launch_contract_mps(int d, int tau, const void* u, const void* glc, 
                                 cudaStream_t s);
 
 // ---------------------------------------------------------------- observables.cu
-// env_r[b] (b = n..0) and env_l[b] (b = 0..n), complex, masked to ket == bra charges.
-cudaError_t launch_env_right_step(int d, int chi, const void* gamma_b, const int* charge_b,
-                                  const double* lam_b, const void* r_next, void* r_out,
-                                  int rows, int cols, cudaStream_t s);
-cudaError_t launch_env_left_step(int d, int chi, const void* gamma_b, const int* charge_next,
-                                 const double* lam_next, const void* l_cur, void* l_out,
-                                 int rows, int cols, cudaStream_t s);
-cudaError_t launch_env_init(int d, int chi, const int* charge_b, const double* lam_b, void* v,
-                            cudaStream_t s);
-// partial marginal bins: part[site][chunk][d] complex, then reduced into out[site][d].
-cudaError_t launch_marginals(int n, int d, int chi, const void* gamma, const int* charge,
-                             const void* env_l, const void* env_r, const int* dims,
-                             void* part, int chunk_rows, void* out, cudaStream_t s);
-cudaError_t launch_sum_vector(const void* v, int len, void* out, cudaStream_t s);
+// Per bond the positions of the entries with ket == bra charge and Lambda > 0 (list
+// [n+1][chi], count [n+1]); env_r / env_l [n+1][chi] hold environments in list order, of
+// which R_n and L_0 are set here.
+cudaError_t launch_diag_lists(int n, int d, int chi, const int* charge, const double* lam, int* list, int* count,
+                              void* env_r, void* env_l, cudaStream_t s);
+// Step t = 0 .. n - 1: R_{n-1-t} and, with left, L_{t+1}.
+cudaError_t launch_env_step(int n, int chi, int t, int max_rows, bool left, const void* gamma, const int* list,
+                            const int* count, void* env_r, void* env_l, cudaStream_t s);
+// Marginals (nchunk chunks of chunk_rows kept rows; nchunk 0: none) into out[n][d] through
+// part[site][chunk][d], and the trace into out[n d].
+cudaError_t launch_marginals(int n, int d, int chi, const void* gamma, const int* charge, const int* list,
+                             const int* count, const void* env_l, const void* env_r, void* part, int chunk_rows,
+                             int nchunk, void* out, cudaStream_t s);

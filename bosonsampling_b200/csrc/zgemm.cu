@@ -1,32 +1,85 @@
 // Grouped complex128 GEMM for the contraction-shaped steps of the BS update
-// (the Theta block products, V = T Y / sigma, W = V^H C).
+// (the Theta block products, the Gram matrices, V = T Y / sigma, W = V^H C).
 //
-// FP64 has no tcgen05 kind on sm_100a, so this is a SIMT DFMA kernel: 64 x 64 output
-// tile per CTA, K staged through shared memory 16 complex at a time with a register
-// prefetch of the next slab, 4 x 4 complex accumulators per thread.  A thread owns
-// rows ty + 16 i and columns tx + 16 j so shared-memory reads are conflict-free
-// broadcasts and global stores are 256-byte coalesced rows.  All groups of one
-// update go in one launch; a CTA finds its group by binary search over tile_start.
-#include "common.cuh"
+// FP64 has no tcgen05 kind on sm_100a, so this runs on the FP64 tensor path (m8n8k4): 64 x 64
+// output tile per CTA, 8 warps of 32 x 16, K in slabs of 8 complex through a ring of three
+// shared-memory stages filled by cp.async (zeros past the edges).  op(A) and B keep their
+// storage order in shared memory, padded so that a fragment load (four k by two rows a
+// quarter warp) falls on distinct banks.  All groups of one launch share the grid; a CTA
+// finds its group by binary search over tile_start.  A Hermitian group (C = A^H A) forms its
+// upper tiles only and writes the others as their adjoints.
+// What bounds it: the FP64 tensor rate for large groups, the slabs' latency for small ones.
+// 128-bit shared-memory reads take 4 cycles of the SM a warp: the vector form (4 x 4 complex
+// a thread) needed as many cycles for its operands as for its arithmetic, the fragments need
+// a fifth.  Measured, all GEMMs of one chi = 1024 update alone: 0.55 ms against 1.05; of two
+// layers at N = 64 (62 updates, beside other kernels): 20 ms against 36 to 44.
+#include "dmma.cuh"
 #include "kernels.h"
 
 namespace {
 
-constexpr int TM = 64, TN = 64, TK = 16, NT = 256;
+constexpr int TM = 64, TN = 64, TK = 8, NT = 256, STAGES = 3;
+constexpr int LDK = TK + 4;    // op(A) = A, stored [m][k]: 4 mod 8
+constexpr int LDM = TM + 2;    // A^H, stored [k][m], and B [k][n]: 2 mod 8
+constexpr int A_ELEMS = TM * LDK > TK * LDM ? TM * LDK : TK * LDM, B_ELEMS = TK * (TN + 2);
+constexpr size_t SMEM = (size_t)STAGES * (A_ELEMS + B_ELEMS) * sizeof(double2);
 
-__device__ __forceinline__ double2 ld2(const cplx* p) {
-  return __ldg(reinterpret_cast<const double2*>(p));
+template <bool OPA>
+__device__ __forceinline__ void tile_loop(const GemmGroup& g, const cplx* __restrict__ a, const cplx* __restrict__ b,
+                                          int m0, int n0, double2* smem, double2 (&re)[4][2], double2 (&im)[4][2]) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int M = g.M, N = g.N, K = g.K;
+  auto stage_a = [&](int s) { return smem + s * (A_ELEMS + B_ELEMS); };
+  auto stage_b = [&](int s) { return smem + s * (A_ELEMS + B_ELEMS) + A_ELEMS; };
+  auto fill = [&](int s, int k0) {
+    double2 *as = stage_a(s), *bs = stage_b(s);
+#pragma unroll
+    for (int i = 0; i < TM * TK / NT; ++i) {
+      const int e = tid + i * NT;
+      if (OPA) {
+        const int k = e / TM, m = e % TM;
+        const bool ok = m0 + m < M && k0 + k < K;
+        cp_async16(as + k * LDM + m, ok ? a + (int64_t)(k0 + k) * g.lda + m0 + m : a, ok);
+      } else {
+        const int m = e / TK, k = e % TK;
+        const bool ok = m0 + m < M && k0 + k < K;
+        cp_async16(as + m * LDK + k, ok ? a + (int64_t)(m0 + m) * g.lda + k0 + k : a, ok);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < TK * TN / NT; ++i) {
+      const int e = tid + i * NT, k = e / TN, n = e % TN;
+      const bool ok = n0 + n < N && k0 + k < K;
+      cp_async16(bs + k * (TN + 2) + n, ok ? b + (int64_t)(k0 + k) * g.ldb + n0 + n : b, ok);
+    }
+  };
+  const int wm = (warp >> 2) * 32, wn = (warp & 3) * 16, li = lane >> 2, lk = lane & 3;
+  const bool live = m0 + wm < M && n0 + wn < N;   // a warp's tile past the edge does nothing
+  const int slabs = (K + TK - 1) / TK;
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) {
+    if (s < slabs) fill(s, s * TK);
+    cp_async_commit();
+  }
+  for (int t = 0; t < slabs; ++t) {
+    cp_async_wait<STAGES - 2>();
+    __syncthreads();
+    if (t + STAGES - 1 < slabs) fill((t + STAGES - 1) % STAGES, (t + STAGES - 1) * TK);
+    cp_async_commit();
+    if (!live) continue;
+    const double2 *as = stage_a(t % STAGES), *bs = stage_b(t % STAGES);
+    cmma_tile<4, 2, TK / 4, OPA>(
+        re, im,
+        [&](int i, int k) { return OPA ? as[(k + lk) * LDM + wm + 8 * i + li] : as[(wm + 8 * i + li) * LDK + k + lk]; },
+        [&](int j, int k) { return bs[(k + lk) * (TN + 2) + wn + 8 * j + li]; });
+  }
 }
 
-__global__ __launch_bounds__(NT) void zgemm_grouped_kernel(const cplx* __restrict__ A,
-                                                           const cplx* __restrict__ B,
-                                                           cplx* __restrict__ C,
-                                                           const double* __restrict__ scale,
-                                                           const GemmGroup* __restrict__ groups,
-                                                           int n_groups,
-                                                           const SectorDesc* __restrict__ sd) {
-  __shared__ double2 As[TK][TM + 1];
-  __shared__ double2 Bs[TK][TN + 1];
+__global__ __launch_bounds__(NT, 2) void zgemm_grouped_kernel(const cplx* __restrict__ A, const cplx* __restrict__ B,
+                                                              cplx* __restrict__ C, const double* __restrict__ scale,
+                                                              const GemmGroup* __restrict__ groups, int n_groups,
+                                                              const SectorDesc* __restrict__ sd) {
+  extern __shared__ __align__(16) double2 smem[];
   __shared__ GemmGroup g;
   const int tid = threadIdx.x;
   if (tid == 0) {
@@ -45,109 +98,36 @@ __global__ __launch_bounds__(NT) void zgemm_grouped_kernel(const cplx* __restric
   }
   __syncthreads();
   const int tile = blockIdx.x - g.tile_start;
-  const int m0 = (tile / g.tiles_n) * TM;
-  const int n0 = (tile % g.tiles_n) * TN;
-  const int M = g.M, N = g.N, K = g.K;
-  if (m0 >= M || n0 >= N) return;   // tiles are laid out for the host's bound
-  const cplx* a = A + g.a_off;
-  const cplx* b = B + g.b_off;
-  const double* ks = g.ks_off >= 0 ? scale + g.ks_off : nullptr;
-
-  // global -> register staging coordinates (4 complex per thread per operand)
-  // opA == 0: A[m][k] row-major, thread loads row ra, k = ka..ka+3
-  // opA == 1: A stored [k][m], thread loads k = ka2, m = ma2..ma2+3 (conjugated)
-  const int ra = tid >> 2, ka = (tid & 3) * 4;
-  const int ka2 = tid >> 4, ma2 = (tid & 15) * 4;
-  const int kb = tid >> 4, nb = (tid & 15) * 4;      // opB == 0: B[k][n]
-  const int nb2 = tid >> 2, kb2 = (tid & 3) * 4;     // opB == 1: B stored [n][k]
-
-  double2 ra_reg[4], rb_reg[4];
-
-  auto load_a = [&](int k0) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      int m, k;
-      if (g.opA == 0) { m = m0 + ra; k = k0 + ka + i; } else { m = m0 + ma2 + i; k = k0 + ka2; }
-      double2 v = make_double2(0.0, 0.0);
-      if (m < M && k < K) {
-        v = (g.opA == 0) ? ld2(a + (int64_t)m * g.lda + k) : ld2(a + (int64_t)k * g.lda + m);
-        if (g.opA == 1) v.y = -v.y;
-        if (ks) { double s = __ldg(ks + k); v.x *= s; v.y *= s; }
-      }
-      ra_reg[i] = v;
-    }
-  };
-  auto load_b = [&](int k0) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      int n, k;
-      if (g.opB == 0) { k = k0 + kb; n = n0 + nb + i; } else { n = n0 + nb2; k = k0 + kb2 + i; }
-      double2 v = make_double2(0.0, 0.0);
-      if (n < N && k < K) {
-        v = (g.opB == 0) ? ld2(b + (int64_t)k * g.ldb + n) : ld2(b + (int64_t)n * g.ldb + k);
-        if (g.opB == 1) v.y = -v.y;
-      }
-      rb_reg[i] = v;
-    }
-  };
-  auto store_ab = [&]() {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (g.opA == 0) As[ka + i][ra] = ra_reg[i]; else As[ka2][ma2 + i] = ra_reg[i];
-      if (g.opB == 0) Bs[kb][nb + i] = rb_reg[i]; else Bs[kb2 + i][nb2] = rb_reg[i];
-    }
-  };
-
-  const int ty = tid >> 4, tx = tid & 15;
-  cplx acc[4][4];
+  const int m0 = (tile / g.tiles_n) * TM, n0 = (tile % g.tiles_n) * TN;
+  // tiles are laid out for the host's bound; a Hermitian group forms n0 >= m0
+  if (m0 >= g.M || n0 >= g.N || (g.herm && n0 < m0)) return;
+  double2 re[4][2], im[4][2];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = cmake(0.0, 0.0);
-
-  load_a(0);
-  load_b(0);
-  for (int k0 = 0; k0 < K; k0 += TK) {
-    __syncthreads();
-    store_ab();
-    __syncthreads();
-    if (k0 + TK < K) { load_a(k0 + TK); load_b(k0 + TK); }
-#pragma unroll 4
-    for (int kk = 0; kk < TK; ++kk) {
-      cplx av[4], bv[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        double2 t = As[kk][ty + 16 * i];
-        av[i] = cmake(t.x, t.y);
-        double2 u = Bs[kk][tx + 16 * i];
-        bv[i] = cmake(u.x, u.y);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) cfma(acc[i][j], av[i], bv[j]);
-    }
-  }
-
-  const double* rs = g.rs_off >= 0 ? scale + g.rs_off : nullptr;
+    for (int j = 0; j < 2; ++j) re[i][j] = im[i][j] = make_double2(0.0, 0.0);
+  if (g.opA) tile_loop<true>(g, A + g.a_off, B + g.b_off, m0, n0, smem, re, im);
+  else tile_loop<false>(g, A + g.a_off, B + g.b_off, m0, n0, smem, re, im);
+  const int lane = tid & 31, warp = tid >> 5;
+  const int row0 = m0 + (warp >> 2) * 32 + (lane >> 2), col0 = n0 + (warp & 3) * 16 + 2 * (lane & 3);
   const double* cs = g.cs_off >= 0 ? scale + g.cs_off : nullptr;
   cplx* c = C + g.c_off;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty + 16 * i;
-    if (m >= M) continue;
-    const double rsv = rs ? rs[m] : 1.0;
+  for (int j = 0; j < 2; ++j)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx + 16 * j;
-      if (n >= N) continue;
-      double f = rsv * (cs ? cs[n] : 1.0);
-      cplx v = cscale(acc[i][j], f);
-      cplx* p = c + (int64_t)m * g.ldc + n;
-      if (g.beta) v = cadd(v, ldc(p));
-      stc(p, v);
+    for (int x = 0; x < 2; ++x) {
+      const int n = col0 + 8 * j + x;
+      if (n >= g.N) continue;
+      const double f = cs ? cs[n] : 1.0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int m = row0 + 8 * i;
+        if (m >= g.M) continue;
+        const cplx v = cmake(f * (x ? re[i][j].y : re[i][j].x), f * (x ? im[i][j].y : im[i][j].x));
+        stc(c + (int64_t)m * g.ldc + n, v);
+        if (g.herm && n0 > m0) stc(c + (int64_t)n * g.ldc + m, cconj(v));
+      }
     }
-  }
 }
 
 }  // namespace
@@ -159,7 +139,10 @@ cudaError_t launch_zgemm_grouped(const void* a, const void* b, void* c, const do
                                  const GemmGroup* groups_dev, int n_groups, int total_tiles,
                                  const SectorDesc* sd_dev, cudaStream_t s) {
   if (total_tiles <= 0 || n_groups <= 0) return cudaSuccess;
-  zgemm_grouped_kernel<<<total_tiles, NT, 0, s>>>(
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(zgemm_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+  if (attr != cudaSuccess) return attr;
+  zgemm_grouped_kernel<<<total_tiles, NT, SMEM, s>>>(
       reinterpret_cast<const cplx*>(a), reinterpret_cast<const cplx*>(b),
       reinterpret_cast<cplx*>(c), scale, groups_dev, n_groups, sd_dev);
   return cudaGetLastError();
