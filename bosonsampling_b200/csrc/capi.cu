@@ -78,7 +78,7 @@ struct bsmpo_ctx {
   DevBuf theta, cbuf, abuf, wbuf, vbuf, sig, keys, perm, tab, tab2, rot, u3, m4, env_l,
       env_r, part, outv, dims, nf2, qbuf, qflag, pbuf, pcnt;
   // Gram / eigen route of the sector SVD (precision != BSMPO_PRECISION_FP64)
-  DevBuf gbuf, eigd, taub, invsig, escr, swp, zbuf, ybuf;
+  DevBuf gbuf, eigd, taub, invsig, escr, swp, zbuf, ybuf, wyt;
   // tensor-core contractions (BSMPO_PRECISION_TF32X3): groups and tensor maps of the
   // V / W GEMMs
   DevBuf tab3;
@@ -1093,10 +1093,11 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
     double* dbuf_d = reinterpret_cast<double*>(h->eigd.p);
     double* ebuf_d = dbuf_d + P.s_elems;
     double* lam_d = ebuf_d + P.s_elems;
-    CK(h, launch_eigvec(sd_d, ns, P.max_k, P.max_k, dbuf_d, ebuf_d, lam_d, reinterpret_cast<double*>(h->escr.p),
+    if ((rc = grow(h, h->wyt, eigvec_t_elems(P.s_elems, ns) * sizeof(cplx)))) return rc;
+    CK(h, launch_eigvec(sd_d, ns, P.max_k, false, dbuf_d, ebuf_d, lam_d, reinterpret_cast<double*>(h->escr.p),
                         reinterpret_cast<unsigned char*>(h->swp.p), reinterpret_cast<double*>(h->zbuf.p), h->gbuf.p,
-                        h->taub.p, h->vbuf.p, h->ybuf.p, st));
-    h->launches += 2;
+                        h->taub.p, h->wyt.p, h->vbuf.p, h->ybuf.p, st));
+    h->launches += 3;
     // V = T Y diag(1/sigma) stays FP64: it divides by sigma (down to ~3e-3 of the largest
     // at the cut), which would magnify a TF32 error into V's orthogonality, and a
     // non-orthonormal V leaks into W = V^H C at the scale of C
@@ -1196,7 +1197,7 @@ void free_workspaces(bsmpo_ctx* h) {
                     &h->perm, &h->tab, &h->tab2, &h->rot, &h->u3, &h->m4,
                     &h->env_l, &h->env_r, &h->part, &h->outv, &h->dims, &h->nf2, &h->qbuf,
                     &h->qflag, &h->pbuf, &h->pcnt, &h->gbuf, &h->eigd, &h->taub, &h->invsig,
-                    &h->escr, &h->swp, &h->zbuf, &h->ybuf, &h->tab3};
+                    &h->escr, &h->swp, &h->zbuf, &h->ybuf, &h->wyt, &h->tab3};
   for (DevBuf* b : bufs)
     if (b->p) cudaFreeAsync(b->p, h->stream);
   cudaStreamSynchronize(h->stream);
@@ -2132,7 +2133,7 @@ int bsmpo_workspace_stats(const bsmpo_ctx* h, int64_t* out) {
                             &c->perm, &c->tab, &c->tab2, &c->rot, &c->u3, &c->m4,
                             &c->env_l, &c->env_r, &c->part, &c->outv, &c->dims, &c->nf2, &c->qbuf,
                             &c->qflag, &c->pbuf, &c->pcnt, &c->gbuf, &c->eigd, &c->taub, &c->invsig,
-                            &c->escr, &c->swp, &c->zbuf, &c->ybuf, &c->tab3};
+                            &c->escr, &c->swp, &c->zbuf, &c->ybuf, &c->wyt, &c->tab3};
     for (const DevBuf* b : bufs) dev += (int64_t)b->bytes;
     const HostStage* hs[] = {&c->stage, &c->stage2, &c->stage3, &c->hres};
     for (const HostStage* b : hs) host += (int64_t)b->bytes;

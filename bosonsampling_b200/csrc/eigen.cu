@@ -27,7 +27,7 @@
 #include <cstdlib>
 #include <type_traits>
 
-#include "common.cuh"
+#include "dmma.cuh"
 #include "kernels.h"
 #include "pipeline.cuh"
 
@@ -83,14 +83,10 @@ __device__ __forceinline__ cplx warp_sum(cplx v) {
 // lane x holds two, and a second product adds the four pairs.  Two matrix instructions and
 // an addition (60 cycles) where five shuffles and additions take 210.
 __device__ __forceinline__ double warp_sum(double v) {
-  double a = 0.0, b = 0.0, t = 0.0, u = 0.0;
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(a), "+d"(b)
-               : "d"(1.0), "d"(v));
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(t), "+d"(u)
-               : "d"(1.0), "d"(a + b));
-  return t;
+  double2 a = make_double2(0.0, 0.0), t = a;
+  dmma8x8x4(a, 1.0, v);
+  dmma8x8x4(t, 1.0, a.x + a.y);
+  return t.x;
 }
 
 // a - (x conj(y) + u conj(z)), eight fused multiply-adds (the rank-2 update of one entry)
@@ -751,18 +747,45 @@ __global__ void __launch_bounds__(TD_NT, 2)
 // ---------------------------------------------------------------------------------
 // 2. Eigenvalues: warp i of sector s finds the i-th largest eigenvalue of (d, e) by
 //    multisection: 32 Sturm counts per pass (one per lane), the interval shrinks 33x.
+//    The counts use the three-term recurrence of the leading minors, p_i = (d_i - x) p_{i-1}
+//    - e_{i-1}^2 p_{i-2} (Givens 1954; Barth, Martin, Wilkinson 1967), on the matrix scaled
+//    to a norm of at most one: two dependent operations a step, where the ratio form has a
+//    division in its chain.  The pair is rescaled by a power of two every BI_RS steps, in
+//    which it can grow by 3^BI_RS and, with e^2 held above BI_E2, shrink by at most
+//    BI_E2^(BI_RS / 2) or eps^BI_RS.  A minor of exactly zero changes the count by one over
+//    its two steps whatever its sign bit.
+//    Measured, all sectors of a chi = 1024 update alone: 144 us against 469 with divisions.
 constexpr int BI_NT = 256;
+constexpr int BI_RS = 8;
+constexpr double BI_E2 = 1e-60;
 
-__device__ __forceinline__ int sturm_count(const double* d, const double* e2, int k, double x,
-                                           double pivmin) {
-  double q = d[0] - x;
-  if (fabs(q) < pivmin) q = -pivmin;
-  int c = q < 0.0;
-  for (int i = 1; i < k; ++i) {
-    q = (d[i] - x) - e2[i - 1] / q;
-    if (fabs(q) < pivmin) q = -pivmin;
-    c += q < 0.0;
+// number of eigenvalues below x of the scaled matrix, de[i] = (d_i, e_{i-1}^2)
+__device__ __forceinline__ int sturm_count(const double2* de, int k, double x) {
+  double pp = 1.0, p = de[0].x - x;
+  int c = (unsigned)__double2hiint(p) >> 31;
+  auto step = [&](double2 v) {
+    const double n = fma(v.x - x, p, -v.y * pp);
+    c += (unsigned)(__double2hiint(n) ^ __double2hiint(p)) >> 31;
+    pp = p;
+    p = n;
+  };
+  auto rescale = [&]() {
+    // the larger of the two to [1, 2)
+    const int h = max(__double2hiint(p) & 0x7ff00000, __double2hiint(pp) & 0x7ff00000);
+    const double f = __hiloint2double(0x7fe00000 - h, 0);
+    p *= f;
+    pp *= f;
+  };
+  int i = 1;
+  for (; i + BI_RS <= k; i += BI_RS) {
+    double2 v[BI_RS];
+#pragma unroll
+    for (int q = 0; q < BI_RS; ++q) v[q] = de[i + q];
+#pragma unroll
+    for (int q = 0; q < BI_RS; ++q) step(v[q]);
+    rescale();
   }
+  for (; i < k; ++i) step(de[i]);
   return c;
 }
 
@@ -770,57 +793,52 @@ __global__ __launch_bounds__(BI_NT) void bisect_kernel(const SectorDesc* __restr
                                                        const double* __restrict__ dbuf,
                                                        const double* __restrict__ ebuf,
                                                        double* __restrict__ lam) {
-  extern __shared__ double bsm[];
+  extern __shared__ double2 de[];
   const SectorDesc& S = sd[blockIdx.y];
   const int k = S.k;
   const int first = blockIdx.x * (BI_NT / 32);
   if (first >= k) return;             // uniform over the CTA
-  double* d = bsm;
-  double* e2 = bsm + k;
   __shared__ double red[2][BI_NT / 32];
-  __shared__ double bounds[3];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const double* dg = dbuf + S.s_off;
   const double* eg = ebuf + S.s_off;
-  double lo = 1e300, hi = -1e300, emax = 0.0;
+  double lo = 1e300, hi = -1e300;
   for (int i = tid; i < k; i += BI_NT) {
     const double di = dg[i];
     const double ea = i > 0 ? fabs(eg[i - 1]) : 0.0, eb = i < k - 1 ? fabs(eg[i]) : 0.0;
-    d[i] = di;
-    if (i < k - 1) e2[i] = eg[i] * eg[i];
+    de[i] = make_double2(di, ea);
     lo = fmin(lo, di - ea - eb);
     hi = fmax(hi, di + ea + eb);
-    emax = fmax(emax, eb * eb);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
     hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    emax = fmax(emax, __shfl_xor_sync(0xffffffffu, emax, o));
   }
   if (lane == 0) { red[0][warp] = lo; red[1][warp] = hi; }
-  __shared__ double red_e[BI_NT / 32];
-  if (lane == 0) red_e[warp] = emax;
   __syncthreads();
-  if (tid == 0) {
-    double a = red[0][0], b = red[1][0], c = red_e[0];
-    for (int w = 1; w < BI_NT / 32; ++w) { a = fmin(a, red[0][w]); b = fmax(b, red[1][w]); c = fmax(c, red_e[w]); }
-    // widen by a few ulps of the bound so the extreme eigenvalues stay inside
-    const double span = fmax(fabs(a), fabs(b));
-    bounds[0] = a - 4.0 * EPS * span - 1e-300;
-    bounds[1] = b + 4.0 * EPS * span + 1e-300;
-    bounds[2] = 2.2250738585072014e-308 * fmax(1.0, c);   // pivmin
+  lo = red[0][0];
+  hi = red[1][0];
+  for (int w = 1; w < BI_NT / 32; ++w) { lo = fmin(lo, red[0][w]); hi = fmax(hi, red[1][w]); }
+  // a power of two above the bound of the spectrum; a zero matrix is left as it is
+  const double span = fmax(fabs(lo), fabs(hi));
+  int ex = 0;
+  if (span > 0.0) frexp(span, &ex);
+  for (int i = tid; i < k; i += BI_NT) {
+    const double e = scalbn(de[i].y, -ex);
+    de[i] = make_double2(scalbn(de[i].x, -ex), fmax(e * e, BI_E2));
   }
   __syncthreads();
   const int i = first + warp;
   if (i >= k) return;
   const int target = k - 1 - i;        // eigenvalues below lambda_(i) (ascending index)
-  const double pivmin = bounds[2];
-  double a = bounds[0], b = bounds[1];
-  const double tol_abs = 4.0 * EPS * fmax(fabs(a), fabs(b)) + 2.0 * pivmin;
+  // widen by a few ulps of the bound so the extreme eigenvalues stay inside
+  const double sspan = scalbn(span, -ex);
+  double a = scalbn(lo, -ex) - 4.0 * EPS * sspan - 1e-300, b = scalbn(hi, -ex) + 4.0 * EPS * sspan + 1e-300;
+  const double tol_abs = 4.0 * EPS * fmax(fabs(a), fabs(b));
   for (int it = 0; it < 16; ++it) {
     const double x = a + (double)(lane + 1) * ((b - a) / 33.0);
-    const int c = sturm_count(d, e2, k, x, pivmin);
+    const int c = sturm_count(de, k, x);
     const unsigned below = __ballot_sync(0xffffffffu, c <= target);
     const int L = __popc(below);       // counts rise with x: lanes 0..L-1 lie below
     const double xl = __shfl_sync(0xffffffffu, x, L > 0 ? L - 1 : 0);
@@ -832,7 +850,7 @@ __global__ __launch_bounds__(BI_NT) void bisect_kernel(const SectorDesc* __restr
     // the selection and sigma = sqrt(lambda) need
     if (b - a <= tol_abs) break;   // warp-uniform
   }
-  if (lane == 0) lam[S.s_off + i] = 0.5 * (a + b);
+  if (lane == 0) lam[S.s_off + i] = scalbn(0.5 * (a + b), ex);
 }
 
 // Monotone order (bisection rounds independently), numerical floor, sigma and 1/sigma.
@@ -905,11 +923,11 @@ __global__ __launch_bounds__(IV_NT) void invit_kernel(const SectorDesc* __restri
                                                       const double* __restrict__ lam,
                                                       double* __restrict__ scratch,
                                                       unsigned char* __restrict__ swp,
-                                                      double* __restrict__ zbuf) {
+                                                      double* __restrict__ zbuf, bool all) {
   extern __shared__ double ism[];
   __shared__ double dots[IV_NT / 32][IV_GT], coef[IV_GT], nrm2[IV_NT / 32];
   const SectorDesc& S = sd[blockIdx.x];
-  const int k = S.k, kept = S.kept;
+  const int k = S.k, kept = all ? k : S.kept;
   if (kept == 0) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double* d = ism;
@@ -1085,52 +1103,180 @@ __global__ __launch_bounds__(IV_NT) void invit_kernel(const SectorDesc* __restri
   }
 }
 
-// 3b. y = Q z = H_0 (H_1 (... H_{k-2} z)), one warp per kept vector; lane holds the
-//     entries l = lane (mod 32).  Writes V = y ([k][kept], X = T^H) or Y for the GEMM.
-constexpr int BT_NT = 128;
+// 3b. y = Q z = H_0 (H_1 (... H_{k-2} z)), the reflectors in blocks of WY_B: H_j0 .. H_{j0+15} =
+//     I - V T V^H (V the block's vectors as columns, T upper triangular).  wy_t_kernel forms
+//     T of every block; backtransform_kernel applies the blocks, last first, to WY_C vectors
+//     held in shared memory: W = V^H Z with the rows split over the warps, W2 = T W,
+//     Z -= V W2, the two products on the FP64 tensor path with the fragments of V read
+//     straight from the Householder vectors (row j of the Gram matrix holds v_j at columns
+//     j + 1 ..).  Writes V = y ([k][kept], X = T^H) or Y for the GEMM.
+//     What bounds it: the block's chain (three barriers and two passes over V from L2); a
+//     pass serves WY_C vectors, where one warp per vector read V once per vector.  Measured,
+//     all sectors of a chi = 1024 update alone: 203 us and 23 for T, against 527.
+constexpr int WY_B = 16;      // reflectors of a block
+constexpr int WY_C = 8;       // vectors of a CTA
+constexpr int WY_NT = 256, WY_NW = WY_NT / 32;
+static_assert(WY_NT == WY_B * WY_B, "a thread to an entry of T");
+constexpr int WY_LDZ = WY_C + 2;   // 2 mod 8: a fragment's four rows on distinct banks
 
-template <int NPL>
-__global__ __launch_bounds__(BT_NT) void backtransform_kernel(const SectorDesc* __restrict__ sd,
-                                                              const cplx* __restrict__ gbuf,
-                                                              const cplx* __restrict__ taubuf,
-                                                              const double* __restrict__ zbuf,
-                                                              cplx* __restrict__ vbuf,
-                                                              cplx* __restrict__ ybuf) {
+// T of block b of sector s
+__device__ __forceinline__ int64_t wy_t_off(const SectorDesc& S, int s, int b) {
+  return WY_B * S.s_off + (int64_t)WY_B * WY_B * (s + b);
+}
+
+// v_j[l], zero outside the reflector
+__device__ __forceinline__ cplx wy_v(const cplx* A, int k, int j, int l) {
+  return j < k - 1 && l > j && l < k ? ldc(A + (int64_t)j * k + l) : cmake(0.0, 0.0);
+}
+
+constexpr int WT_NT = 128;
+__global__ __launch_bounds__(WT_NT) void wy_t_kernel(const SectorDesc* __restrict__ sd, const cplx* __restrict__ gbuf,
+                                                     const cplx* __restrict__ taubuf, cplx* __restrict__ tbuf, bool all) {
+  __shared__ double2 G[WT_NT / 32][WY_B][WY_B + 1];
+  __shared__ cplx T[WY_B][WY_B + 1];
   const SectorDesc& S = sd[blockIdx.y];
-  const int k = S.k, kept = S.kept;
-  const int lane = threadIdx.x & 31;
-  const int t = blockIdx.x * (BT_NT / 32) + (threadIdx.x >> 5);
-  if (t >= kept) return;
+  const int k = S.k, j0 = blockIdx.x * WY_B;
+  if (j0 >= k - 1 || (!all && S.kept == 0)) return;
   const cplx* A = gbuf + S.g_off;
-  const cplx* tau = taubuf + S.s_off;
-  const double* Z = zbuf + S.y_off;
-  cplx y[NPL];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, li = lane >> 2, lk = lane & 3;
+  // G = V^H V, rows j0 + 1 .. k - 1 in quarters
+  double2 re[2][2], im[2][2];
 #pragma unroll
-  for (int c = 0; c < NPL; ++c) {
-    const int l = lane + 32 * c;
-    y[c] = l < k ? cmake(Z[(int64_t)l * kept + t], 0.0) : cmake(0.0, 0.0);
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) re[i][j] = im[i][j] = make_double2(0.0, 0.0);
+  for (int l = j0 + 1 + 4 * warp; l < k; l += 4 * (WT_NT / 32)) {
+    auto frag = [&](int i, int) {
+      const cplx v = wy_v(A, k, j0 + 8 * i + li, l + lk);
+      return make_double2(v.x, v.y);
+    };
+    cmma_tile<2, 2, 1, true>(re, im, frag, frag);
   }
-  for (int j = k - 2; j >= 0; --j) {
-    const cplx* v = A + (int64_t)j * k;     // v_j at columns j+1 .. k-1 (v[j+1] = 1)
-    cplx dot = cmake(0.0, 0.0);
 #pragma unroll
-    for (int c = 0; c < NPL; ++c) {
-      const int l = lane + 32 * c;
-      if (l > j && l < k) ccfma(dot, ldc(v + l), y[c]);
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      G[warp][8 * i + li][8 * j + 2 * lk] = make_double2(re[i][j].x, im[i][j].x);
+      G[warp][8 * i + li][8 * j + 2 * lk + 1] = make_double2(re[i][j].y, im[i][j].y);
     }
-    dot = warp_sum(dot);
-    const cplx f = cmul(tau[j], dot);
-#pragma unroll
-    for (int c = 0; c < NPL; ++c) {
-      const int l = lane + 32 * c;
-      if (l > j && l < k) y[c] = csub(y[c], cmul(f, ldc(v + l)));
+  __syncthreads();
+  if (warp == 0) {
+    // column i of T: tau_i on the diagonal, -tau_i T(:, < i) (V^H v_i) above
+    const cplx* tau = taubuf + S.s_off;
+    for (int i = 0; i < WY_B; ++i) {
+      const cplx ti = j0 + i < k - 1 ? tau[j0 + i] : cmake(0.0, 0.0);
+      if (lane < WY_B) {
+        cplx acc = cmake(0.0, 0.0);
+        for (int c = lane; c < i; ++c) {
+          cplx g = cmake(0.0, 0.0);
+          for (int w = 0; w < WT_NT / 32; ++w) g = cadd(g, cmake(G[w][c][i].x, G[w][c][i].y));
+          cfma(acc, T[lane][c], g);
+        }
+        acc = cmul(ti, acc);
+        T[lane][i] = lane < i ? cmake(-acc.x, -acc.y) : lane == i ? ti : cmake(0.0, 0.0);
+      }
+      __syncwarp();
     }
   }
-  cplx* out = S.left ? vbuf + S.v_off : ybuf + S.y_off;
+  __syncthreads();
+  cplx* out = tbuf + wy_t_off(S, blockIdx.y, blockIdx.x);
+  for (int e = tid; e < WY_B * WY_B; e += WT_NT) stc(out + e, T[e / WY_B][e % WY_B]);
+}
+
+__global__ __launch_bounds__(WY_NT) void backtransform_kernel(const SectorDesc* __restrict__ sd,
+                                                              const cplx* __restrict__ gbuf,
+                                                              const cplx* __restrict__ tbuf,
+                                                              const double* __restrict__ zbuf,
+                                                              cplx* __restrict__ vbuf, cplx* __restrict__ ybuf,
+                                                              bool all) {
+  extern __shared__ __align__(16) double2 Z[];   // [k][WY_LDZ]
+  __shared__ double2 Wp[WY_NW][WY_B][WY_C + 1], W[WY_B][WY_LDZ];
+  const SectorDesc& S = sd[blockIdx.y];
+  const int k = S.k, kept = all ? k : S.kept, c0 = blockIdx.x * WY_C;
+  if (c0 >= kept) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, li = lane >> 2, lk = lane & 3;
+  const cplx* A = gbuf + S.g_off;
+  const double* z = zbuf + S.y_off;
+  for (int e = tid; e < k * WY_C; e += WY_NT) {
+    const int l = e / WY_C, c = e % WY_C;
+    Z[l * WY_LDZ + c] = make_double2(c0 + c < kept ? z[(int64_t)l * kept + c0 + c] : 0.0, 0.0);
+  }
+  const int nb = (k - 1 + WY_B - 1) / WY_B;
+  for (int b = nb - 1; b >= 0; --b) {
+    const int j0 = b * WY_B;
+    const cplx* T = tbuf + wy_t_off(S, blockIdx.y, b);
+    const cplx te = ldc(T + tid);   // this thread's entry of T
+    __syncthreads();
+    // W = V^H Z, four rows a step, the steps over the warps
+    {
+      double2 re[2][1], im[2][1];
 #pragma unroll
-  for (int c = 0; c < NPL; ++c) {
-    const int l = lane + 32 * c;
-    if (l < k) stc(out + (int64_t)l * kept + t, y[c]);
+      for (int i = 0; i < 2; ++i) re[i][0] = im[i][0] = make_double2(0.0, 0.0);
+#pragma unroll 4
+      for (int l = j0 + 1 + 4 * warp; l < k; l += 4 * WY_NW)
+        cmma_tile<2, 1, 1, true>(
+            re, im,
+            [&](int i, int) {
+              const cplx v = wy_v(A, k, j0 + 8 * i + li, l + lk);
+              return make_double2(v.x, v.y);
+            },
+            [&](int, int) { return l + lk < k ? Z[(l + lk) * WY_LDZ + li] : make_double2(0.0, 0.0); });
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        Wp[warp][8 * i + li][2 * lk] = make_double2(re[i][0].x, im[i][0].x);
+        Wp[warp][8 * i + li][2 * lk + 1] = make_double2(re[i][0].y, im[i][0].y);
+      }
+    }
+    __syncthreads();
+    // the warps' parts summed, then W2 = T W
+    if (tid < WY_B * WY_C) {
+      const int j = tid / WY_C, c = tid % WY_C;
+      double2 s = make_double2(0.0, 0.0);
+#pragma unroll
+      for (int w = 0; w < WY_NW; ++w) { s.x += Wp[w][j][c].x; s.y += Wp[w][j][c].y; }
+      W[j][c] = s;
+    }
+    // T into the parts' place once they are read
+    __syncthreads();
+    cplx* Ts = reinterpret_cast<cplx*>(&Wp[0][0][0]);
+    stc(Ts + tid, te);
+    __syncthreads();
+    cplx w2 = cmake(0.0, 0.0);
+    if (tid < WY_B * WY_C) {
+      const int j = tid / WY_C, c = tid % WY_C;
+      for (int q = j; q < WY_B; ++q) cfma(w2, ldc(Ts + j * WY_B + q), cmake(W[q][c].x, W[q][c].y));
+    }
+    __syncthreads();
+    if (tid < WY_B * WY_C) W[tid / WY_C][tid % WY_C] = make_double2(w2.x, w2.y);
+    __syncthreads();
+    // Z -= V W2, eight rows a tile
+    for (int l0 = j0 + 1 + 8 * warp; l0 < k; l0 += 8 * WY_NW) {
+      double2 re[1][1], im[1][1];
+      re[0][0] = im[0][0] = make_double2(0.0, 0.0);
+      cmma_tile<1, 1, WY_B / 4, false>(
+          re, im,
+          [&](int, int q) {
+            const cplx v = wy_v(A, k, j0 + q + lk, l0 + li);
+            return make_double2(v.x, v.y);
+          },
+          [&](int, int q) { return W[q + lk][li]; });
+      if (l0 + li < k) {
+        double2* p = Z + (l0 + li) * WY_LDZ + 2 * lk;
+        p[0].x -= re[0][0].x;
+        p[0].y -= im[0][0].x;
+        p[1].x -= re[0][0].y;
+        p[1].y -= im[0][0].y;
+      }
+    }
+  }
+  __syncthreads();
+  cplx* out = S.left && !all ? vbuf + S.v_off : ybuf + S.y_off;
+  for (int e = tid; e < k * WY_C; e += WY_NT) {
+    const int l = e / WY_C, c = e % WY_C;
+    if (c0 + c < kept) {
+      const double2 v = Z[l * WY_LDZ + c];
+      stc(out + (int64_t)l * kept + c0 + c, cmake(v.x, v.y));
+    }
   }
 }
 
@@ -1242,29 +1388,35 @@ cudaError_t launch_bisect(const SectorDesc* sd_dev, int n_sectors, int kmax, con
   return cudaGetLastError();
 }
 
-cudaError_t launch_eigvec(const SectorDesc* sd_dev, int n_sectors, int kmax, int kept_max,
+size_t eigvec_t_elems(int64_t s_elems, int n_sectors) {
+  return (size_t)(WY_B * s_elems + (int64_t)WY_B * WY_B * 2 * n_sectors);
+}
+
+cudaError_t launch_eigvec(const SectorDesc* sd_dev, int n_sectors, int kmax, bool all,
                           const double* dbuf, const double* ebuf, const double* lam,
                           double* scratch, unsigned char* swp, double* zbuf, const void* gbuf,
-                          const void* taubuf, void* vbuf, void* ybuf, cudaStream_t s) {
-  if (n_sectors <= 0 || kept_max <= 0) return cudaSuccess;
-  const size_t smem = (size_t)2 * kmax * sizeof(double);
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(invit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  invit_kernel<<<n_sectors, IV_NT, smem, s>>>(sd_dev, dbuf, ebuf, lam, scratch, swp, zbuf);
+                          const void* taubuf, void* tbuf, void* vbuf, void* ybuf, cudaStream_t s) {
+  if (n_sectors <= 0 || kmax <= 0) return cudaSuccess;
+  static const cudaError_t attr = [] {
+    const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(backtransform_kernel, dyn, eigen_max_k() * WY_LDZ * (int)sizeof(double2));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(invit_kernel, dyn, 2 * eigen_max_k() * (int)sizeof(double));
+    return e;
+  }();
+  if (attr != cudaSuccess) return attr;
+  invit_kernel<<<n_sectors, IV_NT, (size_t)2 * kmax * sizeof(double), s>>>(sd_dev, dbuf, ebuf, lam, scratch, swp, zbuf,
+                                                                          all);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  dim3 grid(ceil_div(kept_max, BT_NT / 32), n_sectors);
   const cplx* G = reinterpret_cast<const cplx*>(gbuf);
-  const cplx* T = reinterpret_cast<const cplx*>(taubuf);
-  cplx* V = reinterpret_cast<cplx*>(vbuf);
-  cplx* Y = reinterpret_cast<cplx*>(ybuf);
-  const int npl = ceil_div(kmax, 32);
-  if (npl <= 4) backtransform_kernel<4><<<grid, BT_NT, 0, s>>>(sd_dev, G, T, zbuf, V, Y);
-  else if (npl <= 8) backtransform_kernel<8><<<grid, BT_NT, 0, s>>>(sd_dev, G, T, zbuf, V, Y);
-  else if (npl <= 16) backtransform_kernel<16><<<grid, BT_NT, 0, s>>>(sd_dev, G, T, zbuf, V, Y);
-  else if (npl <= 32) backtransform_kernel<32><<<grid, BT_NT, 0, s>>>(sd_dev, G, T, zbuf, V, Y);
-  else return cudaErrorInvalidValue;
+  cplx* T = reinterpret_cast<cplx*>(tbuf);
+  if (kmax > 1) {
+    wy_t_kernel<<<dim3(ceil_div(kmax - 1, WY_B), n_sectors), WT_NT, 0, s>>>(
+        sd_dev, G, reinterpret_cast<const cplx*>(taubuf), T, all);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  backtransform_kernel<<<dim3(ceil_div(kmax, WY_C), n_sectors), WY_NT, (size_t)kmax * WY_LDZ * sizeof(double2), s>>>(
+      sd_dev, G, T, zbuf, reinterpret_cast<cplx*>(vbuf), reinterpret_cast<cplx*>(ybuf), all);
   return cudaGetLastError();
 }

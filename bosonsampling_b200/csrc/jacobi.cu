@@ -19,18 +19,10 @@
 // noise (the null space of a rank-deficient block); it takes part in no rotation and
 // its singular value is reported as 0, as is a column below tol times its partner
 // in a pair test.  Without this, noise columns never test orthogonal.
-#include "common.cuh"
+#include "dmma.cuh"
 #include "kernels.h"
 
 namespace {
-
-// D += A B on the FP64 tensor path, m8n8k4: a = A[lane>>2][lane&3],
-// b = B[lane&3][lane>>2], d = (D[lane>>2][2(lane&3)], D[lane>>2][2(lane&3)+1])
-__device__ __forceinline__ void dmma(double2& d, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(d.x), "+d"(d.y)
-               : "d"(a), "d"(b));
-}
 
 constexpr int JB = 16;        // columns per block
 constexpr int JC = 2 * JB;    // columns per block pair
@@ -213,10 +205,10 @@ __global__ __launch_bounds__(JNT) void jacobi_gram_kernel(const SectorDesc* __re
       const int I = jj == 0 ? I0 : I1, J = jj == 0 ? J0 : J1;
       const double2 a = r < ng ? S.u.tile[r][8 * I + li] : make_double2(0.0, 0.0);
       const double2 b = r < ng ? S.u.tile[r][8 * J + li] : make_double2(0.0, 0.0);
-      dmma(gre[jj], a.x, b.x);
-      dmma(gre[jj], a.y, b.y);
-      dmma(gim[jj], a.x, b.y);
-      dmma(gim[jj], -a.y, b.x);
+      dmma8x8x4(gre[jj], a.x, b.x);
+      dmma8x8x4(gre[jj], a.y, b.y);
+      dmma8x8x4(gim[jj], a.x, b.y);
+      dmma8x8x4(gim[jj], -a.y, b.x);
     }
   }
   __syncthreads();   // the tile is dead; G takes its place
@@ -464,9 +456,9 @@ __global__ __launch_bounds__(JNT) void jacobi_apply_kernel(const SectorDesc* __r
       for (int c = 0; c < 4; ++c) {
         const double2 q = Qs[4 * kk + lk][8 * c + li];
         const double qs = Qsum[4 * kk + lk][8 * c + li];
-        dmma(t1[c], tv[kk].x, q.x);
-        dmma(t2[c], tv[kk].y, q.y);
-        dmma(t3[c], ts, qs);
+        dmma8x8x4(t1[c], tv[kk].x, q.x);
+        dmma8x8x4(t2[c], tv[kk].y, q.y);
+        dmma8x8x4(t3[c], ts, qs);
       }
     }
     if (row < nr) {
@@ -582,12 +574,12 @@ inline size_t js_smem(int rows, int k) { return (size_t)js_ld(rows) * k * sizeof
 __device__ __forceinline__ void sum4(double& a, double& b, double& gx, double& gy) {
   const int lane = threadIdx.x & 31, n = (lane >> 2) & 3;
   double2 s0 = make_double2(0, 0), s1 = s0, s2 = s0, s3 = s0, t = s0;
-  dmma(s0, 1.0, a);
-  dmma(s1, 1.0, b);
-  dmma(s2, 1.0, gx);
-  dmma(s3, 1.0, gy);
+  dmma8x8x4(s0, 1.0, a);
+  dmma8x8x4(s1, 1.0, b);
+  dmma8x8x4(s2, 1.0, gx);
+  dmma8x8x4(s3, 1.0, gy);
   const double e0 = s0.x + s0.y, e1 = s1.x + s1.y, e2 = s2.x + s2.y, e3 = s3.x + s3.y;
-  dmma(t, 1.0, n == 0 ? e0 : n == 1 ? e1 : n == 2 ? e2 : e3);
+  dmma8x8x4(t, 1.0, n == 0 ? e0 : n == 1 ? e1 : n == 2 ? e2 : e3);
   // lanes with an even lane & 3 hold (a, b), the others (gx, gy)
   const double ox = __shfl_xor_sync(0xffffffffu, t.x, 1), oy = __shfl_xor_sync(0xffffffffu, t.y, 1);
   const bool ab = (lane & 1) == 0;
@@ -704,7 +696,11 @@ __global__ __launch_bounds__(NT) void jacobi_small_kernel(const SectorDesc* __re
       int mine = 0;
       for (int step = 0; step < n - 1; ++step) {
         for (int P = warp; P < n / 2; P += NW) {
-          int p = circle_at(P, step, n), q = circle_at(n - 1 - P, step, n);
+          // circle_at without its division
+          int p = P + step, q = n - 1 - P + step;
+          if (p > n - 1) p -= n - 1;
+          if (q > n - 1) q -= n - 1;
+          if (P == 0) p = 0;
           if (p > q) { const int x = p; p = q; q = x; }
           if (q >= k) continue;          // the padding column
           double2 *x = X + p * ld, *y = X + q * ld;
@@ -761,9 +757,9 @@ __global__ __launch_bounds__(NT) void jacobi_small_kernel(const SectorDesc* __re
 int jacobi_block_cols() { return JB; }
 
 // The whole SVD in one CTA, by the shape of the Jacobi matrix.  Measured against the blocked
-// form's rounds (two launches of 45 us a round and sweep): k = 9, 958 rows 121 us (270);
-// k = 17, 128 rows 101 (270); k = 28, 128 rows 236 (315), 256 rows 336 (315); k = 48, 128 rows
-// 768 (1,080), 256 rows 1,000 (945); k = 64, 128 rows 1,195 (1,080).
+// form's rounds (two launches of 45 us a round and sweep), us: k = 9, 958 rows 121 (270);
+// k = 17, 128 rows 90 (270); k = 28, 128 rows 209 (315), 256 rows 306 (315), 400 rows 447
+// (315); k = 48, 128 rows 543 (1,080), 192 rows 664 (945); k = 64, 128 rows 1,195 (1,080).
 bool jacobi_is_small(int rows, int k) {
   return (k <= 16 || (k <= 32 && rows <= 256) || (k <= JS_KMAX && rows <= 192)) && js_smem(rows, k) <= 220 * 1024;
 }
@@ -775,17 +771,21 @@ cudaError_t launch_jacobi_small(const SectorDesc* sd_dev, const int* list_dev, i
   static const cudaError_t attr = [] {
     cudaError_t e = cudaFuncSetAttribute(jacobi_small_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, 221 * 1024);
     if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(jacobi_small_kernel<768>, cudaFuncAttributeMaxDynamicSharedMemorySize, 221 * 1024);
+    if (e == cudaSuccess)
       e = cudaFuncSetAttribute(jacobi_small_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, 221 * 1024);
     return e;
   }();
   if (attr != cudaSuccess) return attr;
   const size_t smem = (size_t)max_rows_k * sizeof(double2) + JS_KMAX * sizeof(double);
   cplx* A = reinterpret_cast<cplx*>(abuf);
-  // a warp to a column pair: 8 warps cover a step of up to 16 columns
+  // a warp to a column pair of a step
   if (max_k <= 16)
     jacobi_small_kernel<256><<<count, 256, smem, s>>>(sd_dev, list_dev, A, max_sweeps, sig, perm, fail, executed);
-  else
+  else if (max_k <= 32)
     jacobi_small_kernel<512><<<count, 512, smem, s>>>(sd_dev, list_dev, A, max_sweeps, sig, perm, fail, executed);
+  else
+    jacobi_small_kernel<768><<<count, 768, smem, s>>>(sd_dev, list_dev, A, max_sweeps, sig, perm, fail, executed);
   return cudaGetLastError();
 }
 int jacobi_small_elems(int rows, int k) { return js_ld(rows) * k; }

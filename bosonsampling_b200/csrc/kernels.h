@@ -196,11 +196,13 @@ cudaError_t launch_bisect(const SectorDesc* sd_dev, int n_sectors, int kmax, con
                           const double* ebuf, double* lam, double* sig, double* invsig,
                           cudaStream_t s);
 // eigenvectors of the kept eigenvalues (sd[s].kept): V ([k][kept] at v_off) of the
-// sectors with X = T^H, Y ([k][kept] at y_off) of the others
-cudaError_t launch_eigvec(const SectorDesc* sd_dev, int n_sectors, int kmax, int kept_max,
+// sectors with X = T^H, Y ([k][kept] at y_off) of the others; with `all`, of every eigenvalue
+// and all at y_off ([k][k]).  tbuf: eigvec_t_elems complex entries.
+size_t eigvec_t_elems(int64_t s_elems, int n_sectors);
+cudaError_t launch_eigvec(const SectorDesc* sd_dev, int n_sectors, int kmax, bool all,
                           const double* dbuf, const double* ebuf, const double* lam,
                           double* scratch, unsigned char* swp, double* zbuf, const void* gbuf,
-                          const void* taubuf, void* vbuf, void* ybuf, cudaStream_t s);
+                          const void* taubuf, void* tbuf, void* vbuf, void* ybuf, cudaStream_t s);
 
 // ---------------------------------------------------------------- tcgemm.cu
 // One group of the tensor-core (tcgen05, 3 x TF32) grouped complex GEMM:
