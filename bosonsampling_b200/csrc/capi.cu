@@ -258,6 +258,10 @@ struct Plan {
   std::vector<GemmGroup> gg;
   std::vector<GemmGroup> ggram;   // Gram G_s = X^H X of every sector (Gram route)
   std::vector<GemmGroup> gv, gw;  // V = T Y diag(1/sigma) (Gram route, X = T) and W = V^H C
+  // Jacobi route, preconditioned sectors: Y^H Y, Y M and X Y (ggram their Gram matrices,
+  // tdlist the sectors by size class behind the others, n_pre of them)
+  std::vector<GemmGroup> gyy, gym, gxy;
+  int ym_tiles = 0, xy_tiles = 0, n_pre = 0, pre_k = 0, pre_elems = 0;
   // sectors by tridiagonalisation size class (Gram route); the small sectors, then the
   // others (Jacobi)
   std::vector<int> tdlist;
@@ -274,6 +278,7 @@ struct Plan {
   int64_t g_elems = 0, y_elems = 0;
   std::vector<double> flops_theta;   // per update
   bool gram = false;                 // the group's route (one for all of its updates)
+  bool pre = false;                  // Jacobi: the blocked sectors start from preconditioned matrices
 };
 
 // Orders a round's work entries (most rounds per sweep first: those sectors set the
@@ -316,20 +321,28 @@ int64_t candidates(bsmpo_ctx* h, int mode) {
   return sum;
 }
 
-// Whether an update takes the Gram route.  That route drops singular values below ~2e-6
-// of a sector's largest.  Where the update does not truncate to chi that is pure loss
-// (W = V^H C carries them through 1 / Lambda_R), so such updates take the exact Jacobi
-// SVD: where the candidates cannot exceed chi, or (gram_policy 2) where the centre bond
-// holds fewer than chi vectors (it was not truncated by the last update on it and is
-// unlikely to be by this one).
-bool gram_route(bsmpo_ctx* h, int mode) {
-  if (h->precision == BSMPO_PRECISION_FP64 || candidates(h, mode) <= h->chi) return false;
-  if (h->gram_policy < 2) return true;
+// How an update's sector SVD is computed.  The Gram route drops singular values below ~2e-6
+// of a sector's largest, and a preconditioned Jacobi SVD (X Y in place of X) determines them
+// to ~eps of the largest, where the plain one keeps them to high relative accuracy.  Where the
+// update does not truncate to chi the small values stay in the state (W = V^H C carries
+// them through 1 / Lambda_R), so such updates take the plain Jacobi SVD: where the
+// candidates cannot exceed chi, or (Gram route, gram_policy 2) where the centre bond holds
+// fewer than chi vectors (it was not truncated by the last update on it and is unlikely
+// to be by this one).
+enum class Route { plain, preconditioned, gram };
+
+Route route_of(bsmpo_ctx* h, int mode) {
+  if (candidates(h, mode) <= h->chi) return Route::plain;
+  if (h->precision == BSMPO_PRECISION_FP64) return Route::preconditioned;
+  if (h->gram_policy < 2) return Route::gram;
   const int dd = h->d * h->d;
   int64_t centre = 0;
   for (int q = 0; q < dd; ++q) centre += mirror(h)[(size_t)(mode + 1) * dd + q];
-  return centre >= h->chi;
+  return centre >= h->chi ? Route::gram : Route::plain;
 }
+
+// Jacobi route: whether a sector of the blocked form starts from a preconditioned matrix.
+bool preconditioned(const SectorDesc& S) { return !jacobi_is_small(S.rows_tot, S.k) && S.k <= eigen_max_k(); }
 
 // Adds the update at `mode` to the plan.
 int add_update(bsmpo_ctx* h, int mode, int64_t gate_off, Plan& P) {
@@ -378,6 +391,8 @@ int add_update(bsmpo_ctx* h, int mode, int64_t gate_off, Plan& P) {
       S.rows_tot = S.left ? n + m : m;
       S.c_off = P.c_elems; P.c_elems += (int64_t)m * n;
       S.a_off = P.a_elems; P.a_elems += (int64_t)S.rows_tot * S.k;
+      S.t_off = S.a_off;
+      if (!P.gram && P.pre && preconditioned(S)) { S.t_off = P.a_elems; P.a_elems += (int64_t)S.rows_g * S.k; }
       S.s_off = P.s_elems; P.s_elems += S.k;
       S.w_off = P.w_elems; P.w_elems += (int64_t)S.k * n;
       S.v_off = P.v_elems; P.v_elems += (int64_t)m * S.k;
@@ -497,7 +512,7 @@ int add_update(bsmpo_ctx* h, int mode, int64_t gate_off, Plan& P) {
     g.a_off = S.v_off; g.b_off = S.c_off; g.c_off = S.w_off;
     g.cs_off = -1;
     P.gw.push_back(g);
-    if (P.gram) {
+    if (P.gram || S.t_off != S.a_off) {
       // Gram G_s = X^H X, X = the first rows_g rows of the sector's Jacobi matrix
       // ([rows_g][k] row-major: T, or T^H when |L| < |R|)
       GemmGroup r;
@@ -508,10 +523,24 @@ int add_update(bsmpo_ctx* h, int mode, int64_t gate_off, Plan& P) {
       r.tiles_n = ceil_div(S.k, TNt);
       r.tile_start = P.gram_tiles;
       P.gram_tiles += ceil_div(S.k, TMt) * r.tiles_n;
-      r.a_off = S.a_off; r.b_off = S.a_off; r.c_off = S.g_off;
+      r.a_off = S.t_off; r.b_off = S.t_off; r.c_off = S.g_off;
       r.cs_off = -1;
       P.ggram.push_back(r);
-      if (!S.left) {
+      if (!P.gram) {
+        // S = Y^H Y (tiles as the Gram's), Y' = Y M, X' = X Y
+        GemmGroup y = r;
+        y.K = S.k;
+        y.a_off = y.b_off = S.y_off;
+        P.gyy.push_back(y);
+        y.opA = y.herm = 0;
+        y.b_off = S.g_off; y.c_off = S.y_off;
+        P.gym.push_back(y);
+        y.M = S.rows_g;
+        y.tile_start = P.xy_tiles;
+        P.xy_tiles += ceil_div(S.rows_g, TMt) * y.tiles_n;
+        y.a_off = S.t_off; y.b_off = S.y_off; y.c_off = S.a_off;
+        P.gxy.push_back(y);
+      } else if (!S.left) {
         // V [m][kept] = T [m][k] Y [k][kept] diag(1 / sigma)
         GemmGroup v;
         std::memset(&v, 0, sizeof(v));
@@ -533,22 +562,28 @@ int add_update(bsmpo_ctx* h, int mode, int64_t gate_off, Plan& P) {
 // The sector-wise work lists, once every update of the group is in the plan.
 void finish_plan(bsmpo_ctx* h, Plan& P) {
   const int ns = (int)P.sd.size();
-  if (P.gram) {
+  // the sectors of `from` by tridiagonalisation size class, largest first within a class:
+  // the last CTAs to start are the shortest
+  auto by_class = [&](const std::vector<int>& from) {
     for (int c = 0; c < TD_CLASSES; ++c) {
       const size_t first = P.tdlist.size();
-      for (int s = 0; s < ns; ++s)
+      for (int s : from)
         if (tridiag_class(P.sd[s].k) == c) P.tdlist.push_back(s);
-      // largest first: the last CTAs to start are the shortest
       std::stable_sort(P.tdlist.begin() + first, P.tdlist.end(),
                        [&](int x, int y) { return P.sd[x].k > P.sd[y].k; });
       P.td_count[c] = (int)(P.tdlist.size() - first);
       P.td_kmax[c] = P.td_count[c] ? P.sd[P.tdlist[first]].k : 0;
     }
+  };
+  if (P.gram) {
+    std::vector<int> every(ns);
+    for (int s = 0; s < ns; ++s) every[s] = s;
+    by_class(every);
     return;
   }
   const int JBc = jacobi_block_cols();
   const int rmax = std::min(h->jac_rows, jacobi_rows_per_part());
-  std::vector<int> big;
+  std::vector<int> big, pre;
   for (int s = 0; s < ns; ++s) {
     const SectorDesc& S = P.sd[s];
     if (S.left) P.max_left_m2 = std::max(P.max_left_m2, S.m * S.m);
@@ -560,6 +595,11 @@ void finish_plan(bsmpo_ctx* h, Plan& P) {
     }
     big.push_back(s);
     P.big_k = std::max(P.big_k, S.k);
+    if (S.t_off != S.a_off) {
+      pre.push_back(s);
+      P.pre_k = std::max(P.pre_k, S.k);
+      P.pre_elems = std::max(P.pre_elems, S.rows_tot * S.k);
+    }
     JacobiWork w;
     std::memset(&w, 0, sizeof(w));
     w.sector = s;
@@ -582,13 +622,15 @@ void finish_plan(bsmpo_ctx* h, Plan& P) {
   });
   P.n_small = (int)P.tdlist.size();
   P.tdlist.insert(P.tdlist.end(), big.begin(), big.end());
+  P.n_pre = (int)pre.size();
+  by_class(pre);
   std::vector<JacobiWork> all(P.jw);
   jacobi_launch_list(all, &P.gram_ctas, &P.apply_ctas, &P.jac_slots);
 }
 
 // packs plan tables into the pinned stage and copies them to the device table buffer
 struct TabLayout {
-  size_t tab, tidx, td, sd, pairs, gg, ggram, gv, gw, tdlist, tcmaps, tcg, jw, res, total;
+  size_t tab, tidx, td, sd, pairs, gg, ggram, gv, gw, gyy, gym, gxy, tdlist, tcmaps, tcg, jw, res, total;
 };
 
 // The words that come back from the device at the end of a group's update, at L.res of the
@@ -627,6 +669,9 @@ TabLayout layout_of(const Plan& P, const ResLayout& R) {
   L.ggram = place(P.ggram.size() * sizeof(GemmGroup));
   L.gv = place(P.gv.size() * sizeof(GemmGroup));
   L.gw = place(P.gw.size() * sizeof(GemmGroup));
+  L.gyy = place(P.gyy.size() * sizeof(GemmGroup));
+  L.gym = place(P.gym.size() * sizeof(GemmGroup));
+  L.gxy = place(P.gxy.size() * sizeof(GemmGroup));
   L.tdlist = place(P.tdlist.size() * sizeof(int));
   L.tcmaps = place(P.tcmaps.size());
   L.tcg = place(P.tcg.size() * sizeof(TcGroup));
@@ -663,23 +708,17 @@ struct StageClock {
   }
 };
 
-// 3a. The Gram route's eigenvalues: Gram matrices, tridiagonalisation, bisection.
-int gram_eigenvalues(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, const GemmGroup* ggram_d,
-                     const int* tdlist_d, int* err_d) {
-  const int ns = (int)P.sd.size();
+// Gram matrices and Householder tridiagonalisation of the plan's classes (Gram route: every
+// sector; Jacobi route: the preconditioned ones); list_d: their sectors by class.
+int gram_tridiagonal(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, const GemmGroup* ggram_d, const int* list_d,
+                     int* err_d) {
   cudaStream_t st = h->stream;
   int rc;
-  if (P.max_k > eigen_max_k())
-    return fail(h, BSMPO_ECAPACITY, "a sector of dimension " + std::to_string(P.max_k) +
-                                        " exceeds the Gram route's limit " + std::to_string(eigen_max_k()));
   if ((rc = grow(h, h->gbuf, std::max<int64_t>(P.g_elems, 1) * sizeof(cplx)))) return rc;
   if ((rc = grow(h, h->eigd, std::max<int64_t>(3 * P.s_elems, 1) * sizeof(double)))) return rc;
   if ((rc = grow(h, h->taub, std::max<int64_t>(P.s_elems, 1) * sizeof(cplx)))) return rc;
-  if ((rc = grow(h, h->invsig, std::max<int64_t>(P.s_elems, 1) * sizeof(double)))) return rc;
   double* dbuf_d = reinterpret_cast<double*>(h->eigd.p);
   double* ebuf_d = dbuf_d + P.s_elems;
-  double* lam_d = ebuf_d + P.s_elems;
-  if (h->timing) CK(h, cudaEventRecord(h->ev0, st));
   CKL(h, launch_zgemm_grouped(h->abuf.p, h->abuf.p, h->gbuf.p, nullptr, ggram_d, (int)P.ggram.size(), P.gram_tiles,
                               nullptr, st));
   // the largest class present on the update's stream, the others dealt out to the side
@@ -698,7 +737,7 @@ int gram_eigenvalues(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, const 
     ++slot;
   }
   const bool fork = used[0] || used[1] || used[2];
-  if (h->timing) {
+  if (h->timing && P.gram) {
     if (!h->td_ev0) {
       CK(h, cudaEventCreate(&h->td_ev0));
       CK(h, cudaEventCreate(&h->td_ev1));
@@ -710,7 +749,7 @@ int gram_eigenvalues(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, const 
     for (int i = 0; i < 3; ++i)
       if (used[i]) CK(h, cudaStreamWaitEvent(h->aux[i], h->fork_ev, 0));
   }
-  CK(h, launch_tridiag(sd_d, tdlist_d, P.td_count, P.td_kmax, h->gbuf.p, dbuf_d, ebuf_d, h->taub.p, err_d, ts));
+  CK(h, launch_tridiag(sd_d, list_d, P.td_count, P.td_kmax, h->gbuf.p, dbuf_d, ebuf_d, h->taub.p, err_d, ts));
   for (int i = 0; i < 3; ++i)
     if (used[i]) {
       CK(h, cudaEventRecord(h->join_ev[i], h->aux[i]));
@@ -718,12 +757,70 @@ int gram_eigenvalues(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, const 
     }
   // the last class takes two kernels
   for (int c = 0; c < TD_CLASSES; ++c) h->launches += P.td_count[c] > 0 ? 1 + (c == TD_CLASSES - 1) : 0;
-  if (h->timing) CK(h, cudaEventRecord(h->td_ev1, st));
+  if (h->timing && P.gram) CK(h, cudaEventRecord(h->td_ev1, st));
+  return BSMPO_OK;
+}
+
+// scratch of the eigenvectors
+int grow_eigvec(bsmpo_ctx* h, const Plan& P) {
+  const size_t ye = (size_t)std::max<int64_t>(P.y_elems, 1);
+  int rc;
+  if ((rc = grow(h, h->escr, 4 * ye * sizeof(double)))) return rc;
+  if ((rc = grow(h, h->swp, ye))) return rc;
+  if ((rc = grow(h, h->zbuf, ye * sizeof(double)))) return rc;
+  return grow(h, h->ybuf, ye * sizeof(cplx));
+}
+
+// 3a. The Gram route's eigenvalues: Gram matrices, tridiagonalisation, bisection.
+int gram_eigenvalues(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, const GemmGroup* ggram_d,
+                     const int* tdlist_d, int* err_d) {
+  const int ns = (int)P.sd.size();
+  cudaStream_t st = h->stream;
+  int rc;
+  if (P.max_k > eigen_max_k())
+    return fail(h, BSMPO_ECAPACITY, "a sector of dimension " + std::to_string(P.max_k) +
+                                        " exceeds the Gram route's limit " + std::to_string(eigen_max_k()));
+  if ((rc = grow(h, h->invsig, std::max<int64_t>(P.s_elems, 1) * sizeof(double)))) return rc;
+  if (h->timing) CK(h, cudaEventRecord(h->ev0, st));
+  if ((rc = gram_tridiagonal(h, P, sd_d, ggram_d, tdlist_d, err_d))) return rc;
+  double* dbuf_d = reinterpret_cast<double*>(h->eigd.p);
+  double* ebuf_d = dbuf_d + P.s_elems;
+  double* lam_d = ebuf_d + P.s_elems;
   CK(h, launch_bisect(sd_d, ns, P.max_k, dbuf_d, ebuf_d, lam_d, reinterpret_cast<double*>(h->sig.p),
                       reinterpret_cast<double*>(h->invsig.p), st));
   h->launches += 2;
   if (h->timing) CK(h, cudaEventRecord(h->ev1, st));
   h->last_sweeps = 0;
+  return BSMPO_OK;
+}
+
+// The matrices the blocked Jacobi rounds of the preconditioned sectors start from: X Y with
+// a unitary Y close to the eigenvectors of X^H X.
+int precondition(bsmpo_ctx* h, const Plan& P, SectorDesc* sd_d, const GemmGroup* ggram_d, const GemmGroup* gyy_d,
+                 const GemmGroup* gym_d, const GemmGroup* gxy_d, const int* list_d, int* err_d) {
+  cudaStream_t st = h->stream;
+  const int n = P.n_pre;
+  int rc;
+  if ((rc = gram_tridiagonal(h, P, sd_d, ggram_d, list_d, err_d))) return rc;
+  if ((rc = grow_eigvec(h, P))) return rc;
+  if ((rc = grow(h, h->wyt, precondition_t_elems(P.s_elems, (int)P.sd.size()) * sizeof(cplx)))) return rc;
+  double* dbuf_d = reinterpret_cast<double*>(h->eigd.p);
+  double* ebuf_d = dbuf_d + P.s_elems;
+  CK(h, launch_precondition_basis(sd_d, list_d, n, P.pre_k, dbuf_d, ebuf_d, ebuf_d + P.s_elems,
+                                  reinterpret_cast<double*>(h->escr.p), reinterpret_cast<unsigned char*>(h->swp.p),
+                                  reinterpret_cast<double*>(h->zbuf.p), h->gbuf.p, h->taub.p, h->wyt.p, h->ybuf.p, st));
+  h->launches += 5;
+  // three Newton-Schulz steps between ybuf and the inverse iteration's scratch (2 k^2
+  // complex a sector), ending in the latter; the Gram matrices' place holds Y^H Y
+  void *y = h->ybuf.p, *y2 = h->escr.p;
+  for (int it = 0; it < 3; ++it) {
+    CKL(h, launch_zgemm_grouped(y, y, h->gbuf.p, nullptr, gyy_d, n, P.gram_tiles, nullptr, st));
+    CKL(h, launch_newton_schulz(sd_d, list_d, n, P.pre_k, h->gbuf.p, it == 2, st));
+    CKL(h, launch_zgemm_grouped(y, h->gbuf.p, y2, nullptr, gym_d, n, P.gram_tiles, nullptr, st));
+    std::swap(y, y2);
+  }
+  CKL(h, launch_zgemm_grouped(h->abuf.p, y, h->abuf.p, nullptr, gxy_d, n, P.xy_tiles, nullptr, st));
+  CKL(h, launch_precondition_finish(sd_d, list_d, n, P.pre_elems, y, h->abuf.p, st));
   return BSMPO_OK;
 }
 
@@ -753,9 +850,9 @@ int gram_timing(bsmpo_ctx* h, const Plan& P) {
 }
 
 // 3b. One-sided Jacobi of every sector of the group: the small sectors in one launch, the
-// others in blocked rounds.
-int jacobi_svd(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, char* jw_d, const int* list_d, char* res_d,
-               const ResLayout& R) {
+// others in blocked rounds.  gg_d: the preconditioner's GEMM groups (X^H X, Y^H Y, Y M, X Y).
+int jacobi_svd(bsmpo_ctx* h, const Plan& P, SectorDesc* sd_d, char* jw_d, const int* list_d, const GemmGroup* const* gg_d,
+               char* res_d, const ResLayout& R) {
   const int ns = (int)P.sd.size(), n_big = (int)P.jw.size();
   cudaStream_t st = h->stream;
   int rc;
@@ -765,6 +862,9 @@ int jacobi_svd(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, char* jw_d, 
   double* sig = reinterpret_cast<double*>(h->sig.p);
   int* perm = reinterpret_cast<int*>(h->perm.p);
   if (h->timing) CK(h, cudaEventRecord(h->ev0, st));
+  if (P.n_pre && (rc = precondition(h, P, sd_d, gg_d[0], gg_d[1], gg_d[2], gg_d[3], list_d + P.n_small + n_big,
+                                    reinterpret_cast<int*>(res_d + R.err))))
+    return rc;
   // beside the blocked rounds, where there are any, on the first side stream
   cudaStream_t small_st = st;
   if (P.n_small && n_big && h->td_fork > 0) {
@@ -965,7 +1065,9 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
   const int d = h->d, chi = h->chi, dd = d * d;
   cudaStream_t st = h->stream;
   Plan P;
-  P.gram = gram_route(h, jobs[0].mode);
+  const Route route = route_of(h, jobs[0].mode);
+  P.gram = route == Route::gram;
+  P.pre = route == Route::preconditioned;
   const cplx* u3_base = jobs[0].u3;
   for (int j = 0; j < nj; ++j)
     if ((rc = add_update(h, jobs[j].mode, jobs[j].u3 - u3_base, P))) return rc;
@@ -994,6 +1096,9 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
   put(hs, L.ggram, P.ggram);
   put(hs, L.gv, P.gv);
   put(hs, L.gw, P.gw);
+  put(hs, L.gyy, P.gyy);
+  put(hs, L.gym, P.gym);
+  put(hs, L.gxy, P.gxy);
   put(hs, L.tdlist, P.tdlist);
   put(hs, L.tcmaps, P.tcmaps);
   put(hs, L.tcg, P.tcg);
@@ -1044,8 +1149,9 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
   int* kept_d = reinterpret_cast<int*>(res_d + R.kept);
   double* trunc_d = reinterpret_cast<double*>(res_d + R.trunc);
   if (!h->wait_ev) CK(h, cudaEventCreateWithFlags(&h->wait_ev, cudaEventBlockingSync | cudaEventDisableTiming));
+  const GemmGroup* pre_d[4] = {groups_at(L.ggram), groups_at(L.gyy), groups_at(L.gym), groups_at(L.gxy)};
   rc = P.gram ? gram_eigenvalues(h, P, sd_d, groups_at(L.ggram), list_d, tcerr_d)
-              : jacobi_svd(h, P, sd_d, dt + L.jw, list_d, res_d, R);
+              : jacobi_svd(h, P, sd_d, dt + L.jw, list_d, pre_d, res_d, R);
   if (rc || (rc = clk.mark(3))) return rc;
   auto select = [&]() -> int {
     CKL(h, launch_select(tab_d, sd_d, nj, ns, reinterpret_cast<double*>(h->sig.p),
@@ -1075,7 +1181,7 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
       char* t2 = static_cast<char*>(h->tab2.p);
       CK(h, cudaMemcpyAsync(t2, h->stage3.p, bytes, cudaMemcpyHostToDevice, st));
       CKL(h, launch_identity_rows(sd_d, ns, J.max_left_m2, h->abuf.p, st));
-      if ((rc = jacobi_svd(h, J, sd_d, t2, reinterpret_cast<const int*>(t2 + jbytes), res_d, R))) return rc;
+      if ((rc = jacobi_svd(h, J, sd_d, t2, reinterpret_cast<const int*>(t2 + jbytes), nullptr, res_d, R))) return rc;
       P.gram = false;
       if ((rc = select())) return rc;
     }
@@ -1085,19 +1191,14 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
   // V = T Y diag(1/sigma) where X = T) and W = V^H C; the kernels read the kept counts on
   // the device, so the host does not wait for them before these launches
   if (P.gram) {
-    const size_t ye = (size_t)std::max<int64_t>(P.y_elems, 1);
-    if ((rc = grow(h, h->escr, 4 * ye * sizeof(double)))) return rc;
-    if ((rc = grow(h, h->swp, ye))) return rc;
-    if ((rc = grow(h, h->zbuf, ye * sizeof(double)))) return rc;
-    if ((rc = grow(h, h->ybuf, ye * sizeof(cplx)))) return rc;
+    if ((rc = grow_eigvec(h, P))) return rc;
     double* dbuf_d = reinterpret_cast<double*>(h->eigd.p);
     double* ebuf_d = dbuf_d + P.s_elems;
     double* lam_d = ebuf_d + P.s_elems;
-    if ((rc = grow(h, h->wyt, eigvec_t_elems(P.s_elems, ns) * sizeof(cplx)))) return rc;
-    CK(h, launch_eigvec(sd_d, ns, P.max_k, false, dbuf_d, ebuf_d, lam_d, reinterpret_cast<double*>(h->escr.p),
+    CK(h, launch_eigvec(sd_d, ns, P.max_k, dbuf_d, ebuf_d, lam_d, reinterpret_cast<double*>(h->escr.p),
                         reinterpret_cast<unsigned char*>(h->swp.p), reinterpret_cast<double*>(h->zbuf.p), h->gbuf.p,
-                        h->taub.p, h->wyt.p, h->vbuf.p, h->ybuf.p, st));
-    h->launches += 3;
+                        h->taub.p, h->vbuf.p, h->ybuf.p, st));
+    h->launches += 2;
     // V = T Y diag(1/sigma) stays FP64: it divides by sigma (down to ~3e-3 of the largest
     // at the cut), which would magnify a TF32 error into V's orthogonality, and a
     // non-orthonormal V leaks into W = V^H C at the scale of C
@@ -1367,10 +1468,10 @@ int run_mesh_concurrent(bsmpo_ctx* h, int n_bs, const int* modes, const cplx* u3
           done_ev.push_back(mine);
           lane_of.push_back(wk);
           jobs.clear();
-          const bool route = gram_route(w, modes[ready[0]]);
+          const Route route = route_of(w, modes[ready[0]]);
           for (size_t i = 0; i < ready.size() && (int)jobs.size() < share;) {
             const int k = ready[i];
-            if (gram_route(w, modes[k]) != route) { ++i; continue; }
+            if (route_of(w, modes[k]) != route) { ++i; continue; }
             ready.erase(ready.begin() + i);
             Job j;
             j.mode = modes[k];

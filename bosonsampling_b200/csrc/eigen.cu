@@ -9,9 +9,8 @@
 //   1. Householder reduction of G to a real symmetric tridiagonal (d, e): G = Q T Q^H,
 //      Q = H_0 ... H_{k-2}, H_j = I - tau_j v_j v_j^H (LAPACK's zhetd2 conventions,
 //      lower storage), one thread-block cluster per sector, rows owned cyclically by
-//      the cluster's CTAs, the rank-2 update of step j - 1 fused with the matrix-vector
-//      product of step j (one read and one write of the trailing matrix per step), one
-//      cluster barrier per step;
+//      the cluster's CTAs and kept in their shared memory, the rank-2 update of step j - 1
+//      fused with the matrix-vector product of step j, one cluster barrier per step;
 //   2. every eigenvalue by multisection of Sturm counts (one warp per eigenvalue, 32
 //      points per pass), sigma = sqrt(lambda), zero below the numerical floor;
 //   3. after the global top-chi selection: eigenvectors of the kept eigenvalues by
@@ -339,8 +338,7 @@ __global__ void __launch_bounds__(NT + 32)
       cplx tau = cmake(0.0, 0.0), sc = tau;
       if (xn2 != 0.0 || alpha.y != 0.0) {
         beta = -copysign(sqrt(fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, xn2))), alpha.x);
-        const double rb = 1.0 / beta;
-        tau = cmake((beta - alpha.x) * rb, -alpha.y * rb);
+        tau = cmake((beta - alpha.x) / beta, -alpha.y / beta);
         sc = cdiv(cmake(1.0, 0.0), cmake(alpha.x - beta, alpha.y));
       }
       if (lane == 0) {
@@ -457,9 +455,8 @@ __global__ void __launch_bounds__(NT + 32)
 // ---------------------------------------------------------------------------------
 // 1b. The first k - TD_RES_MAX steps of the larger sectors, rows streamed from L2; the
 //    resident kernel takes over there (a step costs about 10 us here at k = 445, 30 at 1,024,
-//    and 3.6 in the resident kernel).  Cluster c handles sector list[c]; its cl CTAs (1, 2, 4 or 8,
-//    by sector size: a small sector would spend its steps waiting at barriers of a big
-//    cluster) own the rows i = rank (mod cl).  Every CTA holds the reflector vectors
+//    and 3.6 in the resident kernel).  Cluster c handles sector list[c]; its TD_CL CTAs own
+//    the rows i = rank (mod TD_CL).  Every CTA holds the reflector vectors
 //    and a copy of the row being reduced, so one cluster barrier per step suffices.
 //    Step j (trailing size t = k - j - 1):
 //    R   every CTA (warp 0): row j as the previous pass left it, minus the pending
@@ -789,12 +786,16 @@ __device__ __forceinline__ int sturm_count(const double2* de, int k, double x) {
   return c;
 }
 
+// a launch's sectors: all of them, or a list
+__device__ __forceinline__ int sector_of(const int* list, int i) { return list ? list[i] : i; }
+
 __global__ __launch_bounds__(BI_NT) void bisect_kernel(const SectorDesc* __restrict__ sd,
+                                                       const int* __restrict__ list,
                                                        const double* __restrict__ dbuf,
                                                        const double* __restrict__ ebuf,
                                                        double* __restrict__ lam) {
   extern __shared__ double2 de[];
-  const SectorDesc& S = sd[blockIdx.y];
+  const SectorDesc& S = sd[sector_of(list, blockIdx.y)];
   const int k = S.k;
   const int first = blockIdx.x * (BI_NT / 32);
   if (first >= k) return;             // uniform over the CTA
@@ -908,6 +909,7 @@ __global__ __launch_bounds__(FI_NT) void eig_finish_kernel(const SectorDesc* __r
 constexpr int IV_NT = 128;
 constexpr int IV_B = 8;        // steps of a batch
 constexpr int IV_GT = 32;      // group members one pass of the orthogonalisation takes
+constexpr double IV_GAP_ALL = 1e-10;   // orthogonalise_kernel's groups, of the norm
 
 __device__ __forceinline__ double start_entry(int l, int t) {
   unsigned h = (unsigned)l * 2654435761u ^ ((unsigned)t * 40503u + 0x9e3779b9u);
@@ -918,6 +920,7 @@ __device__ __forceinline__ double start_entry(int l, int t) {
 }
 
 __global__ __launch_bounds__(IV_NT) void invit_kernel(const SectorDesc* __restrict__ sd,
+                                                      const int* __restrict__ list,
                                                       const double* __restrict__ dbuf,
                                                       const double* __restrict__ ebuf,
                                                       const double* __restrict__ lam,
@@ -926,7 +929,7 @@ __global__ __launch_bounds__(IV_NT) void invit_kernel(const SectorDesc* __restri
                                                       double* __restrict__ zbuf, bool all) {
   extern __shared__ double ism[];
   __shared__ double dots[IV_NT / 32][IV_GT], coef[IV_GT], nrm2[IV_NT / 32];
-  const SectorDesc& S = sd[blockIdx.x];
+  const SectorDesc& S = sd[sector_of(list, blockIdx.x)];
   const int k = S.k, kept = all ? k : S.kept;
   if (kept == 0) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -950,7 +953,8 @@ __global__ __launch_bounds__(IV_NT) void invit_kernel(const SectorDesc* __restri
   double* Z = zbuf + S.y_off;
   __syncthreads();
   bool grouped = false;
-  for (int m = tid; m < kept; m += IV_NT) grouped |= m > 0 && lv[m - 1] - lv[m] <= gaptol;
+  // with `all`, orthogonalise_kernel does the groups
+  for (int m = tid; m < kept && !all; m += IV_NT) grouped |= m > 0 && lv[m - 1] - lv[m] <= gaptol;
   grouped = __syncthreads_or(grouped);
   for (int m = tid; m < kept; m += IV_NT) {
     // factor T - lambda I
@@ -1103,16 +1107,122 @@ __global__ __launch_bounds__(IV_NT) void invit_kernel(const SectorDesc* __restri
   }
 }
 
-// 3b. y = Q z = H_0 (H_1 (... H_{k-2} z)), the reflectors in blocks of WY_B: H_j0 .. H_{j0+15} =
-//     I - V T V^H (V the block's vectors as columns, T upper triangular).  wy_t_kernel forms
-//     T of every block; backtransform_kernel applies the blocks, last first, to WY_C vectors
-//     held in shared memory: W = V^H Z with the rows split over the warps, W2 = T W,
-//     Z -= V W2, the two products on the FP64 tensor path with the fragments of V read
-//     straight from the Householder vectors (row j of the Gram matrix holds v_j at columns
-//     j + 1 ..).  Writes V = y ([k][kept], X = T^H) or Y for the GEMM.
-//     What bounds it: the block's chain (three barriers and two passes over V from L2); a
-//     pass serves WY_C vectors, where one warp per vector read V once per vector.  Measured,
-//     all sectors of a chi = 1024 update alone: 203 us and 23 for T, against 527.
+// 3b. y = Q z = H_0 (H_1 (... H_{k-2} z)), one warp per kept vector, lane holding the entries
+//     l = lane (mod 32) in registers; the reflectors' vectors come through shared memory, BT_R
+//     rows at a time and one block ahead (cp.async, zeros outside the reflector, so the
+//     products need no tests).  Writes V = y ([k][kept], X = T^H) or Y for the GEMM.
+//     What bounds it: a reflector's chain (loads, dot product, warp sum, update) and its
+//     instructions; the chunks of 32 entries are unrolled for the number still reached (in
+//     steps of two), so they carry no tests.  Measured, all sectors of a chi = 1024 update
+//     alone: 193 us, 527 with the vectors read from L2 by every warp, a test per chunk
+//     and sums by shuffles.
+constexpr int BT_NT = 128, BT_NW = BT_NT / 32;
+constexpr int BT_R = 4;        // reflectors of a block
+
+// Reflectors r = BT_R - 1 .. 0 of a block on a lane's entries y[i], chunk nc - 1 - i, of
+// which the first N can be reached; v: this lane's entry of the first reflector's last chunk.
+template <int N, int NPL>
+__device__ __forceinline__ void bt_block(cplx (&y)[NPL], const double2* v0, int ks, const cplx* taus) {
+  constexpr bool HOLD = N <= 16;       // v in registers between the two products
+#pragma unroll 1
+  for (int r = BT_R - 1; r >= 0; --r) {
+    const double2* v = v0 + r * ks;
+    const cplx tj = ldc(taus + r);
+    double2 x[HOLD ? N : 1];
+    cplx dot[2] = {cmake(0.0, 0.0), cmake(0.0, 0.0)};
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const double2 e = v[-32 * i];
+      if (HOLD) x[HOLD ? i : 0] = e;
+      ccfma(dot[i & 1], cmake(e.x, e.y), y[i]);
+    }
+    const cplx f = cmul(tj, cmake(warp_sum(dot[0].x + dot[1].x), warp_sum(dot[0].y + dot[1].y)));
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const double2 e = HOLD ? x[HOLD ? i : 0] : v[-32 * i];
+      y[i].x = fma(-f.x, e.x, fma(f.y, e.y, y[i].x));
+      y[i].y = fma(-f.x, e.y, fma(-f.y, e.x, y[i].y));
+    }
+  }
+}
+
+template <int N, int NPL>
+__device__ __forceinline__ void bt_blocks(int n, cplx (&y)[NPL], const double2* v0, int ks, const cplx* taus) {
+  if constexpr (N > 2) {
+    if (n <= N - 2) return bt_blocks<N - 2, NPL>(n, y, v0, ks, taus);
+  }
+  bt_block<N, NPL>(y, v0, ks, taus);
+}
+
+template <int NPL>
+__global__ __launch_bounds__(BT_NT) void backtransform_kernel(const SectorDesc* __restrict__ sd,
+                                                              const cplx* __restrict__ gbuf,
+                                                              const cplx* __restrict__ taubuf,
+                                                              const double* __restrict__ zbuf,
+                                                              cplx* __restrict__ vbuf, cplx* __restrict__ ybuf) {
+  extern __shared__ __align__(16) double2 vs[];   // [2][BT_R][ks], then tau [ks]
+  const SectorDesc& S = sd[blockIdx.y];
+  const int k = S.k, kept = S.kept;
+  if ((int)blockIdx.x * BT_NW >= kept) return;    // uniform over the CTA
+  const int tid = threadIdx.x, lane = tid & 31, t = blockIdx.x * BT_NW + (tid >> 5);
+  const bool live = t < kept;
+  const int nc = ((k + 63) >> 6) << 1, ks = nc << 5;   // chunks, an even number
+  const cplx* A = gbuf + S.g_off;
+  const cplx* tau = taubuf + S.s_off;
+  const double* Z = zbuf + S.y_off;
+  cplx y[NPL];
+#pragma unroll
+  for (int i = 0; i < NPL; ++i) {
+    const int l = lane + 32 * (nc - 1 - i);
+    y[i] = cmake(live && l >= 0 && l < k ? Z[(int64_t)l * kept + t] : 0.0, 0.0);
+  }
+  cplx* taus = reinterpret_cast<cplx*>(vs + 2 * BT_R * ks);
+  for (int j = tid; j < ks; j += BT_NT) stc(taus + j, j < k - 1 ? ldc(tau + j) : cmake(0.0, 0.0));
+  const int nb = (k - 1 + BT_R - 1) / BT_R;
+  // block b: v_j of j = b BT_R .. (at columns j+1 .. k-1 of row j, v[j+1] = 1), from the first
+  // pair of chunks that it reaches
+  auto fill = [&](int b) {
+    const int l0 = (b * BT_R + 1) & ~63;
+    for (int r = 0; r < BT_R; ++r) {
+      const int j = b * BT_R + r;
+      double2* dst = vs + ((b & 1) * BT_R + r) * ks;
+      const cplx* src = A + (int64_t)j * k;
+      for (int l = l0 + tid; l < ks; l += BT_NT) {
+        const bool ok = l > j && l < k && j < k - 1;
+        cp_async16(dst + l, ok ? src + l : A, ok);
+      }
+    }
+  };
+  if (nb > 0) fill(nb - 1);
+  cp_async_commit();
+  for (int b = nb - 1; b >= 0; --b) {
+    if (b > 0) fill(b - 1);
+    cp_async_commit();
+    cp_async_wait<1>();
+    __syncthreads();
+    bt_blocks<NPL, NPL>(nc - 2 * ((b * BT_R + 1) >> 6), y, vs + (b & 1) * BT_R * ks + 32 * (nc - 1) + lane, ks,
+                        taus + b * BT_R);
+    __syncthreads();
+  }
+  if (!live) return;
+  cplx* out = S.left ? vbuf + S.v_off : ybuf + S.y_off;
+#pragma unroll
+  for (int i = 0; i < NPL; ++i) {
+    const int l = lane + 32 * (nc - 1 - i);
+    if (l >= 0 && l < k) stc(out + (int64_t)l * kept + t, y[i]);
+  }
+}
+
+// 3c. The same for every eigenvector of the preconditioned sectors (section 4), the
+//     reflectors in blocks of WY_B: H_j0 .. H_{j0+15} = I - V T V^H (V the block's vectors as
+//     columns, T upper triangular).  wy_t_kernel forms T of every block; wy_apply_kernel
+//     applies the blocks, last first, to WY_C vectors held in shared memory: W = V^H Z with
+//     the rows split over the warps, W2 = T W, Z -= V W2, the two products on the FP64 tensor
+//     path with the fragments of V read straight from the Householder vectors.
+//     Why not for 3b: its vectors leave the Gram route's marginals three times further off (T
+//     adds its own rounding); here the Newton-Schulz steps take that out again.  Measured,
+//     one layer at N = 64, chi = 1024, every eigenvector: 3.0 ms against 11.5 with 3b's
+//     kernel.
 constexpr int WY_B = 16;      // reflectors of a block
 constexpr int WY_C = 8;       // vectors of a CTA
 constexpr int WY_NT = 256, WY_NW = WY_NT / 32;
@@ -1130,13 +1240,15 @@ __device__ __forceinline__ cplx wy_v(const cplx* A, int k, int j, int l) {
 }
 
 constexpr int WT_NT = 128;
-__global__ __launch_bounds__(WT_NT) void wy_t_kernel(const SectorDesc* __restrict__ sd, const cplx* __restrict__ gbuf,
-                                                     const cplx* __restrict__ taubuf, cplx* __restrict__ tbuf, bool all) {
+__global__ __launch_bounds__(WT_NT) void wy_t_kernel(const SectorDesc* __restrict__ sd, const int* __restrict__ list,
+                                                     const cplx* __restrict__ gbuf,
+                                                     const cplx* __restrict__ taubuf, cplx* __restrict__ tbuf) {
   __shared__ double2 G[WT_NT / 32][WY_B][WY_B + 1];
   __shared__ cplx T[WY_B][WY_B + 1];
-  const SectorDesc& S = sd[blockIdx.y];
+  const int sec = list[blockIdx.y];
+  const SectorDesc& S = sd[sec];
   const int k = S.k, j0 = blockIdx.x * WY_B;
-  if (j0 >= k - 1 || (!all && S.kept == 0)) return;
+  if (j0 >= k - 1) return;
   const cplx* A = gbuf + S.g_off;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, li = lane >> 2, lk = lane & 3;
   // G = V^H V, rows j0 + 1 .. k - 1 in quarters
@@ -1179,32 +1291,33 @@ __global__ __launch_bounds__(WT_NT) void wy_t_kernel(const SectorDesc* __restric
     }
   }
   __syncthreads();
-  cplx* out = tbuf + wy_t_off(S, blockIdx.y, blockIdx.x);
+  cplx* out = tbuf + wy_t_off(S, sec, blockIdx.x);
   for (int e = tid; e < WY_B * WY_B; e += WT_NT) stc(out + e, T[e / WY_B][e % WY_B]);
 }
 
-__global__ __launch_bounds__(WY_NT) void backtransform_kernel(const SectorDesc* __restrict__ sd,
-                                                              const cplx* __restrict__ gbuf,
-                                                              const cplx* __restrict__ tbuf,
-                                                              const double* __restrict__ zbuf,
-                                                              cplx* __restrict__ vbuf, cplx* __restrict__ ybuf,
-                                                              bool all) {
+__global__ __launch_bounds__(WY_NT) void wy_apply_kernel(const SectorDesc* __restrict__ sd,
+                                                         const int* __restrict__ list,
+                                                         const cplx* __restrict__ gbuf,
+                                                         const cplx* __restrict__ tbuf,
+                                                         const double* __restrict__ zbuf,
+                                                         cplx* __restrict__ ybuf) {
   extern __shared__ __align__(16) double2 Z[];   // [k][WY_LDZ]
   __shared__ double2 Wp[WY_NW][WY_B][WY_C + 1], W[WY_B][WY_LDZ];
-  const SectorDesc& S = sd[blockIdx.y];
-  const int k = S.k, kept = all ? k : S.kept, c0 = blockIdx.x * WY_C;
-  if (c0 >= kept) return;
+  const int sec = list[blockIdx.y];
+  const SectorDesc& S = sd[sec];
+  const int k = S.k, c0 = blockIdx.x * WY_C;
+  if (c0 >= k) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, li = lane >> 2, lk = lane & 3;
   const cplx* A = gbuf + S.g_off;
   const double* z = zbuf + S.y_off;
   for (int e = tid; e < k * WY_C; e += WY_NT) {
     const int l = e / WY_C, c = e % WY_C;
-    Z[l * WY_LDZ + c] = make_double2(c0 + c < kept ? z[(int64_t)l * kept + c0 + c] : 0.0, 0.0);
+    Z[l * WY_LDZ + c] = make_double2(c0 + c < k ? z[(int64_t)l * k + c0 + c] : 0.0, 0.0);
   }
   const int nb = (k - 1 + WY_B - 1) / WY_B;
   for (int b = nb - 1; b >= 0; --b) {
     const int j0 = b * WY_B;
-    const cplx* T = tbuf + wy_t_off(S, blockIdx.y, b);
+    const cplx* T = tbuf + wy_t_off(S, sec, b);
     const cplx te = ldc(T + tid);   // this thread's entry of T
     __syncthreads();
     // W = V^H Z, four rows a step, the steps over the warps
@@ -1270,13 +1383,175 @@ __global__ __launch_bounds__(WY_NT) void backtransform_kernel(const SectorDesc* 
     }
   }
   __syncthreads();
-  cplx* out = S.left && !all ? vbuf + S.v_off : ybuf + S.y_off;
+  cplx* out = ybuf + S.y_off;
   for (int e = tid; e < k * WY_C; e += WY_NT) {
     const int l = e / WY_C, c = e % WY_C;
-    if (c0 + c < kept) {
+    if (c0 + c < k) {
       const double2 v = Z[l * WY_LDZ + c];
-      stc(out + (int64_t)l * kept + c0 + c, cmake(v.x, v.y));
+      stc(out + (int64_t)l * k + c0 + c, cmake(v.x, v.y));
     }
+  }
+}
+
+// ---------------------------------------------------------------------------------
+// 4. The preconditioner of the blocked Jacobi SVD (plain path): a unitary Y close to the
+//    eigenvectors of X^H X, so that the columns of X Y are nearly orthogonal and sorted, and
+//    two or three sweeps replace 8 to 18.  Y comes from every eigenvector of the
+//    tridiagonal (invit_kernel with `all`), orthogonalised within groups of close
+//    eigenvalues here and, after the back-transformation, as a whole by three Newton-Schulz
+//    steps Y <- Y (3 I - Y^H Y) / 2, which square the departure from unitarity and leave it
+//    at rounding level.  The SVD itself stays the one-sided Jacobi iteration on X Y with its
+//    own test, so Y decides how fast it converges, not what it converges to.  Measured: one
+//    layer at N = 64, chi = 1024 on the plain path 223 ms without and 63 with it, an N = 24,
+//    chi = 256 circuit 118 and 57; the marginals of N = 16 to 20 circuits are as far from a
+//    64-bit CPU computation as before (1.1e-13 at most).  A sector whose
+//    Y was not unitary to NS_TOL before the last step (flagged in sd[].kept, which the
+//    selection sets later) starts from X itself.
+constexpr int OR_NT = 256, OR_NW = OR_NT / 32;
+constexpr int OR_P = 8;        // vectors of a panel
+constexpr double NS_TOL = 1e-7;
+
+// Panels of OR_P vectors of a group, in order: each against the group's earlier vectors (32 at
+// a time) and within itself (Gram-Schmidt), the whole twice.
+__global__ __launch_bounds__(OR_NT) void orthogonalise_kernel(const SectorDesc* __restrict__ sd,
+                                                              const int* __restrict__ list,
+                                                              const double* __restrict__ lam,
+                                                              double* __restrict__ zbuf) {
+  extern __shared__ double zp[];   // the panel, [k][OR_P]
+  __shared__ double dots[OR_NW][32][OR_P], coef[32][OR_P], part[OR_NW][OR_P];
+  const SectorDesc& S = sd[list[blockIdx.x]];
+  const int k = S.k, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const double* lv = lam + S.s_off;
+  double* Z = zbuf + S.y_off;      // [k][k]
+  const double gaptol = IV_GAP_ALL * fmax(fabs(lv[0]), fabs(lv[k - 1]));
+  int first = 0;
+  while (first < k) {
+    int end = first + 1;
+    while (end < k && lv[end - 1] - lv[end] <= gaptol) ++end;
+    for (int m0 = first; end > first + 1 && m0 < end; m0 += OR_P) {
+      const int np = min(OR_P, end - m0);
+      for (int e = tid; e < k * OR_P; e += OR_NT) {
+        const int i = e / OR_P, p = e % OR_P;
+        zp[e] = p < np ? Z[(int64_t)i * k + m0 + p] : 0.0;
+      }
+      __syncthreads();
+      for (int pass = 0; pass < 2; ++pass) {
+        for (int g0 = first; g0 < m0; g0 += 32) {
+          const int g = g0 + lane;
+          double acc[OR_P];
+#pragma unroll
+          for (int p = 0; p < OR_P; ++p) acc[p] = 0.0;
+          if (g < m0) {
+#pragma unroll 4
+            for (int i = warp; i < k; i += OR_NW) {
+              const double z = Z[(int64_t)i * k + g];
+#pragma unroll
+              for (int p = 0; p < OR_P; ++p) acc[p] = fma(z, zp[i * OR_P + p], acc[p]);
+            }
+          }
+#pragma unroll
+          for (int p = 0; p < OR_P; ++p) dots[warp][lane][p] = acc[p];
+          __syncthreads();
+          {
+            const int c = tid / OR_P, p = tid % OR_P;   // OR_NT = 32 OR_P
+            double s = 0.0;
+            for (int w = 0; w < OR_NW; ++w) s += dots[w][c][p];
+            coef[c][p] = s;
+          }
+          __syncthreads();
+          const int ng = min(32, m0 - g0);
+          for (int i = tid; i < k; i += OR_NT) {
+            double v[OR_P];
+#pragma unroll
+            for (int p = 0; p < OR_P; ++p) v[p] = zp[i * OR_P + p];
+#pragma unroll 4
+            for (int c = 0; c < ng; ++c) {
+              const double z = Z[(int64_t)i * k + g0 + c];
+#pragma unroll
+              for (int p = 0; p < OR_P; ++p) v[p] = fma(-coef[c][p], z, v[p]);
+            }
+#pragma unroll
+            for (int p = 0; p < OR_P; ++p) zp[i * OR_P + p] = v[p];
+          }
+          __syncthreads();
+        }
+        // within the panel: vector p normalised, then taken out of the later ones
+        for (int p = 0; p < np; ++p) {
+          double acc[OR_P];
+#pragma unroll
+          for (int q = 0; q < OR_P; ++q) acc[q] = 0.0;
+          for (int i = tid; i < k; i += OR_NT) {
+            const double z = zp[i * OR_P + p];
+#pragma unroll
+            for (int q = 0; q < OR_P; ++q) acc[q] = fma(z, zp[i * OR_P + q], acc[q]);
+          }
+#pragma unroll
+          for (int q = 0; q < OR_P; ++q) {
+            const double s = warp_sum(acc[q]);
+            if (lane == 0) part[warp][q] = s;
+          }
+          __syncthreads();
+          double tot[OR_P];
+#pragma unroll
+          for (int q = 0; q < OR_P; ++q) {
+            tot[q] = 0.0;
+            for (int w = 0; w < OR_NW; ++w) tot[q] += part[w][q];
+          }
+          double n2 = 0.0;
+#pragma unroll
+          for (int q = 0; q < OR_P; ++q) n2 = q == p ? tot[q] : n2;
+          const double inv = n2 > 0.0 ? 1.0 / n2 : 0.0, rinv = sqrt(inv);
+          for (int i = tid; i < k; i += OR_NT) {
+            const double z = zp[i * OR_P + p];
+#pragma unroll
+            for (int q = 0; q < OR_P; ++q)
+              if (q > p) zp[i * OR_P + q] = fma(-tot[q] * inv, z, zp[i * OR_P + q]);
+            zp[i * OR_P + p] = z * rinv;
+          }
+          __syncthreads();
+        }
+      }
+      for (int e = tid; e < k * OR_P; e += OR_NT) {
+        const int i = e / OR_P, p = e % OR_P;
+        if (p < np) Z[(int64_t)i * k + m0 + p] = zp[e];
+      }
+      __syncthreads();
+    }
+    first = end;
+  }
+}
+
+// S = Y^H Y -> 3/2 I - S / 2 in place; with check, flags a sector where S is not within NS_TOL
+// of I
+__global__ __launch_bounds__(256) void newton_schulz_kernel(SectorDesc* __restrict__ sd, const int* __restrict__ list,
+                                                            cplx* __restrict__ gbuf, bool check) {
+  SectorDesc& S = sd[list[blockIdx.y]];
+  const int k = S.k;
+  cplx* G = gbuf + S.g_off;
+  bool bad = false;
+  for (int e = blockIdx.x * 256 + threadIdx.x; e < k * k; e += gridDim.x * 256) {
+    const double diag = e / k == e % k ? 1.0 : 0.0;
+    const cplx s = ldc(G + e);
+    bad |= !(fabs(s.x - diag) <= NS_TOL && fabs(s.y) <= NS_TOL);
+    stc(G + e, cmake(1.5 * diag - 0.5 * s.x, -0.5 * s.y));
+  }
+  if (check && bad) S.kept = -1;   // every writer writes the same
+}
+
+// Y below X^H Y in the matrices [T^H; I] Y of the `left` sectors; a flagged sector's matrix
+// is [X; I] or X itself
+__global__ __launch_bounds__(256) void precondition_finish_kernel(const SectorDesc* __restrict__ sd,
+                                                                  const int* __restrict__ list,
+                                                                  const cplx* __restrict__ y, cplx* __restrict__ abuf) {
+  const SectorDesc& S = sd[list[blockIdx.y]];
+  const bool bad = S.kept < 0;
+  const int k = S.k, top = S.rows_g * k, total = S.rows_tot * k;
+  for (int e = (bad ? 0 : top) + blockIdx.x * 256 + threadIdx.x; e < total; e += gridDim.x * 256) {
+    const int r = e - top;
+    const cplx v = r < 0 ? ldc(abuf + S.t_off + e)
+                   : bad ? cmake(r / k == r % k ? 1.0 : 0.0, 0.0)
+                         : ldc(y + S.y_off + r);
+    stc(abuf + S.a_off + e, v);
   }
 }
 
@@ -1371,52 +1646,121 @@ cudaError_t launch_tridiag(const SectorDesc* sd_dev, const int* list_dev, const 
   return cudaSuccess;
 }
 
+namespace {
+
+cudaError_t run_bisect(const SectorDesc* sd, const int* list, int n, int kmax, const double* dbuf, const double* ebuf,
+                       double* lam, cudaStream_t s) {
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      bisect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, eigen_max_k() * (int)sizeof(double2));
+  if (attr != cudaSuccess) return attr;
+  bisect_kernel<<<dim3(ceil_div(kmax, BI_NT / 32), n), BI_NT, (size_t)kmax * sizeof(double2), s>>>(sd, list, dbuf, ebuf,
+                                                                                               lam);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
 cudaError_t launch_bisect(const SectorDesc* sd_dev, int n_sectors, int kmax, const double* dbuf,
                           const double* ebuf, double* lam, double* sig, double* invsig,
                           cudaStream_t s) {
   if (n_sectors <= 0 || kmax <= 0) return cudaSuccess;
-  const size_t smem = (size_t)2 * kmax * sizeof(double);
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(bisect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  dim3 grid(ceil_div(kmax, BI_NT / 32), n_sectors);
-  bisect_kernel<<<grid, BI_NT, smem, s>>>(sd_dev, dbuf, ebuf, lam);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = run_bisect(sd_dev, nullptr, n_sectors, kmax, dbuf, ebuf, lam, s);
   if (e != cudaSuccess) return e;
   eig_finish_kernel<<<n_sectors, FI_NT, 0, s>>>(sd_dev, lam, sig, invsig);
   return cudaGetLastError();
 }
 
-size_t eigvec_t_elems(int64_t s_elems, int n_sectors) {
-  return (size_t)(WY_B * s_elems + (int64_t)WY_B * WY_B * 2 * n_sectors);
+namespace {
+
+cudaError_t run_invit(const SectorDesc* sd, const int* list, int n, int kmax, bool all, const double* dbuf,
+                      const double* ebuf, const double* lam, double* scratch, unsigned char* swp, double* zbuf,
+                      cudaStream_t s) {
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      invit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * eigen_max_k() * (int)sizeof(double));
+  if (attr != cudaSuccess) return attr;
+  invit_kernel<<<n, IV_NT, (size_t)2 * kmax * sizeof(double), s>>>(sd, list, dbuf, ebuf, lam, scratch, swp, zbuf, all);
+  return cudaGetLastError();
 }
 
-cudaError_t launch_eigvec(const SectorDesc* sd_dev, int n_sectors, int kmax, bool all,
-                          const double* dbuf, const double* ebuf, const double* lam,
-                          double* scratch, unsigned char* swp, double* zbuf, const void* gbuf,
-                          const void* taubuf, void* tbuf, void* vbuf, void* ybuf, cudaStream_t s) {
+}  // namespace
+
+cudaError_t launch_eigvec(const SectorDesc* sd_dev, int n_sectors, int kmax, const double* dbuf, const double* ebuf,
+                          const double* lam, double* scratch, unsigned char* swp, double* zbuf, const void* gbuf,
+                          const void* taubuf, void* vbuf, void* ybuf, cudaStream_t s) {
   if (n_sectors <= 0 || kmax <= 0) return cudaSuccess;
   static const cudaError_t attr = [] {
     const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaError_t e = cudaFuncSetAttribute(backtransform_kernel, dyn, eigen_max_k() * WY_LDZ * (int)sizeof(double2));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(invit_kernel, dyn, 2 * eigen_max_k() * (int)sizeof(double));
+    const int most = (2 * BT_R + 1) * (eigen_max_k() + 63) * (int)sizeof(double2);
+    cudaError_t e = cudaFuncSetAttribute(backtransform_kernel<4>, dyn, most);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(backtransform_kernel<8>, dyn, most);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(backtransform_kernel<16>, dyn, most);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(backtransform_kernel<32>, dyn, most);
     return e;
   }();
   if (attr != cudaSuccess) return attr;
-  invit_kernel<<<n_sectors, IV_NT, (size_t)2 * kmax * sizeof(double), s>>>(sd_dev, dbuf, ebuf, lam, scratch, swp, zbuf,
-                                                                          all);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = run_invit(sd_dev, nullptr, n_sectors, kmax, false, dbuf, ebuf, lam, scratch, swp, zbuf, s);
   if (e != cudaSuccess) return e;
+  const cplx* G = reinterpret_cast<const cplx*>(gbuf);
+  const cplx* tau = reinterpret_cast<const cplx*>(taubuf);
+  cplx* V = reinterpret_cast<cplx*>(vbuf);
+  cplx* Y = reinterpret_cast<cplx*>(ybuf);
+  const dim3 grid(ceil_div(kmax, BT_NW), n_sectors);
+  const int npl = 2 * ceil_div(kmax, 64);
+  const size_t smem = (size_t)(2 * BT_R + 1) * 32 * npl * sizeof(double2);
+  if (npl <= 4) backtransform_kernel<4><<<grid, BT_NT, smem, s>>>(sd_dev, G, tau, zbuf, V, Y);
+  else if (npl <= 8) backtransform_kernel<8><<<grid, BT_NT, smem, s>>>(sd_dev, G, tau, zbuf, V, Y);
+  else if (npl <= 16) backtransform_kernel<16><<<grid, BT_NT, smem, s>>>(sd_dev, G, tau, zbuf, V, Y);
+  else if (npl <= 32) backtransform_kernel<32><<<grid, BT_NT, smem, s>>>(sd_dev, G, tau, zbuf, V, Y);
+  else return cudaErrorInvalidValue;
+  return cudaGetLastError();
+}
+
+size_t precondition_t_elems(int64_t s_elems, int n_sectors) {
+  return (size_t)(WY_B * s_elems + (int64_t)WY_B * WY_B * n_sectors);
+}
+
+cudaError_t launch_precondition_basis(const SectorDesc* sd_dev, const int* list_dev, int count, int kmax,
+                                      const double* dbuf, const double* ebuf, double* lam, double* scratch,
+                                      unsigned char* swp, double* zbuf, const void* gbuf, const void* taubuf, void* tbuf,
+                                      void* ybuf, cudaStream_t s) {
+  if (count <= 0) return cudaSuccess;
+  static const cudaError_t attr = [] {
+    const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(wy_apply_kernel, dyn, eigen_max_k() * WY_LDZ * (int)sizeof(double2));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(orthogonalise_kernel, dyn, OR_P * eigen_max_k() * (int)sizeof(double));
+    return e;
+  }();
+  if (attr != cudaSuccess) return attr;
+  cudaError_t e = run_bisect(sd_dev, list_dev, count, kmax, dbuf, ebuf, lam, s);
+  if (e != cudaSuccess) return e;
+  e = run_invit(sd_dev, list_dev, count, kmax, true, dbuf, ebuf, lam, scratch, swp, zbuf, s);
+  if (e != cudaSuccess) return e;
+  orthogonalise_kernel<<<count, OR_NT, (size_t)OR_P * kmax * sizeof(double), s>>>(sd_dev, list_dev, lam, zbuf);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   const cplx* G = reinterpret_cast<const cplx*>(gbuf);
   cplx* T = reinterpret_cast<cplx*>(tbuf);
   if (kmax > 1) {
-    wy_t_kernel<<<dim3(ceil_div(kmax - 1, WY_B), n_sectors), WT_NT, 0, s>>>(
-        sd_dev, G, reinterpret_cast<const cplx*>(taubuf), T, all);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    wy_t_kernel<<<dim3(ceil_div(kmax - 1, WY_B), count), WT_NT, 0, s>>>(sd_dev, list_dev, G,
+                                                                        reinterpret_cast<const cplx*>(taubuf), T);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
-  backtransform_kernel<<<dim3(ceil_div(kmax, WY_C), n_sectors), WY_NT, (size_t)kmax * WY_LDZ * sizeof(double2), s>>>(
-      sd_dev, G, T, zbuf, reinterpret_cast<cplx*>(vbuf), reinterpret_cast<cplx*>(ybuf), all);
+  wy_apply_kernel<<<dim3(ceil_div(kmax, WY_C), count), WY_NT, (size_t)kmax * WY_LDZ * sizeof(double2), s>>>(
+      sd_dev, list_dev, G, T, zbuf, reinterpret_cast<cplx*>(ybuf));
+  return cudaGetLastError();
+}
+
+cudaError_t launch_newton_schulz(SectorDesc* sd_dev, const int* list_dev, int count, int kmax, void* gbuf, bool check,
+                                 cudaStream_t s) {
+  if (count <= 0) return cudaSuccess;
+  newton_schulz_kernel<<<dim3(std::min(ceil_div(kmax * kmax, 1024), 64), count), 256, 0, s>>>(
+      sd_dev, list_dev, reinterpret_cast<cplx*>(gbuf), check);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_precondition_finish(const SectorDesc* sd_dev, const int* list_dev, int count, int max_elems,
+                                       const void* ybuf, void* abuf, cudaStream_t s) {
+  if (count <= 0) return cudaSuccess;
+  precondition_finish_kernel<<<dim3(std::min(ceil_div(std::max(max_elems, 1), 1024), 64), count), 256, 0, s>>>(
+      sd_dev, list_dev, reinterpret_cast<const cplx*>(ybuf), reinterpret_cast<cplx*>(abuf));
   return cudaGetLastError();
 }

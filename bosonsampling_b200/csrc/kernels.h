@@ -72,6 +72,8 @@ struct SectorDesc {
   int slot0;           // first slot of this sector on the new bond
   int64_t c_off;       // C[m][n] row-major (complex)
   int64_t a_off;       // Jacobi matrix, row-major [rows_tot][k] (complex)
+  int64_t t_off;       // its first rows_g rows as the mix writes them (a_off, or where a
+                       // preconditioned sector's T or T^H stays)
   int64_t s_off;       // singular values / keys / permutation (k entries)
   int64_t w_off;       // W = V^H C, [kept][n] row-major (complex)
   int64_t v_off;       // V, [m][kept] row-major (complex)
@@ -196,13 +198,24 @@ cudaError_t launch_bisect(const SectorDesc* sd_dev, int n_sectors, int kmax, con
                           const double* ebuf, double* lam, double* sig, double* invsig,
                           cudaStream_t s);
 // eigenvectors of the kept eigenvalues (sd[s].kept): V ([k][kept] at v_off) of the
-// sectors with X = T^H, Y ([k][kept] at y_off) of the others; with `all`, of every eigenvalue
-// and all at y_off ([k][k]).  tbuf: eigvec_t_elems complex entries.
-size_t eigvec_t_elems(int64_t s_elems, int n_sectors);
-cudaError_t launch_eigvec(const SectorDesc* sd_dev, int n_sectors, int kmax, bool all,
-                          const double* dbuf, const double* ebuf, const double* lam,
-                          double* scratch, unsigned char* swp, double* zbuf, const void* gbuf,
-                          const void* taubuf, void* tbuf, void* vbuf, void* ybuf, cudaStream_t s);
+// sectors with X = T^H, Y ([k][kept] at y_off) of the others.
+cudaError_t launch_eigvec(const SectorDesc* sd_dev, int n_sectors, int kmax, const double* dbuf, const double* ebuf,
+                          const double* lam, double* scratch, unsigned char* swp, double* zbuf, const void* gbuf,
+                          const void* taubuf, void* vbuf, void* ybuf, cudaStream_t s);
+// The preconditioner of the blocked Jacobi SVD (see eigen.cu) of the listed sectors, from
+// their tridiagonals: every eigenvector, nearly unitary, to ybuf ([k][k] at y_off); 3/2 I -
+// S / 2 in place of S = Y^H Y (check: a sector whose S is too far from I gets kept = -1); and
+// Y into the matrices [T^H; I] Y, or the unpreconditioned matrix of a flagged sector
+// (max_elems: the largest rows_tot k).  tbuf: precondition_t_elems complex entries.
+size_t precondition_t_elems(int64_t s_elems, int n_sectors);
+cudaError_t launch_precondition_basis(const SectorDesc* sd_dev, const int* list_dev, int count, int kmax,
+                                      const double* dbuf, const double* ebuf, double* lam, double* scratch,
+                                      unsigned char* swp, double* zbuf, const void* gbuf, const void* taubuf, void* tbuf,
+                                      void* ybuf, cudaStream_t s);
+cudaError_t launch_newton_schulz(SectorDesc* sd_dev, const int* list_dev, int count, int kmax, void* gbuf, bool check,
+                                 cudaStream_t s);
+cudaError_t launch_precondition_finish(const SectorDesc* sd_dev, const int* list_dev, int count, int max_elems,
+                                       const void* ybuf, void* abuf, cudaStream_t s);
 
 // ---------------------------------------------------------------- tcgemm.cu
 // One group of the tensor-core (tcgen05, 3 x TF32) grouped complex GEMM:

@@ -91,7 +91,7 @@ __global__ __launch_bounds__(MIX_NT) void mix_kernel(const UpdateTables* __restr
       if (s >= 0) {
         const SectorDesc& S = sd[s];
         cb[i0][i1] = S.c_off;
-        ab[i0][i1] = S.a_off;
+        ab[i0][i1] = S.t_off;
         cn[i0][i1] = S.n;
         ck[i0][i1] = S.k;
         cleft[i0][i1] = S.left;
@@ -149,7 +149,7 @@ __global__ __launch_bounds__(MIX_NT) void mix_kernel(const UpdateTables* __restr
 
 __global__ void identity_rows_kernel(const SectorDesc* __restrict__ sd, cplx* __restrict__ abuf) {
   const SectorDesc& S = sd[blockIdx.y];
-  if (!S.left) return;
+  if (!S.left || S.t_off != S.a_off) return;   // a preconditioned sector gets Y there
   const int m = S.m;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m * m; e += gridDim.x * blockDim.x) {
     const int i = e / m, j = e % m;
