@@ -33,6 +33,7 @@ namespace {
 thread_local std::string g_last_error;
 
 constexpr int MAX_SWEEPS = 40;
+constexpr int WAIT_POLL_US = 400;   // host waits poll this long before they sleep
 constexpr int MESH_LANES = 2;   // streams a mesh's groups of updates are spread over
 
 struct DevBuf {
@@ -155,18 +156,15 @@ int fail(bsmpo_ctx* h, int code, const std::string& msg) {
 // the host mirror of the charge-block sizes (a worker's is its owner's)
 std::vector<int>& mirror(bsmpo_ctx* h) { return h->cnt_shared ? *h->cnt_shared : h->cnt; }
 
-// waits (sleeping) until the handle's stream has drained
-// the forked streams of the tridiagonalisation's size classes and their events, created
-// once (for a worker when it is made, so the order of stream creation, which decides
-// the streams' hardware queues, is fixed)
-int make_fork_streams(bsmpo_ctx* h) {
-  if (h->fork_ev) return BSMPO_OK;
-  if (cudaEventCreateWithFlags(&h->fork_ev, cudaEventDisableTiming) != cudaSuccess) {
+// the first n side streams of the tridiagonalisation's size classes (at most td_fork) and
+// their events, created when a group first needs them: a small circuit's never do
+int make_fork_streams(bsmpo_ctx* h, int n) {
+  if (!h->fork_ev && cudaEventCreateWithFlags(&h->fork_ev, cudaEventDisableTiming) != cudaSuccess) {
     cudaGetLastError();
     h->fork_ev = nullptr;
     return fail(h, BSMPO_ECUDA, "fork event creation failed");
   }
-  for (int i = 0; i < std::min(h->td_fork, 3); ++i) {
+  for (int i = h->n_aux; i < std::min(n, std::min(h->td_fork, 3)); ++i) {
     if (cudaStreamCreateWithFlags(&h->aux[i], cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&h->join_ev[i], cudaEventDisableTiming) != cudaSuccess) {
       cudaGetLastError();
@@ -177,6 +175,20 @@ int make_fork_streams(bsmpo_ctx* h) {
   return BSMPO_OK;
 }
 
+// Waits for an event: a short wait is polled (a sleeping wait wakes up tens of us late, as
+// long as a small update takes), a longer one sleeps, so that the waits of several lanes
+// leave the host cores to the launching threads.
+cudaError_t wait_event(cudaEvent_t ev) {
+  const auto t0 = std::chrono::steady_clock::now();
+  do {
+    const cudaError_t e = cudaEventQuery(ev);
+    if (e != cudaErrorNotReady) return e;
+    cudaGetLastError();   // not ready is recorded, but no error
+  } while (std::chrono::steady_clock::now() - t0 < std::chrono::microseconds(WAIT_POLL_US));
+  return cudaEventSynchronize(ev);
+}
+
+// waits until the handle's stream has drained
 cudaError_t host_wait(bsmpo_ctx* h) {
   if (!h->wait_ev) {
     cudaError_t e = cudaEventCreateWithFlags(&h->wait_ev, cudaEventBlockingSync | cudaEventDisableTiming);
@@ -184,7 +196,7 @@ cudaError_t host_wait(bsmpo_ctx* h) {
   }
   cudaError_t e = cudaEventRecord(h->wait_ev, h->stream);
   if (e != cudaSuccess) return e;
-  return cudaEventSynchronize(h->wait_ev);
+  return wait_event(h->wait_ev);
 }
 
 #define CK(h, call)                                                                    \
@@ -226,8 +238,9 @@ int grow_host(bsmpo_ctx* h, HostStage& b, size_t bytes) {
   if (b.p) h->retired_host.push_back(b.p);
   b.p = nullptr;
   b.bytes = 0;
-  // pinned host memory: rare, generous growth
-  size_t want = std::max<size_t>(align_up(bytes + bytes / 2 + 256, 256), 1 << 20);
+  // pinned host memory: rare, generous growth (pinning costs by the page: 1 MB at least, as
+  // it was, made eight small handles' stages 75 of a batch's 130 ms)
+  size_t want = std::max<size_t>(align_up(2 * bytes, 4096), 1 << 15);
   h->host_grows++;
   CK(h, cudaMallocHost(&b.p, want));
   b.bytes = want;
@@ -723,8 +736,10 @@ int gram_tridiagonal(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, const 
                               nullptr, st));
   // the largest class present on the update's stream, the others dealt out to the side
   // streams (none: all one after another)
-  if (h->td_fork > 0 && (rc = make_fork_streams(h))) return rc;
-  const int naux = std::min(h->td_fork, h->n_aux);
+  int classes = 0;
+  for (int c = 0; c < TD_CLASSES; ++c) classes += P.td_count[c] > 0;
+  if (classes > 1 && (rc = make_fork_streams(h, classes - 1))) return rc;
+  const int naux = std::min(classes - 1, h->n_aux);
   cudaStream_t ts[TD_CLASSES];
   bool used[3] = {false, false, false};
   for (int c = TD_CLASSES - 1, slot = -1; c >= 0; --c) {
@@ -868,7 +883,7 @@ int jacobi_svd(bsmpo_ctx* h, const Plan& P, SectorDesc* sd_d, char* jw_d, const 
   // beside the blocked rounds, where there are any, on the first side stream
   cudaStream_t small_st = st;
   if (P.n_small && n_big && h->td_fork > 0) {
-    if ((rc = make_fork_streams(h))) return rc;
+    if ((rc = make_fork_streams(h, 1))) return rc;
     if (h->n_aux > 0) {
       small_st = h->aux[0];
       CK(h, cudaEventRecord(h->fork_ev, st));
@@ -936,7 +951,7 @@ int jacobi_svd(bsmpo_ctx* h, const Plan& P, SectorDesc* sd_d, char* jw_d, const 
   for (;;) {
     const bool more = t < t_max;
     if (more && (rc = launch_chunk(cur ^ 1))) return rc;
-    CK(h, cudaEventSynchronize(h->poll_ev[cur]));
+    CK(h, wait_event(h->poll_ev[cur]));
     ++checks;
     const int* hrot = hrot_slot[cur];
     bool all = true;
@@ -1162,7 +1177,7 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
   };
   if ((rc = select())) return rc;
   if (P.gram && h->gram_policy >= 1) {
-    CK(h, cudaEventSynchronize(h->wait_ev));
+    CK(h, wait_event(h->wait_ev));
     if (*htc == 0 && hk[ns] < chi && h->cutoff == 0.0) {
       // not truncated to chi (groups of one update under this policy): redo the SVD
       // exactly; the Jacobi matrix is intact
@@ -1210,7 +1225,7 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
                             reinterpret_cast<int*>(h->perm.p), h->vbuf.p, st));
   }
   if (tc_w) {
-    CK(h, cudaEventSynchronize(h->wait_ev));
+    CK(h, wait_event(h->wait_ev));
     if ((rc = tc_w_gemm(h, P, hk, tcerr_d))) return rc;
   } else {
     CKL(h, launch_zgemm_grouped(h->vbuf.p, h->cbuf.p, h->wbuf.p, nullptr, groups_at(L.gw), (int)P.gw.size(),
@@ -1221,7 +1236,7 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
   CKL(h, launch_scatter(tab_d, sd_d, nj, kept_d + ns, chi, h->vbuf.p, h->wbuf.p,
                         reinterpret_cast<double*>(h->sig.p), h->gamma, h->lam, h->charge, st));
   if ((rc = clk.mark(6))) return rc;
-  CK(h, cudaEventSynchronize(h->wait_ev));
+  CK(h, wait_event(h->wait_ev));
   if (*htc != 0)
     return fail(h, BSMPO_ECUDA, "tensor-core GEMM or tridiagonalisation: a pipeline wait expired (error word set)");
   if (htc[1] != 0) return fail(h, BSMPO_ECONVERGE, "Jacobi SVD did not converge (a small sector)");
@@ -1337,11 +1352,6 @@ int make_worker(bsmpo_ctx* h, bsmpo_ctx** out) {
     cudaGetLastError();
     delete w;
     return fail(h, BSMPO_ECUDA, "worker stream creation failed");
-  }
-  if (w->td_fork && make_fork_streams(w) != BSMPO_OK) {
-    const std::string msg = w->err;
-    destroy_worker(w);
-    return fail(h, BSMPO_ECUDA, msg);
   }
   *out = w;
   return BSMPO_OK;
