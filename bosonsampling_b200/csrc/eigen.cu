@@ -821,10 +821,14 @@ __global__ __launch_bounds__(BI_NT) void bisect_kernel(const SectorDesc* __restr
   lo = red[0][0];
   hi = red[1][0];
   for (int w = 1; w < BI_NT / 32; ++w) { lo = fmin(lo, red[0][w]); hi = fmax(hi, red[1][w]); }
-  // a power of two above the bound of the spectrum; a zero matrix is left as it is
   const double span = fmax(fabs(lo), fabs(hi));
-  int ex = 0;
-  if (span > 0.0) frexp(span, &ex);
+  if (span == 0.0) {                   // a zero matrix (uniform over the CTA)
+    if (tid < BI_NT / 32 && first + tid < k) lam[S.s_off + first + tid] = 0.0;
+    return;
+  }
+  // a power of two above the bound of the spectrum
+  int ex;
+  frexp(span, &ex);
   for (int i = tid; i < k; i += BI_NT) {
     const double e = scalbn(de[i].y, -ex);
     de[i] = make_double2(scalbn(de[i].x, -ex), fmax(e * e, BI_E2));
