@@ -112,6 +112,7 @@ struct bsmpo_ctx {
   // streams each are the device's 8 hardware queues (CUDA_DEVICE_MAX_CONNECTIONS' default)
   int td_fork = 3;
   int n_aux = 0;   // side streams created
+  cudaStream_t copy_out = nullptr;   // worker: site copies to the host (meshes over a host state)
   HostStage stage, stage2, hres;
   // last update diagnostics (host)
   std::vector<int> last_cc, last_shape, last_kept, last_k;
@@ -1327,6 +1328,7 @@ void free_workspaces(bsmpo_ctx* h) {
   if (h->wait_ev) cudaEventDestroy(h->wait_ev);
   for (cudaEvent_t& e : h->poll_ev)
     if (e) cudaEventDestroy(e);
+  if (h->copy_out) { cudaStreamSynchronize(h->copy_out); cudaStreamDestroy(h->copy_out); }
   if (h->fork_ev) cudaEventDestroy(h->fork_ev);
   if (h->td_ev0) cudaEventDestroy(h->td_ev0);
   if (h->td_ev1) cudaEventDestroy(h->td_ev1);
@@ -1516,13 +1518,18 @@ int run_mesh_concurrent(bsmpo_ctx* h, int n_bs, const int* modes, const cplx* u3
         for (size_t i = 0; i < jobs.size() && !r; ++i) h->mesh_tw[jobs[i].index] = tw[i];
         if (!r && cudaEventRecord(mine, w->stream) != cudaSuccess)
           r = fail(w, BSMPO_ECUDA, "cudaEventRecord failed");
+        if (hs && !r && !w->copy_out && cudaStreamCreateWithFlags(&w->copy_out, cudaStreamNonBlocking) != cudaSuccess)
+          r = fail(w, BSMPO_ECUDA, "stream creation failed");
+        if (hs && !r && cudaStreamWaitEvent(w->copy_out, mine, 0) != cudaSuccess)
+          r = fail(w, BSMPO_ECUDA, "cudaStreamWaitEvent failed");
         for (const Job& j : jobs)
           for (int site = j.mode; hs && site <= j.mode + 1 && !r; ++site)
-            // the site's final value of this mesh: copied out behind the update
+            // the site's final value of this mesh: copied out behind the update, beside the
+            // lane's next group, whose own sites come in meanwhile
             if (hs->last[site] == j.index &&
                 cudaMemcpyAsync(hs->gamma_out + (size_t)site * hs->site_bytes,
                                 reinterpret_cast<const char*>(h->gamma) + (size_t)site * hs->site_bytes,
-                                hs->site_bytes, cudaMemcpyDeviceToHost, w->stream) != cudaSuccess)
+                                hs->site_bytes, cudaMemcpyDeviceToHost, w->copy_out) != cudaSuccess)
               r = fail(w, BSMPO_ECUDA, "site copy-out failed");
         std::lock_guard<std::mutex> lock(mu);
         ++idle;
@@ -1540,7 +1547,11 @@ int run_mesh_concurrent(bsmpo_ctx* h, int n_bs, const int* modes, const cplx* u3
     });
   for (auto& t : pool) t.join();
   for (int wk = 0; wk < lanes; ++wk) {
-    const cudaError_t e = host_wait(h->workers[wk]);
+    cudaError_t e = host_wait(h->workers[wk]);
+    if (hs && h->workers[wk]->copy_out) {
+      const cudaError_t e2 = cudaStreamSynchronize(h->workers[wk]->copy_out);
+      if (e == cudaSuccess) e = e2;
+    }
     if (e != cudaSuccess && !err_code) { err_code = BSMPO_ECUDA; err_msg = cudaGetErrorString(e); }
   }
   for (cudaEvent_t e : done_ev) cudaEventDestroy(e);
