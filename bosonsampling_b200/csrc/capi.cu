@@ -35,6 +35,7 @@ thread_local std::string g_last_error;
 constexpr int MAX_SWEEPS = 40;
 constexpr int WAIT_POLL_US = 400;   // host waits poll this long before they sleep
 constexpr int MESH_LANES = 2;   // streams a mesh's groups of updates are spread over
+constexpr int MAX_GROUP = 32;   // updates of a group
 
 struct DevBuf {
   void* p = nullptr;
@@ -1399,8 +1400,16 @@ int run_mesh_concurrent(bsmpo_ctx* h, int n_bs, const int* modes, const cplx* u3
   const int d3 = h->d * h->d * h->d;
   int rc;
   const int lanes = std::min(nw, MESH_LANES);
+  // Four updates to a worker up to chi = 512, where an update's launches leave most of the
+  // chip idle and four hold the workspace of one at chi = 1,024.  Circuits with 8 workers,
+  // one and four to a worker, ms: 24 modes chi = 64 9.5 and 8.2, chi = 128 11.7 and 10.3,
+  // chi = 256 fp64 45.9 and 38.8; 32 modes chi = 256 42.3 and 31.2, chi = 384 79.9 and
+  // 67.0, chi = 512 150 and 140, fp64 214 and 168.  Two layers at N = 64, chi = 1,024: no
+  // gain from 32 workers over 16 (46.3 and 46.8) for twice the memory.
+  const int fill = h->chi <= 512 ? 4 : 1;
   // updates per group; a policy that may redo an update's SVD takes them one by one
-  const int cap = h->gram_policy >= 1 && h->precision != BSMPO_PRECISION_FP64 ? 1 : ceil_div(nw, lanes);
+  const int cap = h->gram_policy >= 1 && h->precision != BSMPO_PRECISION_FP64
+                      ? 1 : std::min(MAX_GROUP, fill * ceil_div(nw, lanes));
   while ((int)h->workers.size() < lanes) {
     bsmpo_ctx* w = nullptr;
     if ((rc = make_worker(h, &w))) return rc;
