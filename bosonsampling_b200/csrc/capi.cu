@@ -357,7 +357,7 @@ Route route_of(bsmpo_ctx* h, int mode) {
 }
 
 // Jacobi route: whether a sector of the blocked form starts from a preconditioned matrix.
-bool preconditioned(const SectorDesc& S) { return !jacobi_is_small(S.rows_tot, S.k) && S.k <= eigen_max_k(); }
+bool preconditioned(const SectorDesc& S) { return !jacobi_is_small(S.rows_g, S.k) && S.k <= eigen_max_k(); }
 
 // Adds the update at `mode` to the plan.
 int add_update(bsmpo_ctx* h, int mode, int64_t gate_off, Plan& P) {
@@ -602,9 +602,9 @@ void finish_plan(bsmpo_ctx* h, Plan& P) {
   for (int s = 0; s < ns; ++s) {
     const SectorDesc& S = P.sd[s];
     if (S.left) P.max_left_m2 = std::max(P.max_left_m2, S.m * S.m);
-    if (jacobi_is_small(S.rows_tot, S.k)) {
+    if (jacobi_is_small(S.rows_g, S.k)) {
       P.tdlist.push_back(s);
-      P.small_elems = std::max(P.small_elems, jacobi_small_elems(S.rows_tot, S.k));
+      P.small_elems = std::max(P.small_elems, jacobi_small_elems(S.rows_g, S.k));
       P.small_k = std::max(P.small_k, S.k);
       continue;
     }

@@ -552,103 +552,352 @@ __global__ __launch_bounds__(NNT) void sector_norm_kernel(const SectorDesc* __re
 }
 
 // ---------------------------------------------------------------------------------
-// Small sectors: the whole SVD of a sector in one CTA.  The Jacobi matrix lives in shared
-// memory by columns; a sweep is the circle method over single columns, a warp to a column
-// pair: dot products over the Gram rows, the rotation, its application to all rows, with
-// the tests and the floor of the blocked form above.  All sweeps, the column norms and the
-// sort run here, so such a sector needs no rounds of launches and no convergence polls.
-// What bounds it: the latency of a step (loads, 130 cycles of reduction, 200 of reciprocal
-// square roots, a barrier), k - 1 steps a sweep.  The blocked form pays two launches of
-// ~45 us a round and the host's polls: a 9-mode chi = 50 circuit took 16 ms with it and takes
-// 5.9, one update at chi = 32 1.58 ms and 0.47.
-constexpr int JS_KMAX = 48;
+// Small sectors: the whole SVD of a sector in one CTA, preconditioned by QR with column
+// pivoting (Drmac and Veselic, SIAM J. Matrix Anal. Appl. 29, 2008).  X is the Jacobi matrix's
+// Gram part, rows x k, in shared memory by columns:
+//   X P = Q R;  left sectors (X = T^H): T = P R^H Q^H, so T's left vectors are P times those
+//   of L = R^H; the others (X = T): R^H P2 = Q2 R2, T's left vectors are Q P2 times those of
+//   L = R2^H.
+// One-sided Jacobi on the k columns of L gives L W = U Sigma; its normalised columns are the
+// left vectors, so no rotation is accumulated.  A sweep is the circle method over single
+// columns, eight lanes to a column pair with the columns in their registers: dot products,
+// the rotation, its application, with the tests and the floor of the blocked form above.
+// All sweeps, the norms and the sort run here: no rounds of launches, no convergence polls.
+// What bounds it: a step's latency and its FP64 issue on one SM.  At k = 48 a step of a sweep
+// takes 1,225 cycles (five to seven sweeps of k - 1 steps), a step of a QR 2,250 up to 64 rows
+// and 4,100 up to 128.  Without the factorisations, a warp to a pair over all rows and the
+// accumulated rotations (six to twelve sweeps where the sector is graded), before and after,
+// us: k = 28, 128 rows 209 and 154 (X = T), 230 and 107 (X = T^H); k = 48, 128 rows 545 and
+// 360, 674 and 287; graded sectors of a 24-mode circuit up to 1,090 and 340.  A 24-mode chi =
+// 256 circuit 40.6 ms and 36.3, 32 modes on the Gram route 30.7 and 27.0, 24 modes chi = 64
+// 13.8 and 10.0, chi = 128 31 and 20.5.
+constexpr int JS_KMAX = 64;
+constexpr int JS_SMEM = 216 * 1024;
 
 // leading dimension of a column: odd in units of 16 B, so lanes across columns fall on
 // different banks
 __host__ __device__ inline int js_ld(int rows) { return rows | 1; }
-inline size_t js_smem(int rows, int k) { return (size_t)js_ld(rows) * k * sizeof(double2) + JS_KMAX * sizeof(double); }
+__host__ __device__ inline int js_ldl(int k) { return (k + 15) / 16 * 16 + 1; }   // of L
 
-// (a, b, gx, gy) summed over the warp, in every lane.  Each value's product with ones leaves
-// a lane its four-lane sums of columns 2 (lane & 3) and 2 (lane & 3) + 1; a last product
-// whose right operand is value n in column n adds the four pairs of all values at once.
-__device__ __forceinline__ void sum4(double& a, double& b, double& gx, double& gy) {
-  const int lane = threadIdx.x & 31, n = (lane >> 2) & 3;
-  double2 s0 = make_double2(0, 0), s1 = s0, s2 = s0, s3 = s0, t = s0;
-  dmma8x8x4(s0, 1.0, a);
-  dmma8x8x4(s1, 1.0, b);
-  dmma8x8x4(s2, 1.0, gx);
-  dmma8x8x4(s3, 1.0, gy);
-  const double e0 = s0.x + s0.y, e1 = s1.x + s1.y, e2 = s2.x + s2.y, e3 = s3.x + s3.y;
-  dmma8x8x4(t, 1.0, n == 0 ? e0 : n == 1 ? e1 : n == 2 ? e2 : e3);
-  // lanes with an even lane & 3 hold (a, b), the others (gx, gy)
-  const double ox = __shfl_xor_sync(0xffffffffu, t.x, 1), oy = __shfl_xor_sync(0xffffffffu, t.y, 1);
-  const bool ab = (lane & 1) == 0;
-  a = ab ? t.x : ox;
-  b = ab ? t.y : oy;
-  gx = ab ? ox : t.x;
-  gy = ab ? oy : t.y;
+// a summed over each LPC consecutive lanes (8, 16 or 32), in every one of them: a product
+// with ones leaves lane i & 3 the four-lane sums of columns 2 i and 2 i + 1, lanes 8 i..8 i + 7
+template <int LPC>
+__device__ __forceinline__ double group_sum(double a) {
+  double2 s = make_double2(0, 0);
+  __syncwarp();
+  dmma8x8x4(s, 1.0, a);
+  const double e = s.x + s.y;
+  const int first = (threadIdx.x & 31) / LPC * (LPC / 8);
+  double t = __shfl_sync(0xffffffffu, e, first);
+#pragma unroll
+  for (int i = 1; i < LPC / 8; ++i) t += __shfl_sync(0xffffffffu, e, first + i);
+  return t;
 }
 
-// One column pair: RC chunks of 32 rows held in registers between the dot products and the
-// rotation (0: read again).  Returns whether it rotated.
-template <int RC>
-__device__ __forceinline__ bool js_pair(double2* x, double2* y, int rows_g, int rows, double z2, double t2) {
-  const int lane = threadIdx.x & 31;
-  constexpr int R = RC > 0 ? RC : 1;
-  double2 u[R], v[R];
-  double a = 0.0, b = 0.0, gx = 0.0, gy = 0.0;
-  auto dot = [&](double2 p, double2 q) {
-    a = fma(p.x, p.x, fma(p.y, p.y, a));
-    b = fma(q.x, q.x, fma(q.y, q.y, b));
-    gx = fma(p.x, q.x, fma(p.y, q.y, gx));
-    gy = fma(p.x, q.y, fma(-p.y, q.x, gy));
-  };
-  if (RC > 0) {
-#pragma unroll
-    for (int c = 0; c < R; ++c) {
-      const int r = lane + 32 * c;
-      u[c] = v[c] = make_double2(0.0, 0.0);
-      if (r < rows) { u[c] = x[r]; v[c] = y[r]; }
+// X P = Q R of one matrix: the reflectors H_j = 1 - t_j v_j v_j^H, v_j the rows below j of
+// column piv[j] under v1[j]; R's diagonal rd, its row i < j in row i of column piv[j].
+struct JsQr {
+  double nn[2][JS_KMAX];   // squared norms of the columns' rows below the reduced ones, -1: reduced
+  double2 rd[JS_KMAX], v1[JS_KMAX];
+  double t[JS_KMAX];
+  int piv[JS_KMAX];
+};
+
+// Steps [j0, j1) of the factorisation, whose rows below j lie in chunks F..RPL - 1 of LPC rows
+// (chunk F alone holds rows above them too): no test per chunk, so a column's loads are in
+// flight together.  Returns false where nothing is left to reduce.
+template <int LPC, int RPL, int F>
+__device__ __forceinline__ bool js_qr_steps(double2* X, int ld, int rows, int k, JsQr& q, int n_warps, int j0, int j1) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int GPW = 32 / LPC, R = RPL > 0 ? RPL : 1;
+  const int g = lane / LPC, l = lane % LPC;
+  for (int j = j0; j < j1; ++j) {
+    const double* nn = q.nn[j & 1];
+    double* next = q.nn[(j + 1) & 1];
+    // a largest column, by the leading 32 bits of its norm
+    auto key = [&](int c) { return c >= k ? -2 : nn[c] < 0.0 ? -1 : __double2hiint(nn[c]) & 0x7fffffff; };
+    const int h0 = key(lane), h1 = key(lane + 32);
+    const int hm = __reduce_max_sync(0xffffffffu, max(h0, h1));
+    const unsigned in0 = __ballot_sync(0xffffffffu, h0 == hm), in1 = __ballot_sync(0xffffffffu, h1 == hm);
+    const int p = in0 ? __ffs(in0) - 1 : 31 + __ffs(in1);
+    const double n2 = nn[p];
+    if (n2 < 1e-270) {                 // nothing left (uniform over the CTA): R's other rows are zero
+      if (tid == 0) {
+        int at = j;
+        for (int c = 0; c < k; ++c)
+          if (nn[c] >= 0.0) q.piv[at++] = c;
+      }
+      for (int i = j + tid; i < k; i += 32 * n_warps) {
+        q.rd[i] = q.v1[i] = make_double2(0.0, 0.0);
+        q.t[i] = 0.0;
+      }
+      return false;
     }
+    const double2 *vp = X + p * ld, al = vp[j];
+    double2 v[R];                      // the reflector below its head
+    if (RPL > 0) {
 #pragma unroll
-    for (int c = 0; c < R; ++c)
-      if (lane + 32 * c < rows_g) dot(u[c], v[c]);
-  } else {
-#pragma unroll 4
-    for (int r = lane; r < rows_g; r += 32) dot(x[r], y[r]);
-  }
-  sum4(a, b, gx, gy);
-  const double g2 = gx * gx + gy * gy;
-  if (!(a > z2 && b > z2 && a > t2 * b && b > t2 * a && g2 > t2 * a * b)) return false;   // warp-uniform
-  // the rotation of the blocked form: c, s e^{i alpha} of the small angle
-  const double dd = b - a, ir = rsqrt(fma(dd, dd, 4.0 * g2)), c2 = fma(0.5 * fabs(dd), ir, 0.5), ic = rsqrt(c2);
-  const double c = c2 * ic, f = copysign(ir * ic, dd), sx = f * gx, sy = f * gy;
-  auto turn = [&](double2& p, double2& q) {
-    // p' = c p - conj(s) q, q' = s p + c q
-    const double2 n = make_double2(c * p.x - (sx * q.x + sy * q.y), c * p.y - (sx * q.y - sy * q.x));
-    q = make_double2(fma(c, q.x, sx * p.x - sy * p.y), fma(c, q.y, sx * p.y + sy * p.x));
-    p = n;
-  };
-  if (RC > 0) {
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-      const int r = lane + 32 * k;
-      if (r < rows) {
-        turn(u[k], v[k]);
-        x[r] = u[k];
-        y[r] = v[k];
+      for (int i = F; i < R; ++i) {
+        const int r = l + LPC * i;
+        v[i] = (i > F || r > j) && r < rows ? vp[r] : make_double2(0.0, 0.0);
       }
     }
-  } else {
-#pragma unroll 4
-    for (int r = lane; r < rows; r += 32) {
-      double2 p = x[r], q = y[r];
-      turn(p, q);
-      x[r] = p;
-      y[r] = q;
+    const double a2 = fma(al.x, al.x, al.y * al.y), nx = n2 * rsqrt(n2);
+    double t;
+    double2 v1, beta;
+    if (a2 > 1e-34 * n2) {
+      const double ra = rsqrt(a2), f = nx * ra;
+      t = __drcp_rn(fma(nx, a2 * ra, n2));
+      beta = make_double2(-al.x * f, -al.y * f);
+      v1 = make_double2(al.x - beta.x, al.y - beta.y);
+    } else {
+      // a head below the rounding of nx
+      t = __drcp_rn(n2);
+      beta = make_double2(-nx, 0.0);
+      v1 = make_double2(nx, 0.0);
     }
+    if (tid == 0) {
+      q.piv[j] = p;
+      q.rd[j] = beta;
+      q.v1[j] = v1;
+      q.t[j] = t;
+    }
+    for (int base = warp * GPW; base < k; base += n_warps * GPW) {
+      const int c = base + g;
+      const bool act = c < k && c != p && nn[c] >= 0.0;
+      double2* x = X + (act ? c : p) * ld;
+      double dx = 0.0, dy = 0.0, s = 0.0;
+      auto dot = [&](double2 a, double2 b) {   // conj(a) b
+        dx = fma(a.x, b.x, fma(a.y, b.y, dx));
+        dy = fma(a.x, b.y, fma(-a.y, b.x, dy));
+      };
+      auto sub = [&](double2 a, double2 b) {   // b - w a, w in (dx, dy)
+        return make_double2(fma(-dx, a.x, fma(dy, a.y, b.x)), fma(-dx, a.y, fma(-dy, a.x, b.y)));
+      };
+      const double2 xj = x[j];
+      auto weight = [&] {
+        dx = group_sum<LPC>(dx);
+        dy = group_sum<LPC>(dy);
+        dot(v1, xj);
+        dx *= t;
+        dy *= t;
+      };
+      if (RPL > 0) {
+        double2 u[R];
+#pragma unroll
+        for (int i = F; i < R; ++i) {
+          const int r = l + LPC * i;
+          u[i] = (i > F || r > j) && r < rows ? x[r] : make_double2(0.0, 0.0);
+        }
+#pragma unroll
+        for (int i = F; i < R; ++i) dot(v[i], u[i]);
+        weight();
+#pragma unroll
+        for (int i = F; i < R; ++i) {
+          const int r = l + LPC * i;
+          u[i] = sub(v[i], u[i]);
+          s = fma(u[i].x, u[i].x, fma(u[i].y, u[i].y, s));
+          if (act && (i > F || r > j) && r < rows) x[r] = u[i];
+        }
+      } else {
+        for (int r = j + 1 + l; r < rows; r += LPC) dot(vp[r], x[r]);
+        weight();
+        for (int r = j + 1 + l; r < rows; r += LPC) {
+          const double2 o = sub(vp[r], x[r]);
+          if (act) x[r] = o;
+          s = fma(o.x, o.x, fma(o.y, o.y, s));
+        }
+      }
+      if (act && l == 0) x[j] = sub(v1, xj);
+      s = group_sum<LPC>(s);
+      if (l == 0 && c < k) next[c] = act ? s : -1.0;
+    }
+    __syncwarp();
+    asm volatile("bar.sync 1, %0;" ::"r"(32 * n_warps) : "memory");
   }
   return true;
+}
+
+template <int LPC, int RPL, int F>
+__device__ __forceinline__ void js_qr_from(double2* X, int ld, int rows, int k, JsQr& q, int n_warps) {
+  // rows below j start in chunk F for j + 1 in [LPC F, LPC (F + 1))
+  if (!js_qr_steps<LPC, RPL, F>(X, ld, rows, k, q, n_warps, max(LPC * F - 1, 0), min(LPC * (F + 1) - 1, k))) return;
+  if constexpr (LPC * (F + 1) - 1 < JS_KMAX && F + 1 < RPL) {
+    if (LPC * (F + 1) - 1 < k) js_qr_from<LPC, RPL, F + 1>(X, ld, rows, k, q, n_warps);
+  } else if constexpr (LPC * (F + 1) - 1 < JS_KMAX) {
+    // rows = k = LPC RPL: the last column has no rows below its head
+    js_qr_steps<LPC, RPL, RPL - 1>(X, ld, rows, k, q, n_warps, LPC * (F + 1) - 1, k);
+  }
+}
+
+// The factorisation; q.nn[0] holds the squared column norms.  LPC lanes take a column, its
+// rows in their registers (up to LPC RPL rows; RPL 0: read twice): its dot product with
+// the reflector, its update, and the norm of what is left of it, summed anew.  No more warps
+// than the columns need take part: each computes the reflector's scalars.
+template <int LPC, int RPL>
+__device__ void js_qr(double2* X, int ld, int rows, int k, JsQr& q, int n_warps) {
+  n_warps = min(n_warps, (k + 32 / LPC - 1) / (32 / LPC));
+  if ((int)(threadIdx.x >> 5) < n_warps) {
+    if constexpr (RPL > 0) js_qr_from<LPC, RPL, 0>(X, ld, rows, k, q, n_warps);
+    else js_qr_steps<LPC, 0, 0>(X, ld, rows, k, q, n_warps, 0, k);
+  }
+  __syncthreads();
+}
+
+// y = H_j1 .. H_j0 y (j1 the lower) of a column's rows in registers; chunks F.. hold rows j..
+template <int LPC, int RPL, int F>
+__device__ __forceinline__ void js_q_steps(const double2* X, int ld, int rows, const JsQr& q, double2 (&y)[RPL], int j0, int j1) {
+  const int l = threadIdx.x % LPC;
+  constexpr bool KEEP = RPL <= 8;      // the reflector in registers too
+  for (int j = j0; j >= j1; --j) {
+    const double2* x = X + q.piv[j] * ld;
+    const double2 v1 = q.v1[j];
+    const double t = q.t[j];
+    auto at = [&](int i) {
+      const int r = l + LPC * i;
+      const double2 w = (i > F || r > j) && r < rows ? x[r] : make_double2(0.0, 0.0);
+      return i == F && r == j ? v1 : w;
+    };
+    double2 v[KEEP ? RPL : 1];
+    double dx = 0.0, dy = 0.0;
+    if (KEEP) {
+#pragma unroll
+      for (int i = F; i < RPL; ++i) v[KEEP ? i : 0] = at(i);
+    }
+#pragma unroll
+    for (int i = F; i < RPL; ++i) {
+      const double2 w = KEEP ? v[KEEP ? i : 0] : at(i);
+      dx = fma(w.x, y[i].x, fma(w.y, y[i].y, dx));
+      dy = fma(w.x, y[i].y, fma(-w.y, y[i].x, dy));
+    }
+    dx = t * group_sum<LPC>(dx);
+    dy = t * group_sum<LPC>(dy);
+#pragma unroll
+    for (int i = F; i < RPL; ++i) {
+      const double2 w = KEEP ? v[KEEP ? i : 0] : at(i);
+      y[i] = make_double2(fma(-dx, w.x, fma(dy, w.y, y[i].x)), fma(-dx, w.y, fma(-dy, w.x, y[i].y)));
+    }
+  }
+}
+
+template <int LPC, int RPL, int F>
+__device__ __forceinline__ void js_q_from(const double2* X, int ld, int rows, int k, const JsQr& q, double2 (&y)[RPL]) {
+  js_q_steps<LPC, RPL, F>(X, ld, rows, q, y, min(LPC * (F + 1), k) - 1, LPC * F);
+  if constexpr (F > 0) js_q_from<LPC, RPL, F - 1>(X, ld, rows, k, q, y);
+}
+
+// A's columns = Q [P2 Y; 0], LPC lanes to a column (y0(c, i): entry i of P2 Y's column c), a
+// column's rows in their registers
+template <int LPC, int RPL, typename F>
+__device__ void js_q_apply(const double2* X, int ld, int rows, int k, const JsQr& q, cplx* A, int n_warps, F y0) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int GPW = 32 / LPC;
+  const int g = lane / LPC, l = lane % LPC;
+  for (int base = warp * GPW; base < k; base += n_warps * GPW) {
+    const int c = base + g;
+    double2 y[RPL];
+#pragma unroll
+    for (int i = 0; i < RPL; ++i) {
+      const int r = l + LPC * i;
+      y[i] = r < k && c < k ? y0(c, r) : make_double2(0.0, 0.0);
+    }
+    js_q_from<LPC, RPL, (JS_KMAX - 1) / LPC>(X, ld, rows, k, q, y);
+#pragma unroll
+    for (int i = 0; i < RPL; ++i) {
+      const int r = l + LPC * i;
+      if (r < rows && c < k) stc(A + (int64_t)r * k + c, cmake(y[i].x, y[i].y));
+    }
+  }
+}
+
+// All sweeps over the k columns of L (k rows, zeros up to 8 RL), by the first n_warps warps: four column pairs
+// to a warp, eight lanes and RL rows a lane to a pair.  Returns the sweeps done (max_sweeps
+// + 1: not converged) and adds this lane's rotations to `turned`.
+template <int RL>
+__device__ int js_sweeps(double2* L, int ld, int k, double z2, double t2, int max_sweeps, int n_warps, int* rot,
+                         unsigned long long& turned) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 3, l = lane & 7;
+  const int n = k + (k & 1), P = 4 * warp + g;
+  auto barrier = [&] { asm volatile("bar.sync 1, %0;" ::"r"(32 * n_warps) : "memory"); };
+  for (int sweep = 0;; ++sweep) {
+    if (sweep == max_sweeps) return max_sweeps + 1;
+    int mine = 0;
+    for (int step = 0; step < n - 1; ++step) {
+      // circle_at without its division
+      int p = P + step, q = n - 1 - P + step;
+      if (p > n - 1) p -= n - 1;
+      if (q > n - 1) q -= n - 1;
+      if (P == 0) p = 0;
+      if (p > q) { const int x = p; p = q; q = x; }
+      const bool ok = P < n / 2 && q < k;   // q == k: the padding column
+      double2 *x = L + (ok ? p * ld : 0) + l, *y = L + (ok ? q * ld : 0) + l;
+      double2 u[RL], v[RL];
+      double a = 0.0, b = 0.0, gx = 0.0, gy = 0.0;
+#pragma unroll
+      for (int i = 0; i < RL; ++i) {
+        u[i] = x[8 * i];
+        v[i] = y[8 * i];
+      }
+#pragma unroll
+      for (int i = 0; i < RL; ++i) {
+        a = fma(u[i].x, u[i].x, fma(u[i].y, u[i].y, a));
+        b = fma(v[i].x, v[i].x, fma(v[i].y, v[i].y, b));
+        gx = fma(u[i].x, v[i].x, fma(u[i].y, v[i].y, gx));
+        gy = fma(u[i].x, v[i].y, fma(-u[i].y, v[i].x, gy));
+      }
+      // sums over the eight lanes: a product with ones leaves lane j & 3 the four-lane sums
+      // of columns 2 j and 2 j + 1, which are the lanes of pair j
+      double2 s0 = make_double2(0, 0), s1 = s0, s2 = s0, s3 = s0;
+      __syncwarp();
+      dmma8x8x4(s0, 1.0, a);
+      dmma8x8x4(s1, 1.0, b);
+      dmma8x8x4(s2, 1.0, gx);
+      dmma8x8x4(s3, 1.0, gy);
+      a = __shfl_sync(0xffffffffu, s0.x + s0.y, g);
+      b = __shfl_sync(0xffffffffu, s1.x + s1.y, g);
+      gx = __shfl_sync(0xffffffffu, s2.x + s2.y, g);
+      gy = __shfl_sync(0xffffffffu, s3.x + s3.y, g);
+      const double g2 = fma(gx, gx, gy * gy);
+      const bool turn = ok && a > z2 && b > z2 && a > t2 * b && b > t2 * a && g2 > t2 * a * b;
+      if (turn) {
+        // the rotation of the blocked form: c, s e^{i alpha} of the small angle
+        const double dd = b - a, ir = rsqrt(fma(dd, dd, 4.0 * g2)), c2 = fma(0.5 * fabs(dd), ir, 0.5), ic = rsqrt(c2);
+        const double c = c2 * ic, f = copysign(ir * ic, dd), sx = f * gx, sy = f * gy;
+        ++mine;
+#pragma unroll
+        for (int i = 0; i < RL; ++i) {
+          // u' = c u - conj(s) v, v' = s u + c v
+          x[8 * i] = make_double2(fma(c, u[i].x, fma(-sx, v[i].x, -(sy * v[i].y))),
+                                  fma(c, u[i].y, fma(-sx, v[i].y, sy * v[i].x)));
+          y[8 * i] = make_double2(fma(c, v[i].x, fma(sx, u[i].x, -(sy * u[i].y))),
+                                  fma(c, v[i].y, fma(sx, u[i].y, sy * u[i].x)));
+        }
+      }
+      __syncwarp();
+      barrier();
+    }
+    turned += mine;
+    if (l == 0 && mine) rot[sweep & 1] = 1;
+    __syncwarp();
+    barrier();
+    const bool again = rot[sweep & 1] != 0;
+    if (threadIdx.x == 0) rot[(sweep + 1) & 1] = 0;   // the next sweep's flag, which nobody sets before its barriers
+    if (!again) return sweep + 1;
+  }
+}
+
+// squared norms of a matrix's columns, a warp to a column
+__device__ __forceinline__ void js_norms(const double2* X, int ld, int rows, int k, double* nn, int n_warps) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int c = warp; c < k; c += n_warps) {
+    double s = 0.0;
+    for (int r = lane; r < rows; r += 32) {
+      const double2 v = X[c * ld + r];
+      s = fma(v.x, v.x, fma(v.y, v.y, s));
+    }
+    s = group_sum<32>(s);
+    if (lane == 0) nn[c] = s;
+  }
 }
 
 template <int NT>
@@ -659,84 +908,92 @@ __global__ __launch_bounds__(NT) void jacobi_small_kernel(const SectorDesc* __re
                                                           unsigned long long* __restrict__ executed) {
   constexpr int NW = NT / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double red[NW];
-  __shared__ int rot[2];
+  __shared__ JsQr q1, q2;
+  __shared__ double nrm[JS_KMAX];
+  __shared__ int rot[2], inv2[JS_KMAX];
   const SectorDesc& S = sd[list[blockIdx.x]];
-  const int k = S.k, rows = S.rows_tot, rows_g = S.rows_g, ld = js_ld(rows);
-  double2* X = reinterpret_cast<double2*>(smem_raw);   // column c: X + c ld
-  double* nrm = reinterpret_cast<double*>(X + (size_t)k * ld);
+  const int k = S.k, rows = S.rows_g, ldx = js_ld(rows), ld = js_ldl(k);
+  const bool left = S.left != 0;
+  double2* X = reinterpret_cast<double2*>(smem_raw);   // column c: X + c ldx
+  double2* Y = X + (size_t)k * ldx;                    // L, column c: Y + c ld
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   cplx* A = abuf + S.a_off;
-  double f2 = 0.0;
   for (int e = tid; e < rows * k; e += NT) {
     const int r = e / k, c = e - r * k;
     const cplx v = ldc(A + e);
-    X[c * ld + r] = make_double2(v.x, v.y);
-    if (r < rows_g) f2 += cabs2(v);
+    X[c * ldx + r] = make_double2(v.x, v.y);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) f2 += __shfl_xor_sync(0xffffffffu, f2, o);
-  if (lane == 0) red[warp] = f2;
   if (tid < 2) rot[tid] = 0;
   __syncthreads();
-  f2 = 0.0;
-  for (int w = 0; w < NW; ++w) f2 += red[w];
-  const double zf = 16.0 * 2.220446049250313e-16 * sqrt((double)rows_g), z2 = zf * zf * f2;
-  const double tol = fmax(8.0 * 2.220446049250313e-16, 4.0 * 2.220446049250313e-16 * sqrt((double)rows_g));
+  js_norms(X, ldx, rows, k, q1.nn[0], NW);
+  __syncthreads();
+  double f2 = 0.0;
+  for (int c = 0; c < k; ++c) f2 += q1.nn[0][c];
+  __syncthreads();                                     // q1.nn[0] is overwritten from the second step on
+  const double zf = 16.0 * 2.220446049250313e-16 * sqrt((double)rows), z2 = zf * zf * f2;
+  const double tol = fmax(8.0 * 2.220446049250313e-16, 4.0 * 2.220446049250313e-16 * sqrt((double)k));
   const double t2 = tol * tol;
-  const int n = k + (k & 1), chunks = (rows + 31) / 32;
-  int sweep = 0;
-  unsigned long long turned = 0;
-  if (k > 1)
-    for (;; ++sweep) {
-      if (sweep == max_sweeps) {
-        if (tid == 0) *fail = 1;
-        break;
+  if (rows <= 64) js_qr<8, 8>(X, ldx, rows, k, q1, NW);
+  else if (rows <= 128) js_qr<16, 8>(X, ldx, rows, k, q1, NW);
+  else if (rows <= 256) js_qr<32, 8>(X, ldx, rows, k, q1, NW);
+  else js_qr<32, 0>(X, ldx, rows, k, q1, NW);
+  // L = R^H
+  for (int e = tid; e < ld * k; e += NT) {
+    const int c = e / ld, r = e - c * ld;
+    double2 v = make_double2(0.0, 0.0);
+    if (r < k && r >= c) v = r > c ? X[q1.piv[r] * ldx + c] : q1.rd[c];
+    Y[e] = make_double2(v.x, -v.y);
+  }
+  __syncthreads();
+  if (!left) {
+    js_norms(Y, ld, k, k, q2.nn[0], NW);
+    __syncthreads();
+    js_qr<8, 8>(Y, ld, k, k, q2, NW);
+    // L = R2^H, in place through registers
+    constexpr int PER = (JS_KMAX * JS_KMAX + 511) / 512;
+    double2 keep[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int e = tid + i * NT;
+      keep[i] = make_double2(0.0, 0.0);
+      if (e < k * k) {
+        const int c = e / k, r = e - c * k;
+        if (r >= c) keep[i] = r > c ? Y[q2.piv[r] * ld + c] : q2.rd[c];
       }
-      int mine = 0;
-      for (int step = 0; step < n - 1; ++step) {
-        for (int P = warp; P < n / 2; P += NW) {
-          // circle_at without its division
-          int p = P + step, q = n - 1 - P + step;
-          if (p > n - 1) p -= n - 1;
-          if (q > n - 1) q -= n - 1;
-          if (P == 0) p = 0;
-          if (p > q) { const int x = p; p = q; q = x; }
-          if (q >= k) continue;          // the padding column
-          double2 *x = X + p * ld, *y = X + q * ld;
-          bool r;
-          if (chunks <= 1) r = js_pair<1>(x, y, rows_g, rows, z2, t2);
-          else if (chunks == 2) r = js_pair<2>(x, y, rows_g, rows, z2, t2);
-          else if (chunks <= 4) r = js_pair<4>(x, y, rows_g, rows, z2, t2);
-          else r = js_pair<0>(x, y, rows_g, rows, z2, t2);
-          mine += r;
-        }
-        __syncthreads();
-      }
-      turned += mine;
-      if (lane == 0 && mine) rot[sweep & 1] = 1;
-      __syncthreads();
-      const bool again = rot[sweep & 1] != 0;
-      if (tid == 0) rot[(sweep + 1) & 1] = 0;   // the next sweep's flag, which nobody sets before its barriers
-      if (!again) break;
     }
-  if (lane == 0 && turned) atomicAdd(executed, turned * 4ull * rows);
-  if (tid == 0) {
-    atomicAdd(executed, (unsigned long long)(sweep + 1) * (unsigned)(k * (k - 1) / 2) * 2ull * rows_g);
-    atomicMax(executed + 1, (unsigned long long)(sweep + 1));
+    if (tid < k) inv2[q2.piv[tid]] = tid;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int e = tid + i * NT;
+      if (e < k * k) {
+        const int c = e / k, r = e - c * k;
+        Y[c * ld + r] = make_double2(keep[i].x, -keep[i].y);
+      }
+    }
+    __syncthreads();
+  }
+  const int jw = (k + (k & 1)) / 8 + ((k + (k & 1)) % 8 != 0);   // four pairs a warp
+  if (k > 1 && warp < jw) {
+    unsigned long long turned = 0;
+    int sweeps;
+    if (k <= 16) sweeps = js_sweeps<2>(Y, ld, k, z2, t2, max_sweeps, jw, rot, turned);
+    else if (k <= 32) sweeps = js_sweeps<4>(Y, ld, k, z2, t2, max_sweeps, jw, rot, turned);
+    else if (k <= 48) sweeps = js_sweeps<6>(Y, ld, k, z2, t2, max_sweeps, jw, rot, turned);
+    else sweeps = js_sweeps<8>(Y, ld, k, z2, t2, max_sweeps, jw, rot, turned);
+    if ((lane & 7) == 0 && turned) atomicAdd(executed, turned * 4ull * k);
+    if (tid == 0) {
+      if (sweeps > max_sweeps) *fail = 1;
+      sweeps = min(sweeps, max_sweeps);
+      atomicAdd(executed, (unsigned long long)sweeps * (unsigned)(k * (k - 1) / 2) * 2ull * k + (unsigned long long)k * k * rows);
+      atomicMax(executed + 1, (unsigned long long)sweeps);
+    }
   }
   __syncthreads();
   // column norms (0 below the numerical-rank floor), the descending order (ties by column)
-  for (int c = warp; c < k; c += NW) {
-    double s2 = 0.0;
-    for (int r = lane; r < rows_g; r += 32) {
-      const double2 v = X[c * ld + r];
-      s2 = fma(v.x, v.x, fma(v.y, v.y, s2));
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-    if (lane == 0) nrm[c] = s2 <= z2 ? 0.0 : sqrt(s2);
-  }
+  js_norms(Y, ld, k, k, nrm, NW);
+  __syncthreads();
+  if (tid < k) nrm[tid] = nrm[tid] <= z2 ? 0.0 : sqrt(nrm[tid]);
   __syncthreads();
   if (tid < k) {
     const double s = nrm[tid];
@@ -745,50 +1002,56 @@ __global__ __launch_bounds__(NT) void jacobi_small_kernel(const SectorDesc* __re
     sig[S.s_off + at] = s;
     perm[S.s_off + at] = tid;
   }
-  for (int e = tid; e < rows * k; e += NT) {
-    const int r = e / k, c = e - r * k;
-    const double2 v = X[c * ld + r];
-    stc(A + e, cmake(v.x, v.y));
+  if (left) {
+    // the left vectors, where the blocked form accumulates its rotations
+    for (int e = tid; e < k * k; e += NT) {
+      const int r = e / k, c = e - r * k;
+      const double2 v = Y[c * ld + r];
+      const double is = nrm[c] > 0.0 ? 1.0 / nrm[c] : 0.0;
+      stc(A + (int64_t)(rows + q1.piv[r]) * k + c, cmake(v.x * is, v.y * is));
+    }
+    return;
   }
+  auto y0 = [&](int c, int r) { return Y[c * ld + inv2[r]]; };
+  if (rows <= 64) js_q_apply<8, 8>(X, ldx, rows, k, q1, A, NW, y0);
+  else if (rows <= 128) js_q_apply<16, 8>(X, ldx, rows, k, q1, A, NW, y0);
+  else if (rows <= 256) js_q_apply<32, 8>(X, ldx, rows, k, q1, A, NW, y0);
+  else if (rows <= 512) js_q_apply<32, 16>(X, ldx, rows, k, q1, A, NW, y0);
+  else js_q_apply<32, 32>(X, ldx, rows, k, q1, A, NW, y0);
 }
 
 }  // namespace
 
 int jacobi_block_cols() { return JB; }
 
-// The whole SVD in one CTA, by the shape of the Jacobi matrix.  Measured against the blocked
-// form's rounds (two launches of 45 us a round and sweep), us: k = 9, 958 rows 121 (270);
-// k = 17, 128 rows 90 (270); k = 28, 128 rows 209 (315), 256 rows 306 (315), 400 rows 447
-// (315); k = 48, 128 rows 543 (1,080), 192 rows 664 (945); k = 64, 128 rows 1,195 (1,080).
-bool jacobi_is_small(int rows, int k) {
-  return (k <= 16 || (k <= 32 && rows <= 256) || (k <= JS_KMAX && rows <= 192)) && js_smem(rows, k) <= 220 * 1024;
+// The whole SVD in one CTA: where X and L fit in shared memory and a column of X in a warp's
+// registers (16 or, in the form for 16 columns, 32 a lane).  The blocked form pays two
+// launches of 45 to 60 us a round, three rounds a sweep at k = 64: 64 x 128 945 us and more,
+// here 480 to 620; k = 28, 400 rows 315 and 200 to 350.
+int jacobi_small_elems(int rows_g, int k) { return (js_ld(rows_g) + js_ldl(k)) * k; }
+bool jacobi_is_small(int rows_g, int k) {
+  return k <= JS_KMAX && rows_g <= (k <= 16 ? 1024 : 512) && (size_t)jacobi_small_elems(rows_g, k) * sizeof(double2) <= JS_SMEM;
 }
 
-cudaError_t launch_jacobi_small(const SectorDesc* sd_dev, const int* list_dev, int count, int max_rows_k, int max_k,
+cudaError_t launch_jacobi_small(const SectorDesc* sd_dev, const int* list_dev, int count, int max_elems, int max_k,
                                 void* abuf, int max_sweeps, double* sig, int* perm, int* fail,
                                 unsigned long long* executed, cudaStream_t s) {
   if (count <= 0) return cudaSuccess;
   static const cudaError_t attr = [] {
-    cudaError_t e = cudaFuncSetAttribute(jacobi_small_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, 221 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(jacobi_small_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, JS_SMEM);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(jacobi_small_kernel<768>, cudaFuncAttributeMaxDynamicSharedMemorySize, 221 * 1024);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(jacobi_small_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, 221 * 1024);
+      e = cudaFuncSetAttribute(jacobi_small_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, JS_SMEM);
     return e;
   }();
   if (attr != cudaSuccess) return attr;
-  const size_t smem = (size_t)max_rows_k * sizeof(double2) + JS_KMAX * sizeof(double);
+  const size_t smem = (size_t)max_elems * sizeof(double2);
   cplx* A = reinterpret_cast<cplx*>(abuf);
-  // a warp to a column pair of a step
   if (max_k <= 16)
     jacobi_small_kernel<256><<<count, 256, smem, s>>>(sd_dev, list_dev, A, max_sweeps, sig, perm, fail, executed);
-  else if (max_k <= 32)
-    jacobi_small_kernel<512><<<count, 512, smem, s>>>(sd_dev, list_dev, A, max_sweeps, sig, perm, fail, executed);
   else
-    jacobi_small_kernel<768><<<count, 768, smem, s>>>(sd_dev, list_dev, A, max_sweeps, sig, perm, fail, executed);
+    jacobi_small_kernel<512><<<count, 512, smem, s>>>(sd_dev, list_dev, A, max_sweeps, sig, perm, fail, executed);
   return cudaGetLastError();
 }
-int jacobi_small_elems(int rows, int k) { return js_ld(rows) * k; }
 
 cudaError_t launch_sector_norms(const SectorDesc* sd_dev, const int* list_dev, int count, const void* abuf,
                                 double* nf2, cudaStream_t s) {

@@ -161,12 +161,14 @@ cudaError_t launch_jacobi_round(const SectorDesc* sd_dev, const JacobiWork* work
                                 const double* nf2, double tol, int max_sweeps, void* pbuf,
                                 int* pcnt, void* qbuf, int* qflag, unsigned long long* executed,
                                 cudaStream_t s);
-// Small sectors: the whole SVD (all sweeps, column norms, sort) in one CTA per listed
-// sector.  jacobi_is_small: whether a rows x k Jacobi matrix goes there; max_elems: the
-// largest jacobi_small_elems of the list.  fail is set to 1 where max_sweeps do not
-// converge; executed[0] += complex MACs done, executed[1] = the most sweeps.
-bool jacobi_is_small(int rows, int k);
-int jacobi_small_elems(int rows, int k);
+// Small sectors: the whole SVD (QR, all sweeps, column norms, sort) in one CTA per listed
+// sector.  jacobi_is_small: whether a Jacobi matrix of rows_g Gram rows and k columns goes
+// there; max_elems: the largest jacobi_small_elems of the list.  A left sector's vectors are
+// left in the rows below the Gram rows, the others' scaled columns in the Gram rows.  fail
+// is set to 1 where max_sweeps do not converge; executed[0] += complex MACs done,
+// executed[1] = the most sweeps.
+bool jacobi_is_small(int rows_g, int k);
+int jacobi_small_elems(int rows_g, int k);
 cudaError_t launch_jacobi_small(const SectorDesc* sd_dev, const int* list_dev, int count, int max_elems, int max_k,
                                 void* abuf, int max_sweeps, double* sig, int* perm, int* fail,
                                 unsigned long long* executed, cudaStream_t s);

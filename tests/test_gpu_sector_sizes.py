@@ -114,6 +114,35 @@ def test_singular_values_by_shape(shape, precision):
         at += n
 
 
+# the one-CTA SVD's own limits: columns 1, 2, 16, 17, 64, 65; rows where its registers and its
+# shared memory end, tall and wide
+ONE_CTA = [(1, 1), (2, 2), (3, 17), (16, 16), (17, 16), (32, 33), (48, 33), (64, 64), (63, 128), (128, 64), (64, 65), (65, 64),
+           (65, 65), (130, 56), (56, 130), (17, 512), (512, 17), (513, 17), (16, 800), (800, 16), (13, 1024), (1024, 13), (2, 1025)]
+
+
+@pytest.mark.parametrize("shape", ONE_CTA, ids=lambda s: "%dx%d" % s)
+@pytest.mark.parametrize("rank", [None, 5])
+def test_one_cta_svd(shape, rank):
+    """Graded sectors (right weights over eight decades) that keep every vector: singular values
+    within 64 eps sqrt(size) of the largest, zeros below the numerical rank, and orthonormal
+    kept vectors.  A vector of sigma carries the rounding of its matrix, eps sigma_1 / sigma."""
+    L, R = shape
+    d, k, eps = 2, min(L, R), np.finfo(np.float64).eps
+    K = max(40, k)
+    rng = np.random.default_rng(L * 2000 + R)
+    args = _two_sites(rng, L, K, R, d, rank=rank, spread=8.0)
+    want = _expected(d, *args)
+    info, g, lam, _ = _update("fp64", d, *args, max(4 * k, L, R, K))
+    V, at = g[0][:L], 0
+    for i, cc in enumerate(info["sectors"]):
+        s, w, n = info["sigma"][i], want[cc], info["kept"][i]
+        assert np.all(np.abs(s - w) <= 64 * eps * np.sqrt(max(K, L, R)) * w[0])
+        v = V[:, at:at + n]
+        loss = w[0] / min(s[:n], default=1.0)
+        assert np.abs(v.conj().T @ v - np.eye(n)).max(initial=0.0) <= 64 * eps * max(k, K) * max(loss, 1.0)
+        at += n
+
+
 @pytest.mark.parametrize("precision", ["fp64", "fp64-gram"])
 @pytest.mark.parametrize("rank", [0, 3, 17])
 def test_rank_deficient_sectors(precision, rank):
