@@ -34,7 +34,7 @@ thread_local std::string g_last_error;
 
 constexpr int MAX_SWEEPS = 40;
 constexpr int WAIT_POLL_US = 400;   // host waits poll this long before they sleep
-constexpr int MESH_LANES = 2;   // streams a mesh's groups of updates are spread over
+constexpr int MESH_LANES = 4;   // streams a mesh's groups of updates are spread over, at most
 constexpr int MAX_GROUP = 32;   // updates of a group
 
 struct DevBuf {
@@ -1371,8 +1371,8 @@ void destroy_worker(bsmpo_ctx* w) {
 // conflict when their modes differ by 0 or 1 (shared site); update k depends on the latest
 // earlier update at modes m_k - 1, m_k and m_k + 1 -- nothing else it touches is written
 // by another update (modes 2 apart share only a bond both read).  At most `nw` updates run
-// at once, on MESH_LANES streams (fewer where nw is smaller): a lane takes the
-// lowest-numbered updates whose dependencies have finished (host side: after their host
+// at once (four times as many up to chi = 512), on up to MESH_LANES streams: a lane takes
+// the lowest-numbered updates whose dependencies have finished (host side: after their host
 // mirror entries are written; device side: the lane's stream waits for the events recorded
 // at their ends) as one group, so an update's launches are shared by its layer's other
 // updates and consecutive brick-wall layers overlap.  Every update computes exactly what
@@ -1382,12 +1382,11 @@ void destroy_worker(bsmpo_ctx* w) {
 // N = 64, chi = 1024 with 16 updates at once took 142 ms, in groups on two lanes 92 (with
 // the eigen kernels of that time).
 // The host side of a mesh over a host-resident state: the first update touching site s,
-// first[s], copies the site in on its own stream before it starts, and the last, last[s],
-// copies it out after it ends.  Every later update touching the site depends on the
-// first one (they share a site), and the last one on every earlier one, so the copies
-// need no events of their own; they run in the workers' streams, where they overlap the
-// other workers' updates without extra streams (which would share the device's hardware
-// queues with the workers' streams).
+// first[s], copies the site in on its own stream before it starts; after the last, last[s],
+// the lane's copy stream takes it out, behind the group's event.  Every later update touching
+// the site depends on the first one (they share a site), and the last one on every earlier
+// one, so the copies need no other events.  Copies out on the lane's own stream held back
+// its next group: one layer at N = 40, chi = 500 10.4 ms, so 9.8.
 struct HostStream {
   std::vector<int> first, last;
   const char* gamma_in = nullptr;
@@ -1399,7 +1398,12 @@ int run_mesh_concurrent(bsmpo_ctx* h, int n_bs, const int* modes, const cplx* u3
                         HostStream* hs = nullptr) {
   const int d3 = h->d * h->d * h->d;
   int rc;
-  const int lanes = std::min(nw, MESH_LANES);
+  // Two workers to a lane.  Two, three and four lanes, 8 workers (16 at N = 64), ms: 24 modes
+  // chi = 256 fp64 35.9, 32.9 and 32.1; 32 modes chi = 256 26.0, 25.8 and 24.4, chi = 512 107,
+  // 104 and 97, fp64 148, 132 and 132; two layers at N = 64, chi = 1,024 46.9, 45.3 and 44.8.
+  // Many small circuits side by side, 4 workers each, lose by more lanes (8 circuits of up
+  // to 16 modes, chi = 64: 38, 43 and 50): each has its own streams, threads and workspaces.
+  const int lanes = std::min(MESH_LANES, std::max(std::min(nw, 2), nw / 2));
   // Four updates to a worker up to chi = 512, where an update's launches leave most of the
   // chip idle and four hold the workspace of one at chi = 1,024.  Circuits with 8 workers,
   // one and four to a worker, ms: 24 modes chi = 64 9.5 and 8.2, chi = 128 11.7 and 10.3,

@@ -231,7 +231,7 @@ int bsmpo_mesh_truncation(const bsmpo_ctx* h, double* weights, int cap);
 
 /* Number of updates bsmpo_run_mesh runs at once (1..64, default 8 or the environment
  * variable BSMPO_WORKERS at create; up to chi = 512, where an update's sectors fill a small
- * part of the chip, four times as many).  They run in groups on at most two streams, a
+ * part of the chip, four times as many).  They run in groups on up to four streams, a
  * group's updates in shared launches; each stream has its own workspaces, sized for its
  * largest group (grown on demand, freed by bsmpo_destroy).  Replaces the reference's dispatch
  * of one layer's beam splitters to separate MPI ranks (src/beam_splitter_parallel/
