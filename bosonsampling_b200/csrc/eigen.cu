@@ -1411,20 +1411,24 @@ __global__ __launch_bounds__(WY_NT) void wy_apply_kernel(const SectorDesc* __res
 //    64-bit CPU computation as before (1.1e-13 at most).  A sector whose
 //    Y was not unitary to NS_TOL before the last step (flagged in sd[].kept, which the
 //    selection sets later) starts from X itself.
-constexpr int OR_NT = 256, OR_NW = OR_NT / 32;
+constexpr int OR_NT = 512, OR_NW = OR_NT / 32;
 constexpr int OR_P = 8;        // vectors of a panel
 constexpr double NS_TOL = 1e-7;
 
 // Panels of OR_P vectors of a group, in order: each against the group's earlier vectors (32 at
-// a time) and within itself (Gram-Schmidt), the whole twice.
+// a time, two products on the FP64 tensor path) and within itself (Gram-Schmidt), the whole
+// twice.  What bounds it: the reads of the group's vectors by one CTA, twice a chunk; the
+// sectors below chi's cut share one group of up to a few hundred values.  With scalar
+// products, a thread to a row in the second one (uncoalesced), the largest launch of a layer
+// at N = 64, chi = 1024 took 6.5 ms, now 2.6; one such update 10.9 and 10.1.
 __global__ __launch_bounds__(OR_NT) void orthogonalise_kernel(const SectorDesc* __restrict__ sd,
                                                               const int* __restrict__ list,
                                                               const double* __restrict__ lam,
                                                               double* __restrict__ zbuf) {
-  extern __shared__ double zp[];   // the panel, [k][OR_P]
-  __shared__ double dots[OR_NW][32][OR_P], coef[32][OR_P], part[OR_NW][OR_P];
+  extern __shared__ __align__(16) double zp[];   // the panel, [k][OR_P]
+  __shared__ double dots[OR_NW][32][OR_P], coef[32][OR_P], part[OR_NW][OR_P], tots[OR_P];
   const SectorDesc& S = sd[list[blockIdx.x]];
-  const int k = S.k, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int k = S.k, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, li = lane >> 2, lk = lane & 3;
   const double* lv = lam + S.s_off;
   double* Z = zbuf + S.y_off;      // [k][k]
   const double gaptol = IV_GAP_ALL * fmax(fabs(lv[0]), fabs(lv[k - 1]));
@@ -1441,41 +1445,53 @@ __global__ __launch_bounds__(OR_NT) void orthogonalise_kernel(const SectorDesc* 
       __syncthreads();
       for (int pass = 0; pass < 2; ++pass) {
         for (int g0 = first; g0 < m0; g0 += 32) {
-          const int g = g0 + lane;
-          double acc[OR_P];
+          // Z^T zp by the warps' rows, four at a time
+          double2 acc[4];
 #pragma unroll
-          for (int p = 0; p < OR_P; ++p) acc[p] = 0.0;
-          if (g < m0) {
+          for (int m = 0; m < 4; ++m) acc[m] = make_double2(0.0, 0.0);
 #pragma unroll 4
-            for (int i = warp; i < k; i += OR_NW) {
-              const double z = Z[(int64_t)i * k + g];
+          for (int r0 = 4 * warp; r0 < k; r0 += 4 * OR_NW) {
+            const int i = r0 + lk;
+            const double b = i < k ? zp[i * OR_P + li] : 0.0;
+            double a[4];
 #pragma unroll
-              for (int p = 0; p < OR_P; ++p) acc[p] = fma(z, zp[i * OR_P + p], acc[p]);
+            for (int m = 0; m < 4; ++m) {
+              const int g = g0 + 8 * m + li;
+              a[m] = i < k && g < m0 ? Z[(int64_t)i * k + g] : 0.0;
             }
+            __syncwarp();
+#pragma unroll
+            for (int m = 0; m < 4; ++m) dmma8x8x4(acc[m], a[m], b);
           }
 #pragma unroll
-          for (int p = 0; p < OR_P; ++p) dots[warp][lane][p] = acc[p];
+          for (int m = 0; m < 4; ++m) *reinterpret_cast<double2*>(&dots[warp][8 * m + li][2 * lk]) = acc[m];
           __syncthreads();
-          {
-            const int c = tid / OR_P, p = tid % OR_P;   // OR_NT = 32 OR_P
+          if (tid < 32 * OR_P) {
+            const int c = tid / OR_P, p = tid % OR_P;
             double s = 0.0;
+#pragma unroll
             for (int w = 0; w < OR_NW; ++w) s += dots[w][c][p];
             coef[c][p] = s;
           }
           __syncthreads();
-          const int ng = min(32, m0 - g0);
-          for (int i = tid; i < k; i += OR_NT) {
-            double v[OR_P];
+          // zp - Z (Z^T zp), eight rows at a time
+          double cf[8];
 #pragma unroll
-            for (int p = 0; p < OR_P; ++p) v[p] = zp[i * OR_P + p];
-#pragma unroll 4
-            for (int c = 0; c < ng; ++c) {
-              const double z = Z[(int64_t)i * k + g0 + c];
+          for (int q = 0; q < 8; ++q) cf[q] = coef[4 * q + lk][li];
+#pragma unroll 2
+          for (int r0 = 8 * warp; r0 < k; r0 += 8 * OR_NW) {
+            const int i = r0 + li;
+            double a[8];
 #pragma unroll
-              for (int p = 0; p < OR_P; ++p) v[p] = fma(-coef[c][p], z, v[p]);
+            for (int q = 0; q < 8; ++q) {
+              const int g = g0 + 4 * q + lk;
+              a[q] = i < k && g < m0 ? -Z[(int64_t)i * k + g] : 0.0;
             }
+            double2 v = i < k ? *reinterpret_cast<const double2*>(&zp[i * OR_P + 2 * lk]) : make_double2(0.0, 0.0);
+            __syncwarp();
 #pragma unroll
-            for (int p = 0; p < OR_P; ++p) zp[i * OR_P + p] = v[p];
+            for (int q = 0; q < 8; ++q) dmma8x8x4(v, a[q], cf[q]);
+            if (i < k) *reinterpret_cast<double2*>(&zp[i * OR_P + 2 * lk]) = v;
           }
           __syncthreads();
         }
@@ -1495,12 +1511,16 @@ __global__ __launch_bounds__(OR_NT) void orthogonalise_kernel(const SectorDesc* 
             if (lane == 0) part[warp][q] = s;
           }
           __syncthreads();
+          if (tid < OR_P) {
+            double s = 0.0;
+#pragma unroll
+            for (int w = 0; w < OR_NW; ++w) s += part[w][tid];
+            tots[tid] = s;
+          }
+          __syncthreads();
           double tot[OR_P];
 #pragma unroll
-          for (int q = 0; q < OR_P; ++q) {
-            tot[q] = 0.0;
-            for (int w = 0; w < OR_NW; ++w) tot[q] += part[w][q];
-          }
+          for (int q = 0; q < OR_P; ++q) tot[q] = tots[q];
           double n2 = 0.0;
 #pragma unroll
           for (int q = 0; q < OR_P; ++q) n2 = q == p ? tot[q] : n2;
