@@ -369,7 +369,7 @@ def roofline(args, mine, kernel, fp64_peak, hbm_peak, peaks=None):
         achieved = kernel["bytes"] / (kernel["ms"] / 1e3) / 1e9
         pool = float(peaks["hbm_gbs"]) if peaks and peaks.get("hbm_gbs") else None
         peak = pool if pool else hbm_peak
-        return {"kernel": "tridiag_kernel (Householder tridiagonalisation, four forked size-class launches)",
+        return {"kernel": "tridiag_resident_kernel (Householder tridiagonalisation, forked size-class launches)",
                 "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak if peak else None,
                 "frac_of": "measured",
@@ -632,7 +632,7 @@ def main():
                    "n_range": [min(sp["n"] for sp in specs), max(sp["n"] for sp in specs)],
                    "chis": sorted(set(sp["chi"] for sp in specs)),
                    "concurrency": conc_best, "seconds_by_concurrency": {str(c): round(t, 3) for c, t in best.items()},
-                   "how": "circuits side by side, one handle + host thread + stream each, 4 worker streams per "
+                   "how": "circuits side by side, one handle + host thread + stream each, 4 workers per "
                           "handle (one by one: 8); host wall clock of the meshes, output phases and "
                           "observables, handles created and initialised before"}
 

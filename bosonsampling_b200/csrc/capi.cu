@@ -2,14 +2,15 @@
 //
 // The host keeps a mirror of the per-bond charge-block sizes (they change only when
 // an update writes a new bond, and the update reports its kept counts), so every
-// launch of an update is planned on the host without reading device data; the one
-// device->host synchronisation per update reads the kept counts after selection.
+// launch of a group of updates is planned on the host without reading device data; the
+// kernels behind the selection read the kept counts on the device, and the host waits once
+// per group, for one copy of its results.
 //
-// Per update (bond layout of src/MPO.py:158-303, GPU driver
+// Per group (bond layout of src/MPO.py:158-303, GPU driver
 // src/beam_splitter_parallel/Rank.py:32-206):
 //   Theta grouped GEMM -> gate mix (C per sector and the Jacobi matrix) ->
-//   blocked one-sided Jacobi rounds -> column norms + sort -> top-chi selection ->
-//   [sync: kept counts] -> V extraction -> W = V^H C grouped GEMM -> scatter.
+//   sector SVD (one-CTA Jacobi; preconditioned or plain blocked Jacobi rounds; or Gram ->
+//   tridiagonal -> eigenvalues) -> top-chi selection -> V -> W = V^H C grouped GEMM -> scatter.
 #include <algorithm>
 #include <atomic>
 #include <condition_variable>
@@ -601,7 +602,6 @@ void finish_plan(bsmpo_ctx* h, Plan& P) {
   std::vector<int> big, pre;
   for (int s = 0; s < ns; ++s) {
     const SectorDesc& S = P.sd[s];
-    if (S.left) P.max_left_m2 = std::max(P.max_left_m2, S.m * S.m);
     if (jacobi_is_small(S.rows_g, S.k)) {
       P.tdlist.push_back(s);
       P.small_elems = std::max(P.small_elems, jacobi_small_elems(S.rows_g, S.k));
@@ -609,6 +609,8 @@ void finish_plan(bsmpo_ctx* h, Plan& P) {
       continue;
     }
     big.push_back(s);
+    // the identity below T^H, which accumulates the rotations (the one-CTA form has none)
+    if (S.left) P.max_left_m2 = std::max(P.max_left_m2, S.m * S.m);
     P.big_k = std::max(P.big_k, S.k);
     if (S.t_off != S.a_off) {
       pre.push_back(s);

@@ -211,7 +211,7 @@ int bsmpo_run_mesh(bsmpo_ctx* h, int n_bs, const int* modes, const double* theta
  * (gamma_in [n][chi][chi] complex128, lambda_in [n-1][chi], charge_in [n+1][chi][2], the
  * bsmpo_load_state layout, host memory) is validated, its bonds are copied in, and
  * each site of Gamma is copied in by the first update touching it, on that update's
- * stream, and copied to gamma_out by the last one, so one update's transfers overlap
+ * stream, and to gamma_out behind the last one, so one update's transfers overlap
  * the other updates' compute (both directions need page-locked host memory to run
  * asynchronously).  lambda_out and charge_out are written at the end.  The outputs may
  * alias the inputs.  On return the device holds the same state (as after
