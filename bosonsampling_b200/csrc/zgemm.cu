@@ -1,8 +1,8 @@
 // Grouped complex128 GEMM for the contraction-shaped steps of the BS update
 // (the Theta block products, the Gram matrices, V = T Y / sigma, W = V^H C).
 //
-// FP64 has no tcgen05 kind on sm_100a, so this runs on the FP64 tensor path (m8n8k4): 64 x 64
-// output tile per CTA, 8 warps of 32 x 16, K in slabs of 8 complex through a ring of three
+// FP64 has no tcgen05 kind on sm_100a, so this runs on the FP64 tensor path (m8n8k4): 32 x 32
+// output tile per CTA, 4 warps of 16 x 16, K in slabs of 8 complex through a ring of three
 // shared-memory stages filled by cp.async (zeros past the edges).  op(A) and B keep their
 // storage order in shared memory, padded so that a fragment load (four k by two rows a
 // quarter warp) falls on distinct banks.  All groups of one launch share the grid; a CTA
@@ -11,14 +11,19 @@
 // What bounds it: the FP64 tensor rate for large groups, the slabs' latency for small ones.
 // 128-bit shared-memory reads take 4 cycles of the SM a warp: the vector form (4 x 4 complex
 // a thread) needed as many cycles for its operands as for its arithmetic, the fragments need
-// a fifth.  Measured, all GEMMs of one chi = 1024 update alone: 0.55 ms against 1.05; of two
-// layers at N = 64 (62 updates, beside other kernels): 20 ms against 36 to 44.
+// a quarter.  Measured, all GEMMs of one chi = 1024 update alone: 0.55 ms against 1.05 (64 x 64
+// tiles).  Why 32 x 32: a launch's sectors give 20 to 300 tiles of 64 x 64, less than a wave or
+// a ragged one, and a CTA's slabs wait for loads and barriers that other CTAs of the SM
+// fill.  64 and 32, ms: update at chi = 1024 3.05 and 2.83 (Gram route), 10.1 and 9.7 (fp64);
+// chi = 256 0.638 and 0.582, 1.575 and 1.450; 24 modes chi = 256 33.2 and 29.9; two layers at N =
+// 64, chi = 1024 (thousands of tiles) 45.2 and 43.5.
 #include "dmma.cuh"
 #include "kernels.h"
 
 namespace {
 
-constexpr int TM = 64, TN = 64, TK = 8, NT = 256, STAGES = 3;
+constexpr int TM = 32, TN = 32, TK = 8, NT = 128, STAGES = 3;
+constexpr int MI = 2, NJ = 2;  // 8 x 8 tiles of a warp
 constexpr int LDK = TK + 4;    // op(A) = A, stored [m][k]: 4 mod 8
 constexpr int LDM = TM + 2;    // A^H, stored [k][m], and B [k][n]: 2 mod 8
 constexpr int A_ELEMS = TM * LDK > TK * LDM ? TM * LDK : TK * LDM, B_ELEMS = TK * (TN + 2);
@@ -26,7 +31,7 @@ constexpr size_t SMEM = (size_t)STAGES * (A_ELEMS + B_ELEMS) * sizeof(double2);
 
 template <bool OPA>
 __device__ __forceinline__ void tile_loop(const GemmGroup& g, const cplx* __restrict__ a, const cplx* __restrict__ b,
-                                          int m0, int n0, double2* smem, double2 (&re)[4][2], double2 (&im)[4][2]) {
+                                          int m0, int n0, double2* smem, double2 (&re)[MI][NJ], double2 (&im)[MI][NJ]) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int M = g.M, N = g.N, K = g.K;
   auto stage_a = [&](int s) { return smem + s * (A_ELEMS + B_ELEMS); };
@@ -53,7 +58,7 @@ __device__ __forceinline__ void tile_loop(const GemmGroup& g, const cplx* __rest
       cp_async16(bs + k * (TN + 2) + n, ok ? b + (int64_t)(k0 + k) * g.ldb + n0 + n : b, ok);
     }
   };
-  const int wm = (warp >> 2) * 32, wn = (warp & 3) * 16, li = lane >> 2, lk = lane & 3;
+  const int wm = (warp >> 1) * 16, wn = (warp & 1) * 16, li = lane >> 2, lk = lane & 3;
   const bool live = m0 + wm < M && n0 + wn < N;   // a warp's tile past the edge does nothing
   const int slabs = (K + TK - 1) / TK;
 #pragma unroll
@@ -68,14 +73,14 @@ __device__ __forceinline__ void tile_loop(const GemmGroup& g, const cplx* __rest
     cp_async_commit();
     if (!live) continue;
     const double2 *as = stage_a(t % STAGES), *bs = stage_b(t % STAGES);
-    cmma_tile<4, 2, TK / 4, OPA>(
+    cmma_tile<MI, NJ, TK / 4, OPA>(
         re, im,
         [&](int i, int k) { return OPA ? as[(k + lk) * LDM + wm + 8 * i + li] : as[(wm + 8 * i + li) * LDK + k + lk]; },
         [&](int j, int k) { return bs[(k + lk) * (TN + 2) + wn + 8 * j + li]; });
   }
 }
 
-__global__ __launch_bounds__(NT, 2) void zgemm_grouped_kernel(const cplx* __restrict__ A, const cplx* __restrict__ B,
+__global__ __launch_bounds__(NT, 4) void zgemm_grouped_kernel(const cplx* __restrict__ A, const cplx* __restrict__ B,
                                                               cplx* __restrict__ C, const double* __restrict__ scale,
                                                               const GemmGroup* __restrict__ groups, int n_groups,
                                                               const SectorDesc* __restrict__ sd) {
@@ -101,26 +106,26 @@ __global__ __launch_bounds__(NT, 2) void zgemm_grouped_kernel(const cplx* __rest
   const int m0 = (tile / g.tiles_n) * TM, n0 = (tile % g.tiles_n) * TN;
   // tiles are laid out for the host's bound; a Hermitian group forms n0 >= m0
   if (m0 >= g.M || n0 >= g.N || (g.herm && n0 < m0)) return;
-  double2 re[4][2], im[4][2];
+  double2 re[MI][NJ], im[MI][NJ];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < MI; ++i)
 #pragma unroll
-    for (int j = 0; j < 2; ++j) re[i][j] = im[i][j] = make_double2(0.0, 0.0);
+    for (int j = 0; j < NJ; ++j) re[i][j] = im[i][j] = make_double2(0.0, 0.0);
   if (g.opA) tile_loop<true>(g, A + g.a_off, B + g.b_off, m0, n0, smem, re, im);
   else tile_loop<false>(g, A + g.a_off, B + g.b_off, m0, n0, smem, re, im);
   const int lane = tid & 31, warp = tid >> 5;
-  const int row0 = m0 + (warp >> 2) * 32 + (lane >> 2), col0 = n0 + (warp & 3) * 16 + 2 * (lane & 3);
+  const int row0 = m0 + (warp >> 1) * 16 + (lane >> 2), col0 = n0 + (warp & 1) * 16 + 2 * (lane & 3);
   const double* cs = g.cs_off >= 0 ? scale + g.cs_off : nullptr;
   cplx* c = C + g.c_off;
 #pragma unroll
-  for (int j = 0; j < 2; ++j)
+  for (int j = 0; j < NJ; ++j)
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
       const int n = col0 + 8 * j + x;
       if (n >= g.N) continue;
       const double f = cs ? cs[n] : 1.0;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < MI; ++i) {
         const int m = row0 + 8 * i;
         if (m >= g.M) continue;
         const cplx v = cmake(f * (x ? re[i][j].y : re[i][j].x), f * (x ? im[i][j].y : im[i][j].x));
