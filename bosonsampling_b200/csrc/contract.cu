@@ -12,18 +12,21 @@
 // taken in runs of equal charge (any order of the entries is allowed; an order by charge has
 // the fewest runs): a run's plain products are accumulated on the FP64 tensor path (m8n8k4),
 // and at its end each output adds its weight times the run's sum.  A run that no row and
-// column of the tile can use is not read.  What bounds it: the FP64 tensor rate, at a small
-// grid (32 x 32 tiles, 4 warps, so that a sector of 443 x 389 is 182 CTAs).  Measured there with
-// 1,024 centre entries, d = 5: 93 us; 16 x 16 tiles with the weight applied per entry took 270.
+// column of the tile can use is not read.  What bounds it: the FP64 tensor rate of the SM with
+// the most tiles, so they are small (32 x 16, 4 warps): a sector of 443 x 389 is 350 CTAs.
+// Measured there with 1,024 centre entries, d = 5, with the call and the wait: 188 us; with 32 x
+// 32 tiles (182 CTAs) 206; with 16 x 16 tiles and the weight applied per entry 383.  700 x
+// 1,024 x 300: 180 and 202; 1,500 x 1,024 x 1,400: 411 and 411.
 #include "dmma.cuh"
 #include "kernels.h"
 
 namespace {
 
 static_assert(BSMPO_MAX_D <= 1 << 10, "charges are far below the sentinel");
-constexpr int CT = 32, CK = 8, CNT = 128, CSTAGES = 3;
+constexpr int CT = 32, CN = 16, CK = 8, CNT = 128, CSTAGES = 3;   // rows, columns, centre entries
+constexpr int NJ = CN / 16;                // 8-column tiles of a warp
 constexpr int CWIN = 1024;                 // centre entries whose runs are listed at once
-constexpr int CLDA = CK + 4, CLDB = CT + 2;
+constexpr int CLDA = CK + 4, CLDB = CN + 2;
 constexpr int CSTAGE = CT * CLDA + CK * CLDB;
 
 // (a, b) >= (x, y) in both components
@@ -33,12 +36,12 @@ __device__ __forceinline__ bool ge2(int2 a, int2 b) { return a.x >= b.x && a.y >
 // run's first centre index once re / im hold its sum.  use is called by whole warps.
 template <typename Same, typename Use, typename Fold>
 __device__ __forceinline__ void run_products(const cplx* __restrict__ glc, const cplx* __restrict__ gcr, int len_l,
-                                             int len_c, int len_r, double2* smem, int* runs, double2 (&re)[2][2],
-                                             double2 (&im)[2][2], Same same, Use use, Fold fold) {
+                                             int len_c, int len_r, double2* smem, int* runs, double2 (&re)[2][NJ],
+                                             double2 (&im)[2][NJ], Same same, Use use, Fold fold) {
   __shared__ int wsum[CNT / 32], n_runs;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int m0 = blockIdx.y * CT, n0 = blockIdx.x * CT;
-  const int wm = (warp >> 1) * 16, wn = (warp & 1) * 16, li = lane >> 2, lk = lane & 3;
+  const int m0 = blockIdx.y * CT, n0 = blockIdx.x * CN;
+  const int wm = (warp >> 1) * 16, wn = (warp & 1) * (CN / 2), li = lane >> 2, lk = lane & 3;
   for (int w0 = 0; w0 < len_c; w0 += CWIN) {
     const int w1 = min(w0 + CWIN, len_c);
     // starts of the window's runs, in order
@@ -78,8 +81,8 @@ __device__ __forceinline__ void run_products(const cplx* __restrict__ glc, const
         cp_async16(as + m * CLDA + k, ok ? glc + (int64_t)(m0 + m) * len_c + fk + k : glc, ok);
       }
 #pragma unroll
-      for (int i = 0; i < CT * CK / CNT; ++i) {
-        const int e = tid + i * CNT, k = e / CT, n = e % CT;
+      for (int i = 0; i < CN * CK / CNT; ++i) {
+        const int e = tid + i * CNT, k = e / CN, n = e % CN;
         const bool ok = n0 + n < len_r && fk + k < end;
         cp_async16(bs + k * CLDB + n, ok ? gcr + (int64_t)(fk + k) * len_r + n0 + n : gcr, ok);
       }
@@ -101,7 +104,7 @@ __device__ __forceinline__ void run_products(const cplx* __restrict__ glc, const
       fill((t + CSTAGES - 1) % CSTAGES);
       cp_async_commit();
       const double2 *as = smem + (t % CSTAGES) * CSTAGE, *bs = as + CT * CLDA;
-      cmma_tile<2, 2, CK / 4, false>(
+      cmma_tile<2, NJ, CK / 4, false>(
           re, im, [&](int i, int k) { return as[(wm + 8 * i + li) * CLDA + k + lk]; },
           [&](int j, int k) { return bs[(k + lk) * CLDB + wn + 8 * j + li]; });
       ck += CK;
@@ -110,7 +113,7 @@ __device__ __forceinline__ void run_products(const cplx* __restrict__ glc, const
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
-          for (int j = 0; j < 2; ++j) re[i][j] = im[i][j] = make_double2(0.0, 0.0);
+          for (int j = 0; j < NJ; ++j) re[i][j] = im[i][j] = make_double2(0.0, 0.0);
         cr = next_used(cr + 1);
         if (cr < nr) ck = runs[cr];
       }
@@ -125,7 +128,7 @@ struct TileLane {
   __device__ TileLane() {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     row0 = blockIdx.y * CT + (warp >> 1) * 16 + (lane >> 2);
-    col0 = blockIdx.x * CT + (warp & 1) * 16 + 2 * (lane & 3);
+    col0 = blockIdx.x * CN + (warp & 1) * (CN / 2) + 2 * (lane & 3);
   }
   __device__ int row(int i) const { return row0 + 8 * i; }
   __device__ int col(int j, int x) const { return col0 + 8 * j + x; }
@@ -138,7 +141,7 @@ __global__ __launch_bounds__(CNT) void contract_sector_kernel(int d, int cc0, in
                                                               cplx* __restrict__ out) {
   __shared__ __align__(16) double2 smem[CSTAGES * CSTAGE];
   __shared__ cplx us[BSMPO_MAX_D * BSMPO_MAX_D * BSMPO_MAX_D];
-  __shared__ int2 rows[CT], cols[CT];
+  __shared__ int2 rows[CT], cols[CN];
   __shared__ int runs[CWIN];
   const int tid = threadIdx.x, d3 = d * d * d;
   for (int i = tid; i < d3; i += CNT) us[i] = u[i];
@@ -148,26 +151,29 @@ __global__ __launch_bounds__(CNT) void contract_sector_kernel(int d, int cc0, in
     const int l = blockIdx.y * CT + tid;
     const int2 a = l < len_l ? cl[l] : make_int2(d, d);
     rows[tid] = a.x < d && a.y < d && a.x >= cc0 && a.y >= cc1 ? a : make_int2(-1, -1);
-  } else if (tid < 2 * CT) {
-    const int r = blockIdx.x * CT + tid - CT;
+  } else if (tid < CT + CN) {
+    const int r = blockIdx.x * CN + tid - CT;
     const int2 b = r < len_r ? cr[r] : make_int2(d, d);
     cols[tid - CT] = b.x < d && b.y < d && b.x <= cc0 && b.y <= cc1 ? b : make_int2(BIG, BIG);
   }
   __syncthreads();
   const TileLane T;
-  int2 a[2], b[2][2];
+  int2 a[2], b[NJ][2];
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     a[i] = rows[T.row(i) - blockIdx.y * CT];
-    b[i][0] = cols[T.col(i, 0) - blockIdx.x * CT];
-    b[i][1] = cols[T.col(i, 1) - blockIdx.x * CT];
   }
-  double2 re[2][2], im[2][2];
-  cplx acc[2][2][2];
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    b[j][0] = cols[T.col(j, 0) - blockIdx.x * CN];
+    b[j][1] = cols[T.col(j, 1) - blockIdx.x * CN];
+  }
+  double2 re[2][NJ], im[2][NJ];
+  cplx acc[2][NJ][2];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
+    for (int j = 0; j < NJ; ++j) {
       re[i][j] = im[i][j] = make_double2(0.0, 0.0);
       acc[i][j][0] = acc[i][j][1] = cmake(0.0, 0.0);
     }
@@ -178,7 +184,7 @@ __global__ __launch_bounds__(CNT) void contract_sector_kernel(int d, int cc0, in
         const int2 q = cc[i];
         if (q.x >= d || q.y >= d) return false;
         const int t = threadIdx.x & 31;   // a lane to a row and a column of the tile
-        const bool r = __any_sync(0xffffffffu, ge2(rows[t], q)), c = __any_sync(0xffffffffu, ge2(q, cols[t]));
+        const bool r = __any_sync(0xffffffffu, ge2(rows[t], q)), c = __any_sync(0xffffffffu, ge2(q, cols[t % CN]));
         return r && c;
       },
       [&](int i0) {
@@ -187,7 +193,7 @@ __global__ __launch_bounds__(CNT) void contract_sector_kernel(int d, int cc0, in
         for (int i = 0; i < 2; ++i) {
           if (!ge2(a[i], q)) continue;
 #pragma unroll
-          for (int j = 0; j < 2; ++j)
+          for (int j = 0; j < NJ; ++j)
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
               const int2 c = b[j][x];
@@ -202,7 +208,7 @@ __global__ __launch_bounds__(CNT) void contract_sector_kernel(int d, int cc0, in
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+    for (int j = 0; j < NJ; ++j)
 #pragma unroll
       for (int x = 0; x < 2; ++x)
         if (T.row(i) < len_l && T.col(j, x) < len_r) stc(out + (int64_t)T.row(i) * len_r + T.col(j, x), acc[i][j][x]);
@@ -277,7 +283,7 @@ cudaError_t launch_contract_sector(int d, int cc0, int cc1, const void* u, const
                                    const void* gcr, const int* cl, const int* cc, const int* cr,
                                    int len_l, int len_c, int len_r, void* c, cudaStream_t s) {
   if (len_l <= 0 || len_r <= 0) return cudaSuccess;
-  dim3 grid(ceil_div(len_r, CT), ceil_div(len_l, CT));
+  dim3 grid(ceil_div(len_r, CN), ceil_div(len_l, CT));
   contract_sector_kernel<<<grid, CNT, 0, s>>>(
       d, cc0, cc1, reinterpret_cast<const cplx*>(u), reinterpret_cast<const cplx*>(glc),
       reinterpret_cast<const cplx*>(gcr), reinterpret_cast<const int2*>(cl),
