@@ -597,7 +597,9 @@ __device__ __forceinline__ double group_sum(double a) {
 // X P = Q R of one matrix: the reflectors H_j = 1 - t_j v_j v_j^H, v_j the rows below j of
 // column piv[j] under v1[j]; R's diagonal rd, its row i < j in row i of column piv[j].
 struct JsQr {
-  double nn[2][JS_KMAX];   // squared norms of the columns' rows below the reduced ones, -1: reduced
+  // squared norms of the columns' rows below the reduced ones; reduced: < 0, which a NaN is
+  // not, so piv ends as a permutation whatever the numbers are
+  double nn[2][JS_KMAX];
   double2 rd[JS_KMAX], v1[JS_KMAX];
   double t[JS_KMAX];
   int piv[JS_KMAX];
@@ -625,7 +627,7 @@ __device__ __forceinline__ bool js_qr_steps(double2* X, int ld, int rows, int k,
       if (tid == 0) {
         int at = j;
         for (int c = 0; c < k; ++c)
-          if (nn[c] >= 0.0) q.piv[at++] = c;
+          if (!(nn[c] < 0.0)) q.piv[at++] = c;
       }
       for (int i = j + tid; i < k; i += 32 * n_warps) {
         q.rd[i] = q.v1[i] = make_double2(0.0, 0.0);
@@ -664,7 +666,7 @@ __device__ __forceinline__ bool js_qr_steps(double2* X, int ld, int rows, int k,
     }
     for (int base = warp * GPW; base < k; base += n_warps * GPW) {
       const int c = base + g;
-      const bool act = c < k && c != p && nn[c] >= 0.0;
+      const bool act = c < k && c != p && !(nn[c] < 0.0);
       double2* x = X + (act ? c : p) * ld;
       double dx = 0.0, dy = 0.0, s = 0.0;
       auto dot = [&](double2 a, double2 b) {   // conj(a) b
@@ -929,8 +931,33 @@ __global__ __launch_bounds__(NT) void jacobi_small_kernel(const SectorDesc* __re
   __syncthreads();
   double f2 = 0.0;
   for (int c = 0; c < k; ++c) f2 += q1.nn[0][c];
-  __syncthreads();                                     // q1.nn[0] is overwritten from the second step on
   const double zf = 16.0 * 2.220446049250313e-16 * sqrt((double)rows), z2 = zf * zf * f2;
+  // singular values from the squared norms in nrm (0 below the numerical-rank floor, -1 for a
+  // NaN), in descending order (ties by column): perm is a permutation whatever nrm holds
+  auto finish = [&] {
+    if (tid < k) {
+      const double s = nrm[tid];
+      nrm[tid] = s <= z2 ? 0.0 : s >= 0.0 ? sqrt(s) : -1.0;
+    }
+    __syncthreads();
+    if (tid < k) {
+      const double s = nrm[tid];
+      int at = 0;
+      for (int c = 0; c < k; ++c) at += nrm[c] > s || (nrm[c] == s && c < tid);
+      sig[S.s_off + at] = s;
+      perm[S.s_off + at] = tid;
+    }
+  };
+  if (!(f2 <= 1.7976931348623157e308)) {
+    // a NaN or an infinity in X (uniform over the CTA): as in the blocked form, whose tests
+    // are all false then, no column is rotated
+    if (tid < k) nrm[tid] = q1.nn[0][tid];
+    __syncthreads();
+    finish();
+    for (int e = tid; left && e < k * k; e += NT) stc(A + (int64_t)rows * k + e, cmake(e / k == e % k ? 1.0 : 0.0, 0.0));
+    return;
+  }
+  __syncthreads();                                     // q1.nn[0] is overwritten from the second step on
   const double tol = fmax(8.0 * 2.220446049250313e-16, 4.0 * 2.220446049250313e-16 * sqrt((double)k));
   const double t2 = tol * tol;
   if (rows <= 64) js_qr<8, 8>(X, ldx, rows, k, q1, NW);
@@ -990,18 +1017,9 @@ __global__ __launch_bounds__(NT) void jacobi_small_kernel(const SectorDesc* __re
     }
   }
   __syncthreads();
-  // column norms (0 below the numerical-rank floor), the descending order (ties by column)
   js_norms(Y, ld, k, k, nrm, NW);
   __syncthreads();
-  if (tid < k) nrm[tid] = nrm[tid] <= z2 ? 0.0 : sqrt(nrm[tid]);
-  __syncthreads();
-  if (tid < k) {
-    const double s = nrm[tid];
-    int at = 0;
-    for (int c = 0; c < k; ++c) at += nrm[c] > s || (nrm[c] == s && c < tid);
-    sig[S.s_off + at] = s;
-    perm[S.s_off + at] = tid;
-  }
+  finish();
   if (left) {
     // the left vectors, where the blocked form accumulates its rotations
     for (int e = tid; e < k * k; e += NT) {
