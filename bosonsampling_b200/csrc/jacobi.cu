@@ -573,6 +573,7 @@ __global__ __launch_bounds__(NNT) void sector_norm_kernel(const SectorDesc* __re
 // 13.8 and 10.0, chi = 128 31 and 20.5.
 constexpr int JS_KMAX = 64;
 constexpr int JS_SMEM = 216 * 1024;
+constexpr int JS_EX = 100;     // binary exponents of X's largest entry that need no scaling
 
 // leading dimension of a column: odd in units of 16 B, so lanes across columns fall on
 // different banks
@@ -623,7 +624,7 @@ __device__ __forceinline__ bool js_qr_steps(double2* X, int ld, int rows, int k,
     const unsigned in0 = __ballot_sync(0xffffffffu, h0 == hm), in1 = __ballot_sync(0xffffffffu, h1 == hm);
     const int p = in0 ? __ffs(in0) - 1 : 31 + __ffs(in1);
     const double n2 = nn[p];
-    if (n2 < 1e-270) {                 // nothing left (uniform over the CTA): R's other rows are zero
+    if (n2 < 1e-270) {                 // nothing left (f2 >= 2^-200; uniform over the CTA): R's other rows are zero
       if (tid == 0) {
         int at = j;
         for (int c = 0; c < k; ++c)
@@ -912,7 +913,7 @@ __global__ __launch_bounds__(NT) void jacobi_small_kernel(const SectorDesc* __re
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ JsQr q1, q2;
   __shared__ double nrm[JS_KMAX];
-  __shared__ int rot[2], inv2[JS_KMAX];
+  __shared__ int rot[2], inv2[JS_KMAX], top;
   const SectorDesc& S = sd[list[blockIdx.x]];
   const int k = S.k, rows = S.rows_g, ldx = js_ld(rows), ld = js_ldl(k);
   const bool left = S.left != 0;
@@ -920,13 +921,31 @@ __global__ __launch_bounds__(NT) void jacobi_small_kernel(const SectorDesc* __re
   double2* Y = X + (size_t)k * ldx;                    // L, column c: Y + c ld
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   cplx* A = abuf + S.a_off;
+  if (tid < 2) rot[tid] = 0;
+  if (tid == 0) top = 0;
+  __syncthreads();
+  int hi = 0;                                          // largest leading word of an entry's magnitude
   for (int e = tid; e < rows * k; e += NT) {
     const int r = e / k, c = e - r * k;
     const cplx v = ldc(A + e);
     X[c * ldx + r] = make_double2(v.x, v.y);
+    hi = max(hi, max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff));
   }
-  if (tid < 2) rot[tid] = 0;
+  __syncwarp();
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if (lane == 0) atomicMax(&top, hi);
   __syncthreads();
+  // X 2^-ex where squares of its entries could leave the exponent's range (uniform over the
+  // CTA), so the result does not depend on the scale; undone in the values and in X = T's columns
+  int ex = (top >> 20) - 1023;
+  if (top == 0 || top >= 0x7ff00000 || abs(ex) <= JS_EX) ex = 0;
+  if (ex != 0) {
+    for (int e = tid; e < rows * k; e += NT) {
+      double2* x = X + (e % k) * ldx + e / k;
+      *x = make_double2(scalbn(x->x, -ex), scalbn(x->y, -ex));
+    }
+    __syncthreads();
+  }
   js_norms(X, ldx, rows, k, q1.nn[0], NW);
   __syncthreads();
   double f2 = 0.0;
@@ -944,7 +963,7 @@ __global__ __launch_bounds__(NT) void jacobi_small_kernel(const SectorDesc* __re
       const double s = nrm[tid];
       int at = 0;
       for (int c = 0; c < k; ++c) at += nrm[c] > s || (nrm[c] == s && c < tid);
-      sig[S.s_off + at] = s;
+      sig[S.s_off + at] = ex != 0 ? scalbn(s, ex) : s;
       perm[S.s_off + at] = tid;
     }
   };
@@ -1029,6 +1048,10 @@ __global__ __launch_bounds__(NT) void jacobi_small_kernel(const SectorDesc* __re
       stc(A + (int64_t)(rows + q1.piv[r]) * k + c, cmake(v.x * is, v.y * is));
     }
     return;
+  }
+  if (ex != 0) {
+    for (int e = tid; e < ld * k; e += NT) Y[e] = make_double2(scalbn(Y[e].x, ex), scalbn(Y[e].y, ex));
+    __syncthreads();
   }
   auto y0 = [&](int c, int r) { return Y[c * ld + inv2[r]]; };
   if (rows <= 64) js_q_apply<8, 8>(X, ldx, rows, k, q1, A, NW, y0);
