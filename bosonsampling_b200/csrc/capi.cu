@@ -100,6 +100,9 @@ struct bsmpo_ctx {
   // cannot exceed chi; 1 also after a selection that keeps fewer than chi; 2 also where
   // the centre bond holds fewer than chi vectors
   int gram_policy = 0;
+  // BSMPO_TEST_ERROR (tests only, read at create): 1, 2 sets an error word behind the SVD of
+  // the next update (an expired wait; no convergence), once
+  int test_error = 0;
   // which contractions of BSMPO_PRECISION_TF32X3 go on the tensor cores (BSMPO_TC_MASK,
   // read at create): bit 0 the Theta block products, bit 1 W = V^H C; the others FP64.
   // Default: Theta only.  W = V^H C is formed at the scale of C (columns carry
@@ -1172,6 +1175,10 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
   rc = P.gram ? gram_eigenvalues(h, P, sd_d, groups_at(L.ggram), list_d, tcerr_d)
               : jacobi_svd(h, P, sd_d, dt + L.jw, list_d, pre_d, res_d, R);
   if (rc || (rc = clk.mark(3))) return rc;
+  if (h->test_error == 1 || h->test_error == 2) {
+    CK(h, cudaMemsetAsync(tcerr_d + h->test_error - 1, 1, sizeof(int), st));
+    h->test_error = 0;
+  }
   auto select = [&]() -> int {
     CKL(h, launch_select(tab_d, sd_d, nj, ns, reinterpret_cast<double*>(h->sig.p),
                          reinterpret_cast<double*>(h->keys.p), h->cutoff, chi, kept_d, trunc_d, st));
@@ -1236,8 +1243,9 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
                                 P.w_tiles, sd_d, st));
   }
   if ((rc = clk.mark(5))) return rc;
-  // 6. scatter into Gamma[mode], Gamma[mode+1], Lambda / charge of bond mode+1
-  CKL(h, launch_scatter(tab_d, sd_d, nj, kept_d + ns, chi, h->vbuf.p, h->wbuf.p,
+  // 6. scatter into Gamma[mode], Gamma[mode+1], Lambda / charge of bond mode+1 (nothing is
+  // written where an error word is set: the state stays that of the host mirror)
+  CKL(h, launch_scatter(tab_d, sd_d, nj, kept_d + ns, tcerr_d, chi, h->vbuf.p, h->wbuf.p,
                         reinterpret_cast<double*>(h->sig.p), h->gamma, h->lam, h->charge, st));
   if ((rc = clk.mark(6))) return rc;
   CK(h, wait_event(h->wait_ev));
@@ -1429,6 +1437,7 @@ int run_mesh_concurrent(bsmpo_ctx* h, int n_bs, const int* modes, const cplx* u3
     w->tc_mask = h->tc_mask;
     w->td_fork = h->td_fork;
     w->jac_rows = h->jac_rows;
+    w->test_error = h->test_error;
     w->timing = h->timing;
     if (w->timing && !w->ev0) {
       CK(h, cudaEventCreate(&w->ev0));
@@ -1436,6 +1445,7 @@ int run_mesh_concurrent(bsmpo_ctx* h, int n_bs, const int* modes, const cplx* u3
     }
     w->last_index = -1;
   }
+  h->test_error = 0;
   // dependencies
   std::vector<int> pred((size_t)3 * n_bs, -1), remaining(n_bs, 0);
   std::vector<std::vector<int>> succ(n_bs);
@@ -1776,6 +1786,8 @@ int bsmpo_create(int n, int d, int chi, int flags, bsmpo_ctx** out) {
   if (gp && gp[0] >= '0' && gp[0] <= '2') h->gram_policy = gp[0] - '0';
   const char* tf = std::getenv("BSMPO_TD_FORK");
   if (tf && tf[0] >= '0' && tf[0] <= '3') h->td_fork = tf[0] - '0';
+  const char* te = std::getenv("BSMPO_TEST_ERROR");
+  if (te && te[0] >= '1' && te[0] <= '2') h->test_error = te[0] - '0';
   const char* nwk = std::getenv("BSMPO_WORKERS");
   if (nwk && std::atoi(nwk) >= 1 && std::atoi(nwk) <= 64) h->n_workers = std::atoi(nwk);
   *out = h;

@@ -124,9 +124,10 @@ cudaError_t launch_extract_v(const SectorDesc* sd_dev, int n_sectors, int max_el
                              const void* abuf, const double* sig, const int* perm, void* vbuf,
                              cudaStream_t s);
 // New Gamma_L (= Gamma[mode]), Gamma_R (= Gamma[mode+1]), Lambda and charges of bond mode+1
-// of every update; gamma, lam, charge: the whole state's; totals: kept vectors per update.
+// of every update; gamma, lam, charge: the whole state's; totals: kept vectors per update;
+// err: two words on the device, nothing is written unless both are zero.
 cudaError_t launch_scatter(const UpdateTables* tab_dev, const SectorDesc* sd_dev, int n_updates,
-                           const int* totals, int chi, const void* vbuf, const void* wbuf,
+                           const int* totals, const int* err, int chi, const void* vbuf, const void* wbuf,
                            const double* sig, void* gamma, double* lam, int* charge,
                            cudaStream_t s);
 // exp(i phi (n_ket - n_bra)) on every element of one site tensor.

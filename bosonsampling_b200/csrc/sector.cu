@@ -355,12 +355,14 @@ constexpr int SC_NT = 256;
 __global__ __launch_bounds__(SC_NT) void scatter_kernel(const UpdateTables* __restrict__ tabs,
                                                         const SectorDesc* __restrict__ sds,
                                                         const int* __restrict__ totals,
+                                                        const int* __restrict__ err,
                                                         const cplx* __restrict__ vbuf,
                                                         const cplx* __restrict__ wbuf,
                                                         const double* __restrict__ sig,
                                                         cplx* __restrict__ gamma,
                                                         double* __restrict__ lam,
                                                         int2* __restrict__ charge) {
+  if (err[0] != 0 || err[1] != 0) return;   // a failed group leaves the state as it is
   const UpdateTables* tab = tabs + blockIdx.y;
   const SectorDesc* sd = sds + tab->sec0;
   const int ns = tab->n_sectors, total_kept = totals[blockIdx.y];
@@ -506,13 +508,13 @@ cudaError_t launch_extract_v(const SectorDesc* sd_dev, int n_sectors, int max_el
 }
 
 cudaError_t launch_scatter(const UpdateTables* tab_dev, const SectorDesc* sd_dev, int n_updates,
-                           const int* totals, int chi, const void* vbuf, const void* wbuf,
+                           const int* totals, const int* err, int chi, const void* vbuf, const void* wbuf,
                            const double* sig, void* gamma, double* lam, int* charge, cudaStream_t s) {
   if (n_updates <= 0) return cudaSuccess;
   const int64_t total = 2 * (int64_t)chi * chi + chi;
   const int blocks = (int)std::min<int64_t>((total + SC_NT - 1) / SC_NT, 148 * 16);
   scatter_kernel<<<dim3(blocks, n_updates), SC_NT, 0, s>>>(
-      tab_dev, sd_dev, totals, reinterpret_cast<const cplx*>(vbuf), reinterpret_cast<const cplx*>(wbuf), sig,
+      tab_dev, sd_dev, totals, err, reinterpret_cast<const cplx*>(vbuf), reinterpret_cast<const cplx*>(wbuf), sig,
       reinterpret_cast<cplx*>(gamma), lam, reinterpret_cast<int2*>(charge));
   return cudaGetLastError();
 }
