@@ -101,7 +101,8 @@ struct bsmpo_ctx {
   // the centre bond holds fewer than chi vectors
   int gram_policy = 0;
   // BSMPO_TEST_ERROR (tests only, read at create): 1, 2 sets an error word behind the SVD of
-  // the next update (an expired wait; no convergence), once
+  // the next update (an expired wait; no convergence), 3 the first behind its tensor-core
+  // W = V^H C, once
   int test_error = 0;
   // which contractions of BSMPO_PRECISION_TF32X3 go on the tensor cores (BSMPO_TC_MASK,
   // read at create): bit 0 the Theta block products, bit 1 W = V^H C; the others FP64.
@@ -1238,6 +1239,13 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
   if (tc_w) {
     CK(h, wait_event(h->wait_ev));
     if ((rc = tc_w_gemm(h, P, hk, tcerr_d))) return rc;
+    if (h->test_error == 3) {
+      CK(h, cudaMemsetAsync(tcerr_d, 1, sizeof(int), st));
+      h->test_error = 0;
+    }
+    // the error words again: the results above were copied before this GEMM's waits
+    CK(h, cudaMemcpyAsync(hres + R.err, tcerr_d, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(h, cudaEventRecord(h->wait_ev, st));
   } else {
     CKL(h, launch_zgemm_grouped(h->vbuf.p, h->cbuf.p, h->wbuf.p, nullptr, groups_at(L.gw), (int)P.gw.size(),
                                 P.w_tiles, sd_d, st));
@@ -1787,7 +1795,7 @@ int bsmpo_create(int n, int d, int chi, int flags, bsmpo_ctx** out) {
   const char* tf = std::getenv("BSMPO_TD_FORK");
   if (tf && tf[0] >= '0' && tf[0] <= '3') h->td_fork = tf[0] - '0';
   const char* te = std::getenv("BSMPO_TEST_ERROR");
-  if (te && te[0] >= '1' && te[0] <= '2') h->test_error = te[0] - '0';
+  if (te && te[0] >= '1' && te[0] <= '3') h->test_error = te[0] - '0';
   const char* nwk = std::getenv("BSMPO_WORKERS");
   if (nwk && std::atoi(nwk) >= 1 && std::atoi(nwk) <= 64) h->n_workers = std::atoi(nwk);
   *out = h;

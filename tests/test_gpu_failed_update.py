@@ -84,3 +84,24 @@ def test_mesh_that_fails(word, workers, state, monkeypatch):
         sim.load_host(*after)
         sim.run_mesh(*_mesh(8, 6))
         assert _equal(_host(sim), got)
+
+
+def test_expired_wait_of_the_last_gemm(state, monkeypatch):
+    """W = V^H C on the tensor cores: a wait of its own that expires is this update's error."""
+    monkeypatch.setenv("BSMPO_TC_MASK", "3")
+    monkeypatch.setenv("BSMPO_TEST_ERROR", "3")
+    S = interferometer.t_block(0.7, 0.4)
+    with engine.MPOSimulator(N, D, CHI) as sim:
+        sim.set_precision("tf32x3")
+        sim.load_host(*state)
+        with pytest.raises(RuntimeError, match="wait expired"):
+            sim.bs_update(5, S)
+        assert _equal(_host(sim), state)
+        sim.bs_update(5, S)
+        got = _host(sim)
+    monkeypatch.delenv("BSMPO_TEST_ERROR")
+    with engine.MPOSimulator(N, D, CHI) as sim:
+        sim.set_precision("tf32x3")
+        sim.load_host(*state)
+        sim.bs_update(5, S)
+        assert _equal(_host(sim), got)
