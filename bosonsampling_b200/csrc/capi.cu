@@ -102,7 +102,7 @@ struct bsmpo_ctx {
   int gram_policy = 0;
   // BSMPO_TEST_ERROR (tests only, read at create): 1, 2 sets an error word behind the SVD of
   // the next update (an expired wait; no convergence), 3 the first behind its tensor-core
-  // W = V^H C, once
+  // W = V^H C, once; 10 + m: device allocation m fails, once
   int test_error = 0;
   // which contractions of BSMPO_PRECISION_TF32X3 go on the tensor cores (BSMPO_TC_MASK,
   // read at create): bit 0 the Theta block products, bit 1 W = V^H C; the others FP64.
@@ -230,7 +230,9 @@ int grow(bsmpo_ctx* h, DevBuf& b, size_t bytes) {
   size_t want = 4096;
   while (want < bytes + 256) want <<= 1;
   h->dev_grows++;
-  if (cudaMallocFromPoolAsync(&b.p, want, h->pool, h->stream) != cudaSuccess) {
+  const bool refused = h->test_error >= 10 && --h->test_error == 9;
+  if (refused) h->test_error = 0;
+  if (refused || cudaMallocFromPoolAsync(&b.p, want, h->pool, h->stream) != cudaSuccess) {
     cudaGetLastError();
     b.p = nullptr;
     return fail(h, BSMPO_ENOMEM, "device allocation of " + std::to_string(want) + " bytes failed");
@@ -882,6 +884,21 @@ int jacobi_svd(bsmpo_ctx* h, const Plan& P, SectorDesc* sd_d, char* jw_d, const 
   char* hres = static_cast<char*>(h->hres.p);
   unsigned long long* work_d = reinterpret_cast<unsigned long long*>(res_d + R.work);
   if ((rc = grow(h, h->perm, std::max<int64_t>(P.s_elems, 1) * sizeof(int)))) return rc;
+  // every workspace before the small sectors' launch: a side stream still at work when a buffer
+  // is given back would not be waited for
+  const size_t jw_bytes = align_up(std::max<size_t>(P.jw.size(), 1) * sizeof(JacobiWork), 256);
+  if (n_big) {
+    const size_t pair_elems = (size_t)4 * jacobi_block_cols() * jacobi_block_cols();
+    if ((rc = grow(h, h->rot, (size_t)3 * ns * sizeof(int)))) return rc;
+    if ((rc = grow(h, h->nf2, (size_t)ns * sizeof(double)))) return rc;
+    if ((rc = grow(h, h->qbuf, std::max(P.jac_slots, 1) * pair_elems * sizeof(cplx)))) return rc;
+    if ((rc = grow(h, h->qflag, std::max(P.jac_slots, 1) * sizeof(int)))) return rc;
+    if ((rc = grow(h, h->pcnt, std::max(P.jac_slots, 1) * sizeof(int)))) return rc;
+    if ((rc = grow(h, h->pbuf, std::max(P.gram_ctas, 1) * pair_elems * sizeof(cplx)))) return rc;
+    if ((rc = grow_host(h, h->stage2, 2 * jw_bytes))) return rc;
+    for (cudaEvent_t& e : h->poll_ev)
+      if (!e) CK(h, cudaEventCreateWithFlags(&e, cudaEventBlockingSync | cudaEventDisableTiming));
+  }
   double* sig = reinterpret_cast<double*>(h->sig.p);
   int* perm = reinterpret_cast<int*>(h->perm.p);
   if (h->timing) CK(h, cudaEventRecord(h->ev0, st));
@@ -907,13 +924,6 @@ int jacobi_svd(bsmpo_ctx* h, const Plan& P, SectorDesc* sd_d, char* jw_d, const 
     if (h->timing) CK(h, cudaEventRecord(h->ev1, st));
     return BSMPO_OK;
   }
-  const size_t pair_elems = (size_t)4 * jacobi_block_cols() * jacobi_block_cols();
-  if ((rc = grow(h, h->rot, (size_t)3 * ns * sizeof(int)))) return rc;
-  if ((rc = grow(h, h->nf2, (size_t)ns * sizeof(double)))) return rc;
-  if ((rc = grow(h, h->qbuf, std::max(P.jac_slots, 1) * pair_elems * sizeof(cplx)))) return rc;
-  if ((rc = grow(h, h->qflag, std::max(P.jac_slots, 1) * sizeof(int)))) return rc;
-  if ((rc = grow(h, h->pcnt, std::max(P.jac_slots, 1) * sizeof(int)))) return rc;
-  if ((rc = grow(h, h->pbuf, std::max(P.gram_ctas, 1) * pair_elems * sizeof(cplx)))) return rc;
   double* nf2 = reinterpret_cast<double*>(h->nf2.p);
   CKL(h, launch_sector_norms(sd_d, list_d + P.n_small, n_big, h->abuf.p, nf2, st));
   CK(h, cudaMemsetAsync(h->rot.p, 0, (size_t)3 * ns * sizeof(int), st));
@@ -927,11 +937,7 @@ int jacobi_svd(bsmpo_ctx* h, const Plan& P, SectorDesc* sd_d, char* jw_d, const 
   // and compacted launch tables alternate between two pinned slots.
   int* hrot_slot[2] = {reinterpret_cast<int*>(hres + R.rot), nullptr};
   hrot_slot[1] = hrot_slot[0] + 3 * ns;
-  const size_t jw_bytes = align_up(std::max<size_t>(P.jw.size(), 1) * sizeof(JacobiWork), 256);
-  if ((rc = grow_host(h, h->stage2, 2 * jw_bytes))) return rc;
   char* jw_stage[2] = {static_cast<char*>(h->stage2.p), static_cast<char*>(h->stage2.p) + jw_bytes};
-  for (cudaEvent_t& e : h->poll_ev)
-    if (!e) CK(h, cudaEventCreateWithFlags(&e, cudaEventBlockingSync | cudaEventDisableTiming));
   int t = 0;
   const int t_max = MAX_SWEEPS * std::max(1, P.max_rounds);
   bool converged = false;
@@ -1795,7 +1801,7 @@ int bsmpo_create(int n, int d, int chi, int flags, bsmpo_ctx** out) {
   const char* tf = std::getenv("BSMPO_TD_FORK");
   if (tf && tf[0] >= '0' && tf[0] <= '3') h->td_fork = tf[0] - '0';
   const char* te = std::getenv("BSMPO_TEST_ERROR");
-  if (te && te[0] >= '1' && te[0] <= '3') h->test_error = te[0] - '0';
+  if (te && std::atoi(te) > 0) h->test_error = std::atoi(te);
   const char* nwk = std::getenv("BSMPO_WORKERS");
   if (nwk && std::atoi(nwk) >= 1 && std::atoi(nwk) <= 64) h->n_workers = std::atoi(nwk);
   *out = h;

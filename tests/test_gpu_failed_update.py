@@ -105,3 +105,30 @@ def test_expired_wait_of_the_last_gemm(state, monkeypatch):
         sim.load_host(*state)
         sim.bs_update(5, S)
         assert _equal(_host(sim), got)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp64-gram"])
+def test_every_allocation_that_fails(precision, state, monkeypatch):
+    """Whichever workspace cannot be had, small sectors' kernels beside the others included: an
+    error, the state as it was, and the next update as in a new handle."""
+    S = interferometer.t_block(0.7, 0.4)
+    with engine.MPOSimulator(N, D, CHI) as sim:
+        sim.set_precision(precision)
+        sim.load_host(*state)
+        sim.bs_update(5, S)
+        want = _host(sim)
+    failed = 0
+    for m in range(60):
+        monkeypatch.setenv("BSMPO_TEST_ERROR", str(10 + m))
+        with engine.MPOSimulator(N, D, CHI) as sim:
+            sim.set_precision(precision)
+            sim.load_host(*state)
+            try:
+                sim.bs_update(5, S)
+            except RuntimeError as e:
+                assert "allocation" in str(e)
+                failed += 1
+                assert _equal(_host(sim), state)
+                sim.bs_update(5, S)
+            assert _equal(_host(sim), want)
+    assert 10 <= failed < 60
