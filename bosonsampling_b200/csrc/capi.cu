@@ -122,7 +122,9 @@ struct bsmpo_ctx {
   HostStage stage, stage2, hres;
   // last update diagnostics (host)
   std::vector<int> last_cc, last_shape, last_kept, last_k;
-  int64_t last_sig_off = 0;   // first singular value of that update in `sig`
+  int64_t last_sig_off = 0;   // first singular value of that update in `sig`, or
+  bool last_sig_kept = false; // in `dsig` (meshes: the lane's later groups overwrite `sig`)
+  DevBuf dsig;
   double last_trunc = 0.0, last_gemm = 0.0, last_svd = 0.0, last_bytes = 0.0;
   int last_sweeps = 0;
   // opt-in stage timing (BSMPO_PROFILE=1): synchronises after every stage
@@ -147,7 +149,7 @@ struct bsmpo_ctx {
   std::vector<bsmpo_ctx*> workers;
   int n_workers = 8;      // BSMPO_WORKERS / bsmpo_set_workers
   const bsmpo_ctx* diag = nullptr;
-  int last_index = -1;    // worker: mesh index of the last update it ran
+  bool ran_last = false;  // worker: it ran the last update of the mesh
   std::vector<double> mesh_tw;   // truncation weight of every update of the last mesh
   int64_t route_count[2] = {0, 0};   // updates solved by Jacobi [0] and by the Gram route [1]
 };
@@ -1083,9 +1085,10 @@ int tc_w_gemm(bsmpo_ctx* h, const Plan& P, const int* hk, int* err_d) {
 
 // Updates at the modes of `jobs` (disjoint sites, one route), all in the same launches.
 // Every sector computes exactly what it computes in a group of its own; trunc[j], if
-// given, receives job j's truncation weight.  Returns with the kept counts on the host
+// given, receives job j's truncation weight.  The diagnostics of job `diag` (-1: none) are
+// recorded, its singular values in a buffer of their own if keep_sig.  Returns with the kept counts on the host
 // (the plan of a following update needs them) and the group's last kernels in flight.
-int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
+int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc, int diag, bool keep_sig) {
   int rc = BSMPO_OK;
   for (int j = 0; j < nj; ++j)
     if ((rc = check_mode(h, jobs[j].mode))) return rc;
@@ -1110,6 +1113,7 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
   if ((rc = grow(h, h->vbuf, std::max<int64_t>(P.v_elems, 1) * sizeof(cplx)))) return rc;
   if ((rc = grow(h, h->sig, std::max<int64_t>(P.s_elems, 1) * sizeof(double)))) return rc;
   if ((rc = grow(h, h->keys, std::max<int64_t>(P.s_elems, 1) * sizeof(double)))) return rc;
+  if (keep_sig && diag >= 0 && (rc = grow(h, h->dsig, P.s_elems * sizeof(double)))) return rc;
   const ResLayout R = result_layout(ns, nj);
   const TabLayout L = layout_of(P, R);
   if ((rc = grow(h, h->tab, L.total))) return rc;
@@ -1274,7 +1278,7 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
     const UpdateTables& T = P.tab[j];
     std::vector<int>& cnt = mirror(h);
     if (trunc) trunc[j] = htw[j];
-    if (j == nj - 1) {
+    if (j == diag) {
       double nl = 0, nc = 0, nr = 0, flops_w = 0.0, svd_flops = 0.0;
       for (int q = 0; q < dd; ++q) {
         nl += cnt[(size_t)T.mode * dd + q];
@@ -1285,6 +1289,14 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc) {
       h->last_bytes = 16.0 * (nl * nc + nc * nr + (nl + nr) * hk[ns + j]);
       h->last_ns = T.n_sectors;
       h->last_sig_off = P.sd[T.sec0].s_off;
+      h->last_sig_kept = keep_sig;
+      if (keep_sig) {
+        int64_t len = 0;
+        for (int i = 0; i < T.n_sectors; ++i) len += P.sd[T.sec0 + i].k;
+        CK(h, cudaMemcpyAsync(h->dsig.p, reinterpret_cast<const double*>(h->sig.p) + h->last_sig_off,
+                              len * sizeof(double), cudaMemcpyDeviceToDevice, st));
+        h->last_sig_off = 0;
+      }
       h->last_cc.assign(2 * T.n_sectors, 0);
       h->last_shape.assign(2 * T.n_sectors, 0);
       h->last_kept.assign(T.n_sectors, 0);
@@ -1321,7 +1333,7 @@ int bs_update_impl(bsmpo_ctx* h, int mode, const cplx* u3_dev) {
   Job job;
   job.mode = mode;
   job.u3 = u3_dev;
-  return update_group(h, &job, 1, nullptr);
+  return update_group(h, &job, 1, nullptr, 0, false);
 }
 
 M8 transpose_to_m8(const double* S) {
@@ -1335,7 +1347,7 @@ M8 transpose_to_m8(const double* S) {
 }
 
 void free_workspaces(bsmpo_ctx* h) {
-  DevBuf* bufs[] = {&h->theta, &h->cbuf, &h->abuf, &h->wbuf, &h->vbuf, &h->sig, &h->keys,
+  DevBuf* bufs[] = {&h->theta, &h->cbuf, &h->abuf, &h->wbuf, &h->vbuf, &h->sig, &h->dsig, &h->keys,
                     &h->perm, &h->tab, &h->tab2, &h->rot, &h->u3, &h->m4,
                     &h->env_l, &h->env_r, &h->part, &h->outv, &h->dims, &h->nf2, &h->qbuf,
                     &h->qflag, &h->pbuf, &h->pcnt, &h->gbuf, &h->eigd, &h->taub, &h->invsig,
@@ -1457,7 +1469,7 @@ int run_mesh_concurrent(bsmpo_ctx* h, int n_bs, const int* modes, const cplx* u3
       CK(h, cudaEventCreate(&w->ev0));
       CK(h, cudaEventCreate(&w->ev1));
     }
-    w->last_index = -1;
+    w->ran_last = false;
   }
   h->test_error = 0;
   // dependencies
@@ -1552,7 +1564,8 @@ int run_mesh_concurrent(bsmpo_ctx* h, int n_bs, const int* modes, const cplx* u3
                                 cudaMemcpyHostToDevice, w->stream) != cudaSuccess)
               r = fail(w, BSMPO_ECUDA, "site copy-in failed");
         tw.assign(jobs.size(), 0.0);
-        if (!r) r = update_group(w, jobs.data(), (int)jobs.size(), tw.data());
+        const int diag = jobs.back().index == n_bs - 1 ? (int)jobs.size() - 1 : -1;
+        if (!r) r = update_group(w, jobs.data(), (int)jobs.size(), tw.data(), diag, true);
         // each update's weight is written by the one lane that ran it
         for (size_t i = 0; i < jobs.size() && !r; ++i) h->mesh_tw[jobs[i].index] = tw[i];
         if (!r && cudaEventRecord(mine, w->stream) != cudaSuccess)
@@ -1575,7 +1588,7 @@ int run_mesh_concurrent(bsmpo_ctx* h, int n_bs, const int* modes, const cplx* u3
         if (r) {
           if (!err_code) { err_code = r; err_msg = w->err; }
         } else {
-          w->last_index = jobs.back().index;
+          if (diag >= 0) w->ran_last = true;
           finished += (int)jobs.size();
           for (const Job& j : jobs)
             for (int s2 : succ[j.index])
@@ -1596,7 +1609,6 @@ int run_mesh_concurrent(bsmpo_ctx* h, int n_bs, const int* modes, const cplx* u3
   for (cudaEvent_t e : done_ev) cudaEventDestroy(e);
   if (err_code) return fail(h, err_code, err_msg);
   // counters and the last update's diagnostics
-  int best = -1;
   for (int k = 0; k < lanes; ++k) {
     bsmpo_ctx* w = h->workers[k];
     h->launches += w->launches;
@@ -1615,7 +1627,7 @@ int run_mesh_concurrent(bsmpo_ctx* h, int n_bs, const int* modes, const cplx* u3
     w->launches = w->updates = w->jacobi_rounds = w->jac_launches = 0;
     w->jac_ms = w->jac_flops = 0.0;
     for (int q = 0; q < 8; ++q) w->stage_ms[q] = 0.0;
-    if (w->last_index > best) { best = w->last_index; h->diag = w; }
+    if (w->ran_last) h->diag = w;
   }
   return BSMPO_OK;
 }
@@ -2255,7 +2267,8 @@ int bsmpo_last_update_info(const bsmpo_ctx* hc, int* n_sectors, int* sector_cc, 
     int64_t tot = 0;
     for (int k : h->last_k) tot += k;
     if (tot > sigma_cap) return fail(const_cast<bsmpo_ctx*>(hc), BSMPO_ECAPACITY, "sigma buffer too small");
-    CK(h, cudaMemcpyAsync(sigma, reinterpret_cast<const double*>(h->sig.p) + h->last_sig_off, tot * sizeof(double),
+    const DevBuf& from = h->last_sig_kept ? h->dsig : h->sig;
+    CK(h, cudaMemcpyAsync(sigma, reinterpret_cast<const double*>(from.p) + h->last_sig_off, tot * sizeof(double),
                           cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
   }
@@ -2292,7 +2305,7 @@ int bsmpo_workspace_stats(const bsmpo_ctx* h, int64_t* out) {
   // bytes held by the handle and its workers
   int64_t dev = 0, host = 0;
   auto add = [&](const bsmpo_ctx* c) {
-    const DevBuf* bufs[] = {&c->theta, &c->cbuf, &c->abuf, &c->wbuf, &c->vbuf, &c->sig, &c->keys,
+    const DevBuf* bufs[] = {&c->theta, &c->cbuf, &c->abuf, &c->wbuf, &c->vbuf, &c->sig, &c->dsig, &c->keys,
                             &c->perm, &c->tab, &c->tab2, &c->rot, &c->u3, &c->m4,
                             &c->env_l, &c->env_r, &c->part, &c->outv, &c->dims, &c->nf2, &c->qbuf,
                             &c->qflag, &c->pbuf, &c->pcnt, &c->gbuf, &c->eigd, &c->taub, &c->invsig,
