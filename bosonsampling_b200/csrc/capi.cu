@@ -346,13 +346,14 @@ int64_t candidates(bsmpo_ctx* h, int mode) {
 }
 
 // How an update's sector SVD is computed.  The Gram route drops singular values below ~2e-6
-// of a sector's largest, and a preconditioned Jacobi SVD (X Y in place of X) determines them
-// to ~eps of the largest, where the plain one keeps them to high relative accuracy.  Where the
-// update does not truncate to chi the small values stay in the state (W = V^H C carries
-// them through 1 / Lambda_R), so such updates take the plain Jacobi SVD: where the
-// candidates cannot exceed chi, or (Gram route, gram_policy 2) where the centre bond holds
-// fewer than chi vectors (it was not truncated by the last update on it and is unlikely
-// to be by this one).
+// of a sector's largest, and a preconditioned Jacobi SVD (X Y in place of X) loses relative
+// accuracy far below a sector's largest value, where the plain one keeps it.  Where the update
+// does not truncate to chi the small values stay in the state (W = V^H C carries them through
+// 1 / Lambda_R), so such updates take the plain Jacobi SVD: where the candidates cannot
+// exceed chi, or (Gram route, gram_policy 2) where the centre bond holds fewer than chi
+// vectors (it was not truncated by the last update on it and is unlikely to be by this one).
+// A preconditioned update that turns out to keep such values is done again with the plain form
+// (the selection tells; see PRE_MIN).
 enum class Route { plain, preconditioned, gram };
 
 Route route_of(bsmpo_ctx* h, int mode) {
@@ -667,8 +668,8 @@ struct ResLayout {
 
 ResLayout result_layout(int ns, int nj) {
   ResLayout R;
-  R.kept = 0;                                                  // int[ns] kept, int[nj] totals
-  R.trunc = align_up((size_t)(ns + nj) * sizeof(int), 16);     // double[nj]
+  R.kept = 0;                                                  // int[ns] kept, int[nj] totals, int[nj] to redo
+  R.trunc = align_up((size_t)(ns + 2 * nj) * sizeof(int), 16); // double[nj]
   R.err = R.trunc + nj * sizeof(double);                       // int: a pipeline wait expired; int: no convergence
   // unsigned long long[4]: pair-Gram rows, rotated rows; small sectors: complex MACs, sweeps
   R.work = align_up(R.err + 2 * sizeof(int), 16);
@@ -1088,16 +1089,18 @@ int tc_w_gemm(bsmpo_ctx* h, const Plan& P, const int* hk, int* err_d) {
 // given, receives job j's truncation weight.  The diagnostics of job `diag` (-1: none) are
 // recorded, its singular values in a buffer of their own if keep_sig.  Returns with the kept counts on the host
 // (the plan of a following update needs them) and the group's last kernels in flight.
-int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc, int diag, bool keep_sig) {
+// An update of the preconditioned form that keeps a value too small for it (see PRE_MIN) is
+// left out of the scatter and done again with the plain one (plain: no preconditioner).
+int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc, int diag, bool keep_sig, bool plain = false) {
   int rc = BSMPO_OK;
   for (int j = 0; j < nj; ++j)
     if ((rc = check_mode(h, jobs[j].mode))) return rc;
   StageClock clk(h);
-  h->updates += nj;
+  if (!plain) h->updates += nj;
   const int d = h->d, chi = h->chi, dd = d * d;
   cudaStream_t st = h->stream;
   Plan P;
-  const Route route = route_of(h, jobs[0].mode);
+  const Route route = plain ? Route::plain : route_of(h, jobs[0].mode);
   P.gram = route == Route::gram;
   P.pre = route == Route::preconditioned;
   const cplx* u3_base = jobs[0].u3;
@@ -1270,11 +1273,15 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc, int diag,
   if (*htc != 0)
     return fail(h, BSMPO_ECUDA, "tensor-core GEMM or tridiagonalisation: a pipeline wait expired (error word set)");
   if (htc[1] != 0) return fail(h, BSMPO_ECONVERGE, "Jacobi SVD did not converge (a small sector)");
-  h->route_count[P.gram ? 1 : 0] += nj;
+  std::vector<int> again;   // jobs to redo
+  for (int j = 0; j < nj; ++j)
+    if (hk[ns + nj + j] != 0) again.push_back(j);
+  h->route_count[P.gram ? 1 : 0] += nj - (int)again.size();
   if (!P.gram) h->last_sweeps = std::max(h->last_sweeps, (int)hwork[3]);
   if (h->timing && (rc = P.gram ? gram_timing(h, P) : jacobi_timing(h, hwork))) return rc;
   // host mirror, truncation weights, and the diagnostics of the group's last update
   for (int j = 0; j < nj; ++j) {
+    if (hk[ns + nj + j] != 0) continue;
     const UpdateTables& T = P.tab[j];
     std::vector<int>& cnt = mirror(h);
     if (trunc) trunc[j] = htw[j];
@@ -1325,6 +1332,17 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc, int diag,
       const SectorDesc& S = P.sd[T.sec0 + i];
       cM[S.cc0 * d + S.cc1] = hk[T.sec0 + i];
     }
+  }
+  if (!again.empty()) {
+    std::vector<Job> rest;
+    std::vector<double> tw(again.size());
+    int rest_diag = -1;
+    for (int j : again) {
+      if (j == diag) rest_diag = (int)rest.size();
+      rest.push_back(jobs[j]);
+    }
+    if ((rc = update_group(h, rest.data(), (int)rest.size(), tw.data(), rest_diag, keep_sig, true))) return rc;
+    for (size_t i = 0; trunc && i < again.size(); ++i) trunc[again[i]] = tw[i];
   }
   return BSMPO_OK;
 }

@@ -1413,7 +1413,7 @@ __global__ __launch_bounds__(WY_NT) void wy_apply_kernel(const SectorDesc* __res
 //    selection sets later) starts from X itself.
 constexpr int OR_NT = 512, OR_NW = OR_NT / 32;
 constexpr int OR_P = 8;        // vectors of a panel
-constexpr double NS_TOL = 1e-7;
+constexpr double NS_TOL = 1e-11;   // (k NS_TOL)^2 is below eps; about 1e-15 in use
 
 // Panels of OR_P vectors of a group, in order: each against the group's earlier vectors (32 at
 // a time, two products on the FP64 tensor path) and within itself (Gram-Schmidt), the whole

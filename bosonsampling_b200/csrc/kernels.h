@@ -115,7 +115,8 @@ cudaError_t launch_identity_rows(const SectorDesc* sd_dev, int n_sectors, int ma
                                  void* abuf, cudaStream_t s);
 // Deterministic top-chi with ket/bra pair symmetrisation, one CTA per update; writes kept
 // counts into sd_dev[s].kept and kept_out[s], slot starts, every update's total into
-// kept_out[n_sectors + u] and its truncation weight into trunc_out[u].
+// kept_out[n_sectors + u], whether it must be done again without the preconditioner into
+// kept_out[n_sectors + n_updates + u], and its truncation weight into trunc_out[u].
 cudaError_t launch_select(const UpdateTables* tab_dev, SectorDesc* sd_dev, int n_updates,
                           int n_sectors, const double* sig, double* keys, double cutoff, int chi,
                           int* kept_out, double* trunc_out, cudaStream_t s);
@@ -124,8 +125,9 @@ cudaError_t launch_extract_v(const SectorDesc* sd_dev, int n_sectors, int max_el
                              const void* abuf, const double* sig, const int* perm, void* vbuf,
                              cudaStream_t s);
 // New Gamma_L (= Gamma[mode]), Gamma_R (= Gamma[mode+1]), Lambda and charges of bond mode+1
-// of every update; gamma, lam, charge: the whole state's; totals: kept vectors per update;
-// err: two words on the device, nothing is written unless both are zero.
+// of every update not to be done again; gamma, lam, charge: the whole state's; totals: kept
+// vectors per update, then the words of those to be done again; err: two words on the
+// device, nothing is written unless both are zero.
 cudaError_t launch_scatter(const UpdateTables* tab_dev, const SectorDesc* sd_dev, int n_updates,
                            const int* totals, const int* err, int chi, const void* vbuf, const void* wbuf,
                            const double* sig, void* gamma, double* lam, int* charge,

@@ -176,6 +176,14 @@ __device__ __forceinline__ int count_ge(const double* key, int k, double v) {
   return lo;
 }
 
+// An update done with preconditioned matrices is done again from the plain ones where it
+// keeps singular values below PRE_MIN of their sector's largest.  The preconditioner mixes the
+// columns of values below ~1e-7 of the largest, a null space among them, and a column reduced
+// to the numerical-rank floor z takes part in no more rotations, so it can leave (z / sigma)^2
+// of a value sigma out.  At z of 4e-14 (100 rows) that is rounding at 1e-5; at 1e-8 the kept
+// values of a rank-deficient 120 x 100 sector were 6.8e-11 off, without it 5.3e-14 (relative;
+// values above 1e-5: 1e-15 and 1e-14).
+constexpr double PRE_MIN = 1e-5;
 constexpr int SEL_NT = 512;
 constexpr int SEL_CAP = 5120;   // candidates whose keys are kept in shared memory
 
@@ -194,7 +202,7 @@ __global__ __launch_bounds__(SEL_NT) void select_kernel(const UpdateTables* __re
   __shared__ double tws[BSMPO_MAX_Q], smax_s;
   __shared__ int ks[BSMPO_MAX_Q], pair_s[BSMPO_MAX_Q], gt_s[BSMPO_MAX_Q], kept_s[BSMPO_MAX_Q], cut_s[BSMPO_MAX_Q];
   __shared__ int64_t offs[BSMPO_MAX_Q];
-  __shared__ int hist[256], ncand, digit, above;
+  __shared__ int hist[256], ncand, digit, above, redo;
   const UpdateTables* tab = tabs + blockIdx.x;
   const int sec0 = tab->sec0, ns = tab->n_sectors;
   SectorDesc* sd = sds + sec0;
@@ -205,7 +213,7 @@ __global__ __launch_bounds__(SEL_NT) void select_kernel(const UpdateTables* __re
     offs[tid] = sd[tid].s_off;
     pair_s[tid] = tab->pair_of[tid] - sec0;   // own index of the swapped sector, negative: none
   }
-  if (tid == 0) ncand = 0;
+  if (tid == 0) ncand = redo = 0;
   __syncthreads();
   const int64_t off0 = offs[0];
   const int total = (int)(offs[ns - 1] + ks[ns - 1] - off0);
@@ -318,12 +326,17 @@ __global__ __launch_bounds__(SEL_NT) void select_kernel(const UpdateTables* __re
   if (own) {
     int slot = 0;
     for (int i = 0; i < tid; ++i) slot += kept_s[i];
+    // a preconditioned sector (not flagged to start from X) that keeps too small a value
+    const double* v = sig + offs[tid];
+    if (sd[tid].t_off != sd[tid].a_off && sd[tid].kept >= 0 && kept_s[tid] > 0 && v[kept_s[tid] - 1] < PRE_MIN * v[0]) redo = 1;
     sd[tid].kept = kept_s[tid];
     sd[tid].slot0 = slot;
     kept_out[tid] = kept_s[tid];
     if (tid == ns - 1) kept_all[n_sectors + blockIdx.x] = slot + kept_s[tid];
   }
+  __syncthreads();
   if (tid == 0) {
+    kept_all[n_sectors + gridDim.x + blockIdx.x] = redo;
     double tw = 0.0;
     for (int i = 0; i < ns; ++i) tw += tws[i];
     trunc_all[blockIdx.x] = tw;
@@ -362,7 +375,8 @@ __global__ __launch_bounds__(SC_NT) void scatter_kernel(const UpdateTables* __re
                                                         cplx* __restrict__ gamma,
                                                         double* __restrict__ lam,
                                                         int2* __restrict__ charge) {
-  if (err[0] != 0 || err[1] != 0) return;   // a failed group leaves the state as it is
+  // a failed group, or an update to be done again, leaves the state as it is
+  if (err[0] != 0 || err[1] != 0 || totals[gridDim.y + blockIdx.y] != 0) return;
   const UpdateTables* tab = tabs + blockIdx.y;
   const SectorDesc* sd = sds + tab->sec0;
   const int ns = tab->n_sectors, total_kept = totals[blockIdx.y];
