@@ -421,8 +421,10 @@ int add_update(bsmpo_ctx* h, int mode, int64_t gate_off, Plan& P) {
       S.s_off = P.s_elems; P.s_elems += S.k;
       S.w_off = P.w_elems; P.w_elems += (int64_t)S.k * n;
       S.v_off = P.v_elems; P.v_elems += (int64_t)m * S.k;
-      S.g_off = P.g_elems; P.g_elems += (int64_t)S.k * S.k;
-      S.y_off = P.y_elems; P.y_elems += (int64_t)S.k * S.k;
+      if (P.gram || S.t_off != S.a_off) {
+        S.g_off = P.g_elems; P.g_elems += (int64_t)S.k * S.k;
+        S.y_off = P.y_elems; P.y_elems += (int64_t)S.k * S.k;
+      }
       T.sidx[cc0 * d + cc1] = (int)P.sd.size();
       P.sd.push_back(S);
     }

@@ -77,8 +77,9 @@ struct SectorDesc {
   int64_t s_off;       // singular values / keys / permutation (k entries)
   int64_t w_off;       // W = V^H C, [kept][n] row-major (complex)
   int64_t v_off;       // V, [m][kept] row-major (complex)
-  int64_t g_off;       // Gram / Householder vectors, [k][k] (complex; Gram route only)
-  int64_t y_off;       // k x k slots (Gram route): eigenvectors [k][kept], scratch
+  // Gram route and preconditioned sectors only:
+  int64_t g_off;       // Gram / Householder vectors, [k][k] (complex)
+  int64_t y_off;       // k x k slots: eigenvectors [k][kept], scratch
   int row_start[BSMPO_MAX_D];   // row of L_s where left group a0 (a1 >= cc1 part) starts
   int col_start[BSMPO_MAX_D];   // column of R_s where right group b0 (b1 <= cc1 part) starts
 };
