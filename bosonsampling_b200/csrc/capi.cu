@@ -621,7 +621,7 @@ void finish_plan(bsmpo_ctx* h, Plan& P) {
     }
     big.push_back(s);
     // the identity below T^H, which accumulates the rotations (the one-CTA form has none)
-    if (S.left) P.max_left_m2 = std::max(P.max_left_m2, S.m * S.m);
+    if (S.left && S.t_off == S.a_off) P.max_left_m2 = std::max(P.max_left_m2, S.m * S.m);
     P.big_k = std::max(P.big_k, S.k);
     if (S.t_off != S.a_off) {
       pre.push_back(s);
@@ -1173,7 +1173,8 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc, int diag,
                                 P.gemm_tiles, nullptr, st));
   if ((rc = clk.mark(1))) return rc;
   // 2. identity rows of [T^H; I] and the gate mix
-  if (!P.gram) CKL(h, launch_identity_rows(sd_d, ns, P.max_left_m2, h->abuf.p, st));
+  if (!P.gram && P.max_left_m2 > 0)
+    CKL(h, launch_identity_rows(sd_d, list_d + P.n_small, (int)P.jw.size(), P.max_left_m2, h->abuf.p, st));
   CKL(h, launch_mix_d(d, tab_d, tidx_d, td_d, sd_d, pairs_d, (int)P.pairs.size(), P.mix_tiles, u3_base, h->theta.p,
                       h->lam, h->cbuf.p, h->abuf.p, st));
   if ((rc = clk.mark(2))) return rc;
@@ -1222,8 +1223,10 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc, int diag,
       put(h->stage3.p, jbytes, J.tdlist);
       char* t2 = static_cast<char*>(h->tab2.p);
       CK(h, cudaMemcpyAsync(t2, h->stage3.p, bytes, cudaMemcpyHostToDevice, st));
-      CKL(h, launch_identity_rows(sd_d, ns, J.max_left_m2, h->abuf.p, st));
-      if ((rc = jacobi_svd(h, J, sd_d, t2, reinterpret_cast<const int*>(t2 + jbytes), nullptr, res_d, R))) return rc;
+      const int* list2 = reinterpret_cast<const int*>(t2 + jbytes);
+      if (J.max_left_m2 > 0)
+        CKL(h, launch_identity_rows(sd_d, list2 + J.n_small, (int)J.jw.size(), J.max_left_m2, h->abuf.p, st));
+      if ((rc = jacobi_svd(h, J, sd_d, t2, list2, nullptr, res_d, R))) return rc;
       P.gram = false;
       if ((rc = select())) return rc;
     }

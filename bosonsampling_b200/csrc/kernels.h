@@ -111,8 +111,9 @@ cudaError_t launch_mix_d(int d, const UpdateTables* tab_dev, const int* tidx_dev
                          const MixPair* pairs_dev, int n_pairs, int total_tiles, const void* u3,
                          const void* theta, const double* lam, void* cbuf, void* abuf,
                          cudaStream_t s);
-// Identity rows of [T^H; I_m] for the `left` sectors.
-cudaError_t launch_identity_rows(const SectorDesc* sd_dev, int n_sectors, int max_elems,
+// Identity rows of [T^H; I_m] for the `left` sectors of a list (the blocked ones), but for the
+// preconditioned ones.
+cudaError_t launch_identity_rows(const SectorDesc* sd_dev, const int* list_dev, int count, int max_elems,
                                  void* abuf, cudaStream_t s);
 // Deterministic top-chi with ket/bra pair symmetrisation, one CTA per update; writes kept
 // counts into sd_dev[s].kept and kept_out[s], slot starts, every update's total into

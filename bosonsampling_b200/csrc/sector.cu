@@ -147,8 +147,9 @@ __global__ __launch_bounds__(MIX_NT) void mix_kernel(const UpdateTables* __restr
   }
 }
 
-__global__ void identity_rows_kernel(const SectorDesc* __restrict__ sd, cplx* __restrict__ abuf) {
-  const SectorDesc& S = sd[blockIdx.y];
+__global__ void identity_rows_kernel(const SectorDesc* __restrict__ sd, const int* __restrict__ list,
+                                     cplx* __restrict__ abuf) {
+  const SectorDesc& S = sd[list[blockIdx.y]];
   if (!S.left || S.t_off != S.a_off) return;   // a preconditioned sector gets Y there
   const int m = S.m;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m * m; e += gridDim.x * blockDim.x) {
@@ -494,11 +495,11 @@ cudaError_t launch_mix_d(int d, const UpdateTables* tab_dev, const int* tidx_dev
   return cudaGetLastError();
 }
 
-cudaError_t launch_identity_rows(const SectorDesc* sd_dev, int n_sectors, int max_elems,
+cudaError_t launch_identity_rows(const SectorDesc* sd_dev, const int* list_dev, int count, int max_elems,
                                  void* abuf, cudaStream_t s) {
-  if (n_sectors <= 0 || max_elems <= 0) return cudaSuccess;
-  dim3 grid(min(ceil_div(max_elems, 256), 1024), n_sectors);
-  identity_rows_kernel<<<grid, 256, 0, s>>>(sd_dev, reinterpret_cast<cplx*>(abuf));
+  if (count <= 0 || max_elems <= 0) return cudaSuccess;
+  dim3 grid(min(ceil_div(max_elems, 256), 1024), count);
+  identity_rows_kernel<<<grid, 256, 0, s>>>(sd_dev, list_dev, reinterpret_cast<cplx*>(abuf));
   return cudaGetLastError();
 }
 
