@@ -341,12 +341,6 @@ def run_reference(args):
     return 0
 
 
-# DRAM bytes (read + write) of one tridiag_kernel launch of the largest size class
-# (8-CTA clusters, the biggest sector of a centre update at chi = 1024), from the ncu
-# capture summarised under profiles/ (cold cache)
-TRIDIAG_TRAFFIC = 2941184   # 2.836 MB read + 0.105 MB written
-
-
 def measured_peaks(path=os.path.join(ROOT, "MEASURED_PEAKS.json")):
     """The pool's measured peaks (copy bandwidth ``hbm_gbs``, bf16 GEMM), or None."""
     try:
@@ -359,18 +353,23 @@ def measured_peaks(path=os.path.join(ROOT, "MEASURED_PEAKS.json")):
 
 def roofline(args, mine, kernel, fp64_peak, hbm_peak, peaks=None):
     """The dominant kernel's roofline.  Gram route: the Householder tridiagonalisation
-    (tridiag_kernel, 66-71% of the update's kernel time), whose fused passes stream the
-    trailing matrix once per step (read + write, 32 B per complex entry): achieved
-    bytes / device time of the phase, one worker, against the pool's measured copy
-    bandwidth (``peaks["hbm_gbs"]``), or the copy bandwidth measured in this run when
-    that is absent (both reported).  Plain path: the Jacobi rounds' FP64 flops against
-    DGEMM measured in this run (the pool's file holds no FP64 figure)."""
+    (tridiag_resident_kernel, the largest part of the update's kernel time).  The matrix stays
+    in shared memory, so neither HBM nor FP64 bounds it but the latency of a step:
+    ``us_per_step`` is the phase's device time, one worker, over the steps of the largest
+    sector of every update.  ``achieved`` / ``peak`` place that against a reduction that
+    streams its trailing matrix once per step (read + write, 32 B per complex entry): those
+    bytes over the phase's time, beside the pool's measured copy bandwidth
+    (``peaks["hbm_gbs"]``), or the copy bandwidth measured in this run when that is absent (both
+    reported).  Plain path: the Jacobi rounds' FP64 flops against DGEMM measured in this run
+    (the pool's file holds no FP64 figure)."""
     if kernel is not None and kernel["ms"] > 0:
         achieved = kernel["bytes"] / (kernel["ms"] / 1e3) / 1e9
         pool = float(peaks["hbm_gbs"]) if peaks and peaks.get("hbm_gbs") else None
         peak = pool if pool else hbm_peak
+        steps = kernel.get("steps")
         return {"kernel": "tridiag_resident_kernel (Householder tridiagonalisation, forked size-class launches)",
-                "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                "bound": "latency", "us_per_step": 1e3 * kernel["ms"] / steps if steps else None, "steps": steps,
+                "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak if peak else None,
                 "frac_of": "measured",
                 "peak_source": ("MEASURED_PEAKS.json hbm_gbs: copy bandwidth measured on this pool's B200s"
@@ -378,11 +377,11 @@ def roofline(args, mine, kernel, fp64_peak, hbm_peak, peaks=None):
                                 "copy bandwidth measured in this run (torch copy of 1 GiB, best of 10)"),
                 "peak_in_run": hbm_peak,
                 "frac_of_in_run": achieved / hbm_peak if hbm_peak else None,
-                "achieved_over": "the phase's device time (CUDA events), one worker, one layer (%d phases)"
-                                 % kernel["phases"],
+                "achieved_over": "the phase's device time (CUDA events), one worker, one layer (%d phases); bytes a "
+                                 "streaming reduction would move, read from shared memory here" % kernel["phases"],
                 "bytes": kernel["bytes"], "ms": kernel["ms"],
                 "flops_tflops": kernel["flops"] / (kernel["ms"] / 1e3) / 1e12,
-                "traffic": TRIDIAG_TRAFFIC, "traffic_unit": "bytes per launch (largest class)"}
+                "traffic": None}
     achieved = mine["svd_flops"] / mine["seconds"] / 1e12 if mine["seconds"] > 0 else None
     return {"kernel": SVD_KERNELS[args.precision], "bound": "tensor", "achieved": achieved, "peak": fp64_peak,
             "unit": "TFLOP/s", "frac": (achieved / fp64_peak) if achieved and fp64_peak else None,
@@ -517,11 +516,16 @@ def main():
         sim.set_workers(1)
         run_layers(sim, args.start_layer, args.warmup)
         sim.set_timing(True)
-        run_layers(sim, first, 1, partial=True)
+        steps = 0        # of every update's largest sector on the Gram route
+        for m, t, p in layer_ops(first, 1, partial=True):
+            routed = sim.svd_routes()[1]
+            sim.bs_update(m, interferometer.t_block(t, p))
+            if sim.svd_routes()[1] > routed:
+                steps += max(min(shape) for shape in sim.last_update_info()["shape"])
         torch.cuda.synchronize()
         td_ms, td_bytes, td_flops, td_phases = sim.tridiag_timing()
         sim.set_timing(False)
-        kernel = {"ms": td_ms, "bytes": td_bytes, "flops": td_flops, "phases": td_phases}
+        kernel = {"ms": td_ms, "bytes": td_bytes, "flops": td_flops, "phases": td_phases, "steps": steps}
 
     # ---- end to end through the public API with host buffers, over the same K layers: per
     # step (layer) the state goes host -> device, the layer runs, the state comes back
