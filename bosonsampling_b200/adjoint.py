@@ -406,11 +406,11 @@ class DiffCircuit:
     ``phases``: the output phase screen (it leaves the marginals unchanged but is part of
     the forward).  The forward runs on the library (``precision``, default the plain FP64
     path), one update after another, keeping for each update the two sites and three
-    bonds it reads and the two sites and bond it writes (4 chi^2 complex numbers): the
-    backward needs the forward's own output basis -- inside degenerate multiplets of
-    singular values the library's result is not bitwise the same between its concurrent
-    and sequential schedules, so recomputing a segment from a stored MPO could hand the
-    adjoint a different (equally valid) basis than the one its incoming gradient refers to."""
+    bonds it reads and the two sites and bond it writes (4 chi^2 complex numbers), so the
+    backward has the forward's own output basis without a second forward: the incoming
+    gradient refers to that basis, which inside degenerate multiplets of singular values is
+    any of many (every schedule of the updates computes the same bits, so a segment
+    recomputed from a stored state would have it too, at the price of its updates)."""
 
     def __init__(self, n, d, chi, photon_modes, mesh, phases, precision="fp64", workers=8):
         self.n, self.d, self.chi = n, d, chi

@@ -14,9 +14,10 @@
 // and at its end each output adds its weight times the run's sum.  A run that no row and
 // column of the tile can use is not read.  What bounds it: the FP64 tensor rate of the SM with
 // the most tiles, so they are small (32 x 16, 4 warps): a sector of 443 x 389 is 350 CTAs.
-// Measured there with 1,024 centre entries, d = 5, with the call and the wait: 188 us; with 32 x
-// 32 tiles (182 CTAs) 206, of which the kernel 93 (16 x 16 tiles with the weight applied per
-// entry: 270).  700 x 1,024 x 300: 180 and 202; 1,500 x 1,024 x 1,400: 411 and 411.
+// Measured there with 1,024 centre entries, d = 5: the kernel 81 us, the call with its wait 162
+// us, 116 among others.  When the tiles were chosen, calls with their wait, 32 x 16 and 32 x
+// 32 tiles (182 CTAs): 188 and 206 us; 700 x 1,024 x 300: 180 and 202; 1,500 x 1,024 x 1,400: 411
+// and 411 (16 x 16 tiles with the weight applied per entry: the kernel alone 270 at the first).
 #include "dmma.cuh"
 #include "kernels.h"
 

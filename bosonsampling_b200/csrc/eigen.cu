@@ -1406,11 +1406,13 @@ __global__ __launch_bounds__(WY_NT) void wy_apply_kernel(const SectorDesc* __res
 //    steps Y <- Y (3 I - Y^H Y) / 2, which square the departure from unitarity and leave it
 //    at rounding level.  The SVD itself stays the one-sided Jacobi iteration on X Y with its
 //    own test, so Y decides how fast it converges, not what it converges to.  Measured: one
-//    layer at N = 64, chi = 1024 on the plain path 223 ms without and 63 with it, an N = 24,
-//    chi = 256 circuit 118 and 57; the marginals of N = 16 to 20 circuits are as far from a
-//    64-bit CPU computation as before (1.1e-13 at most).  A sector whose
-//    Y was not unitary to NS_TOL before the last step (flagged in sd[].kept, which the
-//    selection sets later) starts from X itself.
+//    layer at N = 64, chi = 1024 on the plain path 223 ms without and 56 with it, an N = 24,
+//    chi = 256 circuit 118 and 57 (30 with the later one-CTA form of its small sectors); the
+//    marginals of N = 13 to 20 circuits are 9.9e-15 from a 64-bit CPU computation at most,
+//    1.5e-13 without.  A sector whose Y was not unitary to NS_TOL before the last step
+//    (flagged in sd[].kept, which the selection sets later) starts from X itself; an update
+//    that keeps values far below a sector's largest is done again without Y (PRE_MIN,
+//    sector.cu).
 constexpr int OR_NT = 512, OR_NW = OR_NT / 32;
 constexpr int OR_P = 8;        // vectors of a panel
 constexpr double NS_TOL = 1e-11;   // (k NS_TOL)^2 is below eps; about 1e-15 in use

@@ -77,7 +77,8 @@ class MPOSimulator:
         self._chk(self.L.bsmpo_set_precision(self.h, self.PRECISIONS[precision]))
 
     def set_workers(self, n_workers):
-        """Beam splitters of one brick-wall layer that ``run_mesh`` runs at once."""
+        """Beam splitters that ``run_mesh`` runs at once, in groups on up to four streams (up to
+        chi = 512 four times as many, with their workspaces)."""
         self._chk(self.L.bsmpo_set_workers(self.h, int(n_workers)))
 
     def close(self):
@@ -363,8 +364,8 @@ def batch_cost(spec):
 def run_batch(specs, concurrency=8, precision="fp64-gram", workers=4, timing=None, largest_first=False):
     """Runs independent circuits (``batch_circuits`` entries) side by side on the current
     device: ``concurrency`` circuits at a time, each on its own handle, host thread and
-    stream (the library's calls release the GIL), each handle overlapping its own updates
-    on ``workers`` streams.  Handles are created and initialised first and released last,
+    stream (the library's calls release the GIL), each handle running its own updates in groups
+    (``workers``, see ``MPOSimulator.set_workers``).  Handles are created and initialised first and released last,
     outside the concurrent phase (allocating or freeing device memory synchronises the
     whole device).  ``largest_first`` starts the circuits in decreasing ``batch_cost``
     (longest-first list scheduling: the batch does not end on one large circuit running

@@ -189,7 +189,8 @@ int bsmpo_canonicalize(bsmpo_ctx* h);
  * RankWorker.RankProcess (src/beam_splitter_parallel/Rank.py:32-206) and
  * InitializationMPO.Update (src/MPO.py:158-303), fully on the device.
  * S: host double[8], the 2x2 single-particle unitary acting on the state
- * (a photon entering mode j leaves mode i with amplitude S[i][j]). */
+ * (a photon entering mode j leaves mode i with amplitude S[i][j]).  On an error the state
+ * is as it was. */
 int bsmpo_bs_update(bsmpo_ctx* h, int mode, const double* S);
 
 /* Same with an explicit device tensor U[new_a][new_b][old_a] (complex128 d^3), e.g.
@@ -201,7 +202,8 @@ int bsmpo_bs_update_tensor(bsmpo_ctx* h, int mode, const void* u);
  * on (modes[i], modes[i]+1), in the given order.  Host arrays.  Consecutive entries
  * whose modes differ pairwise by 2 or more (a brick-wall layer) touch disjoint sites
  * and run concurrently on the handle's workers (bsmpo_set_workers); the result is the
- * same as applying them one by one.  Returns with all work complete. */
+ * same as applying them one by one.  Returns with all work complete; on an error, with
+ * every bond either updated or as it was. */
 int bsmpo_run_mesh(bsmpo_ctx* h, int n_bs, const int* modes, const double* theta,
                    const double* phi);
 
@@ -256,7 +258,8 @@ int bsmpo_last_update_info(const bsmpo_ctx* h, int* n_sectors, int* sector_cc, i
                            double* trunc_weight);
 
 /* Work counters of the last update (host): algorithmic flops of the contraction
- * GEMMs and of the SVD step, and the bytes the update had to move at minimum. */
+ * GEMMs and of the SVD step (the Jacobi form: one sweep's times the sweeps of the slowest
+ * sector, of its group in a mesh), and the bytes the update had to move at minimum. */
 int bsmpo_last_update_work(const bsmpo_ctx* h, double* gemm_flops, double* svd_flops,
                            double* min_bytes);
 
