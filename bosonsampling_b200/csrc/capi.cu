@@ -36,7 +36,7 @@ thread_local std::string g_last_error;
 constexpr int MAX_SWEEPS = 40;
 constexpr int WAIT_POLL_US = 400;   // host waits poll this long before they sleep
 constexpr int MESH_LANES = 4;   // streams a mesh's groups of updates are spread over, at most
-constexpr int MAX_GROUP = 32;   // updates of a group
+constexpr int MAX_GROUP = 32;   // updates of a group (at most a lane to each, see better_plain)
 
 struct DevBuf {
   void* p = nullptr;
@@ -557,6 +557,8 @@ int add_update(bsmpo_ctx* h, int mode, int64_t gate_off, Plan& P) {
         // S = Y^H Y (tiles as the Gram's), Y' = Y M, X' = X Y
         GemmGroup y = r;
         y.K = S.k;
+        y.sec = s;
+        y.kdim = 3;
         y.a_off = y.b_off = S.y_off;
         P.gyy.push_back(y);
         y.opA = y.herm = 0;
@@ -826,8 +828,8 @@ int gram_eigenvalues(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, const 
 
 // The matrices the blocked Jacobi rounds of the preconditioned sectors start from: X Y with
 // a unitary Y close to the eigenvectors of X^H X.
-int precondition(bsmpo_ctx* h, const Plan& P, SectorDesc* sd_d, const GemmGroup* ggram_d, const GemmGroup* gyy_d,
-                 const GemmGroup* gym_d, const GemmGroup* gxy_d, const int* list_d, int* err_d) {
+int precondition(bsmpo_ctx* h, const Plan& P, const UpdateTables* tab_d, SectorDesc* sd_d, const GemmGroup* ggram_d,
+                 const GemmGroup* gyy_d, const GemmGroup* gym_d, const GemmGroup* gxy_d, const int* list_d, int* err_d) {
   cudaStream_t st = h->stream;
   const int n = P.n_pre;
   int rc;
@@ -836,20 +838,21 @@ int precondition(bsmpo_ctx* h, const Plan& P, SectorDesc* sd_d, const GemmGroup*
   if ((rc = grow(h, h->wyt, precondition_t_elems(P.s_elems, (int)P.sd.size()) * sizeof(cplx)))) return rc;
   double* dbuf_d = reinterpret_cast<double*>(h->eigd.p);
   double* ebuf_d = dbuf_d + P.s_elems;
-  CK(h, launch_precondition_basis(sd_d, list_d, n, P.pre_k, dbuf_d, ebuf_d, ebuf_d + P.s_elems,
-                                  reinterpret_cast<double*>(h->escr.p), reinterpret_cast<unsigned char*>(h->swp.p),
-                                  reinterpret_cast<double*>(h->zbuf.p), h->gbuf.p, h->taub.p, h->wyt.p, h->ybuf.p, st));
+  CK(h, launch_precondition_basis(tab_d, sd_d, (int)P.tab.size(), list_d, n, P.pre_k, h->cutoff, h->chi, dbuf_d, ebuf_d,
+                                  ebuf_d + P.s_elems, reinterpret_cast<double*>(h->escr.p),
+                                  reinterpret_cast<unsigned char*>(h->swp.p), reinterpret_cast<double*>(h->zbuf.p),
+                                  h->gbuf.p, h->taub.p, h->wyt.p, h->ybuf.p, st));
   h->launches += 5;
   // three Newton-Schulz steps between ybuf and the inverse iteration's scratch (2 k^2
   // complex a sector), ending in the latter; the Gram matrices' place holds Y^H Y
   void *y = h->ybuf.p, *y2 = h->escr.p;
   for (int it = 0; it < 3; ++it) {
-    CKL(h, launch_zgemm_grouped(y, y, h->gbuf.p, nullptr, gyy_d, n, P.gram_tiles, nullptr, st));
+    CKL(h, launch_zgemm_grouped(y, y, h->gbuf.p, nullptr, gyy_d, n, P.gram_tiles, sd_d, st));
     CKL(h, launch_newton_schulz(sd_d, list_d, n, P.pre_k, h->gbuf.p, it == 2, st));
-    CKL(h, launch_zgemm_grouped(y, h->gbuf.p, y2, nullptr, gym_d, n, P.gram_tiles, nullptr, st));
+    CKL(h, launch_zgemm_grouped(y, h->gbuf.p, y2, nullptr, gym_d, n, P.gram_tiles, sd_d, st));
     std::swap(y, y2);
   }
-  CKL(h, launch_zgemm_grouped(h->abuf.p, y, h->abuf.p, nullptr, gxy_d, n, P.xy_tiles, nullptr, st));
+  CKL(h, launch_zgemm_grouped(h->abuf.p, y, h->abuf.p, nullptr, gxy_d, n, P.xy_tiles, sd_d, st));
   CKL(h, launch_precondition_finish(sd_d, list_d, n, P.pre_elems, y, h->abuf.p, st));
   return BSMPO_OK;
 }
@@ -881,8 +884,8 @@ int gram_timing(bsmpo_ctx* h, const Plan& P) {
 
 // 3b. One-sided Jacobi of every sector of the group: the small sectors in one launch, the
 // others in blocked rounds.  gg_d: the preconditioner's GEMM groups (X^H X, Y^H Y, Y M, X Y).
-int jacobi_svd(bsmpo_ctx* h, const Plan& P, SectorDesc* sd_d, char* jw_d, const int* list_d, const GemmGroup* const* gg_d,
-               char* res_d, const ResLayout& R) {
+int jacobi_svd(bsmpo_ctx* h, const Plan& P, const UpdateTables* tab_d, SectorDesc* sd_d, char* jw_d, const int* list_d,
+               const GemmGroup* const* gg_d, char* res_d, const ResLayout& R) {
   const int ns = (int)P.sd.size(), n_big = (int)P.jw.size();
   cudaStream_t st = h->stream;
   int rc;
@@ -907,7 +910,7 @@ int jacobi_svd(bsmpo_ctx* h, const Plan& P, SectorDesc* sd_d, char* jw_d, const 
   double* sig = reinterpret_cast<double*>(h->sig.p);
   int* perm = reinterpret_cast<int*>(h->perm.p);
   if (h->timing) CK(h, cudaEventRecord(h->ev0, st));
-  if (P.n_pre && (rc = precondition(h, P, sd_d, gg_d[0], gg_d[1], gg_d[2], gg_d[3], list_d + P.n_small + n_big,
+  if (P.n_pre && (rc = precondition(h, P, tab_d, sd_d, gg_d[0], gg_d[1], gg_d[2], gg_d[3], list_d + P.n_small + n_big,
                                     reinterpret_cast<int*>(res_d + R.err))))
     return rc;
   // beside the blocked rounds, where there are any, on the first side stream
@@ -1190,7 +1193,7 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc, int diag,
   if (!h->wait_ev) CK(h, cudaEventCreateWithFlags(&h->wait_ev, cudaEventBlockingSync | cudaEventDisableTiming));
   const GemmGroup* pre_d[4] = {groups_at(L.ggram), groups_at(L.gyy), groups_at(L.gym), groups_at(L.gxy)};
   rc = P.gram ? gram_eigenvalues(h, P, sd_d, groups_at(L.ggram), list_d, tcerr_d)
-              : jacobi_svd(h, P, sd_d, dt + L.jw, list_d, pre_d, res_d, R);
+              : jacobi_svd(h, P, tab_d, sd_d, dt + L.jw, list_d, pre_d, res_d, R);
   if (rc || (rc = clk.mark(3))) return rc;
   if (h->test_error == 1 || h->test_error == 2) {
     CK(h, cudaMemsetAsync(tcerr_d + h->test_error - 1, 1, sizeof(int), st));
@@ -1226,7 +1229,7 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc, int diag,
       const int* list2 = reinterpret_cast<const int*>(t2 + jbytes);
       if (J.max_left_m2 > 0)
         CKL(h, launch_identity_rows(sd_d, list2 + J.n_small, (int)J.jw.size(), J.max_left_m2, h->abuf.p, st));
-      if ((rc = jacobi_svd(h, J, sd_d, t2, list2, nullptr, res_d, R))) return rc;
+      if ((rc = jacobi_svd(h, J, tab_d, sd_d, t2, list2, nullptr, res_d, R))) return rc;
       P.gram = false;
       if ((rc = select())) return rc;
     }

@@ -923,19 +923,78 @@ __device__ __forceinline__ double start_entry(int l, int t) {
   return ((double)(h & 0xffffu) + 0.5) / 32768.0 - 1.0;
 }
 
-__global__ __launch_bounds__(IV_NT) void invit_kernel(const SectorDesc* __restrict__ sd,
-                                                      const int* __restrict__ list,
+// Whether the eigenvalues show a sector to be better left as it is than preconditioned (whole
+// warp): where fewer than chi values of its update lie above PRE_MIN of its largest and some
+// of its own lie between that and the eigenvalues' floor, those would be kept and the update
+// done again; where all values are equal within 5%, X's columns are nearly orthogonal.  Only a
+// matter of time: what is kept too small after all is found by the selection.  Update of four
+// 420 x 420 sectors, values over ten decades, chi = 1,260: 17.3 ms without the preconditioner,
+// 50.0 with it and the second run, 18.9 left as they are; all values equal: 1.6, 11.2 and 2.9.
+__device__ __forceinline__ bool better_plain(const SectorDesc* __restrict__ sds, int sec,
+                                             const UpdateTables* __restrict__ tabs, int n_updates,
+                                             const double* __restrict__ lam, double cutoff, int chi) {
+  const int lane = threadIdx.x & 31;
+  // its update: the last one that starts at or before it (a group has at most 32)
+  const unsigned m = __ballot_sync(0xffffffffu, lane < n_updates && tabs[lane].sec0 <= sec);
+  const UpdateTables* tab = tabs + (31 - __clz(m));
+  const SectorDesc* sd = sds + tab->sec0;
+  const int ns = tab->n_sectors, s = sec - tab->sec0, k = sd[s].k;
+  auto pre = [&](int t) { return sd[t].t_off != sd[t].a_off; };
+  auto above = [&](int t, double v) {   // eigenvalues of sector t above v
+    const double* x = lam + sd[t].s_off;
+    int lo = 0, hi = sd[t].k;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (x[mid] > v) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+  };
+  const double l0 = lam[sd[s].s_off], ln = lam[sd[s].s_off + k - 1], x = PRE_MIN * PRE_MIN * l0;
+  int n = 0;
+  double top = 0.0;
+  for (int t = lane; t < ns; t += 32) {
+    n += pre(t) ? above(t, x) : sd[t].k;   // the others' values are not known yet
+    top = fmax(top, pre(t) ? lam[sd[t].s_off] : 0.0);
+  }
+  n = __reduce_add_sync(0xffffffffu, n);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+  if (ln > 0.9 * l0) return true;
+  if (n >= chi || cutoff * cutoff * top >= x) return false;
+  const int own = lane < 2 ? above(s, lane == 0 ? 32.0 * EPS * k * l0 : x) : 0;
+  return __shfl_sync(0xffffffffu, own, 0) > __shfl_sync(0xffffffffu, own, 1);
+}
+
+// tabs (preconditioner: every eigenvector, and the sectors better left as they are flagged
+// with kept = -1) or null (the kept ones).
+__global__ __launch_bounds__(IV_NT) void invit_kernel(SectorDesc* __restrict__ sd, const int* __restrict__ list,
+                                                      const UpdateTables* __restrict__ tabs, int n_updates,
+                                                      double cutoff, int chi,
                                                       const double* __restrict__ dbuf,
                                                       const double* __restrict__ ebuf,
                                                       const double* __restrict__ lam,
                                                       double* __restrict__ scratch,
                                                       unsigned char* __restrict__ swp,
-                                                      double* __restrict__ zbuf, bool all) {
+                                                      double* __restrict__ zbuf) {
   extern __shared__ double ism[];
   __shared__ double dots[IV_NT / 32][IV_GT], coef[IV_GT], nrm2[IV_NT / 32];
-  const SectorDesc& S = sd[sector_of(list, blockIdx.x)];
+  __shared__ int left;
+  const bool all = tabs != nullptr;
+  const int sec = sector_of(list, blockIdx.x);
+  const SectorDesc& S = sd[sec];
   const int k = S.k, kept = all ? k : S.kept;
   if (kept == 0) return;
+  if (all) {
+    if (threadIdx.x < 32) {
+      const bool yes = better_plain(sd, sec, tabs, n_updates, lam, cutoff, chi);
+      if (threadIdx.x == 0) {
+        left = yes;
+        if (yes) sd[sec].kept = -1;
+      }
+    }
+    __syncthreads();
+    if (left) return;
+  }
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double* d = ism;
   double* e = ism + k;
@@ -1252,7 +1311,7 @@ __global__ __launch_bounds__(WT_NT) void wy_t_kernel(const SectorDesc* __restric
   const int sec = list[blockIdx.y];
   const SectorDesc& S = sd[sec];
   const int k = S.k, j0 = blockIdx.x * WY_B;
-  if (j0 >= k - 1) return;
+  if (j0 >= k - 1 || S.kept < 0) return;
   const cplx* A = gbuf + S.g_off;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, li = lane >> 2, lk = lane & 3;
   // G = V^H V, rows j0 + 1 .. k - 1 in quarters
@@ -1310,7 +1369,7 @@ __global__ __launch_bounds__(WY_NT) void wy_apply_kernel(const SectorDesc* __res
   const int sec = list[blockIdx.y];
   const SectorDesc& S = sd[sec];
   const int k = S.k, c0 = blockIdx.x * WY_C;
-  if (c0 >= k) return;
+  if (c0 >= k || S.kept < 0) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, li = lane >> 2, lk = lane & 3;
   const cplx* A = gbuf + S.g_off;
   const double* z = zbuf + S.y_off;
@@ -1411,8 +1470,7 @@ __global__ __launch_bounds__(WY_NT) void wy_apply_kernel(const SectorDesc* __res
 //    marginals of N = 13 to 20 circuits are 9.9e-15 from a 64-bit CPU computation at most,
 //    1.5e-13 without.  A sector whose Y was not unitary to NS_TOL before the last step
 //    (flagged in sd[].kept, which the selection sets later) starts from X itself; an update
-//    that keeps values far below a sector's largest is done again without Y (PRE_MIN,
-//    sector.cu).
+//    that keeps values far below a sector's largest is done again without Y (PRE_MIN).
 constexpr int OR_NT = 512, OR_NW = OR_NT / 32;
 constexpr int OR_P = 8;        // vectors of a panel
 constexpr double NS_TOL = 1e-11;   // (k NS_TOL)^2 is below eps; about 1e-15 in use
@@ -1430,6 +1488,7 @@ __global__ __launch_bounds__(OR_NT) void orthogonalise_kernel(const SectorDesc* 
   extern __shared__ __align__(16) double zp[];   // the panel, [k][OR_P]
   __shared__ double dots[OR_NW][32][OR_P], coef[32][OR_P], part[OR_NW][OR_P], tots[OR_P];
   const SectorDesc& S = sd[list[blockIdx.x]];
+  if (S.kept < 0) return;
   const int k = S.k, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, li = lane >> 2, lk = lane & 3;
   const double* lv = lam + S.s_off;
   double* Z = zbuf + S.y_off;      // [k][k]
@@ -1552,6 +1611,7 @@ __global__ __launch_bounds__(OR_NT) void orthogonalise_kernel(const SectorDesc* 
 __global__ __launch_bounds__(256) void newton_schulz_kernel(SectorDesc* __restrict__ sd, const int* __restrict__ list,
                                                             cplx* __restrict__ gbuf, bool check) {
   SectorDesc& S = sd[list[blockIdx.y]];
+  if (!check && S.kept < 0) return;
   const int k = S.k;
   cplx* G = gbuf + S.g_off;
   bool bad = false;
@@ -1698,19 +1758,20 @@ cudaError_t launch_bisect(const SectorDesc* sd_dev, int n_sectors, int kmax, con
 
 namespace {
 
-cudaError_t run_invit(const SectorDesc* sd, const int* list, int n, int kmax, bool all, const double* dbuf,
-                      const double* ebuf, const double* lam, double* scratch, unsigned char* swp, double* zbuf,
+cudaError_t run_invit(SectorDesc* sd, const int* list, int n, int kmax, const UpdateTables* tabs, int n_updates,
+                      double cutoff, int chi, const double* dbuf, const double* ebuf, const double* lam, double* scratch, unsigned char* swp, double* zbuf,
                       cudaStream_t s) {
   static const cudaError_t attr = cudaFuncSetAttribute(
       invit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * eigen_max_k() * (int)sizeof(double));
   if (attr != cudaSuccess) return attr;
-  invit_kernel<<<n, IV_NT, (size_t)2 * kmax * sizeof(double), s>>>(sd, list, dbuf, ebuf, lam, scratch, swp, zbuf, all);
+  invit_kernel<<<n, IV_NT, (size_t)2 * kmax * sizeof(double), s>>>(sd, list, tabs, n_updates, cutoff, chi, dbuf, ebuf, lam,
+                                                               scratch, swp, zbuf);
   return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t launch_eigvec(const SectorDesc* sd_dev, int n_sectors, int kmax, const double* dbuf, const double* ebuf,
+cudaError_t launch_eigvec(SectorDesc* sd_dev, int n_sectors, int kmax, const double* dbuf, const double* ebuf,
                           const double* lam, double* scratch, unsigned char* swp, double* zbuf, const void* gbuf,
                           const void* taubuf, void* vbuf, void* ybuf, cudaStream_t s) {
   if (n_sectors <= 0 || kmax <= 0) return cudaSuccess;
@@ -1724,7 +1785,8 @@ cudaError_t launch_eigvec(const SectorDesc* sd_dev, int n_sectors, int kmax, con
     return e;
   }();
   if (attr != cudaSuccess) return attr;
-  const cudaError_t e = run_invit(sd_dev, nullptr, n_sectors, kmax, false, dbuf, ebuf, lam, scratch, swp, zbuf, s);
+  const cudaError_t e = run_invit(sd_dev, nullptr, n_sectors, kmax, nullptr, 0, 0.0, 0, dbuf, ebuf, lam, scratch, swp,
+                                  zbuf, s);
   if (e != cudaSuccess) return e;
   const cplx* G = reinterpret_cast<const cplx*>(gbuf);
   const cplx* tau = reinterpret_cast<const cplx*>(taubuf);
@@ -1745,7 +1807,8 @@ size_t precondition_t_elems(int64_t s_elems, int n_sectors) {
   return (size_t)(WY_B * s_elems + (int64_t)WY_B * WY_B * n_sectors);
 }
 
-cudaError_t launch_precondition_basis(const SectorDesc* sd_dev, const int* list_dev, int count, int kmax,
+cudaError_t launch_precondition_basis(const UpdateTables* tab_dev, SectorDesc* sd_dev, int n_updates,
+                                      const int* list_dev, int count, int kmax, double cutoff, int chi,
                                       const double* dbuf, const double* ebuf, double* lam, double* scratch,
                                       unsigned char* swp, double* zbuf, const void* gbuf, const void* taubuf, void* tbuf,
                                       void* ybuf, cudaStream_t s) {
@@ -1759,7 +1822,7 @@ cudaError_t launch_precondition_basis(const SectorDesc* sd_dev, const int* list_
   if (attr != cudaSuccess) return attr;
   cudaError_t e = run_bisect(sd_dev, list_dev, count, kmax, dbuf, ebuf, lam, s);
   if (e != cudaSuccess) return e;
-  e = run_invit(sd_dev, list_dev, count, kmax, true, dbuf, ebuf, lam, scratch, swp, zbuf, s);
+  e = run_invit(sd_dev, list_dev, count, kmax, tab_dev, n_updates, cutoff, chi, dbuf, ebuf, lam, scratch, swp, zbuf, s);
   if (e != cudaSuccess) return e;
   orthogonalise_kernel<<<count, OR_NT, (size_t)OR_P * kmax * sizeof(double), s>>>(sd_dev, list_dev, lam, zbuf);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;

@@ -40,7 +40,8 @@ struct GemmGroup {
   int tiles_n;       // ceil(N / tile N)
   int tile_start;    // first flat tile index of this group
   int sec;           // >= 0: a dimension is sector sec's kept count, read on the device
-  int kdim;          // (1: M and lda; 2: N, ldb and ldc); the host's value is its bound
+  int kdim;          // (1: M and lda; 2: N, ldb and ldc); the host's value is its bound.
+                     // 3: nothing is done where the kept count is negative
   int64_t a_off, b_off, c_off;
   int64_t cs_off;
 };
@@ -115,6 +116,14 @@ cudaError_t launch_mix_d(int d, const UpdateTables* tab_dev, const int* tidx_dev
 // preconditioned ones.
 cudaError_t launch_identity_rows(const SectorDesc* sd_dev, const int* list_dev, int count, int max_elems,
                                  void* abuf, cudaStream_t s);
+// An update done with preconditioned matrices is done again from the plain ones where it
+// keeps singular values below PRE_MIN of their sector's largest.  The preconditioner mixes the
+// columns of values below ~1e-7 of the largest, a null space among them, and a column reduced
+// to the numerical-rank floor z takes part in no more rotations, so it can leave (z / sigma)^2
+// of a value sigma out.  At z of 4e-14 (100 rows) that is rounding at 1e-5; at 1e-8 the kept
+// values of a rank-deficient 120 x 100 sector were 6.8e-11 off, without it 5.3e-14 (relative;
+// values above 1e-5: 1e-15 and 1e-14).
+constexpr double PRE_MIN = 1e-5;
 // Deterministic top-chi with ket/bra pair symmetrisation, one CTA per update; writes kept
 // counts into sd_dev[s].kept and kept_out[s], slot starts, every update's total into
 // kept_out[n_sectors + u], whether it must be done again without the preconditioner into
@@ -206,16 +215,18 @@ cudaError_t launch_bisect(const SectorDesc* sd_dev, int n_sectors, int kmax, con
                           cudaStream_t s);
 // eigenvectors of the kept eigenvalues (sd[s].kept): V ([k][kept] at v_off) of the
 // sectors with X = T^H, Y ([k][kept] at y_off) of the others.
-cudaError_t launch_eigvec(const SectorDesc* sd_dev, int n_sectors, int kmax, const double* dbuf, const double* ebuf,
+cudaError_t launch_eigvec(SectorDesc* sd_dev, int n_sectors, int kmax, const double* dbuf, const double* ebuf,
                           const double* lam, double* scratch, unsigned char* swp, double* zbuf, const void* gbuf,
                           const void* taubuf, void* vbuf, void* ybuf, cudaStream_t s);
 // The preconditioner of the blocked Jacobi SVD (see eigen.cu) of the listed sectors, from
-// their tridiagonals: every eigenvector, nearly unitary, to ybuf ([k][k] at y_off); 3/2 I -
-// S / 2 in place of S = Y^H Y (check: a sector whose S is too far from I gets kept = -1); and
-// Y into the matrices [T^H; I] Y, or the unpreconditioned matrix of a flagged sector
+// their tridiagonals: the eigenvalues (lam, descending) and the sectors better left as they
+// are, flagged with kept = -1; every eigenvector, nearly unitary, to ybuf ([k][k] at y_off);
+// 3/2 I - S / 2 in place of S = Y^H Y (check: a sector whose S is too far from I is flagged);
+// and Y into the matrices [T^H; I] Y, or the unpreconditioned matrix of a flagged sector
 // (max_elems: the largest rows_tot k).  tbuf: precondition_t_elems complex entries.
 size_t precondition_t_elems(int64_t s_elems, int n_sectors);
-cudaError_t launch_precondition_basis(const SectorDesc* sd_dev, const int* list_dev, int count, int kmax,
+cudaError_t launch_precondition_basis(const UpdateTables* tab_dev, SectorDesc* sd_dev, int n_updates,
+                                      const int* list_dev, int count, int kmax, double cutoff, int chi,
                                       const double* dbuf, const double* ebuf, double* lam, double* scratch,
                                       unsigned char* swp, double* zbuf, const void* gbuf, const void* taubuf, void* tbuf,
                                       void* ybuf, cudaStream_t s);

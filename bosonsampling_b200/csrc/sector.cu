@@ -177,14 +177,6 @@ __device__ __forceinline__ int count_ge(const double* key, int k, double v) {
   return lo;
 }
 
-// An update done with preconditioned matrices is done again from the plain ones where it
-// keeps singular values below PRE_MIN of their sector's largest.  The preconditioner mixes the
-// columns of values below ~1e-7 of the largest, a null space among them, and a column reduced
-// to the numerical-rank floor z takes part in no more rotations, so it can leave (z / sigma)^2
-// of a value sigma out.  At z of 4e-14 (100 rows) that is rounding at 1e-5; at 1e-8 the kept
-// values of a rank-deficient 120 x 100 sector were 6.8e-11 off, without it 5.3e-14 (relative;
-// values above 1e-5: 1e-15 and 1e-14).
-constexpr double PRE_MIN = 1e-5;
 constexpr int SEL_NT = 512;
 constexpr int SEL_CAP = 5120;   // candidates whose keys are kept in shared memory
 

@@ -98,6 +98,7 @@ __global__ __launch_bounds__(NT, 4) void zgemm_grouped_kernel(const cplx* __rest
     if (g.sec >= 0) {
       const int kept = sd[g.sec].kept;
       if (g.kdim == 1) { g.M = kept; g.lda = kept; }
+      else if (g.kdim == 3) { g.M = kept < 0 ? 0 : g.M; }
       else { g.N = kept; g.ldb = kept; g.ldc = kept; }
     }
   }

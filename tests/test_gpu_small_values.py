@@ -69,3 +69,28 @@ def test_kept_values(L, R, K, decades, chi):
     kappa = float(s[0] / s[min(K, L, R) - 1])
     assert 0 < n <= min(K, L, R)
     assert np.max(np.abs(info["sigma"][i][:n] - want) / want) <= 64 * eps * kappa
+
+
+@pytest.mark.parametrize("k,size", [(66, 90), (100, 100), (150, 70), (200, 240)])
+@pytest.mark.parametrize("near", [0.0, 1e-9, 0.3])
+def test_nearly_equal_values(k, size, near):
+    """Sectors whose columns are orthogonal or nearly so: all values the same, or within `near`.
+    Singular values within 64 eps sqrt(size) of the largest, kept vectors orthonormal."""
+    d, L, R, eps = 2, k, size, np.finfo(float).eps
+    n = min(L, R)
+    rng = np.random.default_rng(k + size)
+    gl = np.linalg.qr(rng.standard_normal((L, L)) + 1j * rng.standard_normal((L, L)))[0][:, :n]
+    gr = (np.linalg.qr(rng.standard_normal((R, R)) + 1j * rng.standard_normal((R, R)))[0][:n] *
+          (1 + near * rng.random(n))[:, None])
+    q = [(0, 0)] * n
+    chi = 2 * n
+    info, g, _, _ = _update("fp64", d, d - 1, q, gl, gr, np.ones(R), max(chi, L, R))
+    U = fock.update_tensor(interferometer.t_block(THETA, PHI), d)
+    at = 0
+    for (c0, c1), s, m in zip(info["sectors"], info["sigma"], info["kept"]):
+        T = gl @ gr * (U[1 - c0, c0, 1] * np.conj(U[1 - c1, c1, 1]))
+        want = np.linalg.svd(T, compute_uv=False)
+        assert np.abs(s - want).max() <= 64 * eps * np.sqrt(max(L, R)) * want[0]
+        v = g[0][:L, at:at + m]
+        assert np.abs(v.conj().T @ v - np.eye(m)).max(initial=0.0) <= 4 * eps * np.sqrt(max(L, R)) * n
+        at += m
