@@ -9,15 +9,20 @@
 // contracts charge blocks as GEMMs instead.
 //
 // The weight depends on the centre entry through its charge only.  So the centre entries are
-// taken in runs of equal charge (any order of the entries is allowed; an order by charge has
-// the fewest runs): a run's plain products are accumulated on the FP64 tensor path (m8n8k4),
+// taken in runs of equal charge (any order of the entries is allowed; a window of them with more
+// runs than there are charges is put in an order by charge first, stably): a run's plain
+// products are accumulated on the FP64 tensor path (m8n8k4),
 // and at its end each output adds its weight times the run's sum.  A run that no row and
 // column of the tile can use is not read.  What bounds it: the FP64 tensor rate of the SM with
 // the most tiles, so they are small (32 x 16, 4 warps): a sector of 443 x 389 is 350 CTAs.
-// Measured there with 1,024 centre entries, d = 5: the kernel 81 us, the call with its wait 162
+// Measured there with 1,024 centre entries, d = 5: the kernel 74 us, the call with its wait 162
 // us, 116 among others.  When the tiles were chosen, calls with their wait, 32 x 16 and 32 x
 // 32 tiles (182 CTAs): 188 and 206 us; 700 x 1,024 x 300: 180 and 202; 1,500 x 1,024 x 1,400: 411
 // and 411 (16 x 16 tiles with the weight applied per entry: the kernel alone 270 at the first).
+// Entries in random order, calls with their wait, most of it the expansion of the change list on
+// the host: 443 x 1,024 x 389 1,226 us, 2,222 with every entry a run of its own, 1,313 with the
+// weight applied per entry.  The grouping's tables lie in the stages and the run list: 3 KB of
+// shared memory more cost entries in order 2%.
 #include "dmma.cuh"
 #include "kernels.h"
 
@@ -35,11 +40,18 @@ __device__ __forceinline__ bool ge2(int2 a, int2 b) { return a.x >= b.x && a.y >
 
 // The product of one tile over the centre entries, run by run: fold(q) is called with the
 // run's first centre index once re / im hold its sum.  use is called by whole warps.
-template <typename Same, typename Use, typename Fold>
+// code(i): entry i's charge as a number below CODES.
+constexpr int CODES = BSMPO_MAX_Q + 1;
+template <typename Same, typename Code, typename Use, typename Fold>
 __device__ __forceinline__ void run_products(const cplx* __restrict__ glc, const cplx* __restrict__ gcr, int len_l,
-                                             int len_c, int len_r, double2* smem, int* runs, double2 (&re)[2][NJ],
-                                             double2 (&im)[2][NJ], Same same, Use use, Fold fold) {
+                                             int len_c, int len_r, int most_runs, double2* smem, int* runs, double2 (&re)[2][NJ],
+                                             double2 (&im)[2][NJ], Same same, Code code, Use use,
+                                             Fold fold) {
   __shared__ int wsum[CNT / 32], n_runs;
+  // to group a window: counts in the stages, and its entries by position behind its few runs
+  int *at_code = reinterpret_cast<int*>(smem), (*in_warp)[CODES] = reinterpret_cast<int(*)[CODES]>(at_code + CODES);
+  unsigned short* order = reinterpret_cast<unsigned short*>(runs + CWIN / 2);
+  static_assert(CODES <= CWIN / 2 && (CNT / 32 + 1) * CODES * sizeof(int) <= CSTAGE * sizeof(double2), "no room");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int m0 = blockIdx.y * CT, n0 = blockIdx.x * CN;
   const int wm = (warp >> 1) * 16, wn = (warp & 1) * (CN / 2), li = lane >> 2, lk = lane & 3;
@@ -62,63 +74,105 @@ __device__ __forceinline__ void run_products(const cplx* __restrict__ glc, const
         for (int w = 0; w < CNT / 32; ++w) n_runs += wsum[w];
       __syncthreads();
     }
-    const int nr = n_runs;
-    // slabs of CK entries within a run, over the window's used runs; (run, k) walk in
-    // step for the fills and the products
-    auto end_of = [&](int r) { return r + 1 < nr ? runs[r + 1] : w1; };
-    auto next_used = [&](int r) {
-      while (r < nr && !use(runs[r])) ++r;
-      return r;
-    };
-    int fr = next_used(0), fk = fr < nr ? runs[fr] : 0;   // next slab to fill
-    auto fill = [&](int s) {
-      if (fr >= nr) return;
-      const int end = end_of(fr);
-      double2 *as = smem + s * CSTAGE, *bs = as + CT * CLDA;
-#pragma unroll
-      for (int i = 0; i < CT * CK / CNT; ++i) {
-        const int e = tid + i * CNT, m = e / CK, k = e % CK;
-        const bool ok = m0 + m < len_l && fk + k < end;
-        cp_async16(as + m * CLDA + k, ok ? glc + (int64_t)(m0 + m) * len_c + fk + k : glc, ok);
-      }
-#pragma unroll
-      for (int i = 0; i < CN * CK / CNT; ++i) {
-        const int e = tid + i * CNT, k = e / CN, n = e % CN;
-        const bool ok = n0 + n < len_r && fk + k < end;
-        cp_async16(bs + k * CLDB + n, ok ? gcr + (int64_t)(fk + k) * len_r + n0 + n : gcr, ok);
-      }
-      fk += CK;
-      if (fk >= end) {
-        fr = next_used(fr + 1);
-        if (fr < nr) fk = runs[fr];
-      }
-    };
-    int cr = fr, ck = fk;                                 // next slab to multiply
-#pragma unroll
-    for (int s = 0; s < CSTAGES - 1; ++s) {
-      fill(s);
-      cp_async_commit();
-    }
-    for (int t = 0; cr < nr; ++t) {
-      cp_async_wait<CSTAGES - 2>();
+    const bool grouped = n_runs > most_runs;   // uniform
+    if (grouped) {
+      for (int c = tid; c < CODES; c += CNT) at_code[c] = 0;
+      for (int c = tid; c < CNT / 32 * CODES; c += CNT) in_warp[0][c] = 0;
       __syncthreads();
-      fill((t + CSTAGES - 1) % CSTAGES);
-      cp_async_commit();
-      const double2 *as = smem + (t % CSTAGES) * CSTAGE, *bs = as + CT * CLDA;
-      cmma_tile<2, NJ, CK / 4, false>(
-          re, im, [&](int i, int k) { return as[(wm + 8 * i + li) * CLDA + k + lk]; },
-          [&](int j, int k) { return bs[(k + lk) * CLDB + wn + 8 * j + li]; });
-      ck += CK;
-      if (ck >= end_of(cr)) {
-        fold(runs[cr]);
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-          for (int j = 0; j < NJ; ++j) re[i][j] = im[i][j] = make_double2(0.0, 0.0);
-        cr = next_used(cr + 1);
-        if (cr < nr) ck = runs[cr];
+      for (int i = w0 + tid; i < w1; i += CNT) atomicAdd(&at_code[code(i)], 1);
+      __syncthreads();
+      if (tid == 0) {
+        int at = 0, n = 0;
+        for (int c = 0; c < CODES; ++c) {
+          const int len = at_code[c];
+          at_code[c] = at;
+          if (len > 0) runs[n++] = w0 + at;
+          at += len;
+        }
+        n_runs = n;
+      }
+      __syncthreads();
+      for (int i0 = w0; i0 < w1; i0 += CNT) {
+        // an entry's place: behind those of its code in the chunks, warps and lanes before it
+        const int i = i0 + tid, c = i < w1 ? code(i) : CODES;
+        const unsigned m = __match_any_sync(0xffffffffu, c), before = m & ((1u << lane) - 1);
+        if (i < w1 && before == 0) in_warp[warp][c] = __popc(m);
+        __syncthreads();
+        if (i < w1) {
+          int at = at_code[c] + __popc(before);
+          for (int w = 0; w < warp; ++w) at += in_warp[w][c];
+          order[at] = (unsigned short)(i - w0);
+        }
+        __syncthreads();
+        for (int x = tid; x < CODES; x += CNT)
+          for (int w = 0; w < CNT / 32; ++w) {
+            at_code[x] += in_warp[w][x];
+            in_warp[w][x] = 0;
+          }
+        __syncthreads();
       }
     }
+    const int nr = n_runs;
+    auto products = [&](auto entry) {   // entry at position i of the window
+      // slabs of CK entries within a run, over the window's used runs; (run, k) walk in
+      // step for the fills and the products
+      auto end_of = [&](int r) { return r + 1 < nr ? runs[r + 1] : w1; };
+      auto next_used = [&](int r) {
+        while (r < nr && !use(entry(runs[r]))) ++r;
+        return r;
+      };
+      int fr = next_used(0), fk = fr < nr ? runs[fr] : 0;   // next slab to fill
+      auto fill = [&](int s) {
+        if (fr >= nr) return;
+        const int end = end_of(fr);
+        double2 *as = smem + s * CSTAGE, *bs = as + CT * CLDA;
+#pragma unroll
+        for (int i = 0; i < CT * CK / CNT; ++i) {
+          const int e = tid + i * CNT, m = e / CK, k = e % CK;
+          const bool ok = m0 + m < len_l && fk + k < end;
+          cp_async16(as + m * CLDA + k, ok ? glc + (int64_t)(m0 + m) * len_c + entry(fk + k) : glc, ok);
+        }
+#pragma unroll
+        for (int i = 0; i < CN * CK / CNT; ++i) {
+          const int e = tid + i * CNT, k = e / CN, n = e % CN;
+          const bool ok = n0 + n < len_r && fk + k < end;
+          cp_async16(bs + k * CLDB + n, ok ? gcr + (int64_t)entry(fk + k) * len_r + n0 + n : gcr, ok);
+        }
+        fk += CK;
+        if (fk >= end) {
+          fr = next_used(fr + 1);
+          if (fr < nr) fk = runs[fr];
+        }
+      };
+      int cr = fr, ck = fk;                                 // next slab to multiply
+#pragma unroll
+      for (int s = 0; s < CSTAGES - 1; ++s) {
+        fill(s);
+        cp_async_commit();
+      }
+      for (int t = 0; cr < nr; ++t) {
+        cp_async_wait<CSTAGES - 2>();
+        __syncthreads();
+        fill((t + CSTAGES - 1) % CSTAGES);
+        cp_async_commit();
+        const double2 *as = smem + (t % CSTAGES) * CSTAGE, *bs = as + CT * CLDA;
+        cmma_tile<2, NJ, CK / 4, false>(
+            re, im, [&](int i, int k) { return as[(wm + 8 * i + li) * CLDA + k + lk]; },
+            [&](int j, int k) { return bs[(k + lk) * CLDB + wn + 8 * j + li]; });
+        ck += CK;
+        if (ck >= end_of(cr)) {
+          fold(entry(runs[cr]));
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) re[i][j] = im[i][j] = make_double2(0.0, 0.0);
+          cr = next_used(cr + 1);
+          if (cr < nr) ck = runs[cr];
+        }
+      }
+    };
+    if (grouped) products([&](int i) { return w0 + order[i - w0]; });
+    else products([](int i) { return i; });
     __syncthreads();   // the stages and the run list are free for the next window
   }
 }
@@ -155,7 +209,7 @@ __global__ __launch_bounds__(CNT) void contract_sector_kernel(int d, int cc0, in
   } else if (tid < CT + CN) {
     const int r = blockIdx.x * CN + tid - CT;
     const int2 b = r < len_r ? cr[r] : make_int2(d, d);
-    cols[tid - CT] = b.x < d && b.y < d && b.x <= cc0 && b.y <= cc1 ? b : make_int2(BIG, BIG);
+    cols[tid - CT] = b.x >= 0 && b.y >= 0 && b.x <= cc0 && b.y <= cc1 ? b : make_int2(BIG, BIG);
   }
   __syncthreads();
   const TileLane T;
@@ -179,11 +233,12 @@ __global__ __launch_bounds__(CNT) void contract_sector_kernel(int d, int cc0, in
       acc[i][j][0] = acc[i][j][1] = cmake(0.0, 0.0);
     }
   run_products(
-      glc, gcr, len_l, len_c, len_r, smem, runs, re, im,
+      glc, gcr, len_l, len_c, len_r, d * d + 1, smem, runs, re, im,
       [&](int i, int j) { return cc[i].x == cc[j].x && cc[i].y == cc[j].y; },
+      [&](int i) { return cc[i].x < 0 || cc[i].y < 0 || cc[i].x >= d || cc[i].y >= d ? CODES - 1 : cc[i].x * d + cc[i].y; },
       [&](int i) {
         const int2 q = cc[i];
-        if (q.x >= d || q.y >= d) return false;
+        if (q.x < 0 || q.y < 0 || q.x >= d || q.y >= d) return false;
         const int t = threadIdx.x & 31;   // a lane to a row and a column of the tile
         const bool r = __any_sync(0xffffffffu, ge2(rows[t], q)), c = __any_sync(0xffffffffu, ge2(q, cols[t % CN]));
         return r && c;
