@@ -102,7 +102,8 @@ struct bsmpo_ctx {
   int gram_policy = 0;
   // BSMPO_TEST_ERROR (tests only, read at create): 1, 2 sets an error word behind the SVD of
   // the next update (an expired wait; no convergence), 3 the first behind its tensor-core
-  // W = V^H C, once; 10 + m: device allocation m fails, once
+  // W = V^H C, once; 4: the next preconditioned Jacobi SVD does not converge, 5: nor
+  // does the plain one after it; 10 + m: device allocation m fails, once
   int test_error = 0;
   // which contractions of BSMPO_PRECISION_TF32X3 go on the tensor cores (BSMPO_TC_MASK,
   // read at create): bit 0 the Theta block products, bit 1 W = V^H C; the others FP64.
@@ -355,6 +356,8 @@ int64_t candidates(bsmpo_ctx* h, int mode) {
 // A preconditioned update that turns out to keep such values is done again with the plain form
 // (the selection tells; see PRE_MIN).
 enum class Route { plain, preconditioned, gram };
+// What update_group does with updates of the preconditioned route: see there.
+enum class Form { choose, plain, preconditioned };
 
 Route route_of(bsmpo_ctx* h, int mode) {
   if (candidates(h, mode) <= h->chi) return Route::plain;
@@ -827,9 +830,11 @@ int gram_eigenvalues(bsmpo_ctx* h, const Plan& P, const SectorDesc* sd_d, const 
 }
 
 // The matrices the blocked Jacobi rounds of the preconditioned sectors start from: X Y with
-// a unitary Y close to the eigenvectors of X^H X.
-int precondition(bsmpo_ctx* h, const Plan& P, const UpdateTables* tab_d, SectorDesc* sd_d, const GemmGroup* ggram_d,
-                 const GemmGroup* gyy_d, const GemmGroup* gym_d, const GemmGroup* gxy_d, const int* list_d, int* err_d) {
+// a unitary Y close to the eigenvectors of X^H X.  may_flag: X itself where small values are
+// seen to be kept (better_plain; it keeps a group of chi < 0 as it is).
+int precondition(bsmpo_ctx* h, const Plan& P, bool may_flag, const UpdateTables* tab_d, SectorDesc* sd_d,
+                 const GemmGroup* ggram_d, const GemmGroup* gyy_d, const GemmGroup* gym_d, const GemmGroup* gxy_d,
+                 const int* list_d, int* err_d) {
   cudaStream_t st = h->stream;
   const int n = P.n_pre;
   int rc;
@@ -838,7 +843,7 @@ int precondition(bsmpo_ctx* h, const Plan& P, const UpdateTables* tab_d, SectorD
   if ((rc = grow(h, h->wyt, precondition_t_elems(P.s_elems, (int)P.sd.size()) * sizeof(cplx)))) return rc;
   double* dbuf_d = reinterpret_cast<double*>(h->eigd.p);
   double* ebuf_d = dbuf_d + P.s_elems;
-  CK(h, launch_precondition_basis(tab_d, sd_d, (int)P.tab.size(), list_d, n, P.pre_k, h->cutoff, h->chi, dbuf_d, ebuf_d,
+  CK(h, launch_precondition_basis(tab_d, sd_d, (int)P.tab.size(), list_d, n, P.pre_k, h->cutoff, may_flag ? h->chi : -1, dbuf_d, ebuf_d,
                                   ebuf_d + P.s_elems, reinterpret_cast<double*>(h->escr.p),
                                   reinterpret_cast<unsigned char*>(h->swp.p), reinterpret_cast<double*>(h->zbuf.p),
                                   h->gbuf.p, h->taub.p, h->wyt.p, h->ybuf.p, st));
@@ -883,9 +888,9 @@ int gram_timing(bsmpo_ctx* h, const Plan& P) {
 }
 
 // 3b. One-sided Jacobi of every sector of the group: the small sectors in one launch, the
-// others in blocked rounds.  gg_d: the preconditioner's GEMM groups (X^H X, Y^H Y, Y M, X Y).
-int jacobi_svd(bsmpo_ctx* h, const Plan& P, const UpdateTables* tab_d, SectorDesc* sd_d, char* jw_d, const int* list_d,
-               const GemmGroup* const* gg_d, char* res_d, const ResLayout& R) {
+// others in blocked rounds.  may_flag: see precondition; gg_d: the preconditioner's GEMM groups (X^H X, Y^H Y, Y M, X Y).
+int jacobi_svd(bsmpo_ctx* h, const Plan& P, bool may_flag, const UpdateTables* tab_d, SectorDesc* sd_d, char* jw_d,
+               const int* list_d, const GemmGroup* const* gg_d, char* res_d, const ResLayout& R) {
   const int ns = (int)P.sd.size(), n_big = (int)P.jw.size();
   cudaStream_t st = h->stream;
   int rc;
@@ -910,7 +915,7 @@ int jacobi_svd(bsmpo_ctx* h, const Plan& P, const UpdateTables* tab_d, SectorDes
   double* sig = reinterpret_cast<double*>(h->sig.p);
   int* perm = reinterpret_cast<int*>(h->perm.p);
   if (h->timing) CK(h, cudaEventRecord(h->ev0, st));
-  if (P.n_pre && (rc = precondition(h, P, tab_d, sd_d, gg_d[0], gg_d[1], gg_d[2], gg_d[3], list_d + P.n_small + n_big,
+  if (P.n_pre && (rc = precondition(h, P, may_flag, tab_d, sd_d, gg_d[0], gg_d[1], gg_d[2], gg_d[3], list_d + P.n_small + n_big,
                                     reinterpret_cast<int*>(res_d + R.err))))
     return rc;
   // beside the blocked rounds, where there are any, on the first side stream
@@ -1008,6 +1013,16 @@ int jacobi_svd(bsmpo_ctx* h, const Plan& P, const UpdateTables* tab_d, SectorDes
     h->last_sweeps = std::max(h->last_sweeps, conv_at[w] >= 0 ? conv_at[w] : t / P.jw[w].rounds);
   h->jacobi_rounds += t;   // launched rounds, including the drained chunk
   if (h->timing) h->jac_launches += t;
+  if (h->test_error == 4 && P.n_pre) {
+    converged = false;
+    h->test_error = 0;
+  } else if (h->test_error == 5 && P.n_pre) {
+    converged = false;
+    h->test_error = 6;
+  } else if (h->test_error == 6) {
+    converged = false;
+    h->test_error = 0;
+  }
   if (!converged) {
     std::string msg = "Jacobi SVD did not converge";
     for (int w = 0; w < n_big; ++w) {
@@ -1092,20 +1107,25 @@ int tc_w_gemm(bsmpo_ctx* h, const Plan& P, const int* hk, int* err_d) {
 // Updates at the modes of `jobs` (disjoint sites, one route), all in the same launches.
 // Every sector computes exactly what it computes in a group of its own; trunc[j], if
 // given, receives job j's truncation weight.  The diagnostics of job `diag` (-1: none) are
-// recorded, its singular values in a buffer of their own if keep_sig.  Returns with the kept counts on the host
-// (the plan of a following update needs them) and the group's last kernels in flight.
-// An update of the preconditioned form that keeps a value too small for it (see PRE_MIN) is
-// left out of the scatter and done again with the plain one (plain: no preconditioner).
-int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc, int diag, bool keep_sig, bool plain = false) {
+// recorded, its singular values in a buffer of their own if keep_sig.  Returns with the kept
+// counts on the host (the plan of a following update needs them) and the group's last kernels
+// in flight.
+// Form::choose: an update of the preconditioned form that keeps a value too small for it (see
+// PRE_MIN) is left out of the scatter and done again with Form::plain, without the
+// preconditioner; so is a group that does not converge.  Where the plain form does not
+// converge either (a strongly graded matrix can take it more than MAX_SWEEPS), the
+// preconditioned one stands whatever is kept.
+int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc, int diag, bool keep_sig,
+                 Form form = Form::choose) {
   int rc = BSMPO_OK;
   for (int j = 0; j < nj; ++j)
     if ((rc = check_mode(h, jobs[j].mode))) return rc;
   StageClock clk(h);
-  if (!plain) h->updates += nj;
+  if (form == Form::choose) h->updates += nj;
   const int d = h->d, chi = h->chi, dd = d * d;
   cudaStream_t st = h->stream;
   Plan P;
-  const Route route = plain ? Route::plain : route_of(h, jobs[0].mode);
+  const Route route = form == Form::plain ? Route::plain : route_of(h, jobs[0].mode);
   P.gram = route == Route::gram;
   P.pre = route == Route::preconditioned;
   const cplx* u3_base = jobs[0].u3;
@@ -1193,7 +1213,14 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc, int diag,
   if (!h->wait_ev) CK(h, cudaEventCreateWithFlags(&h->wait_ev, cudaEventBlockingSync | cudaEventDisableTiming));
   const GemmGroup* pre_d[4] = {groups_at(L.ggram), groups_at(L.gyy), groups_at(L.gym), groups_at(L.gxy)};
   rc = P.gram ? gram_eigenvalues(h, P, sd_d, groups_at(L.ggram), list_d, tcerr_d)
-              : jacobi_svd(h, P, tab_d, sd_d, dt + L.jw, list_d, pre_d, res_d, R);
+              : jacobi_svd(h, P, form == Form::choose, tab_d, sd_d, dt + L.jw, list_d, pre_d, res_d, R);
+  // done again from the start: no error word is set and nothing has been written
+  auto redo = [&](const Job* which, int n, double* weights, int which_diag) {
+    const int r = update_group(h, which, n, weights, which_diag, keep_sig, Form::plain);
+    if (r != BSMPO_ECONVERGE) return r;
+    return update_group(h, which, n, weights, which_diag, keep_sig, Form::preconditioned);
+  };
+  if (rc == BSMPO_ECONVERGE && P.n_pre && form == Form::choose) return redo(jobs, nj, trunc, diag);
   if (rc || (rc = clk.mark(3))) return rc;
   if (h->test_error == 1 || h->test_error == 2) {
     CK(h, cudaMemsetAsync(tcerr_d + h->test_error - 1, 1, sizeof(int), st));
@@ -1201,7 +1228,8 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc, int diag,
   }
   auto select = [&]() -> int {
     CKL(h, launch_select(tab_d, sd_d, nj, ns, reinterpret_cast<double*>(h->sig.p),
-                         reinterpret_cast<double*>(h->keys.p), h->cutoff, chi, kept_d, trunc_d, st));
+                         reinterpret_cast<double*>(h->keys.p), h->cutoff, chi,
+                         form == Form::choose ? PRE_MIN : 0.0, kept_d, trunc_d, st));
     CK(h, cudaMemcpyAsync(hres, res_d, R.total, cudaMemcpyDeviceToHost, st));
     CK(h, cudaEventRecord(h->wait_ev, st));
     return BSMPO_OK;
@@ -1229,7 +1257,7 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc, int diag,
       const int* list2 = reinterpret_cast<const int*>(t2 + jbytes);
       if (J.max_left_m2 > 0)
         CKL(h, launch_identity_rows(sd_d, list2 + J.n_small, (int)J.jw.size(), J.max_left_m2, h->abuf.p, st));
-      if ((rc = jacobi_svd(h, J, tab_d, sd_d, t2, list2, nullptr, res_d, R))) return rc;
+      if ((rc = jacobi_svd(h, J, false, tab_d, sd_d, t2, list2, nullptr, res_d, R))) return rc;
       P.gram = false;
       if ((rc = select())) return rc;
     }
@@ -1349,7 +1377,7 @@ int update_group(bsmpo_ctx* h, const Job* jobs, int nj, double* trunc, int diag,
       if (j == diag) rest_diag = (int)rest.size();
       rest.push_back(jobs[j]);
     }
-    if ((rc = update_group(h, rest.data(), (int)rest.size(), tw.data(), rest_diag, keep_sig, true))) return rc;
+    if ((rc = redo(rest.data(), (int)rest.size(), tw.data(), rest_diag))) return rc;
     for (size_t i = 0; trunc && i < again.size(); ++i) trunc[again[i]] = tw[i];
   }
   return BSMPO_OK;

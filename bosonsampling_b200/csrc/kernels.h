@@ -127,10 +127,10 @@ constexpr double PRE_MIN = 1e-5;
 // Deterministic top-chi with ket/bra pair symmetrisation, one CTA per update; writes kept
 // counts into sd_dev[s].kept and kept_out[s], slot starts, every update's total into
 // kept_out[n_sectors + u], whether it must be done again without the preconditioner into
-// kept_out[n_sectors + n_updates + u], and its truncation weight into trunc_out[u].
+// kept_out[n_sectors + n_updates + u] (it keeps a value below pre_min of its sector's largest), and its truncation weight into trunc_out[u].
 cudaError_t launch_select(const UpdateTables* tab_dev, SectorDesc* sd_dev, int n_updates,
                           int n_sectors, const double* sig, double* keys, double cutoff, int chi,
-                          int* kept_out, double* trunc_out, cudaStream_t s);
+                          double pre_min, int* kept_out, double* trunc_out, cudaStream_t s);
 // conj(V) rows for the kept vectors of every sector.
 cudaError_t launch_extract_v(const SectorDesc* sd_dev, int n_sectors, int max_elems,
                              const void* abuf, const double* sig, const int* perm, void* vbuf,

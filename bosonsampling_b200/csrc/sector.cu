@@ -189,7 +189,7 @@ __global__ __launch_bounds__(SEL_NT) void select_kernel(const UpdateTables* __re
                                                         SectorDesc* __restrict__ sds, int n_sectors,
                                                         const double* __restrict__ sig,
                                                         double* __restrict__ keys, double cutoff,
-                                                        int chi, int* __restrict__ kept_all,
+                                                        int chi, double pre_min, int* __restrict__ kept_all,
                                                         double* __restrict__ trunc_all) {
   __shared__ double skey[SEL_CAP];
   __shared__ double tws[BSMPO_MAX_Q], smax_s;
@@ -321,7 +321,8 @@ __global__ __launch_bounds__(SEL_NT) void select_kernel(const UpdateTables* __re
     for (int i = 0; i < tid; ++i) slot += kept_s[i];
     // a preconditioned sector (not flagged to start from X) that keeps too small a value
     const double* v = sig + offs[tid];
-    if (sd[tid].t_off != sd[tid].a_off && sd[tid].kept >= 0 && kept_s[tid] > 0 && v[kept_s[tid] - 1] < PRE_MIN * v[0]) redo = 1;
+    if (sd[tid].t_off != sd[tid].a_off && sd[tid].kept >= 0 && kept_s[tid] > 0 && v[kept_s[tid] - 1] < pre_min * v[0])
+      redo = 1;
     sd[tid].kept = kept_s[tid];
     sd[tid].slot0 = slot;
     kept_out[tid] = kept_s[tid];
@@ -496,10 +497,10 @@ cudaError_t launch_identity_rows(const SectorDesc* sd_dev, const int* list_dev, 
 }
 
 cudaError_t launch_select(const UpdateTables* tab_dev, SectorDesc* sd_dev, int n_updates, int n_sectors,
-                          const double* sig, double* keys, double cutoff, int chi, int* kept_out,
+                          const double* sig, double* keys, double cutoff, int chi, double pre_min, int* kept_out,
                           double* trunc_out, cudaStream_t s) {
   if (n_updates <= 0) return cudaSuccess;
-  select_kernel<<<n_updates, SEL_NT, 0, s>>>(tab_dev, sd_dev, n_sectors, sig, keys, cutoff, chi, kept_out,
+  select_kernel<<<n_updates, SEL_NT, 0, s>>>(tab_dev, sd_dev, n_sectors, sig, keys, cutoff, chi, pre_min, kept_out,
                                              trunc_out);
   return cudaGetLastError();
 }

@@ -132,3 +132,26 @@ def test_every_allocation_that_fails(precision, state, monkeypatch):
                 sim.bs_update(5, S)
             assert _equal(_host(sim), want)
     assert 10 <= failed < 60
+
+
+@pytest.mark.parametrize("workers", [1, 4])
+def test_preconditioned_form_that_does_not_converge(workers, monkeypatch):
+    """Its updates are done again from the matrices themselves: no error, and the result without the
+    failure to rounding (Lambda within 1e-12 of the largest).  Where those do not converge either
+    the preconditioned result stands."""
+    n, d, chi = 16, 4, 300
+    _, bs, _ = interferometer.circuit(n, 4)
+    ops = [b for b in bs if b[0] < 9]
+    out = []
+    for word in (None, "4", "5"):
+        if word:
+            monkeypatch.setenv("BSMPO_TEST_ERROR", word)
+        with engine.MPOSimulator(n, d, chi) as sim:
+            sim.set_workers(workers)
+            sim.init_single_photons(range(0, n, 2), 0.37)
+            sim.run_mesh([b[1] for b in ops], [b[2] for b in ops], [b[3] for b in ops])
+            out.append((_host(sim), sim.observables()))
+    (a, oa), (b, ob), (c, oc) = out
+    assert not np.array_equal(a[0], b[0]) and _equal(a, c)
+    assert np.abs(np.sort(a[1], axis=1) - np.sort(b[1], axis=1)).max() <= 1e-12 * a[1].max()
+    assert np.abs(oa[1] - ob[1]).max() <= 1e-12 * abs(oa[0])
