@@ -1387,7 +1387,11 @@ int bs_update_impl(bsmpo_ctx* h, int mode, const cplx* u3_dev) {
   Job job;
   job.mode = mode;
   job.u3 = u3_dev;
-  return update_group(h, &job, 1, nullptr, 0, false);
+  const int rc = update_group(h, &job, 1, nullptr, 0, false);
+  // copies from the host stages may still be queued behind the kernels of the update before
+  // (meshes wait for their lanes); the next update overwrites the stages
+  if (rc) host_wait(h);
+  return rc;
 }
 
 M8 transpose_to_m8(const double* S) {

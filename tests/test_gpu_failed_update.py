@@ -134,6 +134,28 @@ def test_every_allocation_that_fails(precision, state, monkeypatch):
     assert 10 <= failed < 60
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp64-gram"])
+def test_next_update_follows_a_failed_one_at_once(precision, state, monkeypatch):
+    """The tables of an update that fails behind another's kernels are not overwritten by the
+    next update's while their copy is queued."""
+    S = interferometer.t_block(0.7, 0.4)
+    results = []
+    for m in (None, *range(60)):
+        if m is not None:
+            monkeypatch.setenv("BSMPO_TEST_ERROR", str(10 + m))
+        with engine.MPOSimulator(N, D, CHI) as sim:
+            sim.set_precision(precision)
+            sim.load_host(*state)
+            for mode in (4, 5, 6, 2, 3):
+                try:
+                    sim.bs_update(mode, S)
+                except RuntimeError as e:
+                    assert "allocation" in str(e)
+                    sim.bs_update(mode, S)
+            results.append(_host(sim))
+    assert all(_equal(results[0], r) for r in results[1:])
+
+
 @pytest.mark.parametrize("workers", [1, 4])
 def test_preconditioned_form_that_does_not_converge(workers, monkeypatch):
     """Its updates are done again from the matrices themselves: no error, and the result without the
