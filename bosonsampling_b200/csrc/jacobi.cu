@@ -576,7 +576,8 @@ constexpr int JS_KMAX = 64;
 // two factorisations of one to four columns add more rounding than they take away sweeps.
 // Mean relative error of 1, 2, 3 and 4 square columns' values, 1e-16: 1.9, 1.7, 2.1 and 2.5 with
 // the factorisations, 0.9, 1.2, 1.8 and 2.0 without; Lambda of a chi = 32 update under way 3.0e-15
-// and 2.3e-15 off, at equal time (235 us).
+// and 2.3e-15 off, at equal time (235 us).  Updates of four such sectors, us, with and without: 1,000
+// x 3 215 and 192, 4 x 300 108 and 104, 3 x 1,000 132 and 147 (a warp to a pair is long there).
 constexpr int JS_TINY = 4;
 constexpr int JS_SMEM = 216 * 1024;
 constexpr int JS_EX = 100;     // binary exponents of X's largest entry that need no scaling
@@ -895,6 +896,16 @@ __device__ int js_sweeps(double2* L, int ld, int k, double z2, double t2, int ma
   }
 }
 
+// a summed over the warp, in every lane: the second product with ones adds the four pairs that
+// the first leaves in a row (no shuffles)
+__device__ __forceinline__ double lane_sum(double a) {
+  double2 s = make_double2(0, 0), t = s;
+  __syncwarp();
+  dmma8x8x4(s, 1.0, a);
+  dmma8x8x4(t, 1.0, s.x + s.y);
+  return t.x;
+}
+
 // All sweeps over up to JS_TINY columns of X as they are, a warp to a pair: the rotations
 // also go to the nv rows of V (below the identity they started from).  Returns as js_sweeps.
 __device__ int js_sweeps_tiny(double2* X, int ldx, int rows, double2* V, int ldv, int nv, int k, double z2, double t2,
@@ -910,6 +921,7 @@ __device__ int js_sweeps_tiny(double2* X, int ldx, int rows, double2* V, int ldv
       if (q < k) {                     // q == k: the padding column
         double2 *x = X + p * ldx, *y = X + q * ldx;
         double a = 0.0, b = 0.0, gx = 0.0, gy = 0.0;
+#pragma unroll 4
         for (int r = lane; r < rows; r += 32) {
           const double2 u = x[r], v = y[r];
           a = fma(u.x, u.x, fma(u.y, u.y, a));
@@ -917,16 +929,17 @@ __device__ int js_sweeps_tiny(double2* X, int ldx, int rows, double2* V, int ldv
           gx = fma(u.x, v.x, fma(u.y, v.y, gx));
           gy = fma(u.x, v.y, fma(-u.y, v.x, gy));
         }
-        a = group_sum<32>(a);
-        b = group_sum<32>(b);
-        gx = group_sum<32>(gx);
-        gy = group_sum<32>(gy);
+        a = lane_sum(a);
+        b = lane_sum(b);
+        gx = lane_sum(gx);
+        gy = lane_sum(gy);
         const double g2 = fma(gx, gx, gy * gy);
         if (a > z2 && b > z2 && a > t2 * b && b > t2 * a && g2 > t2 * a * b) {
           const double dd = b - a, ir = rsqrt(fma(dd, dd, 4.0 * g2)), c2 = fma(0.5 * fabs(dd), ir, 0.5), ic = rsqrt(c2);
           const double c = c2 * ic, f = copysign(ir * ic, dd), sx = f * gx, sy = f * gy;
           ++mine;
           auto turn = [&](double2* x, double2* y, int n_rows) {
+#pragma unroll 4
             for (int r = lane; r < n_rows; r += 32) {
               const double2 u = x[r], v = y[r];
               x[r] = make_double2(fma(c, u.x, fma(-sx, v.x, -(sy * v.y))), fma(c, u.y, fma(-sx, v.y, sy * v.x)));
